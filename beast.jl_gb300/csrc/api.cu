@@ -932,31 +932,42 @@ static double dev_norm(beast_ctx* ctx, int64_t n, const double* x, double* scrat
   return std::sqrt(h);
 }
 
-// copy A into F (c64 for the mixed path, c128 otherwise) and factor F in place
+// leading dimension of a factor copy: whole 128-byte lines per column (16 complex FP32, 8 complex
+// FP64 elements).  The TMA maps of the tensor-core updates need 16-byte column strides, which an
+// odd n does not give in complex FP32 (a c64 copy with ld n = 9001 fell back to CUDA-core updates:
+// 57 ms of a 64 ms solve, against 2.3 ms at n = 9000)
+static int64_t factor_ld(int64_t n, int fdt) {
+  const int64_t el = fdt == BEAST_C64 ? 16 : 8;
+  return (n + el - 1) / el * el;
+}
+
+// copy A into F (c64 for the mixed path, c128 otherwise; leading dimension factor_ld) and factor
+// F in place
 static int factor_copy(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dtype, void* F,
                        int fdt, bool pivot, bool sym, beast_lu** out) {
   cudaStream_t st = ctx->stream;
+  const int64_t ldf = factor_ld(n, fdt);
   if (fdt == BEAST_C64) {
     if (a_dtype == BEAST_C64 && sym) {  // the symmetric factorisation reads the block-lower part only
       ProfScope ps(ctx, PK_CONVERT, (double)n * n * 8);
-      BEAST_CUDA_TRY(ctx, copy_lower_c64(n, A, lda, F, n, st));
+      BEAST_CUDA_TRY(ctx, copy_lower_c64(n, A, lda, F, ldf, st));
     } else if (a_dtype == BEAST_C64) {
-      BEAST_CUDA_TRY(ctx, cudaMemcpy2DAsync(F, n * 8, A, lda * 8, n * 8, n, cudaMemcpyDeviceToDevice, st));
+      BEAST_CUDA_TRY(ctx, cudaMemcpy2DAsync(F, ldf * 8, A, lda * 8, n * 8, n, cudaMemcpyDeviceToDevice, st));
     } else if (sym) {
       ProfScope ps(ctx, PK_CONVERT, (double)n * n * 12);
-      BEAST_CUDA_TRY(ctx, convert_lower_c128_to_c64(n, A, lda, F, n, st));
+      BEAST_CUDA_TRY(ctx, convert_lower_c128_to_c64(n, A, lda, F, ldf, st));
     } else {
       ProfScope ps(ctx, PK_CONVERT, (double)n * n * 24);
-      BEAST_CUDA_TRY(ctx, convert_c128_to_c64(n, n, (const double*)A, lda, (float*)F, n, st));
+      BEAST_CUDA_TRY(ctx, convert_c128_to_c64(n, n, (const double*)A, lda, (float*)F, ldf, st));
     }
   } else {
     ARG_CHECK(ctx, a_dtype == BEAST_C128, "plain FP64 solve needs a c128 matrix");
-    BEAST_CUDA_TRY(ctx, cudaMemcpy2DAsync(F, n * 16, A, lda * 16, n * 16, n, cudaMemcpyDeviceToDevice, st));
+    BEAST_CUDA_TRY(ctx, cudaMemcpy2DAsync(F, ldf * 16, A, lda * 16, n * 16, n, cudaMemcpyDeviceToDevice, st));
   }
   beast_lu* lu = new beast_lu();
   lu->ctx = ctx;
   lu->n = n;
-  lu->lda = n;
+  lu->lda = ldf;
   lu->dtype = fdt;
   lu->A = F;
   cudaError_t e = cudaMalloc(&lu->ipiv, lu_aux_bytes(n, fdt));
@@ -964,7 +975,7 @@ static int factor_copy(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, in
     delete lu;
     return beast_fail(ctx, BEAST_ERR_OOM, "pivot allocation failed");
   }
-  int rc = lu_factor_dev(ctx, n, F, n, fdt, lu->ipiv, &lu->info, pivot, sym);
+  int rc = lu_factor_dev(ctx, n, F, ldf, fdt, lu->ipiv, &lu->info, pivot, sym);
   if (rc == BEAST_OK && lu->info > 0)
     rc = beast_fail(ctx, BEAST_ERR_SINGULAR, "zero pivot in column " + std::to_string(lu->info));
   if (rc) {
@@ -1004,7 +1015,7 @@ static void system_release(beast_ctx* ctx, DenseSystem& S) {
 static int system_factor(beast_ctx* ctx, DenseSystem& S) {
   cudaStream_t st = ctx->stream;
   const int64_t n = S.n;
-  const size_t fel = S.mixed ? 8 : 16;
+  const size_t fbytes = (size_t)n * factor_ld(n, S.mixed ? BEAST_C64 : BEAST_C128) * (S.mixed ? 8 : 16);
   if (S.lu) {
     beast_lu_free(S.lu);
     S.lu = nullptr;
@@ -1014,7 +1025,7 @@ static int system_factor(beast_ctx* ctx, DenseSystem& S) {
     // mapped; when the factor copy would not fit next to them, hand them back first (the
     // next assembly grows its workspace again)
     size_t fr = 0, tot = 0;
-    const size_t want = (size_t)n * n * fel + ((size_t)1 << 31);
+    const size_t want = fbytes + ((size_t)1 << 31);
     if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr < want) {
       cudaMemPool_t pool;
       BEAST_CUDA_TRY(ctx, cudaStreamSynchronize(st));
@@ -1025,7 +1036,7 @@ static int system_factor(beast_ctx* ctx, DenseSystem& S) {
       }
       if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     }
-    BEAST_CUDA_TRY(ctx, cudaMallocAsync(&S.F, (size_t)n * n * fel, st));
+    BEAST_CUDA_TRY(ctx, cudaMallocAsync(&S.F, fbytes, st));
   }
   ctx->last_factor_mode = S.mode;
   return factor_copy(ctx, n, S.A, S.lda, S.a_dtype, S.F, S.mixed ? BEAST_C64 : BEAST_C128, S.mode == 0, S.mode == 2,
@@ -1078,7 +1089,7 @@ static int system_solve(beast_ctx* ctx, DenseSystem& S, const double* b, double*
       double bn = dev_norm(ctx, n, bk, nrm);
       if (!S.mixed) {
         BEAST_CUDA_TRY(ctx, vec_copy(n, bk, xk, st));
-        rc = lu_solve_dev(ctx, n, S.F, n, BEAST_C128, S.lu->ipiv, xk, n, 1);
+        rc = lu_solve_dev(ctx, n, S.F, S.lu->lda, BEAST_C128, S.lu->ipiv, xk, n, 1);
         if (rc) break;
         BEAST_CUDA_TRY(ctx, vec_copy(n, bk, r, st));
         {
@@ -1097,7 +1108,7 @@ static int system_solve(beast_ctx* ctx, DenseSystem& S, const double* b, double*
       int slow = 0;
       while (true) {
         BEAST_CUDA_TRY(ctx, convert_c128_to_c64(n, 1, r, n, d32, n, st));
-        rc = lu_solve_dev(ctx, n, S.F, n, BEAST_C64, S.lu->ipiv, d32, n, 1);
+        rc = lu_solve_dev(ctx, n, S.F, S.lu->lda, BEAST_C64, S.lu->ipiv, d32, n, 1);
         if (rc) break;
         BEAST_CUDA_TRY(ctx, convert_c64_to_c128(n, 1, d32, n, d, n, st));
         BEAST_CUDA_TRY(ctx, vec_axpy(n, 1.0, 0.0, d, xk, st));
@@ -1354,7 +1365,8 @@ int beast_system_create(beast_ctx* ctx, const beast_op_desc* op, const beast_qs_
     beast_system_free(y);
     return rc;
   }
-  y->bytes = (size_t)n * n * el + (size_t)n * n * (precision == BEAST_FP64 ? 16 : 8) + lu_aux_bytes(n, y->S.mixed ? BEAST_C64 : BEAST_C128);
+  const int fdt = y->S.mixed ? BEAST_C64 : BEAST_C128;
+  y->bytes = (size_t)n * n * el + (size_t)n * factor_ld(n, fdt) * (fdt == BEAST_C64 ? 8 : 16) + lu_aux_bytes(n, fdt);
   *out = y;
   return BEAST_OK;
 }
