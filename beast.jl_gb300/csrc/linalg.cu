@@ -44,6 +44,10 @@ int tc_gemm_sub(beast_ctx* ctx, float2* Mat, int64_t lda, int64_t rowA, int64_t 
                 bool prepped);
 int tc_gemm_sym(beast_ctx* ctx, float2* Mat, int64_t lda, int64_t rowA, int64_t colA, int64_t rowB, int64_t M0,
                 int64_t N0, int K, bool lower, void* work, size_t work_bytes, bool prepped, int64_t a_skip = 0);
+size_t tc_gemm64_work_bytes(int64_t M, int64_t N, int K);
+int tc_gemm64_sub(beast_ctx* ctx, double2* C, int64_t ldc, const double2* A, int64_t lda, const double2* B, int64_t ldb,
+                  int64_t M, int64_t N, int K, void* work, size_t work_bytes);
+bool tc_gemm64_supported();
 
 namespace {
 
@@ -1917,6 +1921,10 @@ struct LUSteps {
   bool gemm2_tc(int64_t m0, int64_t n0, int64_t n1, int k, const void* tcwork) const {
     return sizeof(T) == 8 && tcwork && m0 >= 64 && n0 + n1 >= 64 && k % 32 == 0;
   }
+  // complex FP64: digit-sliced tensor-core products (tc_gemm64.cu) for every update (a 32 x 32
+  // block with K = 64 takes 50 us there and 440 us on the FP64 units of one SM); the FP64 units
+  // only without the workspace
+  bool gemm64_tc(int k, const void* tcwork) const { return sizeof(T) == 16 && tcwork && k % 32 == 0; }
   // prepped: the FP16 operands are already in tcwork (k_panel_apply wrote them)
   int gemm2(int64_t r0, int64_t m0, int64_t c0, int64_t n0, int64_t m1, int64_t n1, int64_t k0, int k,
             void* tcwork, bool prepped = false) {
@@ -1925,10 +1933,17 @@ struct LUSteps {
     if (tc)  // brackets its operand preparation and its tensor-core launch separately
       return tc_gemm_sub(ctx, reinterpret_cast<float2*>(A), lda, r0, k0, c0, m0, n0, m1, n1, k, tcwork,
                          tcwork_bytes, prepped);
-    ProfScope ps(ctx, PK_GEMM, 8.0 * (double)k * ((double)m0 * n0 + (double)m1 * n1));
     const int64_t ms[2] = {m0, m1}, cs[2] = {c0, c0 + n0}, ns[2] = {n0, n1};
     for (int r = 0; r < 2; ++r) {
       if (ms[r] <= 0 || ns[r] <= 0) continue;
+      if (gemm64_tc(k, tcwork)) {
+        double2* Ad = reinterpret_cast<double2*>(A);
+        int rc = tc_gemm64_sub(ctx, Ad + r0 + cs[r] * lda, lda, Ad + r0 + k0 * lda, lda, Ad + k0 + cs[r] * lda, lda, ms[r],
+                               ns[r], k, tcwork, tcwork_bytes);
+        if (rc) return rc;
+        continue;
+      }
+      ProfScope ps(ctx, PK_GEMM, 8.0 * (double)k * (double)ms[r] * ns[r]);
       dim3 g((unsigned)((ms[r] + GT - 1) / GT), (unsigned)((ns[r] + GT - 1) / GT));
       k_gemm_sub<T, R><<<g, 256, 0, st>>>(A + r0 + cs[r] * lda, lda, A + r0 + k0 * lda, lda, A + k0 + cs[r] * lda,
                                           lda, ms[r], ns[r], k);
@@ -2071,6 +2086,15 @@ int lu_factor_t(beast_ctx* ctx, int64_t n, T* A, int64_t lda, int* ipiv, int* in
   if (sizeof(T) == 8 && tc_gemm_supported(A, lda, NB) && n > NB) {
     tcwork_bytes = tc_gemm_work_bytes(n, n, NB);
     BEAST_CUDA_TRY(ctx, cudaMallocAsync(&tcwork, tcwork_bytes, st));
+  }
+  // complex FP64: the digit slices of the largest update; without the memory for them the updates
+  // stay on the FP64 units
+  if (sizeof(T) == 16 && pivot && n > nb && tc_gemm64_supported()) {
+    tcwork_bytes = tc_gemm64_work_bytes(n, n, NB);
+    if (cudaMallocAsync(&tcwork, tcwork_bytes, st) != cudaSuccess) {
+      cudaGetLastError();
+      tcwork = nullptr;
+    }
   }
   LUSteps<T, R> S{ctx, A, lda, n, ipiv, st, tcwork_bytes};
   // lookahead (symmetric path with tensor-core updates; BEAST_LU_LOOKAHEAD=1): while a panel's

@@ -1,0 +1,373 @@
+// tc_gemm64.cu -- the trailing updates of the complex FP64 LU on the FP16 tensor cores.
+//
+//   C -= A B   with C (M x N), A (M x K), B (K x N) complex128, column-major
+//
+// GB300 runs FP64 at 1/1500 of its FP16 tensor rate (measured: the shared-memory tiled FP64 kernel
+// this replaces ran at 0.69 TFLOP/s, 90% of an FP64 solve of order 6007).  Each operand row /
+// column is therefore written as eight 7-bit digits of a fixed-point number (slice64.h; Ozaki et
+// al., Numer. Algorithms 59 (2012), with the tensor-core form of Mukunoki et al., ISC 2020) and
+// the product summed digit by digit:
+//   C' = sum_l 2^(-12 - 7 l) D_l,   D_l = sum_{i + j = l} A'_i B'_j,   l = 0 .. 7
+// on the real 2x2 form of the complex product (the layout of tc_gemm.cu: A' has rows 2m, 2m+1
+// = [[re, -im], [im, re]], B' columns hold (re, im) per k).  D_l is a sum of at most (l + 1) 2K
+// products of magnitude at most 2^12: with K <= 256 an integer of at most 2^24, exact in the FP32
+// accumulators.  What is dropped (digits beyond 2^-56 of the row's and the column's largest
+// magnitude, pairs i + j > 7) is below the rounding of an FP64 sum of the same length: measured
+// against 64-bit products in tests/test_gpu_lu_paths.py.
+//
+// k_tc_gemm64: persistent CTAs over 128 x TNT tiles of C'; the levels run from the smallest
+// contribution (l = 7) to the largest, each as one K loop over its l + 1 digit pairs through the
+// 4-stage TMA ring into one of two TMEM accumulators, while four epilogue warps add the previous
+// level to C (one FP64 addition per value: -D 2^sh is built from the bits of D).  A tile's C
+// values belong to one CTA and are added to in a fixed order: the result is deterministic.
+//   measured (one GB300): M = N = 5000, K = 1024 in 8.8 ms, 23.2 TFLOP/s of FP64 products (835
+//   TFLOP/s of FP16 ones) where the FP64 units gave 0.69; the order-6007 solve's updates 827 -> 47 ms.
+//   bound: the tensor pipe at large M, N (36 digit pairs: 72 K MACs per real value of C against
+//   8 FP64 additions, which take 0.85 of the time of the MMAs at K = 256); the FP64 additions at
+//   K = 64.
+//   TNT = 256 when its tiles fill the SMs; 64 below (the last blocks of a factorisation and small
+//   matrices): four times the CTAs share the additions and the digit loops.
+#include <algorithm>
+
+#include "internal.h"
+#include "slice64.h"
+#include "tc_ptx.h"
+
+namespace {
+
+using slice64::SLICES;
+
+constexpr int TM = 128, TK = 64, STAGES = 4;
+constexpr int KMAX = 256;  // complex columns of A per launch: (l + 1) 2K 2^12 <= 2^24 for l = 7
+constexpr int A_BYTES = TM * TK * 2;
+constexpr int GROUP = 8;  // row tiles taken together, column by column
+
+template <int TNT>
+struct Tile {
+  static constexpr int B_BYTES = TNT * TK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+};
+
+// tile index -> first real row and first column: groups of GROUP row tiles, column by column
+__device__ __forceinline__ void tile_at(int tile, int ntm, int ntn, int& mt, int& nt) {
+  const int per = GROUP * ntn, g = tile / per, l = tile - g * per;
+  const int rows = min(GROUP, ntm - g * GROUP);
+  mt = g * GROUP + l % rows;
+  nt = l / rows;
+}
+
+// M2 = 2M real rows of C' at Cr (ldr doubles per column), N columns; A' slice i at rows i M2, B'
+// slice j at rows j N of their tensor maps; nk stages of TK halves per digit pair
+template <int TNT>
+__global__ void __launch_bounds__(192, 1)
+    k_tc_gemm64(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double* Cr,
+                int64_t ldr, int M2, int N, const int* __restrict__ ea, const int* __restrict__ eb, int nk, int* status) {
+  constexpr int STAGE_BYTES = Tile<TNT>::STAGE_BYTES;
+  extern __shared__ unsigned char smraw[];
+  const uint32_t base = (smem_u32(smraw) + 1023u) & ~1023u;
+  unsigned char* gbase = smraw + (base - smem_u32(smraw));
+  // full[STAGES], empty[STAGES], tfull[2], tempty[2], done
+  uint64_t* bars = reinterpret_cast<uint64_t*>(gbase + STAGES * STAGE_BYTES);
+  const int B_FULL = 0, B_EMPTY = STAGES, B_TFULL = 2 * STAGES, B_TEMPTY = 2 * STAGES + 2, B_DONE = 2 * STAGES + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 7);
+  __shared__ int s_abort_mem;
+  volatile int* s_abort = &s_abort_mem;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ntm = (M2 + TM - 1) / TM, ntn = (N + TNT - 1) / TNT, ntiles = ntm * ntn;
+
+  if (threadIdx.x == 0) {
+    *s_abort = 0;
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(bars + B_FULL + s), 1);
+      mbar_init(smem_u32(bars + B_EMPTY + s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(bars + B_TFULL + a), 1);
+      mbar_init(smem_u32(bars + B_TEMPTY + a), 4);  // one arrival per epilogue warp
+    }
+    mbar_init(smem_u32(bars + B_DONE), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(2 * TNT)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0 && lane == 0) {
+    // ---- TMA producer
+    uint32_t it = 0;
+    for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x) {
+      int mt, nt;
+      tile_at(tile, ntm, ntn, mt, nt);
+      for (int l = SLICES - 1; l >= 0 && !*s_abort; --l)
+        for (int i = 0; i <= l && !*s_abort; ++i)
+          for (int kb = 0; kb < nk; ++kb, ++it) {
+            const int s = it % STAGES;
+            if (!mbar_wait(smem_u32(bars + B_EMPTY + s), ((it / STAGES) & 1) ^ 1, status, s_abort)) break;
+            const uint32_t sa = base + s * STAGE_BYTES, full = smem_u32(bars + B_FULL + s);
+            mbar_expect_tx(full, STAGE_BYTES);
+            tma_load_2d(sa, &tmA, kb * TK, i * M2 + mt * TM, full);
+            tma_load_2d(sa + A_BYTES, &tmB, kb * TK, (l - i) * N + nt * TNT, full);
+          }
+    }
+    // no copy may still be landing in shared memory when the CTA exits (bounded, whatever the
+    // abort state)
+    int no_abort = 0;
+    for (uint32_t j = it > (uint32_t)STAGES ? it - STAGES : 0; j < it; ++j)
+      mbar_wait(smem_u32(bars + B_FULL + j % STAGES), (j / STAGES) & 1, status, &no_abort);
+  } else if (warp == 1 && lane == 0) {
+    // ---- MMA issuer: D f32, A / B f16, both K-major, M = 128, N = TNT
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(TNT >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+    uint32_t it = 0;
+    int t = 0;  // levels of all tiles, in order
+    for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x)
+      for (int l = SLICES - 1; l >= 0 && !*s_abort; --l, ++t) {
+        const int a = t & 1;
+        if (!mbar_wait(smem_u32(bars + B_TEMPTY + a), ((t >> 1) & 1) ^ 1, status, s_abort)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + (uint32_t)(a * TNT);
+        const int steps = (l + 1) * nk;
+        for (int kb = 0; kb < steps; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(smem_u32(bars + B_FULL + s), (it / STAGES) & 1, status, s_abort)) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sa = base + s * STAGE_BYTES, sb = sa + A_BYTES;
+#pragma unroll
+          for (int kk = 0; kk < TK / 16; ++kk)
+            mma_f16(acc, smem_desc(sa + kk * 32), smem_desc(sb + kk * 32), idesc, (kb | kk) ? 1u : 0u);
+          mma_commit(smem_u32(bars + B_EMPTY + s));
+        }
+        if (*s_abort) break;
+        mma_commit(smem_u32(bars + B_TFULL + a));
+      }
+    // every MMA issued above has completed once this phase does (waited for even after an abort)
+    mma_commit(smem_u32(bars + B_DONE));
+    int no_abort = 0;
+    mbar_wait(smem_u32(bars + B_DONE), 0, status, &no_abort);
+  } else if (warp >= 2) {
+    // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. +31, a thread one real row of the tile
+    const int q = warp & 3;
+    int t = 0;
+    bool live = true;
+    for (int tile = blockIdx.x; tile < ntiles && live; tile += gridDim.x) {
+      int mt, nt;
+      tile_at(tile, ntm, ntn, mt, nt);
+      const int row = mt * TM + q * 32 + lane, n0 = nt * TNT;
+      const bool in = row < M2;
+      const int er = in ? ea[row >> 1] : 0;
+      double* c0 = Cr + row + (int64_t)n0 * ldr;
+      const int ncol = min(TNT, N - n0);
+      for (int l = SLICES - 1; l >= 0; --l, ++t) {
+        const int a = t & 1;
+        if (!mbar_wait(smem_u32(bars + B_TFULL + a), (t >> 1) & 1, status, s_abort)) {
+          live = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * TNT);
+        const int sh0 = er - 12 - 7 * l;
+        for (int c = 0; c < ncol; c += 16) {
+          float v[16];
+          double z[16];
+          tmem_ld16(tb + (uint32_t)c, v);
+          // exponents of the 16 columns, one per lane
+          const int ec = c + (lane & 15) < ncol ? eb[n0 + c + (lane & 15)] : 0;
+          double* cc = c0 + (int64_t)c * ldr;
+          if (ncol - c >= 16) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) z[j] = in ? cc[j * ldr] : 0.0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              z[j] += slice64::neg_scaled(v[j], sh0 + __shfl_sync(0xffffffffu, ec, j));
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (in) cc[j * ldr] = z[j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const double p = slice64::neg_scaled(v[j], sh0 + __shfl_sync(0xffffffffu, ec, j));
+              if (in && j < ncol - c) cc[j * ldr] += p;
+            }
+          }
+        }
+        // accumulator read: hand it back to the MMA warp
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bars + B_TEMPTY + a)) : "memory");
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TNT) : "memory");
+  }
+}
+
+// the digit pair (lo half, hi half) as two FP16 numbers: 1536 + d is exact in the half's last ten
+// bits
+__device__ __forceinline__ __half2 digits_h2(int lo, int hi) {
+  const uint32_t u = (uint32_t)((0x6600 + lo) & 0xFFFF) | ((uint32_t)(0x6600 + hi) << 16);
+  __half2 h;
+  memcpy(&h, &u, 4);
+  return __hsub2(h, __half2half2(__ushort_as_half((unsigned short)0x6600)));
+}
+
+// A' slices of 32 rows of A per CTA: row maxima, then 32 x 64 tiles transposed through shared
+// memory so that every warp writes whole row segments of each slice
+__device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, int M, int K, __half2* Ap, int* ea) {
+  __shared__ uint32_t red[8][33];
+  __shared__ double2 tile[32][65];
+  __shared__ int s_e[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int m0 = bid * 32, m = m0 + lane;
+  uint32_t mx = 0;
+  if (m < M)
+    for (int k = w; k < K; k += 8) {
+      const double2 a = A[m + (int64_t)k * lda];
+      mx = max(mx, max(slice64::abs_hi(a.x), slice64::abs_hi(a.y)));
+    }
+  red[w][lane] = mx;
+  __syncthreads();
+  if (w == 0) {
+    for (int j = 1; j < 8; ++j) mx = max(mx, red[j][lane]);
+    s_e[lane] = slice64::row_exponent(mx);
+    if (m < M) ea[m] = s_e[lane];
+  }
+  __syncthreads();
+  for (int k0 = 0; k0 < K; k0 += 64) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = k0 + w + 8 * j;
+      tile[lane][w + 8 * j] = (m < M && k < K) ? A[m + (int64_t)k * lda] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+      const int r = w + 8 * i, mr = m0 + r;
+      if (mr < M) {
+        const int e = s_e[r];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int kk = lane + 32 * h, k = k0 + kk;
+          if (k < K) {
+            const double2 a = tile[r][kk];
+            int dr[SLICES], di[SLICES];
+            slice64::digits(slice64::fixed55(a.x, e), dr);
+            slice64::digits(slice64::fixed55(a.y, e), di);
+            __half2* row0 = Ap + (int64_t)(2 * mr) * K + k;  // 2K halves = K half2 per row
+#pragma unroll
+            for (int s = 0; s < SLICES; ++s) {
+              row0[(int64_t)s * 2 * M * K] = digits_h2(dr[s], -di[s]);
+              row0[(int64_t)s * 2 * M * K + K] = digits_h2(di[s], dr[s]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// B' slices, one warp per column
+__device__ __forceinline__ void slice_b(int bid, const double2* B, int64_t ldb, int K, int N, __half2* Bp, int* eb) {
+  const int lane = threadIdx.x & 31;
+  const int j = bid * 8 + (threadIdx.x >> 5);
+  if (j >= N) return;
+  const double2* col = B + (int64_t)j * ldb;
+  uint32_t mx = 0;
+  for (int k = lane; k < K; k += 32) mx = max(mx, max(slice64::abs_hi(col[k].x), slice64::abs_hi(col[k].y)));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const int e = slice64::row_exponent(mx);
+  if (lane == 0) eb[j] = e;
+  for (int k = lane; k < K; k += 32) {
+    const double2 b = col[k];
+    int dr[SLICES], di[SLICES];
+    slice64::digits(slice64::fixed55(b.x, e), dr);
+    slice64::digits(slice64::fixed55(b.y, e), di);
+#pragma unroll
+    for (int s = 0; s < SLICES; ++s) Bp[((int64_t)s * N + j) * K + k] = digits_h2(dr[s], di[s]);
+  }
+}
+
+// both operands in one launch: CTAs [0, nA) 32 rows of A each, the rest 8 columns of B each
+__global__ void __launch_bounds__(256) k_slice(const double2* A, int64_t lda, const double2* B, int64_t ldb, int M,
+                                               int N, int K, __half2* Ap, int* ea, __half2* Bp, int* eb, int nA) {
+  if ((int)blockIdx.x < nA)
+    slice_a(blockIdx.x, A, lda, M, K, Ap, ea);
+  else
+    slice_b(blockIdx.x - nA, B, ldb, K, N, Bp, eb);
+}
+
+size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+template <int TNT>
+int run(beast_ctx* ctx, const CUtensorMap& tmA, const __half2* Bp, double* Cr, int64_t ldr, int M2, int N, int K,
+        const int* ea, const int* eb) {
+  CUtensorMap tmB;
+  if (!make_map(&tmB, Bp, (uint64_t)2 * K, (uint64_t)SLICES * N, (uint64_t)2 * K * 2, TK, TNT, true,
+                CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
+    return beast_fail(ctx, BEAST_ERR_CUDA, "tensor map encode (B' slices) failed");
+  BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tc_gemm64<TNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<TNT>::SMEM));
+  const int tiles = ((M2 + TM - 1) / TM) * ((N + TNT - 1) / TNT);
+  k_tc_gemm64<TNT><<<std::min(tiles, std::max(1, ctx->num_sms)), 192, Tile<TNT>::SMEM, ctx->stream>>>(
+      tmA, tmB, Cr, ldr, M2, N, ea, eb, 2 * K / TK, ctx->d_flag);
+  BEAST_CUDA_TRY(ctx, cudaGetLastError());
+  return BEAST_OK;
+}
+
+}  // namespace
+
+// bytes of workspace of an update with at most M rows and N columns
+size_t tc_gemm64_work_bytes(int64_t M, int64_t N, int K) {
+  const int64_t k = std::min(K, KMAX);
+  return al256((size_t)SLICES * M * k * 8) + al256((size_t)SLICES * N * k * 4) + al256((size_t)M * 4) + al256((size_t)N * 4);
+}
+
+// C -= A B (complex128): C at (M x N, ldc), A (M x K, lda), B (K x N, ldb), K a multiple of 32,
+// taken KMAX columns at a time.  A wait that runs out sets bit 4 of the context's status word.
+int tc_gemm64_sub(beast_ctx* ctx, double2* C, int64_t ldc, const double2* A, int64_t lda, const double2* B, int64_t ldb,
+                  int64_t M, int64_t N, int K, void* work, size_t work_bytes) {
+  if (K % 32 != 0 || 2 * M * SLICES > INT32_MAX || N * SLICES > INT32_MAX || tc_gemm64_work_bytes(M, N, K) > work_bytes)
+    return beast_fail(ctx, BEAST_ERR_ARG, "sliced FP64 update: unsupported block");
+  for (int k0 = 0; k0 < K; k0 += KMAX) {
+    const int k = std::min(KMAX, K - k0);
+    char* w = static_cast<char*>(work);
+    __half2* Ap = reinterpret_cast<__half2*>(w);
+    w += al256((size_t)SLICES * M * k * 8);
+    __half2* Bp = reinterpret_cast<__half2*>(w);
+    w += al256((size_t)SLICES * N * k * 4);
+    int* ea = reinterpret_cast<int*>(w);
+    int* eb = reinterpret_cast<int*>(w + al256((size_t)M * 4));
+    {
+      // operands read once, 8 digits of 2 (A') and 1 (B') FP16 pairs written per element
+      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (16 + 64) + (double)N * k * (16 + 32));
+      const int nA = (int)((M + 31) / 32), nB = (int)((N + 7) / 8);
+      k_slice<<<(unsigned)(nA + nB), 256, 0, ctx->stream>>>(A + (int64_t)k0 * lda, lda, B + k0, ldb, (int)M, (int)N, k, Ap,
+                                                            ea, Bp, eb, nA);
+      BEAST_CUDA_TRY(ctx, cudaGetLastError());
+    }
+    CUtensorMap tmA;
+    if (!make_map(&tmA, Ap, (uint64_t)2 * k, (uint64_t)SLICES * 2 * M, (uint64_t)2 * k * 2, TK, TM, true,
+                  CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
+      return beast_fail(ctx, BEAST_ERR_CUDA, "tensor map encode (A' slices) failed");
+    ProfScope ps(ctx, PK_TCGEMM, 8.0 * k * (double)M * N);
+    const int64_t wide = ((2 * M + TM - 1) / TM) * ((N + 255) / 256);
+    double* Cr = reinterpret_cast<double*>(C);
+    const int rc = wide >= ctx->num_sms ? run<256>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb)
+                                        : run<64>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb);
+    if (rc) return rc;
+  }
+  return BEAST_OK;
+}
+
+bool tc_gemm64_supported() { return encode_fn() != nullptr; }
