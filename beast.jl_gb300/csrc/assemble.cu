@@ -22,6 +22,7 @@
 #include <cmath>
 
 #include "fsplit.h"
+#include "green64.h"
 #include "internal.h"
 #include "se_p1.h"
 #include "far_df.h"
@@ -185,6 +186,8 @@ struct FarParams {
   int* near_count;
   int* flag;
   TriRuleDev ro, ri;
+  int qt, fmt;     // trial cells staged per CTA, Zcell format (k_far64)
+  g64::Wave wave;  // the wavenumber (k_far64)
 };
 
 // Zcell rows / columns (-1: the block entry is not stored)
@@ -514,6 +517,358 @@ __global__ void __launch_bounds__(FAR_THREADS) k_far(FarParams P) {
 }
 
 // ------------------------------------------------------------------------------------
+// far pairs in FP64
+// ------------------------------------------------------------------------------------
+// One test cell per thread against P.qt trial cells staged in shared memory, as k_far.  What bounds
+// it is the number of FP64 instructions (the pipe takes one warp instruction in 16 cycles per
+// quarter SM at best; loads, FP32 and integer work hide under it), so the pair is arranged to need
+// few of them:
+//   - a kernel value costs seven for 1/R, R, cos, sin (green64.h) where rsqrt and sincos cost 35;
+//   - every block is a combination of the moments T_mn = sum_ab w_a w_b K(x_a, y_b) lambda_m(x_a)
+//     lambda_n(y_b) over the cells' barycentric coordinates (the RT shapes are linear in them):
+//     three real sums per inner point (1, u, v) and real part, nine per outer point, the third
+//     coordinate by difference at the end; n x K, quadratic in the test point, takes three more
+//     (|xi|^2 with the test point's offset xi from its centroid);
+//   - the double layers' normal component does not depend on the point in the normal's own plane;
+//   - 1/(4 pi), the areas and the shapes' 1/2A enter once per block.
+// Measured (EFIE, 3380 cells): see the launch rule below.
+struct Far64Rec {
+  double sig[3][3];  // trial vertices minus centroid
+  double c[3], n[3];
+  double area, lim;  // lim: near-test radius (radius + threshold distance)
+};
+constexpr int FAR64_PT = 6;  // eta (3), w, w u, w v per inner rule point
+
+template <int OPK, int TK, int BK>
+__global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
+  constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL || OPK == BEAST_MW_NXDL;
+  constexpr bool GRAD = OPK != BEAST_MW_SL && OPK != BEAST_HH_SL;
+  constexpr int NT = TK == BEAST_P0 ? 1 : 3, NB = BK == BEAST_P0 ? 1 : 3;
+  constexpr int NX = OPK == BEAST_MW_NXDL ? 3 : 0;  // |xi|^2 moments
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int ni = P.ri.n, no = P.ro.n, qt = P.qt;
+  g64::Entry* tab = reinterpret_cast<g64::Entry*>(smraw);
+  Far64Rec* rec = reinterpret_cast<Far64Rec*>(tab + g64::TABLE);
+  double* pts = reinterpret_cast<double*>(rec + qt);        // [qt][ni][FAR64_PT]
+  double* sxi = pts + (size_t)qt * ni * FAR64_PT;           // [no][3][FAR_THREADS]: xi_a per thread
+  __shared__ double ro_s[RULE_MAXPTS][3];                   // w, w u, w v
+  __shared__ int s_zc[FAR_QT][3];
+  g64::load_table(tab);
+  const int q0 = blockIdx.y * qt;
+  const int nqt = min(qt, P.nq - q0);
+  for (int k = threadIdx.x; k < no; k += blockDim.x) {
+    ro_s[k][0] = P.ro.w[k];
+    ro_s[k][1] = P.ro.w[k] * P.ro.u[k];
+    ro_s[k][2] = P.ro.w[k] * P.ro.v[k];
+  }
+  for (int k = threadIdx.x; k < nqt * (1 + ni); k += blockDim.x) {
+    const int qi = k / (1 + ni), b = k % (1 + ni);
+    const int qc = P.qcells[q0 + qi];
+    const double* g = P.bgeo + (int64_t)qc * GEO_STRIDE;
+    if (b == 0) {
+      Far64Rec& r = rec[qi];
+      for (int j = 0; j < 9; ++j) r.sig[j / 3][j % 3] = g[j] - g[9 + j % 3];
+      for (int j = 0; j < 3; ++j) {
+        r.c[j] = g[9 + j];
+        r.n[j] = g[12 + j];
+      }
+      r.area = g[15];
+      r.lim = (double)P.bgeof[4 * qc + 3] + sqrt(fmax(near_threshold2(P.qs_kind, P.k2, g[15]), 0.0));
+    } else {
+      const double u = P.ri.u[b - 1], v = P.ri.v[b - 1], t = 1.0 - u - v, w = P.ri.w[b - 1];
+      double* pt = pts + ((size_t)qi * ni + b - 1) * FAR64_PT;
+      for (int j = 0; j < 3; ++j) pt[j] = u * (g[j] - g[9 + j]) + v * (g[3 + j] - g[9 + j]) + t * (g[6 + j] - g[9 + j]);
+      pt[3] = w;
+      pt[4] = w * u;
+      pt[5] = w * v;
+    }
+  }
+  for (int k = threadIdx.x; k < nqt * 3; k += blockDim.x) s_zc[k / 3][k % 3] = (int)zcol_of(P.zcol, q0 + k / 3, NB, k % 3);
+  const int64_t pp = blockIdx.x * (int64_t)FAR_THREADS + threadIdx.x;
+  const bool live = pp < P.np;
+  const int64_t p = live ? P.tperm[pp] : 0;
+  const double* tg = P.tgeo + p * GEO_STRIDE;
+  const V3<double> cp = mk(tg[9], tg[10], tg[11]);
+  auto tau = [&](int i) { return mk(tg[3 * i] - cp.x, tg[3 * i + 1] - cp.y, tg[3 * i + 2] - cp.z); };
+  for (int a = 0; a < no; ++a) {
+    const V3<double> xi = P.ro.u[a] * tau(0) + P.ro.v[a] * tau(1) + (1.0 - P.ro.u[a] - P.ro.v[a]) * tau(2);
+    sxi[(3 * a) * FAR_THREADS + threadIdx.x] = xi.x;
+    sxi[(3 * a + 1) * FAR_THREADS + threadIdx.x] = xi.y;
+    sxi[(3 * a + 2) * FAR_THREADS + threadIdx.x] = xi.z;
+  }
+  __syncthreads();
+  if (!live) return;
+  int64_t zr[3];
+  for (int i = 0; i < 3; ++i) zr[i] = i < NT ? zrow_of(P.zrow, pp, NT, i) : -1;
+  const double radp = P.tgeof[4 * p + 3];
+  const double gr = P.op.gr, sg = P.op.gi < 0.0 ? -1.0 : 1.0;
+  const V3<double> nn = mk(tg[12], tg[13], tg[14]);
+
+  for (int qi = 0; qi < nqt; ++qi) {
+    const Far64Rec& rq = rec[qi];
+    const int ql = q0 + qi;
+    const V3<double> d = mk(cp.x - rq.c[0], cp.y - rq.c[1], cp.z - rq.c[2]);
+    // near test: candidate filter on the centroid distance, exact classification (k_far)
+    {
+      const double lim = radp + rq.lim;
+      if (dot(d, d) <= lim * lim * 1.0001 + 1e-30) {
+        int cls = 4;
+        if (P.qs_kind != BEAST_QS_DOUBLENUM) {
+          const Geo t = load_geo(tg);
+          const Geo s = load_geo(P.bgeo + (int64_t)P.qcells[ql] * GEO_STRIDE);
+          cls = refines_class(classify_exact(t, s, P.qs_kind, P.k2), P.qs_kind);
+        }
+        if (cls != 0) {
+          const int idx = atomicAdd(P.near_count, 1);
+          if (idx < P.near_cap)
+            P.near[idx] = NearPair{(int)pp, ql, cls, 0};
+          else
+            atomicOr(P.flag, 1);
+          for (int i = 0; i < NT; ++i)
+            for (int j = 0; j < NB; ++j)
+              store_c<double>(P.zcell, zidx(zr[i], s_zc[qi][j], P.ldc), C2<double>{0, 0}, P.fmt);
+          continue;
+        }
+      }
+    }
+    const double* pq = pts + (size_t)qi * ni * FAR64_PT;
+    const V3<double> nq = mk(rq.n[0], rq.n[1], rq.n[2]);
+    // moments over (1, u, v) of the test and (1, u, v) of the trial cell
+    C2<double> M[NT][NB], X[3];
+#pragma unroll
+    for (int m = 0; m < NT; ++m)
+#pragma unroll
+      for (int n = 0; n < NB; ++n) M[m][n] = C2<double>{0, 0};
+    X[0] = X[1] = X[2] = C2<double>{0, 0};
+    for (int a = 0; a < no; ++a) {
+      const V3<double> xi = mk(sxi[(3 * a) * FAR_THREADS + threadIdx.x], sxi[(3 * a + 1) * FAR_THREADS + threadIdx.x],
+                               sxi[(3 * a + 2) * FAR_THREADS + threadIdx.x]);
+      const V3<double> dx = d + xi;
+      C2<double> U[3];
+      U[0] = U[1] = U[2] = C2<double>{0, 0};
+#pragma unroll 2
+      for (int b = 0; b < ni; ++b) {
+        const double* pb = pq + b * FAR64_PT;
+        const V3<double> r = dx - mk(pb[0], pb[1], pb[2]);
+        const g64::Value v = g64::eval(dot(r, r), P.wave, tab);
+        double amp = v.iR;
+        if (gr != 0.0) amp *= exp(-gr * v.R);
+        double kr, ki;  // single layer: 4 pi G, the imaginary part times -sg; gradient: -4 pi c, times sg
+        if (GRAD) {
+          const double p1 = v.iR + gr, q = amp * v.iR;
+          kr = fma(p1, v.c, P.wave.k * v.s);
+          ki = fma(P.wave.k, v.c, -(p1 * v.s));
+          double f = q;
+          if (OPK == BEAST_HH_DLT) f *= dot(nn, r);
+          kr *= f;
+          ki *= f;
+        } else {
+          kr = amp * v.c;
+          ki = amp * v.s;
+        }
+        U[0].re = fma(pb[3], kr, U[0].re);
+        U[0].im = fma(pb[3], ki, U[0].im);
+        if (NB == 3) {
+          U[1].re = fma(pb[4], kr, U[1].re);
+          U[1].im = fma(pb[4], ki, U[1].im);
+          U[2].re = fma(pb[5], kr, U[2].re);
+          U[2].im = fma(pb[5], ki, U[2].im);
+        }
+      }
+      if (OPK == BEAST_HH_DL) {
+        const double f = dot(nq, dx);
+#pragma unroll
+        for (int n = 0; n < NB; ++n) U[n] = cscale(f, U[n]);
+      }
+#pragma unroll
+      for (int m = 0; m < NT; ++m)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+          M[m][n].re = fma(ro_s[a][m], U[n].re, M[m][n].re);
+          M[m][n].im = fma(ro_s[a][m], U[n].im, M[m][n].im);
+        }
+      if (NX) {
+        const double f = ro_s[a][0] * dot(xi, xi);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          X[n].re = fma(f, U[n].re, X[n].re);
+          X[n].im = fma(f, U[n].im, X[n].im);
+        }
+      }
+    }
+    const C2<double> M00 = M[0][0];
+    // (1, u, v) -> the three barycentric coordinates, in the order 0 (u), 1 (v), 2
+    if (NB == 3) {
+#pragma unroll
+      for (int m = 0; m < NT; ++m) {
+        const C2<double> t = M[m][0];
+        M[m][0] = M[m][1];
+        M[m][1] = M[m][2];
+        M[m][2] = csub(csub(t, M[m][0]), M[m][1]);
+      }
+      if (NX) {
+        const C2<double> t = X[0];
+        X[0] = X[1];
+        X[1] = X[2];
+        X[2] = csub(csub(t, X[0]), X[1]);
+      }
+    }
+    if (NT == 3) {
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        const C2<double> t = M[0][n];
+        M[0][n] = M[1][n];
+        M[1][n] = M[2][n];
+        M[2][n] = csub(csub(t, M[0][n]), M[1][n]);
+      }
+    }
+    auto put = [&](int i, int j, C2<double> z) { store_c<double>(P.zcell, zidx(zr[i], s_zc[qi][j], P.ldc), z, P.fmt); };
+    if (!RT) {
+      // alpha A_p A_q / (4 pi) T; the gradient's sign: c = -(...)  and the double layer's -n_q . r
+      const double s = I4PI * tg[15] * rq.area * (OPK == BEAST_HH_DLT ? -1.0 : 1.0);
+      const double si = s * (GRAD ? sg : -sg);
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          put(i, j, cmul(C2<double>{P.op.ar, P.op.ai}, C2<double>{s * M[i][j].re, si * M[i][j].im}));
+    } else {
+      V3<double> ta[3], sj[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        ta[i] = tau(i);
+        sj[i] = mk(rq.sig[i][0], rq.sig[i][1], rq.sig[i][2]);
+      }
+      if (OPK == BEAST_MW_SL) {
+        // alpha / 4 sum_{m != i, n != j} T_mn (tau_m - tau_i).(sig_n - sig_j) + beta T: the products
+        // of the edges (01, 02, 12 by index m + i - 1) from four, the rest by differences
+        const V3<double> a0 = ta[0] - ta[2], a1 = ta[1] - ta[2], b0 = sj[0] - sj[2], b1 = sj[1] - sj[2];
+        double g[3][3];  // [test edge][trial edge], edge mi: tau_m - tau_i for m < i
+        g[1][1] = dot(a0, b0);
+        g[1][2] = dot(a0, b1);
+        g[2][1] = dot(a1, b0);
+        g[2][2] = dot(a1, b1);
+        g[0][1] = g[1][1] - g[2][1];
+        g[0][2] = g[1][2] - g[2][2];
+        g[1][0] = g[1][1] - g[1][2];
+        g[2][0] = g[2][1] - g[2][2];
+        g[0][0] = g[0][1] - g[0][2];
+        const double ar = 0.25 * I4PI * P.op.ar, ai = 0.25 * I4PI * P.op.ai;
+        const double m0r = I4PI * M00.re, m0i = -sg * I4PI * M00.im;
+        const double br = P.op.br * m0r - P.op.bi * m0i, bi = P.op.br * m0i + P.op.bi * m0r;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            double fr = 0.0, fi = 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+#pragma unroll
+              for (int n = 0; n < 3; ++n)
+                if (m != i && n != j) {
+                  const double g0 = g[m + i - 1][n + j - 1], e = (m < i) == (n < j) ? g0 : -g0;
+                  fr = fma(e, M[m][n].re, fr);
+                  fi = fma(e, M[m][n].im, fi);
+                }
+            fi = -sg * fi;
+            put(i, j, C2<double>{fma(ar, fr, fma(-ai, fi, br)), fma(ar, fi, fma(ai, fr, bi))});
+          }
+      } else {
+        const double s = -0.25 * I4PI;  // grad G = c r, c = -(gamma + 1/R) G / R
+        if (OPK == BEAST_MW_DL) {
+          // sum_{m != i, n != j} T_mn (tau_m - tau_i).(r_mn x (sig_n - sig_j)), r_mn between vertices
+          C2<double> z[3][3];
+#pragma unroll
+          for (int k = 0; k < 9; ++k) z[k / 3][k % 3] = C2<double>{0, 0};
+#pragma unroll
+          for (int m = 0; m < 3; ++m)
+#pragma unroll
+            for (int n = 0; n < 3; ++n) {
+              const V3<double> rmn = (d + ta[m]) - sj[n];
+#pragma unroll
+              for (int j = 0; j < 3; ++j) {
+                if (j == n) continue;
+                const V3<double> c = cross(rmn, sj[n] - sj[j]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                  if (i == m) continue;
+                  const double e = dot(ta[m] - ta[i], c);
+                  z[i][j].re = fma(e, M[m][n].re, z[i][j].re);
+                  z[i][j].im = fma(e, M[m][n].im, z[i][j].im);
+                }
+              }
+            }
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) put(i, j, C2<double>{s * z[i][j].re, s * sg * z[i][j].im});
+        } else {
+          // n x K (n the test normal): (f.r)(n.g) - (f.g)(n.r) with nu_j = n.sig_j, nd = n.d
+          //   = sum_n lambda_n (nu_n - nu_j) [|xi|^2 + sum_m lambda_m a_im]
+          //     + sum_mn lambda_m lambda_n [(nu_j - nd) (tau_m - tau_i).sig_n + (nd - nu_n) (tau_m - tau_i).sig_j],
+          //   a_im = (tau_m - tau_i).d - tau_i.tau_m
+          const double nd = dot(nn, d);
+          double nu[3], td[3], gs[3][3];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) nu[j] = dot(nn, sj[j]);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            td[i] = dot(ta[i], d);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) gs[i][j] = dot(ta[i], sj[j]);
+          }
+          C2<double> W[3];
+#pragma unroll
+          for (int m = 0; m < 3; ++m) {
+            W[m] = C2<double>{0, 0};
+#pragma unroll
+            for (int n = 0; n < 3; ++n) {
+              W[m].re = fma(nd - nu[n], M[m][n].re, W[m].re);
+              W[m].im = fma(nd - nu[n], M[m][n].im, W[m].im);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            C2<double> B[3], H{0, 0};
+#pragma unroll
+            for (int n = 0; n < 3; ++n) {
+              B[n] = X[n];
+#pragma unroll
+              for (int m = 0; m < 3; ++m) {
+                const double a = (td[m] - td[i]) - dot(ta[i], ta[m]);
+                B[n].re = fma(a, M[m][n].re, B[n].re);
+                B[n].im = fma(a, M[m][n].im, B[n].im);
+                if (m != i) {
+                  H.re = fma(gs[m][n] - gs[i][n], M[m][n].re, H.re);
+                  H.im = fma(gs[m][n] - gs[i][n], M[m][n].im, H.im);
+                }
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+              double zr_ = (nu[j] - nd) * H.re, zi_ = (nu[j] - nd) * H.im;
+#pragma unroll
+              for (int n = 0; n < 3; ++n)
+                if (n != j) {
+                  zr_ = fma(nu[n] - nu[j], B[n].re, zr_);
+                  zi_ = fma(nu[n] - nu[j], B[n].im, zi_);
+                }
+#pragma unroll
+              for (int m = 0; m < 3; ++m)
+                if (m != i) {
+                  zr_ = fma(gs[m][j] - gs[i][j], W[m].re, zr_);
+                  zi_ = fma(gs[m][j] - gs[i][j], W[m].im, zi_);
+                }
+              put(i, j, C2<double>{s * zr_, s * sg * zi_});
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------
 // near pairs (FP64): generic per-point integrand
 // ------------------------------------------------------------------------------------
 struct Shp {
@@ -825,6 +1180,10 @@ struct NearParams {
   int ssdf;  // Sauter-Schwab pairs of RT Maxwell operators in double-float (k_near_ss_df)
   const float2* ssdf_tab[4];  // per class 1..3: node table [7][items] (ss_table)
   int ssdf_items[4];
+  int ss64;  // Sauter-Schwab pairs in k_near_ss64
+  const double* ss64_tab[4];  // per class 1..3: node table [SS64_VALS][items]
+  int ss64_items[4];
+  g64::Wave wave;
   int64_t ldc;
   const int* zrow;  // as in FarParams
   const int* zcol;
@@ -1188,6 +1547,7 @@ DEV void rt_restriction(const Geo& parent, const Geo& ch, double Q[3][3]) {
 // shared memory (lanes read different nodes: a constant-memory read would serialise)
 DEV void near_pair(const NearParams& P, const NearPair np_, const double* s_glx, const double* s_glw, int lane) {
   if (near_is_ss32(P, np_.cls) || near_is_ssdf(P, np_.cls)) return;  // k_near_ss32 / k_near_ss_df
+  if (P.ss64 && np_.cls >= 1 && np_.cls <= 3) return;               // k_near_ss64
   const Geo t = load_geo(P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE);
   const Geo s = load_geo(P.bgeo + (int64_t)(P.qcells ? P.qcells[np_.q] : np_.q) * GEO_STRIDE);
   const int nt = P.tk == BEAST_P0 ? 1 : 3, nb = P.bk == BEAST_P0 ? 1 : 3;
@@ -2165,7 +2525,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch(BatchLaunch L) {
     P.nnear = 0;
     P.zcell = J.Z;
     P.zfmt = L.zfmt;
-    P.ss32 = 0;
+    P.ss32 = P.ss64 = 0;
     P.ldc = J.ldz;
     P.zrow = J.zrow;
     P.zcol = J.zcol;
@@ -2188,12 +2548,38 @@ static cudaError_t far_t(const FarParams& P, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+static int sm_count() {
+  static int n[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  if (n[dev] == 0 && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+  return n[dev];
+}
+
+// The FP64 far kernel.  Trial cells per CTA: FAR_QT for large operators (the staging and the table
+// of a CTA shared by 16 pairs per thread), halved while the grid has less than four CTAs per SM:
+// a thread's pairs run one after the other, and a small operator's few CTAs would leave most of the
+// chip's FP64 units idle.
+template <int OPK, int TK, int BK>
+static cudaError_t far64_t(FarParams P, int fmt, cudaStream_t st) {
+  const int64_t gx = (P.np + FAR_THREADS - 1) / FAR_THREADS;
+  P.qt = FAR_QT;
+  P.fmt = fmt;
+  while (P.qt > 1 && gx * ((P.nq + P.qt - 1) / P.qt) < 4 * (int64_t)sm_count()) P.qt /= 2;
+  P.wave = g64::make_wave(P.op.gi);
+  const size_t sm = sizeof(g64::Entry) * g64::TABLE + P.qt * (sizeof(Far64Rec) + sizeof(double) * FAR64_PT * P.ri.n) +
+                    sizeof(double) * 3 * FAR_THREADS * P.ro.n;
+  cudaError_t e = cudaFuncSetAttribute(k_far64<OPK, TK, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  dim3 grid((unsigned)gx, (unsigned)((P.nq + P.qt - 1) / P.qt));
+  k_far64<OPK, TK, BK><<<grid, FAR_THREADS, sm, st>>>(P);
+  return cudaGetLastError();
+}
+
 template <int OPK, int TK, int BK>
 static cudaError_t far_prec(const FarParams& P, int precision, int fmt, cudaStream_t st) {
   if (precision == BEAST_MIXED) return far_t<OPK, TK, BK, float, ZCELL_C64>(P, st);
-  if (fmt == ZCELL_C64) return far_t<OPK, TK, BK, double, ZCELL_C64>(P, st);
-  if (fmt == ZCELL_DF) return far_t<OPK, TK, BK, double, ZCELL_DF>(P, st);
-  return far_t<OPK, TK, BK, double, ZCELL_C128>(P, st);
+  return far64_t<OPK, TK, BK>(P, fmt, st);
 }
 
 // ---- EFIE far pairs in double-float arithmetic (FP64-quality values on the FP32 pipes) -------
@@ -2837,6 +3223,230 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 5) k_near_ss_df(NearParams P)
   }
 }
 
+// ---- Sauter-Schwab pairs in FP64 (Maxwell single / double layer on RT, Helmholtz operators on
+// P0 / P1; what k_near_ss32 and the double-float kernels do not take)
+// Like k_far64 bound by its number of FP64 instructions; per node:
+//   - the coordinates and the nine products w (1, X0, X1) (1, Y0, Y1) come from a table per rule
+//     (built once per context) instead of the region maps: 4 + 9 loads, no arithmetic;
+//   - x - y from the maps' own factors on the edge vectors: 9 .. 15 operations with |x - y|^2;
+//   - the kernel value on green64.h: 7;
+//   - the moments over the shapes' coordinates (the RT shapes are linear in them): 18.
+// The block is formed once per pair by nine lanes from the moments' totals.
+// A CTA of four warps takes PPC pairs: pairs with SS64_HEAVY nodes or more (common face and edge
+// at the default orders: 3750 and 1536 nodes) one after the other with all warps, then the light
+// ones (common vertex: 162) a warp each.  The split depends on the rule alone, so a pair's sums do
+// not depend on what else is in the list.  PPC = 4; 1 while there are fewer pairs than eight per SM,
+// where the pairs of a CTA one after the other would set the time.
+constexpr int SS64_VALS = 13, SS64_HEAVY = 512;
+__global__ void k_ss64_table(int cls, int n, int items, double* tab) {
+  const int it = blockIdx.x * blockDim.x + threadIdx.x;
+  if (it >= items) return;
+  double X[2], Y[2], D[2], w;
+  ss_node_fd(cls, n, it, c_gl_x + c_gl_off[n - 1], c_gl_w + c_gl_off[n - 1], X, Y, D, &w);
+  // x - y = a et1 + b et2 - c es1 - d es2: class 3 (D0, D1), class 2 (D0, X1, Y1), class 1 all four
+  const double co[4] = {cls == 1 ? X[0] : D[0], cls == 3 ? D[1] : X[1], cls == 1 ? Y[0] : 0.0, cls == 3 ? 0.0 : Y[1]};
+  const double lx[3] = {1.0, X[0], X[1]}, ly[3] = {1.0, Y[0], Y[1]};
+  for (int k = 0; k < 4; ++k) tab[(int64_t)k * items + it] = co[k];
+  for (int m = 0; m < 3; ++m)
+    for (int k = 0; k < 3; ++k) tab[(int64_t)(4 + 3 * m + k) * items + it] = w * lx[m] * ly[k];
+}
+
+template <int OPK, int TK, int BK, int PPC>
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
+  constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL;
+  constexpr bool GRAD = OPK != BEAST_MW_SL && OPK != BEAST_HH_SL;
+  constexpr int NT = TK == BEAST_P0 ? 1 : 3, NB = BK == BEAST_P0 ? 1 : 3, NM = NT * NB;
+  __shared__ __align__(16) g64::Entry tab[g64::TABLE];
+  __shared__ double s_red[NEAR_WARPS][2 * NM][33];
+  __shared__ double s_tot[NEAR_WARPS][2 * NM];
+  __shared__ C2<double> s_T[NEAR_WARPS][NM];
+  g64::load_table(tab);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double gr = P.op.gr, sg = P.op.gi < 0.0 ? -1.0 : 1.0;
+  for (int step = 0; step < 2 * PPC; ++step) {
+    const int64_t e = blockIdx.x * (int64_t)PPC + step % PPC;
+    if (e >= P.nnear) continue;
+    const NearPair np_ = P.near[e];
+    const int cls = np_.cls;
+    if (cls < 1 || cls > 3 || (cls == 3 && dl_type(OPK))) continue;  // other paths / identically zero
+    const int items = P.ss64_items[cls];
+    const bool heavy = items >= SS64_HEAVY;  // uniform over the CTA
+    if (heavy != (step < PPC) || (!heavy && warp != step % PPC)) continue;
+    const Geo t = load_geo(P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE);
+    const Geo s = load_geo(P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE);
+    int pt[3], ps[3];
+    ss_order_warp(t, s, lane, pt, ps);
+    const V3<double> A0 = t.v[pt[0]], A1 = t.v[pt[1]], A2 = t.v[pt[2]];
+    const V3<double> B0 = s.v[ps[0]], B1 = s.v[ps[1]], B2 = s.v[ps[2]];
+    C2<double> M[NM];
+#pragma unroll
+    for (int k = 0; k < NM; ++k) M[k] = C2<double>{0, 0};
+    {
+      const V3<double> et1 = A1 - A0, et2 = A2 - A1, es1 = B1 - B0, es2 = B2 - B1;
+      const double* nodes = P.ss64_tab[cls];
+      const V3<double> nv = OPK == BEAST_HH_DL ? s.n : t.n;
+      for (int it = heavy ? (int)threadIdx.x : lane; it < items; it += heavy ? 32 * NEAR_WARPS : 32) {
+        const double* nd = nodes + it;
+        V3<double> r = nd[0] * et1 + nd[items] * et2;
+        if (cls != 3) {
+          const double y1 = nd[3 * (int64_t)items];
+          r = r - y1 * es2;
+          if (cls == 1) r = r - nd[2 * (int64_t)items] * es1;
+        }
+        const g64::Value v = g64::eval(dot(r, r), P.wave, tab);
+        double amp = v.iR;
+        if (gr != 0.0) amp *= exp(-gr * v.R);
+        double kr, ki;  // as in k_far64
+        if (GRAD) {
+          const double p1 = v.iR + gr;
+          double f = amp * v.iR;
+          kr = fma(p1, v.c, P.wave.k * v.s);
+          ki = fma(P.wave.k, v.c, -(p1 * v.s));
+          if (!RT) f *= dot(nv, r);
+          kr *= f;
+          ki *= f;
+        } else {
+          kr = amp * v.c;
+          ki = amp * v.s;
+        }
+#pragma unroll
+        for (int m = 0; m < NT; ++m)
+#pragma unroll
+          for (int n = 0; n < NB; ++n) {
+            const double w = nd[(int64_t)(4 + 3 * m + n) * items];
+            M[m * NB + n].re = fma(w, kr, M[m * NB + n].re);
+            M[m * NB + n].im = fma(w, ki, M[m * NB + n].im);
+          }
+      }
+    }
+    // totals: lane k sums value k of the 32 lanes (fewer additions than a butterfly per value)
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      s_red[warp][2 * k][lane] = M[k].re;
+      s_red[warp][2 * k + 1][lane] = M[k].im;
+    }
+    __syncwarp();
+    if (lane < 2 * NM) {
+      double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+      for (int l = 0; l < 32; l += 4) {
+        a0 += s_red[warp][lane][l];
+        a1 += s_red[warp][lane][l + 1];
+        a2 += s_red[warp][lane][l + 2];
+        a3 += s_red[warp][lane][l + 3];
+      }
+      s_tot[warp][lane] = (a0 + a1) + (a2 + a3);
+    }
+    if (heavy) {
+      __syncthreads();
+      if (warp == 0 && lane < 2 * NM)
+        s_tot[0][lane] = (s_tot[0][lane] + s_tot[1][lane]) + (s_tot[2][lane] + s_tot[3][lane]);
+      __syncthreads();
+      if (warp > 0) continue;  // (its own rows of s_red and s_tot are read by no other warp)
+    }
+    __syncwarp();
+    // (1, X0, X1) -> barycentric (1 - X0, X0 - X1, X1) on both cells, a shape pair per lane
+    const int m_ = lane / NB, n_ = lane % NB;
+    if (lane < NM) {
+      auto tot = [&](int m, int n) { return C2<double>{s_tot[warp][2 * (m * NB + n)], s_tot[warp][2 * (m * NB + n) + 1]}; };
+      auto row = [&](int m) {
+        return NB == 3 && n_ < 2 ? csub(tot(m, n_), tot(m, n_ + 1)) : tot(m, n_);
+      };
+      C2<double> T = row(m_);
+      if (NT == 3 && m_ < 2) T = csub(T, row(m_ + 1));
+      s_T[warp][lane] = T;
+    }
+    __syncwarp();
+    if (lane < NM) {
+      const int i = NT == 3 ? pt[m_] : 0, j = NB == 3 ? ps[n_] : 0;
+      C2<double> z;
+      if (!RT) {
+        const double c = I4PI * 4.0 * t.area * s.area * (OPK == BEAST_HH_DLT ? -1.0 : 1.0);
+        const C2<double> T = s_T[warp][lane];
+        z = cmul(C2<double>{P.op.ar, P.op.ai}, C2<double>{c * T.re, c * (GRAD ? sg : -sg) * T.im});
+      } else {
+        double fr = 0.0, fi = 0.0;
+        auto tv = [&](int m) { return m == 0 ? A0 : (m == 1 ? A1 : A2); };
+        auto sv = [&](int n) { return n == 0 ? B0 : (n == 1 ? B1 : B2); };
+        const V3<double> ti = tv(m_), sj = sv(n_);
+#pragma unroll
+        for (int dm = 1; dm < 3; ++dm)
+#pragma unroll
+          for (int dn = 1; dn < 3; ++dn) {
+            const int m = (m_ + dm) % 3, n = (n_ + dn) % 3;
+            const V3<double> em = tv(m) - ti, en = sv(n) - sj;
+            const double w = OPK == BEAST_MW_SL ? dot(em, en) : dot(em, cross(tv(m) - sv(n), en));
+            const C2<double> T = s_T[warp][3 * m + n];
+            fr = fma(w, T.re, fr);
+            fi = fma(w, T.im, fi);
+          }
+        if (OPK == BEAST_MW_SL) {
+          const C2<double> f{I4PI * fr, -sg * I4PI * fi}, m0{4.0 * I4PI * s_tot[warp][0], -sg * 4.0 * I4PI * s_tot[warp][1]};
+          z = cadd(cmul(C2<double>{P.op.ar, P.op.ai}, f), cmul(C2<double>{P.op.br, P.op.bi}, m0));
+        } else {
+          z = C2<double>{-I4PI * fr, -I4PI * sg * fi};
+        }
+      }
+      store_c<double>(P.zcell, zidx(zrow_of(P.zrow, np_.p, NT, i), zcol_of(P.zcol, np_.q, NB, j), P.ldc), z, P.zfmt);
+    }
+    __syncwarp();  // s_red, s_tot and s_T are written again by the next pair
+  }
+}
+
+template <int OPK, int TK, int BK>
+static cudaError_t near_ss64_t(const NearParams& P, cudaStream_t st) {
+  if (P.nnear < 8 * sm_count())
+    k_near_ss64<OPK, TK, BK, 1><<<(unsigned)P.nnear, 32 * NEAR_WARPS, 0, st>>>(P);
+  else
+    k_near_ss64<OPK, TK, BK, NEAR_WARPS><<<(unsigned)((P.nnear + NEAR_WARPS - 1) / NEAR_WARPS), 32 * NEAR_WARPS, 0, st>>>(P);
+  return cudaGetLastError();
+}
+
+template <int OPK>
+static cudaError_t near_ss64_hh(const NearParams& P, cudaStream_t st) {
+  if (P.tk == BEAST_P1 && P.bk == BEAST_P1) return near_ss64_t<OPK, BEAST_P1, BEAST_P1>(P, st);
+  if (P.tk == BEAST_P1) return near_ss64_t<OPK, BEAST_P1, BEAST_P0>(P, st);
+  if (P.bk == BEAST_P1) return near_ss64_t<OPK, BEAST_P0, BEAST_P1>(P, st);
+  return near_ss64_t<OPK, BEAST_P0, BEAST_P0>(P, st);
+}
+
+static cudaError_t launch_near_ss64(const NearParams& P, cudaStream_t st) {
+  switch (P.op.kind) {
+    case BEAST_MW_SL: return near_ss64_t<BEAST_MW_SL, BEAST_RT, BEAST_RT>(P, st);
+    case BEAST_MW_DL: return near_ss64_t<BEAST_MW_DL, BEAST_RT, BEAST_RT>(P, st);
+    case BEAST_HH_SL: return near_ss64_hh<BEAST_HH_SL>(P, st);
+    case BEAST_HH_DL: return near_ss64_hh<BEAST_HH_DL>(P, st);
+    default: return near_ss64_hh<BEAST_HH_DLT>(P, st);
+  }
+}
+
+// the node tables of the strategy's orders (class 1..3) from the context's cache, built on first
+// use (after upload_gl)
+static cudaError_t ss64_tables(std::map<int, void*>* cache, const beast_qs_desc& qs, cudaStream_t st, const double** tab,
+                               int* items) {
+  const int ord[4] = {0, qs.ss_vert, qs.ss_edge, qs.ss_face};
+  for (int c = 1; c <= 3; ++c) {
+    const int n = ord[c];
+    items[c] = (c == 1 ? 2 : 6) * n * n * n * n;
+    const int key = 4096 + 64 * c + n;
+    auto f = cache->find(key);
+    if (f == cache->end()) {
+      void* p = nullptr;
+      cudaError_t e = cudaMalloc(&p, sizeof(double) * SS64_VALS * (size_t)items[c]);
+      if (e != cudaSuccess) return e;
+      k_ss64_table<<<(items[c] + 255) / 256, 256, 0, st>>>(c, n, items[c], (double*)p);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) {
+        cudaFree(p);
+        return e;
+      }
+      f = cache->emplace(key, p).first;
+    }
+    tab[c] = (const double*)f->second;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t launch_near(const AsmArgs& a, int nnear, const TriRuleDev& ro, const TriRuleDev& ri,
                         const TriRuleDev& fro, const TriRuleDev& fri, cudaStream_t st) {
   if (nnear <= 0) return cudaSuccess;
@@ -2880,6 +3490,19 @@ cudaError_t launch_near(const AsmArgs& a, int nnear, const TriRuleDev& ro, const
     e = ss_tables(a.ss_tabs, a.qs, st, P.ssdf_tab, P.ssdf_items);
     if (e != cudaSuccess) return e;
   }
+  // every other Sauter-Schwab pair of the operators on RT (not n x K) and P0 / P1
+  const bool rt = a.ts->kind == BEAST_RT && a.bs->kind == BEAST_RT;
+  const bool sl_dl = a.op.kind == BEAST_MW_SL || a.op.kind == BEAST_MW_DL;
+  const bool hh = a.op.kind == BEAST_HH_SL || a.op.kind == BEAST_HH_DL || a.op.kind == BEAST_HH_DLT;
+  P.ss64 = (a.qs.kind == BEAST_QS_WILTON_SAUTER || a.qs.kind == BEAST_QS_SAUTER) && a.ss_tabs != nullptr &&
+           ((rt && sl_dl && !P.ss32) || (hh && a.ts->kind != BEAST_RT && a.bs->kind != BEAST_RT)) && !P.ssdf;
+  // (orders up to 10: a node table of at most 6 MB; without the memory for it, k_near)
+  if (P.ss64 && (a.qs.ss_vert > 10 || a.qs.ss_edge > 10 || a.qs.ss_face > 10 ||
+                 ss64_tables(a.ss_tabs, a.qs, st, P.ss64_tab, P.ss64_items) != cudaSuccess)) {
+    cudaGetLastError();
+    P.ss64 = 0;
+  }
+  P.wave = g64::make_wave(a.op.gi);
   P.bcells = a.bs->cells;
   P.bchildren = a.bs->mesh->children;
   P.bnchild = a.bs->mesh->nchild;
@@ -2902,7 +3525,12 @@ cudaError_t launch_near(const AsmArgs& a, int nnear, const TriRuleDev& ro, const
     else
       k_near_hh_df<0, 0><<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
   }
-  k_near<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
+  if (P.ss64) {
+    e = launch_near_ss64(P, st);
+    if (e != cudaSuccess) return e;
+  }
+  // (DoubleNumSauterQstrat lists touching pairs only: nothing is left for k_near then)
+  if (!(P.ss64 && P.qs.kind == BEAST_QS_SAUTER)) k_near<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
   if (P.qs.kind == BEAST_QS_TEST_REFINES_TRIAL || P.qs.kind == BEAST_QS_TRIAL_REFINES_TEST)
     k_near_refines<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
   return cudaGetLastError();

@@ -1,0 +1,71 @@
+"""GPU: the FP64 far and Sauter-Schwab kernels where their routes differ -- wavenumber of either sign,
+complex, tiny (CUDA's sine), zero and large, rules other than the default's, node counts on either
+side of the one-warp / whole-CTA split, grids of few and of many CTAs -- against the CPU oracle with
+the FP64 contract: 1e-10 per entry with a floor of 1e-3 of the largest entry."""
+import numpy as np
+import pytest
+
+import beastgpu as bg
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(op, X, Y, qs):
+    Z = bg.assemble(op, X, Y, quadstrat=qs, precision=bg.FP64)
+    Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), X, Y)
+    err = np.abs(Z - Zo) / (np.abs(Zo) + 1e-3 * np.abs(Zo).max())
+    assert err.max() < 1e-10
+
+
+def _mesh(level=1, seed=3):
+    return bg.ellipsoid(level, (1.0, 0.8, 1.3), perturb=0.02, rng=seed)
+
+
+WS = bg.DoubleNumWiltonSauterQStrat
+GAMMAS = [2j, -3j, 0.4 + 2j, 1.5, 1e-3j, 60j]
+
+
+@pytest.mark.parametrize("gamma", GAMMAS)
+@pytest.mark.parametrize("kind", ["sl", "dl", "nxdl"])
+def test_maxwell(kind, gamma):
+    X = bg.raviartthomas(_mesh())
+    op = {"sl": bg.Maxwell3D.singlelayer, "dl": bg.Maxwell3D.doublelayer, "nxdl": bg.nxdoublelayer}[kind](gamma=gamma)
+    _check(op, X, X, bg.DoubleNumQStrat(6, 7) if kind == "nxdl" else WS(2, 3, 6, 7, 5, 5, 4, 3))
+
+
+@pytest.mark.parametrize("gamma", GAMMAS + [0.0])
+@pytest.mark.parametrize("kind,spaces", [("sl", "p1p1"), ("dl", "p1p0"), ("dlt", "p0p1"), ("dl", "p0p0"), ("dlt", "p1p1")])
+def test_helmholtz(kind, spaces, gamma):
+    m = _mesh()
+    s = {"p0": bg.lagrangecxd0(m), "p1": bg.lagrangec0d1(m)}
+    H = bg.Helmholtz3D
+    op = {"sl": H.singlelayer, "dl": H.doublelayer, "dlt": H.doublelayer_transposed}[kind](gamma=gamma)
+    _check(op, s[spaces[:2]], s[spaces[2:]], WS(2, 3, 2, 3, 4, 4, 4, 4))
+
+
+@pytest.mark.parametrize("qs", [WS(1, 1, 2, 3, 3, 3, 3, 3), WS(5, 4, 6, 7, 2, 2, 2, 5), WS(8, 10, 6, 7, 5, 5, 4, 4),
+                                WS(2, 3, 6, 7, 5, 11, 4, 3), bg.DoubleNumSauterQstrat(3, 4, 5, 5, 4, 3),
+                                bg.DoubleNumQStrat(5, 4)])  # (equal rules meet at R = 0 on a cell with itself)
+def test_rules(qs):
+    X = bg.raviartthomas(_mesh())
+    _check(bg.Maxwell3D.singlelayer(wavenumber=2.0), X, X, qs)
+    _check(bg.Maxwell3D.doublelayer(wavenumber=2.0), X, X, qs)
+
+
+@pytest.mark.parametrize("test_cells,trial_cells", [(1, 80), (80, 1), (3, 77), (80, 80)])
+def test_small_blocks(test_cells, trial_cells):
+    """P0 functions of part of a mesh: from one pair per thread to the full tile"""
+    X = bg.lagrangecxd0(_mesh())
+    op = bg.Helmholtz3D.doublelayer(wavenumber=2.0)
+    _check(op, X.subset(np.arange(test_cells)), X.subset(np.arange(trial_cells)), WS(2, 3, 2, 3, 4, 4, 4, 4))
+
+
+def test_many_ctas():
+    X = bg.lagrangecxd0(_mesh(level=4))
+    op = bg.Helmholtz3D.doublelayer_transposed(wavenumber=4.0)
+    Z = bg.assemble(op, X, X, precision=bg.FP64)
+    rows = X.subset(np.arange(0, X.numfunctions(), 331))
+    Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*bg.defaultquadstrat(op, X, X).orders()), rows, X)
+    err = np.abs(Z[::331] - Zo) / (np.abs(Zo) + 1e-3 * np.abs(Zo).max())
+    assert err.max() < 1e-10
