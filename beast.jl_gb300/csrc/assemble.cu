@@ -16,6 +16,7 @@
 //             gather: every output entry written once, no atomics, deterministic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -2307,48 +2308,142 @@ __global__ void k_rhs(int kind, int tk, const int64_t* tptr, const int* tcell, c
 // ------------------------------------------------------------------------------------
 // far field (src/postproc.jl:174-211, 273-288; src/maxwell/farfield.jl:60-63)
 // ------------------------------------------------------------------------------------
-__global__ void k_farfield(const double* geo, const int* ad_dof, const double* ad_coef, int maxfn,
-                           int64_t ncells, const double* u, const double* pts, double gr,
-                           double gi, TriRuleDev r, double* ff) {
-  const int p = blockIdx.x;
-  V3<double> yh = mk(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
+// The current's density on a cell is affine, J(x) = J0 + s (x - c) with c the last vertex (a given
+// point: the rounding of a computed one would shift the cell's phase), s = sum_i u_i / 2A, J0 =
+// sum_i u_i (c - v_i) / 2A (u_i: the shape's coefficient): with x - c = u a + v b over the edges a, b
+// from c, a direction needs three moments of the phase on each cell, (1, u, v) e^{gamma y.x}.  k_farfield_cells writes the cells' records once
+// per call, k_farfield sums a chunk of cells for one direction per CTA, k_farfield_sum adds the
+// chunks in order (the chunks depend on the mesh alone).  Bound by FP64 instructions: ten per rule
+// point (two for the phase, two with integer and FP32 work for its sine and cosine, six for the
+// moments).  8000 cells, 721 directions: 4.4 ms; 37.8 with sincos and the shapes evaluated per point.
+struct FarCell {
+  double c[3], a[3], b[3];
+  double sr, si;      // s A
+  double jr[3], ji[3];  // J0 A
+};
+constexpr int FF_THREADS = 128, FF_CHUNK = 512;
+
+__global__ void k_farfield_cells(const double* geo, const int* ad_dof, const double* ad_coef, int maxfn, int64_t ncells,
+                                 const double* u, FarCell* out) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= ncells) return;
+  const Geo g = load_geo(geo + c * GEO_STRIDE);
+  FarCell f;
+  f.sr = f.si = 0.0;
+  V3<double> jr = mk(0.0, 0.0, 0.0), ji = jr;
+  for (int i = 0; i < 3; ++i) {
+    double ur = 0.0, ui = 0.0;
+    for (int k = 0; k < maxfn; ++k) {
+      const int m = ad_dof[(c * 3 + i) * maxfn + k];
+      if (m < 0) continue;
+      const double a = ad_coef[(c * 3 + i) * maxfn + k];
+      ur += a * u[2 * (int64_t)m];
+      ui += a * u[2 * (int64_t)m + 1];
+    }
+    ur *= 0.5;  // A / 2A
+    ui *= 0.5;
+    f.sr += ur;
+    f.si += ui;
+    const V3<double> e = g.v[2] - g.v[i];
+    jr = jr + ur * e;
+    ji = ji + ui * e;
+  }
+  const V3<double> a = g.v[0] - g.v[2], b = g.v[1] - g.v[2];
+  f.c[0] = g.v[2].x; f.c[1] = g.v[2].y; f.c[2] = g.v[2].z;
+  f.a[0] = a.x; f.a[1] = a.y; f.a[2] = a.z;
+  f.b[0] = b.x; f.b[1] = b.y; f.b[2] = b.z;
+  f.jr[0] = jr.x; f.jr[1] = jr.y; f.jr[2] = jr.z;
+  f.ji[0] = ji.x; f.ji[1] = ji.y; f.ji[2] = ji.z;
+  out[c] = f;
+}
+
+__global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, int64_t ncells, const double* pts, double gr,
+                                                         double gi, g64::Wave wave, TriRuleDev r, double* part) {
+  __shared__ __align__(16) g64::Entry tab[g64::TABLE];
+  __shared__ double s_q[RULE_MAXPTS][5];  // u, v, w, w u, w v
+  __shared__ double red[6][FF_THREADS];
+  g64::load_table(tab);
+  for (int k = threadIdx.x; k < r.n; k += FF_THREADS) {
+    const double u = r.u[k], v = r.v[k];
+    s_q[k][0] = u;
+    s_q[k][1] = v;
+    s_q[k][2] = r.w[k];
+    s_q[k][3] = r.w[k] * u;
+    s_q[k][4] = r.w[k] * v;
+  }
+  __syncthreads();
+  const int64_t p = blockIdx.x, npts = gridDim.x;
+  const V3<double> y = mk(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
+  const double sg = gi < 0.0 ? -1.0 : 1.0;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int64_t c = threadIdx.x; c < ncells; c += blockDim.x) {
-    Geo g = load_geo(geo + c * GEO_STRIDE);
+  const int64_t c1 = min(ncells, (blockIdx.y + 1) * (int64_t)FF_CHUNK);
+  for (int64_t c = blockIdx.y * (int64_t)FF_CHUNK + threadIdx.x; c < c1; c += FF_THREADS) {
+    const FarCell& f = cells[c];
+    const V3<double> a = mk(f.a[0], f.a[1], f.a[2]), b = mk(f.b[0], f.b[1], f.b[2]);
+    const double pa = dot(y, a), pb = dot(y, b);
+    // y . c enters the phase of all the cell's points, so its rounding would not average out over
+    // them: a sum of exact products with the rounding errors kept
+    double pc = y.x * f.c[0], pl = fma(y.x, f.c[0], -pc);
+#pragma unroll
+    for (int k = 1; k < 3; ++k) {
+      const double yk = k == 1 ? y.y : y.z, q = yk * f.c[k], t = pc + q, z = t - pc;
+      pl += fma(yk, f.c[k], -q) + ((pc - (t - z)) + (q - z));
+      pc = t;
+    }
+    const double fa = pa * wave.steps, fb = pb * wave.steps, fc = pc * wave.steps;
+    const float rest = (float)fma(pc, wave.steps, -fc) + ((float)pl * (float)wave.steps + (float)pc * wave.rest);
+    C2<double> E0{0, 0}, Eu{0, 0}, Ev{0, 0};
     for (int k = 0; k < r.n; ++k) {
-      double bx[3] = {r.u[k], r.v[k], 1.0 - r.u[k] - r.v[k]};
-      V3<double> x = bx[0] * g.v[0] + bx[1] * g.v[1] + bx[2] * g.v[2];
-      double w = r.w[k] * g.area;
-      double ph = dot(yh, x);
-      C2<double> krn = cexp_d(C2<double>{gr * ph, gi * ph});  // exp(gamma yhat.x)
-      Shp f;
-      shapes(BEAST_RT, g, x, bx, f);
-      for (int i = 0; i < 3; ++i) {
-        C2<double> cu{0, 0};
-        for (int kk = 0; kk < maxfn; ++kk) {
-          int mdof = ad_dof[(c * 3 + i) * maxfn + kk];
-          if (mdof < 0) continue;
-          double a = ad_coef[(c * 3 + i) * maxfn + kk];
-          cu = cadd(cu, cscale(a, C2<double>{u[2 * mdof], u[2 * mdof + 1]}));
-        }
-        C2<double> s = cscale(w, cmul(krn, cu));
-        V3<double> tr = cross(cross(yh, f.v[i]), yh);
-        acc[0] += s.re * tr.x; acc[1] += s.im * tr.x;
-        acc[2] += s.re * tr.y; acc[3] += s.im * tr.y;
-        acc[4] += s.re * tr.z; acc[5] += s.im * tr.z;
+      // (the whole phase per point: the rounding of a cell's phase, applied once to its moments,
+      // would not average out)
+      const double phi = fma(s_q[k][1], fb, fma(s_q[k][0], fa, fc));
+      double cs, sn;
+      if (!g64::turn_signed(phi, rest, tab, cs, sn)) sincos(wave.k * fma(s_q[k][1], pb, fma(s_q[k][0], pa, pc)), &sn, &cs);
+      if (gr != 0.0) {
+        const double m = exp(gr * fma(s_q[k][1], pb, fma(s_q[k][0], pa, pc)));
+        cs *= m;
+        sn *= m;
       }
+      E0.re = fma(s_q[k][2], cs, E0.re);
+      E0.im = fma(s_q[k][2], sn, E0.im);
+      Eu.re = fma(s_q[k][3], cs, Eu.re);
+      Eu.im = fma(s_q[k][3], sn, Eu.im);
+      Ev.re = fma(s_q[k][4], cs, Ev.re);
+      Ev.im = fma(s_q[k][4], sn, Ev.im);
+    }
+    E0.im *= sg;
+    Eu.im *= sg;
+    Ev.im *= sg;
+    const C2<double> s{f.sr, f.si};
+    Eu = cmul(s, Eu);
+    Ev = cmul(s, Ev);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      acc[2 * k] += (E0.re * f.jr[k] - E0.im * f.ji[k]) + (Eu.re * f.a[k] + Ev.re * f.b[k]);
+      acc[2 * k + 1] += (E0.re * f.ji[k] + E0.im * f.jr[k]) + (Eu.im * f.a[k] + Ev.im * f.b[k]);
     }
   }
-  __shared__ double red[6][256];
   for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = acc[k];
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+  for (int o = FF_THREADS / 2; o > 0; o >>= 1) {
     if (threadIdx.x < o)
       for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 6; ++k) ff[6 * p + k] = red[k][0];
+  if (threadIdx.x < 6) part[(blockIdx.y * npts + p) * 6 + threadIdx.x] = red[threadIdx.x][0];
+}
+
+// the chunks' sums, then (y x F) x y
+__global__ void k_farfield_sum(const double* part, int nchunk, int64_t npts, const double* pts, double* ff) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p >= npts) return;
+  double f[6] = {0, 0, 0, 0, 0, 0};
+  for (int c = 0; c < nchunk; ++c)
+    for (int k = 0; k < 6; ++k) f[k] += part[(c * npts + p) * 6 + k];
+  const V3<double> y = mk(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
+  const V3<double> re = cross(cross(y, mk(f[0], f[2], f[4])), y), im = cross(cross(y, mk(f[1], f[3], f[5])), y);
+  double* o = ff + 6 * p;
+  o[0] = re.x; o[1] = im.x; o[2] = re.y; o[3] = im.y; o[4] = re.z; o[5] = im.z;
 }
 
 }  // namespace
@@ -3602,9 +3697,33 @@ cudaError_t launch_rhs(int kind, const beast_space* ts, const double* dir, const
 cudaError_t launch_farfield(const beast_space* s, const double* u, const double* pts, int64_t npts,
                             double gr, double gi, const TriRuleDev& r, double* ff, cudaStream_t st) {
   if (npts == 0) return cudaSuccess;
-  k_farfield<<<(unsigned)npts, 256, 0, st>>>(s->geo, s->ad_dof, s->ad_coeff, s->maxfn, s->ncells, u,
-                                             pts, gr, gi, r, ff);
-  return cudaGetLastError();
+  const int nchunk = (int)((s->ncells + FF_CHUNK - 1) / FF_CHUNK);
+  // directions in slabs whose partial sums take at most 64 MB
+  const int64_t slab = std::max<int64_t>(1, std::min<int64_t>(npts, (64ll << 20) / (48 * std::max(nchunk, 1))));
+  FarCell* cells = nullptr;
+  double* part = nullptr;
+  cudaError_t e = cudaMallocAsync(&cells, sizeof(FarCell) * (size_t)s->ncells + 256, st);
+  if (e != cudaSuccess) return e;
+  e = cudaMallocAsync(&part, sizeof(double) * 6 * (size_t)slab * nchunk + 256, st);
+  if (e != cudaSuccess) {
+    cudaFreeAsync(cells, st);
+    return e;
+  }
+  if (s->ncells > 0)
+    k_farfield_cells<<<(unsigned)((s->ncells + 127) / 128), 128, 0, st>>>(s->geo, s->ad_dof, s->ad_coeff, s->maxfn,
+                                                                          s->ncells, u, cells);
+  const g64::Wave wave = g64::make_wave(gi);
+  for (int64_t p0 = 0; p0 < npts; p0 += slab) {
+    const int64_t n = std::min(slab, npts - p0);
+    if (nchunk > 0)
+      k_farfield<<<dim3((unsigned)n, (unsigned)nchunk), FF_THREADS, 0, st>>>(cells, s->ncells, pts + 3 * p0, gr, gi, wave, r,
+                                                                             part);
+    k_farfield_sum<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, nchunk, n, pts + 3 * p0, ff + 6 * p0);
+  }
+  e = cudaGetLastError();
+  cudaFreeAsync(cells, st);
+  cudaFreeAsync(part, st);
+  return e;
 }
 
 cudaError_t launch_local_impl(int which, const beast_space* ts, const beast_space* bs,

@@ -179,17 +179,10 @@ G64_HD void inv_sqrt(double R2, double& iR, double& R) {
   R = fma(r, half(g), g);
 }
 
-// cos and sin of phi steps (+ rest steps) for phi in [64, 2^30)
-G64_HD void turn(double phi, float rest, const Entry* tab, double& c, double& s) {
-  const uint64_t u = bits(phi);
-  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
-  const int e = (int)(hi >> 20) - 1023;  // 6 .. 29
-  // the mantissa at the top of 64 bits: integer part above bit 63 - e, fraction below
-  const uint32_t xh = ((hi << 11) | (lo >> 21)) | 0x80000000u, xl = lo << 11;
-  const uint32_t n0 = xh >> (31 - e);
-  const uint32_t fh = (xh << (e + 1)) | (xl >> (31 - e)), fl = xl << (e + 1);
-  const uint32_t n = n0 + (fh >> 31);
-  // the fraction in [-1/2, 1/2) as 24 + 32 bits
+// cos and sin of n + f steps, the fraction f in [-1/2, 1/2) as the 64-bit fixed-point number fh:fl
+// (plus rest)
+G64_HD void rotate(uint32_t n, uint32_t fh, uint32_t fl, float rest, const Entry* tab, double& c, double& s) {
+  // the fraction as 24 + 32 bits
   const float fa = fmul((float)(int32_t)(fh & 0xFFFFFF00u), 2.3283064365386963e-10f);
   const float fb = fmaf((float)((fh << 24) | (fl >> 8)), 1.3877787807814457e-17f, rest);
   const float th = fmul(fa, G64_STEP_HI);
@@ -220,6 +213,32 @@ G64_HD void turn(double phi, float rest, const Entry* tab, double& c, double& s)
   const uint64_t us = bits((q & 1) ? c0 : s0), uc = bits((q & 1) ? s0 : c0);
   s = from_bits(us ^ ((uint64_t)(q >> 1) << 63));
   c = from_bits(uc ^ ((uint64_t)(((q + 1) >> 1) & 1) << 63));
+}
+
+// cos and sin of phi steps (+ rest steps) for phi in [64, 2^30)
+G64_HD void turn(double phi, float rest, const Entry* tab, double& c, double& s) {
+  const uint64_t u = bits(phi);
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
+  const int e = (int)(hi >> 20) - 1023;  // 6 .. 29
+  // the mantissa at the top of 64 bits: integer part above bit 63 - e, fraction below
+  const uint32_t xh = ((hi << 11) | (lo >> 21)) | 0x80000000u, xl = lo << 11;
+  const uint32_t fh = (xh << (e + 1)) | (xl >> (31 - e)), fl = xl << (e + 1);
+  rotate((xh >> (31 - e)) + (fh >> 31), fh, fl, rest, tab, c, s);
+}
+
+// the same for any phi (+ rest) with |phi| < 2^30, to 2^-52 absolutely (a small sine keeps no
+// relative accuracy); false: out of range
+G64_HD bool turn_signed(double phi, float rest, const Entry* tab, double& c, double& s) {
+  const uint64_t u = bits(phi);
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
+  const int e = (int)((hi >> 20) & 0x7FF) - 1023;
+  if (e > 29) return false;
+  const uint64_t x = ((uint64_t)(((hi << 11) | (lo >> 21)) | 0x80000000u) << 32) | (lo << 11);
+  const uint64_t f = e >= 0 ? x << (e + 1) : (e > -64 ? x >> (-1 - e) : 0);
+  const uint32_t n0 = e >= 0 ? (uint32_t)(x >> 32) >> (31 - e) : 0u;
+  rotate(n0 + (uint32_t)(f >> 63), (uint32_t)(f >> 32), (uint32_t)f, (u >> 63) ? -rest : rest, tab, c, s);
+  s = from_bits(bits(s) ^ (u & 0x8000000000000000ull));
+  return true;
 }
 
 G64_HD Value eval(double R2, const Wave& w, const Entry* tab) {

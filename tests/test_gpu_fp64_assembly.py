@@ -2,11 +2,15 @@
 complex, tiny (CUDA's sine), zero and large, rules other than the default's, node counts on either
 side of the one-warp / whole-CTA split, grids of few and of many CTAs -- against the CPU oracle with
 the FP64 contract: 1e-10 per entry with a floor of 1e-3 of the largest entry."""
+import os
+import re
+
 import numpy as np
 import pytest
 
 import beastgpu as bg
 import oracle as O
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +73,33 @@ def test_many_ctas():
     Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*bg.defaultquadstrat(op, X, X).orders()), rows, X)
     err = np.abs(Z[::331] - Zo) / (np.abs(Zo) + 1e-3 * np.abs(Zo).max())
     assert err.max() < 1e-10
+
+
+def _farfield_sum(X, u, d, gamma):
+    """the far field as a plain sum over the package's own rule points (the oracle's rule of degree 10
+    agrees with them to about 1e-13, which 80 radians per unit length magnify)"""
+    with open(os.path.join(ROOT, "beast.jl_gb300", "csrc", "rules_gen.h")) as fh:
+        rows = re.findall(r"\{([-0-9.e]+), ([-0-9.e]+), ([-0-9.e]+)\}", fh.read())
+    q = np.array([[float(x) for x in r] for r in rows[88:113]])
+    v, area = X.mesh.vertices[X.mesh.cells], X.mesh.areas()
+    x = np.einsum("qk,ckx->cqx", np.column_stack([q[:, :2], 1 - q[:, 0] - q[:, 1]]), v)
+    J = np.zeros(x.shape, dtype=complex)
+    for i, fn in enumerate(X.fns):
+        for c, r, w in fn:
+            J[c] += u[i] * w * (x[c] - v[c, r]) / (2 * area[c])
+    F = np.array([np.einsum("q,c,cq,cqx->x", q[:, 2], area, np.exp(gamma * (x @ y)), J) for y in d])
+    return np.cross(np.cross(d, F), d)
+
+
+@pytest.mark.parametrize("gamma", [2j, -3j, 0.4 + 2j, 0.5, 80j, 1e-4j])
+@pytest.mark.parametrize("level,npts", [(0, 1), (2, 7), (3, 130)])
+def test_farfield(level, npts, gamma):
+    """one cell chunk and several, the last one partial; directions that are not unit vectors too"""
+    X = bg.raviartthomas(_mesh(level))
+    rng = np.random.default_rng(level)
+    u = rng.normal(size=X.numfunctions()) + 1j * rng.normal(size=X.numfunctions())
+    d = rng.normal(size=(npts, 3))
+    d[::2] /= np.linalg.norm(d[::2], axis=1, keepdims=True)
+    ff = bg.farfield(X, u, d, gamma)
+    fo = _farfield_sum(X, u, d, gamma)
+    assert np.abs(ff - fo).max() <= 1e-12 * np.abs(fo).max()

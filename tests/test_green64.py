@@ -34,6 +34,9 @@ void t_eval(long n, const double* R2, double k, double* out) {
 void t_turn(long n, const double* phi, double* out) {
   for (long i = 0; i < n; ++i) g64::turn(phi[i], 0.f, tab, out[2 * i], out[2 * i + 1]);
 }
+void t_turn_signed(long n, const double* phi, double* out) {
+  for (long i = 0; i < n; ++i) g64::turn_signed(phi[i], 0.f, tab, out[2 * i], out[2 * i + 1]);
+}
 double t_pair(float h, float l) { return g64::pair_to_double(h, l); }
 }
 """
@@ -99,3 +102,16 @@ def test_pair_to_double(lib):
         l = -h * 2.0 ** -26
         assert lib.t_pair(h, l) == h + l
     assert lib.t_pair(0.0, 0.0) == 0.0
+
+
+def test_turn_signed(lib):
+    """any angle below 2^30 steps, of either sign, absolutely"""
+    rng = np.random.default_rng(4)
+    phi = np.concatenate([rng.uniform(-3000, 3000, size=600), rng.uniform(-1, 1, size=200), [0.0, 0.5, -0.5, 1.0, -1.5, 1e-30, 2.0 ** 30 - 1],
+                          2.0 ** rng.uniform(-70, 29, size=200)])
+    out = np.zeros((len(phi), 2))
+    lib.t_turn_signed(C.c_long(len(phi)), phi.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p))
+    mpmath.mp.dps = 40
+    for p, (c, s) in zip(phi, out):
+        th = mpmath.mpf(float(p)) * mpmath.pi / 2048
+        assert abs(c - mpmath.cos(th)) <= 2.0 ** -52 and abs(s - mpmath.sin(th)) <= 2.0 ** -52
