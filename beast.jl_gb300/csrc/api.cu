@@ -167,6 +167,7 @@ int beast_ctx_destroy(beast_ctx* ctx) {
   }
   if (ctx->ws) cudaFree(ctx->ws);
   if (ctx->d_flag) cudaFree(ctx->d_flag);
+  if (ctx->pinned) cudaFreeHost(ctx->pinned);
   for (auto& kv : ctx->ss_tabs) cudaFree(kv.second);
   for (auto& r : ctx->prof) {
     cudaEventDestroy(r.a);
@@ -1198,8 +1199,10 @@ int beast_solve_dense(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int
   return rc;
 }
 
-// restarted GMRES with modified Gram-Schmidt (one dot kernel per basis vector) and Givens
-// rotations on the host (the Hessenberg matrix is tiny)
+// restarted GMRES: classical Gram-Schmidt with one reorthogonalisation (linalg.cu, no host round
+// trip inside an iteration) and Givens rotations on the host (the Hessenberg matrix is tiny).  The
+// host reads an iteration's coefficients while the next basis vector's matvec, queued before the
+// wait, runs: it needs nothing the rotations decide, and after the last iteration it is dropped.
 int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dtype, const double* b,
                 double* x, int bx_loc, double reltol, int restart, int maxiter, int* iters,
                 double* resid) {
@@ -1209,11 +1212,28 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
   if (restart <= 0) restart = (int)std::min<int64_t>(n, 200);
   if (maxiter <= 0) maxiter = (int)n;
   const int m = restart;
+  const int c64 = a_dtype == BEAST_C64;
   double *V = nullptr, *w = nullptr, *db = nullptr, *dx = nullptr, *h = nullptr, *nrm = nullptr;
+  void* work = nullptr;
   BEAST_CUDA_TRY(ctx, cudaMallocAsync(&V, (size_t)n * (m + 1) * 16, st));
   BEAST_CUDA_TRY(ctx, cudaMallocAsync(&w, n * 16, st));
-  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&h, (m + 2) * 16, st));
+  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&h, (size_t)(m + 2) * 32 + 64, st));
   BEAST_CUDA_TRY(ctx, cudaMallocAsync(&nrm, 64, st));
+  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&work, gmres_work_bytes(n, m), st));
+  unsigned int* count = reinterpret_cast<unsigned int*>(nrm + 4);
+  BEAST_CUDA_TRY(ctx, cudaMemsetAsync(nrm, 0, 64, st));
+  const size_t pin = (size_t)(m + 2) * 32 + 64;
+  std::lock_guard<std::mutex> pinned_lock(ctx->pinned_mtx);
+  if (ctx->pinned_size < pin) {
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    ctx->pinned = nullptr;
+    ctx->pinned_size = 0;
+    BEAST_CUDA_TRY(ctx, cudaMallocHost(&ctx->pinned, pin));
+    ctx->pinned_size = pin;
+  }
+  double* hh = static_cast<double*>(ctx->pinned);
+  cudaEvent_t ready;
+  BEAST_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
   if (bx_loc != BEAST_DEVICE) {
     BEAST_CUDA_TRY(ctx, cudaMallocAsync(&db, n * 16, st));
     BEAST_CUDA_TRY(ctx, cudaMallocAsync(&dx, n * 16, st));
@@ -1227,39 +1247,30 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
   double bn = dev_norm(ctx, n, db, nrm);
   int it = 0;
   double rel = 1.0;
-  std::vector<cd> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m), hh(m + 1);
+  std::vector<cd> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
   while (true) {
-    // r = b - A x  into V[:,0]
-    BEAST_CUDA_TRY(ctx, vec_copy(n, db, V, st));
-    BEAST_CUDA_TRY(ctx, gemv_dev(n, A, lda, a_dtype == BEAST_C64, dx, V, -1.0, 1.0, st));
-    double rn = dev_norm(ctx, n, V, nrm);
+    // w = r = b - A x, its norm at nrm
+    BEAST_CUDA_TRY(ctx, vec_copy(n, db, w, st));
+    BEAST_CUDA_TRY(ctx, gemv_dev(n, A, lda, c64, dx, w, -1.0, 1.0, st));
+    double rn = dev_norm(ctx, n, w, nrm);
     rel = bn > 0 ? rn / bn : rn;
     if (rel <= reltol || it >= maxiter || rn == 0.0) break;
-    BEAST_CUDA_TRY(ctx, vec_axpy(n, 1.0 / rn - 1.0, 0.0, V, V, st));  // V0 *= 1/rn
     std::fill(g.begin(), g.end(), cd(0));
     g[0] = rn;
-    int k = 0;
+    int k = 0, slabs = 0;
+    BEAST_CUDA_TRY(ctx, gmres_matvec(n, A, lda, c64, w, nrm, V, work, &slabs, st));
     for (; k < m && it < maxiter; ++k) {
-      double* vk = V + 2 * (int64_t)k * n;
-      double* vk1 = V + 2 * (int64_t)(k + 1) * n;
-      BEAST_CUDA_TRY(ctx, gemv_dev(n, A, lda, a_dtype == BEAST_C64, vk, w, 1.0, 0.0, st));
-      // modified Gram-Schmidt as two classical passes (reorthogonalisation), FP64
-      for (int pass = 0; pass < 2; ++pass) {
-        BEAST_CUDA_TRY(ctx, vec_dots(n, k + 1, V, n, w, h, st));
-        BEAST_CUDA_TRY(ctx, vec_gemv_sub(n, k + 1, V, n, h, w, st));
-        BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(hh.data(), h, (k + 1) * 16, cudaMemcpyDeviceToHost, st));
-        BEAST_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-        for (int j = 0; j <= k; ++j) {
-          if (pass == 0)
-            H[j + (size_t)k * (m + 1)] = hh[j];
-          else
-            H[j + (size_t)k * (m + 1)] += hh[j];
-        }
-      }
-      double hn = dev_norm(ctx, n, w, nrm);
+      BEAST_CUDA_TRY(ctx, gmres_orthogonalise(n, k, m, slabs, V, w, work, count, h, st));
+      const int kk = k + 1;
+      BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(hh, h, (size_t)kk * 32 + 8, cudaMemcpyDeviceToHost, st));
+      BEAST_CUDA_TRY(ctx, cudaEventRecord(ready, st));
+      if (kk < m && it + 1 < maxiter)
+        BEAST_CUDA_TRY(ctx, gmres_matvec(n, A, lda, c64, w, h + 4 * kk, V + 2 * (int64_t)kk * n, work, &slabs, st));
+      BEAST_CUDA_TRY(ctx, cudaEventSynchronize(ready));
+      for (int j = 0; j <= k; ++j)
+        H[j + (size_t)k * (m + 1)] = cd(hh[2 * j], hh[2 * j + 1]) + cd(hh[2 * (kk + j)], hh[2 * (kk + j) + 1]);
+      const double hn = std::sqrt(hh[4 * kk]);
       H[k + 1 + (size_t)k * (m + 1)] = hn;
-      BEAST_CUDA_TRY(ctx, cudaMemsetAsync(vk1, 0, n * 16, st));
-      if (hn > 0) BEAST_CUDA_TRY(ctx, vec_axpy(n, 1.0 / hn, 0.0, w, vk1, st));
       for (int j = 0; j < k; ++j) {
         cd h0 = H[j + (size_t)k * (m + 1)], h1 = H[j + 1 + (size_t)k * (m + 1)];
         H[j + (size_t)k * (m + 1)] = std::conj(cs[j]) * h0 + std::conj(sn[j]) * h1;
@@ -1291,12 +1302,14 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
     BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(h, yh.data(), k * 16, cudaMemcpyHostToDevice, st));
     BEAST_CUDA_TRY(ctx, vec_gemv_sub(n, k, V, n, h, dx, st));
   }
+  cudaEventDestroy(ready);
   if (bx_loc != BEAST_DEVICE) BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(x, dx, n * 16, cudaMemcpyDeviceToHost, st));
   BEAST_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   cudaFreeAsync(V, st);
   cudaFreeAsync(w, st);
   cudaFreeAsync(h, st);
   cudaFreeAsync(nrm, st);
+  cudaFreeAsync(work, st);
   if (bx_loc != BEAST_DEVICE) {
     cudaFreeAsync(db, st);
     cudaFreeAsync(dx, st);

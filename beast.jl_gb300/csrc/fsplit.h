@@ -93,6 +93,21 @@ FS_HD void split_f64(double a, float* hi, float* lo) {
 
 namespace fsplit {
 
+// split_f64 in eight instructions for 2^-73 <= |a| < 2^128 (the low part rounded to nearest from its
+// 29 bits by an integer conversion, which does not run on the FP64 pipe); other values take split_f64
+FS_HD void split_f64_fast(double a, float* hi, float* lo) {
+  const uint64_t u = bits64(a);
+  const uint32_t top = (uint32_t)(u >> 32), low = (uint32_t)u;
+  if (((top >> 20) & 0x7FF) - 950u > 200u) {
+    split_f64(a, hi, lo);
+    return;
+  }
+  const uint32_t sgn = top & 0x80000000u;
+  const uint32_t f = (((top & 0x7FFFFFFFu) - (896u << 20)) << 3) | (low >> 29);
+  *hi = from_bits(f | sgn);
+  *lo = (float)(int32_t)(low & 0x1FFFFFFFu) * from_bits(((f & 0x7F800000u) - (52u << 23)) | sgn);
+}
+
 // a double rounded to the nearest float (ties to even) with integer operations only: the same
 // bits as the conversion instruction for results in the normal float range; results below it
 // (|a| < 2^-126) become 0, results above it +-inf, NaN stays NaN

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -56,6 +57,11 @@ struct beast_ctx {
   cudaEvent_t la_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   // Sauter-Schwab node tables as double-float pairs, built on first use: key 64 class + order
   std::map<int, void*> ss_tabs;
+  // pinned host memory that beast_gmres reads coefficients back through, grown on demand; held
+  // under its mutex (calls of several host threads on one context)
+  std::mutex pinned_mtx;
+  void* pinned = nullptr;
+  size_t pinned_size = 0;
 };
 
 // the lookahead stream and events of ctx (created once); false when they cannot be made
@@ -305,9 +311,13 @@ cudaError_t vec_axpy(int64_t n, double ar, double ai, const double* x, double* y
 cudaError_t vec_copy(int64_t n, const double* x, double* y, cudaStream_t st);
 // reduction: sum of |x|^2 into out (device double), deterministic
 cudaError_t vec_norm2(int64_t n, const double* x, double* out, cudaStream_t st);
-// h[k] = <v_k, w> for k < m (columns of V with ld), FP64
-cudaError_t vec_dots(int64_t n, int m, const double* V, int64_t ldv, const double* w, double* h,
-                     cudaStream_t st);
+// GMRES (linalg.cu): workspace bytes of a solve with restart length m; the normalised basis vector
+// and its matvec; the orthogonalisation (out on the device: 2 (k + 1) complex and one real value)
+size_t gmres_work_bytes(int64_t n, int m);
+cudaError_t gmres_matvec(int64_t n, const void* A, int64_t lda, int a_c64, const double* w, const double* norm2,
+                         double* vk, void* work, int* slabs, cudaStream_t st);
+cudaError_t gmres_orthogonalise(int64_t n, int k, int m, int slabs, const double* V, double* w, void* work,
+                                unsigned int* count, double* out, cudaStream_t st);
 // w -= V h (m columns)
 cudaError_t vec_gemv_sub(int64_t n, int m, const double* V, int64_t ldv, const double* h,
                          double* w, cudaStream_t st);

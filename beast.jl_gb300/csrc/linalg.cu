@@ -1617,7 +1617,9 @@ __global__ void k_permute(const T* in, T* out, const int* perm, int64_t n) {
 }
 
 // ---- FP64 matvec y = alpha A x + beta y  (A c128 or c64) --------------------------------
-constexpr int MV_SLABS = 32;
+// Column slabs of the partial sums (grid.y): as many row blocks x slabs as fill whole waves of the
+// CTAs the chip holds (mv_slabs), up to
+constexpr int MV_MAX_SLABS = 64;
 // x (complex FP64) split into float hi + lo parts: (re_hi, im_hi, re_lo, im_lo)
 __global__ void k_split_x(int64_t n, const double* x, float4* xs) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1644,7 +1646,7 @@ __global__ void k_gemv_partial_c64_df(int64_t n, const float2* A, int64_t lda, c
                                       double* part) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int s = blockIdx.y;
-  int64_t c0 = n * s / MV_SLABS, c1 = n * (s + 1) / MV_SLABS;
+  int64_t c0 = n * s / gridDim.y, c1 = n * (s + 1) / gridDim.y;
   if (i >= n) return;
   float shr = 0.f, slr = 0.f, shi = 0.f, sli = 0.f;
   for (int64_t j = c0; j < c1; ++j) {
@@ -1684,38 +1686,50 @@ __global__ void k_gemv_partial_c64_df(int64_t n, const float2* A, int64_t lda, c
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) {  // a - b, one rounding
   return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
 }
-__device__ __forceinline__ void two_sum2(float2& sh, float2& sl, float2 p) {
-  const float2 t = __fadd2_rn(sh, p);
+// sh + sl += A X with the product's and the sum's rounding errors kept; nX = -X gives the negated
+// product without a negation (the packed operations have no sign modifiers)
+__device__ __forceinline__ void cdf_prod2(float2 A, float2 X, float2 nX, float2& sh, float2& sl) {
+  const float2 np = __fmul2_rn(A, nX);        // -p
+  const float2 e = __ffma2_rn(A, X, np);      // A X - p
+  const float2 t = sub2(sh, np);
   const float2 bb = sub2(t, sh);
-  sl = __fadd2_rn(sl, __fadd2_rn(sub2(sh, sub2(t, bb)), sub2(p, bb)));
+  const float2 v = sub2(sh, sub2(t, bb));     // TwoSum(sh, p): v - (np + bb)
+  sl = __fadd2_rn(sl, __fadd2_rn(v, sub2(e, __fadd2_rn(np, bb))));
   sh = t;
 }
-__device__ __forceinline__ void cdf_acc2(float2 A, float2 B, float2 X1, float2 X2, float2 L1, float2 L2, float2& sh,
-                                         float2& sl) {
-  float2 p = __fmul2_rn(A, X1);
-  float2 e = __ffma2_rn(A, X1, make_float2(-p.x, -p.y));
-  two_sum2(sh, sl, p);
-  sl = __fadd2_rn(sl, e);
-  p = __fmul2_rn(B, X2);
-  e = __ffma2_rn(B, X2, make_float2(-p.x, -p.y));
-  two_sum2(sh, sl, p);
-  sl = __fadd2_rn(sl, e);
-  sl = __ffma2_rn(A, L1, sl);
-  sl = __ffma2_rn(B, L2, sl);
+// one column of the vector as the packed operands of both parts: (x_r, x_i) with A_r, (-x_i, x_r)
+// with A_i, their negatives and the low halves
+struct MvX {
+  float2 X1, X2, n1, n2, L1, L2;
+};
+__device__ __forceinline__ MvX mv_x(float4 v) {
+  MvX x;
+  x.X1 = make_float2(v.x, v.y);
+  x.n1 = make_float2(-v.x, -v.y);
+  x.X2 = make_float2(x.n1.y, v.x);
+  x.n2 = make_float2(v.y, x.n1.x);
+  x.L1 = make_float2(v.z, v.w);
+  x.L2 = make_float2(-v.w, v.z);
+  return x;
+}
+__device__ __forceinline__ void cdf_acc2(float ar, float ai, const MvX& x, float2& sh, float2& sl) {
+  const float2 A = make_float2(ar, ar), B = make_float2(ai, ai);
+  cdf_prod2(A, x.X1, x.n1, sh, sl);
+  cdf_prod2(B, x.X2, x.n2, sh, sl);
+  sl = __ffma2_rn(A, x.L1, sl);
+  sl = __ffma2_rn(B, x.L2, sl);
 }
 __global__ void k_gemv_partial_c64_df2(int64_t n, const float2* A, int64_t lda, const float4* xs,
                                        double* part) {
   const int64_t i = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
   const int s = blockIdx.y;
-  const int64_t c0 = n * s / MV_SLABS, c1 = n * (s + 1) / MV_SLABS;
+  const int64_t c0 = n * s / gridDim.y, c1 = n * (s + 1) / gridDim.y;
   if (i >= n) return;
   const bool two = i + 1 < n;
   float2 h0 = make_float2(0.f, 0.f), l0 = h0, h1 = h0, l1 = h0;
 #pragma unroll 4
   for (int64_t j = c0; j < c1; ++j) {
-    const float4 xv = xs[j];
-    const float2 X1 = make_float2(xv.x, xv.y), X2 = make_float2(-xv.y, xv.x);
-    const float2 L1 = make_float2(xv.z, xv.w), L2 = make_float2(-xv.w, xv.z);
+    const MvX x = mv_x(xs[j]);
     float4 a;
     if (two) {
       a = *reinterpret_cast<const float4*>(A + i + j * lda);
@@ -1723,8 +1737,8 @@ __global__ void k_gemv_partial_c64_df2(int64_t n, const float2* A, int64_t lda, 
       const float2 a0 = A[i + j * lda];
       a = make_float4(a0.x, a0.y, 0.f, 0.f);
     }
-    cdf_acc2(make_float2(a.x, a.x), make_float2(a.y, a.y), X1, X2, L1, L2, h0, l0);
-    cdf_acc2(make_float2(a.z, a.z), make_float2(a.w, a.w), X1, X2, L1, L2, h1, l1);
+    cdf_acc2(a.x, a.y, x, h0, l0);
+    cdf_acc2(a.z, a.w, x, h1, l1);
   }
   part[2 * (s * n + i)] = (double)h0.x + (double)l0.x;
   part[2 * (s * n + i) + 1] = (double)h0.y + (double)l0.y;
@@ -1739,47 +1753,75 @@ __global__ void k_gemv_partial_c64_df2(int64_t n, const float2* A, int64_t lda, 
 // the low parts (hi * x_lo, lo * x_hi) accumulated in FP32 -- the compensated dot product of
 // k_gemv_partial_c64_df2 with the matrix's own low part added.  About 2^-47 relative per
 // product, against a few FP64 multiply-adds per entry at GB300's FP64 rate.
-__global__ void k_gemv_partial_c128_df(int64_t n, const double2* A, int64_t lda, const float4* xs,
-                                       double* part) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Two rows (128 apart) per thread share the vector's loads and operand pairs; the eight matrix
+// loads of four columns are in flight before their arithmetic: 2.72 ms at n = 30720 (5.6 TB/s; one row
+// per thread and 32 slabs: 3.08 ms), 0.200 ms at n = 7213 (0.217).
+constexpr int MV_ROWS = 256;  // rows per CTA of 128 threads
+__global__ void __launch_bounds__(128) k_gemv_partial_c128_df(int64_t n, const double2* A, int64_t lda, const float4* xs,
+                                                              double* part) {
+  const int64_t i0 = blockIdx.x * (int64_t)MV_ROWS + threadIdx.x, i1 = i0 + 128;
   const int s = blockIdx.y;
-  const int64_t c0 = n * s / MV_SLABS, c1 = n * (s + 1) / MV_SLABS;
-  if (i >= n) return;
-  float2 h = make_float2(0.f, 0.f), l = h;
-  auto term = [&](const double2 a, const float4 xv) {
-    const float2 X1 = make_float2(xv.x, xv.y), X2 = make_float2(-xv.y, xv.x);
-    const float2 L1 = make_float2(xv.z, xv.w), L2 = make_float2(-xv.w, xv.z);
-    float2 ar, ai;
-    fsplit::split_f64(a.x, &ar.x, &ar.y);
-    fsplit::split_f64(a.y, &ai.x, &ai.y);
-    cdf_acc2(make_float2(ar.x, ar.x), make_float2(ai.x, ai.x), X1, X2, L1, L2, h, l);
-    l = __ffma2_rn(make_float2(ar.y, ar.y), X1, l);
-    l = __ffma2_rn(make_float2(ai.y, ai.y), X2, l);
+  const int64_t c0 = n * s / gridDim.y, c1 = n * (s + 1) / gridDim.y;
+  const bool in0 = i0 < n, in1 = i1 < n;
+  float2 h0 = make_float2(0.f, 0.f), l0 = h0, h1 = h0, l1 = h0;
+  auto term = [&](float2 ar, float2 ai, const MvX& x, float2& h, float2& l) {
+    cdf_acc2(ar.x, ai.x, x, h, l);
+    l = __ffma2_rn(make_float2(ar.y, ar.y), x.X1, l);
+    l = __ffma2_rn(make_float2(ai.y, ai.y), x.X2, l);
   };
-  // eight streaming loads in flight per thread before their arithmetic (the matrix is read
-  // once per matvec; its latency, not the FP32 work, set the pace with four)
-  const double2* Ai = A + i;
+  const double2 zero = make_double2(0.0, 0.0);
+  const double2 *A0 = A + (in0 ? i0 : 0), *A1 = A + (in1 ? i1 : 0);
+  auto column = [&](const double2 a, const double2 b, const float4 xv) {
+    const MvX x = mv_x(xv);
+    float2 r, i;
+    fsplit::split_f64_fast(a.x, &r.x, &r.y);
+    fsplit::split_f64_fast(a.y, &i.x, &i.y);
+    term(r, i, x, h0, l0);
+    fsplit::split_f64_fast(b.x, &r.x, &r.y);
+    fsplit::split_f64_fast(b.y, &i.x, &i.y);
+    term(r, i, x, h1, l1);
+  };
   int64_t j = c0;
-  for (; j + 8 <= c1; j += 8) {
-    double2 a[8];
+  for (; j + 4 <= c1; j += 4) {
+    double2 a[4], b[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) a[u] = __ldcs(Ai + (j + u) * lda);
+    for (int u = 0; u < 4; ++u) {
+      a[u] = in0 ? __ldcs(A0 + (j + u) * lda) : zero;
+      b[u] = in1 ? __ldcs(A1 + (j + u) * lda) : zero;
+    }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) term(a[u], xs[j + u]);
+    for (int u = 0; u < 4; ++u) column(a[u], b[u], xs[j + u]);
   }
-  for (; j < c1; ++j) term(__ldcs(Ai + j * lda), xs[j]);
-  part[2 * (s * n + i)] = (double)h.x + (double)l.x;
-  part[2 * (s * n + i) + 1] = (double)h.y + (double)l.y;
+  for (; j < c1; ++j) column(in0 ? __ldcs(A0 + j * lda) : zero, in1 ? __ldcs(A1 + j * lda) : zero, xs[j]);
+  if (in0) {
+    part[2 * (s * n + i0)] = (double)h0.x + (double)l0.x;
+    part[2 * (s * n + i0) + 1] = (double)h0.y + (double)l0.y;
+  }
+  if (in1) {
+    part[2 * (s * n + i1)] = (double)h1.x + (double)l1.x;
+    part[2 * (s * n + i1) + 1] = (double)h1.y + (double)l1.y;
+  }
 }
 
-__global__ void k_gemv_reduce(int64_t n, const double* part, double* y, double alpha, double beta) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double sr = 0, si = 0;
-  for (int s = 0; s < MV_SLABS; ++s) {
-    sr += part[2 * (s * n + i)];
-    si += part[2 * (s * n + i) + 1];
-  }
+// y = alpha (sum of the slabs) + beta y: 64 rows per CTA, the slabs of a row dealt over four threads
+__global__ void __launch_bounds__(256) k_gemv_reduce(int64_t n, int slabs, const double* part, double* y, double alpha,
+                                                     double beta) {
+  __shared__ double2 sp[4][64];
+  const int r = threadIdx.x & 63, q = threadIdx.x >> 6;
+  const int64_t i = blockIdx.x * (int64_t)64 + r;
+  double2 a = make_double2(0.0, 0.0);
+  if (i < n)
+#pragma unroll 4
+    for (int s = q; s < slabs; s += 4) {
+      const double2 v = reinterpret_cast<const double2*>(part)[s * n + i];
+      a.x += v.x;
+      a.y += v.y;
+    }
+  sp[q][r] = a;
+  __syncthreads();
+  if (q > 0 || i >= n) return;
+  const double sr = (sp[0][r].x + sp[1][r].x) + (sp[2][r].x + sp[3][r].x);
+  const double si = (sp[0][r].y + sp[1][r].y) + (sp[2][r].y + sp[3][r].y);
   double yr = beta == 0.0 ? 0.0 : beta * y[2 * i], yi = beta == 0.0 ? 0.0 : beta * y[2 * i + 1];
   y[2 * i] = alpha * sr + yr;
   y[2 * i + 1] = alpha * si + yi;
@@ -1842,32 +1884,6 @@ __global__ void k_sum_part(int np, const double* part, double* out) {
   if (threadIdx.x == 0) *out = s[0];
 }
 
-// h[k] = <V_k, w> (conjugated first argument), one block per k
-__global__ void k_dots(int64_t n, const double* V, int64_t ldv, const double* w, double* h) {
-  __shared__ double sr[256], si[256];
-  int k = blockIdx.x;
-  const double* v = V + 2 * (int64_t)k * ldv;
-  double ar = 0, ai = 0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    double vr = v[2 * i], vi = v[2 * i + 1], wr = w[2 * i], wi = w[2 * i + 1];
-    ar += vr * wr + vi * wi;
-    ai += vr * wi - vi * wr;
-  }
-  sr[threadIdx.x] = ar;
-  si[threadIdx.x] = ai;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      sr[threadIdx.x] += sr[threadIdx.x + o];
-      si[threadIdx.x] += si[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    h[2 * k] = sr[0];
-    h[2 * k + 1] = si[0];
-  }
-}
 // w -= sum_k h_k V_k
 __global__ void k_gemv_sub(int64_t n, int m, const double* V, int64_t ldv, const double* h, double* w) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1881,6 +1897,145 @@ __global__ void k_gemv_sub(int64_t n, int m, const double* V, int64_t ldv, const
   }
   w[2 * i] -= sr;
   w[2 * i + 1] -= si;
+}
+
+// ---- the Arnoldi step of GMRES ----------------------------------------------------------
+// One kernel per pass over the basis: a CTA owns GM_ROWS rows of w and
+//   0: forms them from the matvec's slabs,      then dots with V_0 .. V_k
+//   1: subtracts V h of the first pass,          then dots again (the reorthogonalisation)
+//   2: subtracts V h of the second pass,         then the norm
+// with its rows in shared memory between the two halves, and the last CTA to finish adds the
+// CTAs' partial sums in order (deterministic; no second launch, no host round trip).  The whole
+// iteration is then five launches, its coefficients and norm read back once.
+// Dots: a warp takes four basis vectors at a time, its eight partial sums reduced over the lanes
+// by halving (nine additions instead of forty).
+constexpr int GM_ROWS = 64, GM_THREADS = 256;
+
+// out[8 values of a warp]: lane 4 j writes value j's total (j = 0 .. 7, re / im of four vectors)
+__device__ __forceinline__ double gm_reduce8(double* v, int lane) {
+#pragma unroll
+  for (int half = 4, o = 16; half >= 1; half >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double keep = up ? v[i + half] : v[i], give = up ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
+// mode as above; k1 = k + 1 basis vectors; h_in: their coefficients (modes 1, 2); out: k1 complex
+// sums (modes 0, 1) or the squared norm (mode 2); part: [gridDim.x][2 k1]; count: zero at entry and exit
+__global__ void __launch_bounds__(GM_THREADS) k_gm_step(int mode, int64_t n, int k1, int slabs, const double* slab,
+                                                        const double* V, double* w, const double* h_in, double* part,
+                                                        unsigned int* count, double* out) {
+  __shared__ double2 sw[GM_ROWS];
+  __shared__ double2 sp[GM_THREADS / GM_ROWS][GM_ROWS];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = tid % GM_ROWS, q = tid / GM_ROWS;
+  const int64_t r0 = blockIdx.x * (int64_t)GM_ROWS, row = r0 + r;
+  const bool in = row < n;
+  // ---- this CTA's rows of w
+  {
+    double2 a = make_double2(0.0, 0.0);
+    if (in) {
+      if (mode == 0) {
+        for (int s = q; s < slabs; s += GM_THREADS / GM_ROWS) {
+          const double2 v = reinterpret_cast<const double2*>(slab)[s * n + row];
+          a.x += v.x;
+          a.y += v.y;
+        }
+      } else {
+        const double2* h = reinterpret_cast<const double2*>(h_in);
+#pragma unroll 4
+        for (int k = q; k < k1; k += GM_THREADS / GM_ROWS) {
+          const double2 v = reinterpret_cast<const double2*>(V)[k * n + row], c = h[k];
+          a.x = fma(c.x, v.x, fma(-c.y, v.y, a.x));
+          a.y = fma(c.x, v.y, fma(c.y, v.x, a.y));
+        }
+      }
+    }
+    sp[q][r] = a;
+    __syncthreads();
+    if (q == 0) {
+      double2 t = make_double2((sp[0][r].x + sp[1][r].x) + (sp[2][r].x + sp[3][r].x),
+                               (sp[0][r].y + sp[1][r].y) + (sp[2][r].y + sp[3][r].y));
+      if (in) {
+        double2* wr = reinterpret_cast<double2*>(w) + row;
+        if (mode > 0) {
+          const double2 o = *wr;
+          t = make_double2(o.x - t.x, o.y - t.y);
+        }
+        *wr = t;
+      }
+      sw[r] = t;  // (rows beyond n: zero)
+    }
+    __syncthreads();
+  }
+  // ---- partial sums over them
+  const int nv = mode == 2 ? 1 : 2 * k1;
+  double* mine = part + (size_t)blockIdx.x * nv;
+  if (mode == 2) {
+    if (warp == 0) {
+      const double2 a = sw[lane], b = sw[lane + 32];
+      double v = (a.x * a.x + a.y * a.y) + (b.x * b.x + b.y * b.y);
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) mine[0] = v;
+    }
+  } else {
+    const double2 w0 = sw[lane], w1 = sw[lane + 32];
+    const bool in0 = r0 + lane < n, in1 = r0 + lane + 32 < n;
+    const double2 zero = make_double2(0.0, 0.0);
+    for (int k0 = 4 * warp; k0 < k1; k0 += 4 * (GM_THREADS / 32)) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double2* vk = reinterpret_cast<const double2*>(V) + (int64_t)(k0 + u) * n + r0 + lane;
+        const bool ok = k0 + u < k1;
+        const double2 a = ok && in0 ? vk[0] : zero, b = ok && in1 ? vk[32] : zero;
+        v[2 * u] = fma(a.x, w0.x, fma(a.y, w0.y, fma(b.x, w1.x, b.y * w1.y)));
+        v[2 * u + 1] = fma(a.x, w0.y, fma(-a.y, w0.x, fma(b.x, w1.y, -(b.y * w1.x))));
+      }
+      const double t = gm_reduce8(v, lane);
+      const int j = 2 * k0 + (lane >> 2);
+      if ((lane & 3) == 0 && j < nv) mine[j] = t;
+    }
+  }
+  // ---- the last CTA adds the partial sums, in the CTAs' order
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int j = tid; j < nv; j += GM_THREADS) {
+    double a[4] = {0, 0, 0, 0};
+    const int nb = (int)gridDim.x;
+    for (int b = 0; b < nb; b += 16) {  // 16 loads in flight
+      double v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = b + u < nb ? __ldcg(part + (size_t)(b + u) * nv + j) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) a[u & 3] += v[u];
+    }
+    out[j] = (a[0] + a[1]) + (a[2] + a[3]);
+  }
+  if (tid == 0) *count = 0;
+}
+
+// v = w / |w| with |w|^2 on the device (0 for w = 0), and v as float pairs for the next matvec
+__global__ void k_gm_next(int64_t n, const double* w, const double* norm2, double* v, float4* xs) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double nrm = sqrt(*norm2), inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
+  const double2 a = reinterpret_cast<const double2*>(w)[i], b = make_double2(inv * a.x, inv * a.y);
+  reinterpret_cast<double2*>(v)[i] = b;
+  const float rh = (float)b.x, ih = (float)b.y;
+  xs[i] = make_float4(rh, ih, (float)(b.x - (double)rh), (float)(b.y - (double)ih));
 }
 
 template <typename T, typename R>
@@ -2425,30 +2580,92 @@ int trsv_check(beast_ctx* ctx) {
   return BEAST_OK;
 }
 
+// slabs of an n x n matvec: the most slabs (32 below order 2048, where the sum over the slabs
+// counts) whose CTAs fill their waves to 97%, else the count that fills them best.  Many short CTAs
+// even out the ends of the load streams: order 7213 takes 227 us in one full wave of 31 slabs and
+// 205 us in two.
+static int mv_slabs(int64_t n, int64_t row_blocks, const void* kernel) {
+  int dev = 0, sms = 1, occ = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 128, 0) != cudaSuccess || occ < 1) occ = 1;
+  const double cap = (double)sms * occ;
+  int best = 1;
+  double fill = -1.0;
+  for (int s = n < 2048 ? 32 : MV_MAX_SLABS; s >= 8; --s) {
+    if (s > n) continue;
+    const double w = (double)row_blocks * s / cap, f = w / std::ceil(w);
+    if (f >= 0.97) return s;
+    if (f > fill) {
+      fill = f;
+      best = s;
+    }
+  }
+  return best;
+}
+
+// the partial sums of A x over column slabs into part [slabs][n][2]; returns the slab count
+static int gemv_partial(int64_t n, const void* A, int64_t lda, int a_c64, const float4* xs, double* part,
+                        cudaStream_t st) {
+  const bool pair = a_c64 && lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+  const int rows = a_c64 && !pair ? 128 : 256;
+  const int64_t rb = (n + rows - 1) / rows;
+  const void* kern = !a_c64 ? (const void*)k_gemv_partial_c128_df
+                            : (pair ? (const void*)k_gemv_partial_c64_df2 : (const void*)k_gemv_partial_c64_df);
+  const int slabs = mv_slabs(n, rb, kern);
+  dim3 g((unsigned)rb, (unsigned)slabs);
+  if (!a_c64)
+    k_gemv_partial_c128_df<<<g, 128, 0, st>>>(n, (const double2*)A, lda, xs, part);
+  else if (pair)
+    k_gemv_partial_c64_df2<<<g, 128, 0, st>>>(n, (const float2*)A, lda, xs, part);
+  else
+    k_gemv_partial_c64_df<<<g, 128, 0, st>>>(n, (const float2*)A, lda, xs, part);
+  return slabs;
+}
+
 // scratch per call from the device's stream-ordered pool (cheap once the pool holds memory;
 // nothing shared between contexts, streams or devices)
 cudaError_t gemv_dev(int64_t n, const void* A, int64_t lda, int a_c64, const double* x, double* y,
                      double alpha, double beta, cudaStream_t st) {
-  const size_t need = (size_t)MV_SLABS * n * 2 * sizeof(double) + (size_t)n * sizeof(float4) + 256;
+  const size_t need = (size_t)MV_MAX_SLABS * n * 2 * sizeof(double) + (size_t)n * sizeof(float4) + 256;
   double* part = nullptr;
   cudaError_t e = cudaMallocAsync(&part, need, st);
   if (e != cudaSuccess) return e;
-  dim3 g((unsigned)((n + 127) / 128), MV_SLABS);
-  float4* xs = reinterpret_cast<float4*>(part + (size_t)MV_SLABS * n * 2);
+  float4* xs = reinterpret_cast<float4*>(part + (size_t)MV_MAX_SLABS * n * 2);
   k_split_x<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, x, xs);
-  if (a_c64) {
-    if (lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
-      dim3 g2((unsigned)((n + 255) / 256), MV_SLABS);
-      k_gemv_partial_c64_df2<<<g2, 128, 0, st>>>(n, (const float2*)A, lda, xs, part);
-    } else {
-      k_gemv_partial_c64_df<<<g, 128, 0, st>>>(n, (const float2*)A, lda, xs, part);
-    }
-  } else
-    k_gemv_partial_c128_df<<<g, 128, 0, st>>>(n, (const double2*)A, lda, xs, part);
-  k_gemv_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, part, y, alpha, beta);
+  const int slabs = gemv_partial(n, A, lda, a_c64, xs, part, st);
+  k_gemv_reduce<<<(unsigned)((n + 63) / 64), 256, 0, st>>>(n, slabs, part, y, alpha, beta);
   e = cudaGetLastError();
   cudaFreeAsync(part, st);
   return e;
+}
+
+// ---- GMRES on the device: the workspace of one solve and one Arnoldi step
+size_t gmres_work_bytes(int64_t n, int m) {
+  const size_t nb = (size_t)((n + GM_ROWS - 1) / GM_ROWS);
+  return (size_t)MV_MAX_SLABS * n * 16 + (size_t)n * 16 + nb * 2 * (m + 1) * 8 + 4096;
+}
+// v_k = w / |w| (|w|^2 at norm2) and its matvec's slabs
+cudaError_t gmres_matvec(int64_t n, const void* A, int64_t lda, int a_c64, const double* w, const double* norm2,
+                         double* vk, void* work, int* slabs, cudaStream_t st) {
+  double* slab = static_cast<double*>(work);
+  float4* xs = reinterpret_cast<float4*>(slab + (size_t)MV_MAX_SLABS * n * 2);
+  k_gm_next<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, w, norm2, vk, xs);
+  *slabs = gemv_partial(n, A, lda, a_c64, xs, slab, st);
+  return cudaGetLastError();
+}
+// w = A v_k from the slabs, orthogonalised twice against v_0 .. v_k: out = h1 (k + 1 complex), h2, |w|^2
+cudaError_t gmres_orthogonalise(int64_t n, int k, int m, int slabs, const double* V, double* w, void* work,
+                                unsigned int* count, double* out, cudaStream_t st) {
+  double* slab = static_cast<double*>(work);
+  double* part = slab + (size_t)MV_MAX_SLABS * n * 2 + (size_t)n * 2;
+  const unsigned nb = (unsigned)((n + GM_ROWS - 1) / GM_ROWS);
+  double* h2 = out + 2 * (k + 1);
+  k_gm_step<<<nb, GM_THREADS, 0, st>>>(0, n, k + 1, slabs, slab, V, w, nullptr, part, count, out);
+  k_gm_step<<<nb, GM_THREADS, 0, st>>>(1, n, k + 1, slabs, slab, V, w, out, part, count, h2);
+  k_gm_step<<<nb, GM_THREADS, 0, st>>>(2, n, k + 1, slabs, slab, V, w, h2, part, count, h2 + 2 * (k + 1));
+  (void)m;
+  return cudaGetLastError();
 }
 
 cudaError_t copy_lower_c64(int64_t n, const void* A, int64_t lda, void* F, int64_t ldf, cudaStream_t st) {
@@ -2496,12 +2713,6 @@ cudaError_t vec_norm2(int64_t n, const double* x, double* out, cudaStream_t st) 
   e = cudaGetLastError();
   cudaFreeAsync(npart, st);
   return e;
-}
-cudaError_t vec_dots(int64_t n, int m, const double* V, int64_t ldv, const double* w, double* h,
-                     cudaStream_t st) {
-  if (m <= 0) return cudaSuccess;
-  k_dots<<<m, 256, 0, st>>>(n, V, ldv, w, h);
-  return cudaGetLastError();
 }
 cudaError_t vec_gemv_sub(int64_t n, int m, const double* V, int64_t ldv, const double* h, double* w,
                          cudaStream_t st) {

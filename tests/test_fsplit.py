@@ -120,3 +120,28 @@ def test_round_to_float_by_integer_ops(tmp_path):
         ref = a.astype(np.float32)
     ok = (f.view(np.uint32) == ref.view(np.uint32)) | (np.isnan(f) & np.isnan(ref))
     assert ok.all(), a[~ok][:5]
+
+
+def test_fast_split(tmp_path):
+    """split_f64_fast: the same high part, the low part to half a unit of 2^-48 of a over its range;
+    split_f64's results outside it"""
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not available")
+    src, so = tmp_path / "s.cpp", tmp_path / "s.so"
+    src.write_text('#include "fsplit.h"\n'
+                   'extern "C" void t_both(const double* a, long n, float* f) {\n'
+                   '  for (long i = 0; i < n; ++i) {\n'
+                   '    fsplit::split_f64_fast(a[i], f + 4 * i, f + 4 * i + 1);\n'
+                   '    fsplit::split_f64(a[i], f + 4 * i + 2, f + 4 * i + 3);\n  }\n}\n')
+    subprocess.check_call(["g++", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(so)])
+    L = C.CDLL(str(so))
+    rng = np.random.default_rng(5)
+    a = rng.uniform(1, 2, 100000) * 2.0 ** rng.integers(-73, 128, 100000) * rng.choice([-1.0, 1.0], 100000)
+    special = np.array([0.0, -0.0, 2.0 ** -74, 1e-300, 2.0 ** 128, -1e200, np.inf, -np.inf, np.nan])
+    a = np.concatenate([a, special])
+    f = np.zeros((a.size, 4), np.float32)
+    L.t_both(a.ctypes.data_as(C.c_void_p), C.c_long(a.size), f.ctypes.data_as(C.c_void_p))
+    assert np.array_equal(f[:, 0].view(np.uint32), f[:, 2].view(np.uint32))
+    n = a.size - special.size
+    assert np.all(np.abs(a[:n] - (f[:n, 0].astype(float) + f[:n, 1].astype(float))) <= np.abs(a[:n]) * 2.0 ** -48)
+    assert np.array_equal(f[n:, 1].view(np.uint32), f[n:, 3].view(np.uint32))

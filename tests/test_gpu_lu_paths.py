@@ -49,3 +49,23 @@ def test_fp64_solve_is_invariant_under_column_scaling():
     x, _, _ = bg.solve(A, b, precision=bg.FP64)
     y, _, _ = bg.solve(A * s[None, :], b, precision=bg.FP64)
     assert np.array_equal(y * s, x)
+
+
+@pytest.mark.parametrize("n,restart,dtype", [(1, 0, "c128"), (37, 5, "c128"), (63, 0, "c64"), (64, 1, "c128"), (65, 33, "c128"),
+                                             (301, 0, "c64"), (1030, 7, "c128"), (2111, 0, "c128")])
+def test_gmres_at_the_edges_of_its_row_blocks(n, restart, dtype):
+    """orders around the 64-row blocks of the orthogonalisation, restarts down to one vector (a basis
+    of four vectors a warp, partial groups): the residual of the returned solution reaches reltol"""
+    A = (_matrix(n, False, n, dominance=0.0) * 0.3 / max(n, 1) ** 0.5 + 2.0 * np.eye(n)).astype(np.complex64 if dtype == "c64" else np.complex128)
+    b = np.random.default_rng(n + 1).normal(size=n) + 1j * np.random.default_rng(n + 2).normal(size=n)
+    x, it, res = bg.gmres(A, b, reltol=1e-11, restart=restart, maxiter=3000)
+    assert it >= 1 and res <= 1e-11
+    assert np.linalg.norm(A.astype(np.complex128) @ x - b) <= 2e-11 * np.linalg.norm(b)
+
+
+def test_gmres_zero_right_hand_side_and_limit():
+    A = _matrix(70, False, 3, dominance=0.0)
+    x, it, res = bg.gmres(A, np.zeros(70), reltol=1e-10)
+    assert it == 0 and np.array_equal(x, np.zeros(70))
+    with pytest.raises(bg.BeastError):
+        bg.gmres(A, np.ones(70), reltol=1e-14, restart=4, maxiter=6)
