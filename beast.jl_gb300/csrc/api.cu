@@ -1089,9 +1089,11 @@ static int system_solve(beast_ctx* ctx, DenseSystem& S, const double* b, double*
       double* xk = x + 2 * k * n;
       double bn = dev_norm(ctx, n, bk, nrm);
       if (!S.mixed) {
-        BEAST_CUDA_TRY(ctx, vec_copy(n, bk, xk, st));
-        rc = lu_solve_dev(ctx, n, S.F, S.lu->lda, BEAST_C128, S.lu->ipiv, xk, n, 1);
-        if (rc) break;
+        if (k == 0) {  // all right-hand sides side by side
+          BEAST_CUDA_TRY(ctx, vec_copy(n * nrhs, b, x, st));
+          rc = lu_solve_dev(ctx, n, S.F, S.lu->lda, BEAST_C128, S.lu->ipiv, x, n, nrhs);
+          if (rc) break;
+        }
         BEAST_CUDA_TRY(ctx, vec_copy(n, bk, r, st));
         {
           ProfScope ps(ctx, PK_GEMV, (double)n * n * 16, 2);
