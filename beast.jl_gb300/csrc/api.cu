@@ -309,6 +309,15 @@ int beast_mesh_upload(beast_ctx* ctx, const double* verts, int64_t nv, const int
   m->ctx = ctx;
   m->nv = nv;
   m->nc = nc;
+  for (int64_t i = 0; i < nc; ++i) {
+    const double *a = verts + 3 * (int64_t)c[3 * i], *b = verts + 3 * (int64_t)c[3 * i + 1], *g = verts + 3 * (int64_t)c[3 * i + 2];
+    double r2 = 0.0;
+    for (int k = 0; k < 3; ++k) {
+      const double z = (a[k] + b[k] + g[k]) / 3.0;
+      r2 += (a[k] - z) * (a[k] - z) + (b[k] - z) * (b[k] - z) + (g[k] - z) * (g[k] - z);
+    }
+    m->radius += std::sqrt(r2 / 3.0) / nc;
+  }
   cudaError_t e = cudaMalloc(&m->verts, sizeof(double) * 3 * nv);
   if (e == cudaSuccess) e = cudaMalloc(&m->cells, sizeof(int) * 3 * nc);
   if (e == cudaSuccess) e = cudaMemcpyAsync(m->verts, verts, sizeof(double) * 3 * nv, cudaMemcpyHostToDevice, ctx->stream);

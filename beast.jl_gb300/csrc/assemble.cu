@@ -189,6 +189,7 @@ struct FarParams {
   TriRuleDev ro, ri;
   int qt, fmt;     // trial cells staged per CTA, Zcell format (k_far64)
   g64::Wave wave;  // the wavenumber (k_far64)
+  double radius;   // the trial mesh's average cell radius, 0 when not known
 };
 
 // Zcell rows / columns (-1: the block entry is not stored)
@@ -524,15 +525,21 @@ __global__ void __launch_bounds__(FAR_THREADS) k_far(FarParams P) {
 // it is the number of FP64 instructions (the pipe takes one warp instruction in 16 cycles per
 // quarter SM at best; loads, FP32 and integer work hide under it), so the pair is arranged to need
 // few of them:
-//   - a kernel value costs seven for 1/R, R, cos, sin (green64.h) where rsqrt and sincos cost 35;
+//   - a kernel value costs seven for 1/R, R, cos, sin (green64.h) where rsqrt and sincos cost 35,
+//     and five in the integer form (FIX);
 //   - every block is a combination of the moments T_mn = sum_ab w_a w_b K(x_a, y_b) lambda_m(x_a)
 //     lambda_n(y_b) over the cells' barycentric coordinates (the RT shapes are linear in them):
 //     three real sums per inner point (1, u, v) and real part, nine per outer point, the third
 //     coordinate by difference at the end; n x K, quadratic in the test point, takes three more
 //     (|xi|^2 with the test point's offset xi from its centroid);
 //   - the double layers' normal component does not depend on the point in the normal's own plane;
-//   - 1/(4 pi), the areas and the shapes' 1/2A enter once per block.
-// Measured (EFIE, 3380 cells): see the launch rule below.
+//   - 1/(4 pi), the areas and the shapes' 1/2A enter once per block;
+//   - FIX: sines, cosines, products and all sums as 64-bit integers with a power of two per pair (an
+//     integer product is a dozen instructions, an addition two).  What stays in FP64 is the distance,
+//     11 instructions per value, and the block from the moments.
+// Measured (one GB300; CUDA functions, point-wise moments before): EFIE, 3380 cells 20.1 -> 7.8 ms
+// (12.3 without FIX); n x K, 1620 cells 66.8 -> 15.8 (26.2); Helmholtz double layer on
+// P1, 5780 cells 72.6 -> 18.7 (34.3).
 struct Far64Rec {
   double sig[3][3];  // trial vertices minus centroid
   double c[3], n[3];
@@ -540,7 +547,7 @@ struct Far64Rec {
 };
 constexpr int FAR64_PT = 6;  // eta (3), w, w u, w v per inner rule point
 
-template <int OPK, int TK, int BK>
+template <int OPK, int TK, int BK, bool FIX>
 __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
   constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL || OPK == BEAST_MW_NXDL;
   constexpr bool GRAD = OPK != BEAST_MW_SL && OPK != BEAST_HH_SL;
@@ -548,11 +555,17 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
   constexpr int NX = OPK == BEAST_MW_NXDL ? 3 : 0;  // |xi|^2 moments
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ni = P.ri.n, no = P.ro.n, qt = P.qt;
-  g64::Entry* tab = reinterpret_cast<g64::Entry*>(smraw);
+  typedef typename std::conditional<FIX, g64::EntryX, g64::Entry>::type Tab;
+  Tab* tab = reinterpret_cast<Tab*>(smraw);
   Far64Rec* rec = reinterpret_cast<Far64Rec*>(tab + g64::TABLE);
   double* pts = reinterpret_cast<double*>(rec + qt);        // [qt][ni][FAR64_PT]
   double* sxi = pts + (size_t)qt * ni * FAR64_PT;           // [no][3][FAR_THREADS]: xi_a per thread
+  int64_t* sxx = reinterpret_cast<int64_t*>(sxi + (size_t)no * 3 * FAR_THREADS);  // [no][FAR_THREADS]: w |xi|^2 (NX)
+  // FIX: eta and xi in FP32, for the bound on 1/R of a close pair
+  float* ptf = reinterpret_cast<float*>(sxx + (NX ? (size_t)no * FAR_THREADS : 0));  // [qt][ni][3]
+  float* sxf = ptf + (size_t)qt * ni * 3;                                            // [no][3][FAR_THREADS]
   __shared__ double ro_s[RULE_MAXPTS][3];                   // w, w u, w v
+  __shared__ int64_t ro_x[RULE_MAXPTS][3], ri_x[RULE_MAXPTS][3];  // the same as integers, both rules
   __shared__ int s_zc[FAR_QT][3];
   g64::load_table(tab);
   const int q0 = blockIdx.y * qt;
@@ -561,7 +574,15 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
     ro_s[k][0] = P.ro.w[k];
     ro_s[k][1] = P.ro.w[k] * P.ro.u[k];
     ro_s[k][2] = P.ro.w[k] * P.ro.v[k];
+    for (int c = 0; c < 3; ++c) ro_x[k][c] = g64::to_fixed(ro_s[k][c], 1);
   }
+  if (FIX)
+    for (int k = threadIdx.x; k < ni; k += blockDim.x) {
+      const double w = P.ri.w[k];
+      ri_x[k][0] = g64::to_fixed(w, 1);
+      ri_x[k][1] = g64::to_fixed(w * P.ri.u[k], 1);
+      ri_x[k][2] = g64::to_fixed(w * P.ri.v[k], 1);
+    }
   for (int k = threadIdx.x; k < nqt * (1 + ni); k += blockDim.x) {
     const int qi = k / (1 + ni), b = k % (1 + ni);
     const int qc = P.qcells[q0 + qi];
@@ -582,6 +603,8 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
       pt[3] = w;
       pt[4] = w * u;
       pt[5] = w * v;
+      if (FIX)
+        for (int j = 0; j < 3; ++j) ptf[((size_t)qi * ni + b - 1) * 3 + j] = (float)pt[j];
     }
   }
   for (int k = threadIdx.x; k < nqt * 3; k += blockDim.x) s_zc[k / 3][k % 3] = (int)zcol_of(P.zcol, q0 + k / 3, NB, k % 3);
@@ -591,17 +614,25 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
   const double* tg = P.tgeo + p * GEO_STRIDE;
   const V3<double> cp = mk(tg[9], tg[10], tg[11]);
   auto tau = [&](int i) { return mk(tg[3 * i] - cp.x, tg[3 * i + 1] - cp.y, tg[3 * i + 2] - cp.z); };
+  const double radp = P.tgeof[4 * p + 3];
+  const int ex = (int)((__double2hiint(radp * radp) >> 20) & 0x7FF) - 1022;  // radp^2 < 2^ex
   for (int a = 0; a < no; ++a) {
     const V3<double> xi = P.ro.u[a] * tau(0) + P.ro.v[a] * tau(1) + (1.0 - P.ro.u[a] - P.ro.v[a]) * tau(2);
     sxi[(3 * a) * FAR_THREADS + threadIdx.x] = xi.x;
     sxi[(3 * a + 1) * FAR_THREADS + threadIdx.x] = xi.y;
     sxi[(3 * a + 2) * FAR_THREADS + threadIdx.x] = xi.z;
+    if (FIX) {
+      sxf[(3 * a) * FAR_THREADS + threadIdx.x] = (float)xi.x;
+      sxf[(3 * a + 1) * FAR_THREADS + threadIdx.x] = (float)xi.y;
+      sxf[(3 * a + 2) * FAR_THREADS + threadIdx.x] = (float)xi.z;
+    }
+    // (|xi|^2 / radius^2 <= 1, scaled by the radius' power of two)
+    if (FIX && NX) sxx[a * FAR_THREADS + threadIdx.x] = g64::to_fixed(P.ro.w[a] * dot(xi, xi), ex + 1);
   }
   __syncthreads();
   if (!live) return;
   int64_t zr[3];
   for (int i = 0; i < 3; ++i) zr[i] = i < NT ? zrow_of(P.zrow, pp, NT, i) : -1;
-  const double radp = P.tgeof[4 * p + 3];
   const double gr = P.op.gr, sg = P.op.gi < 0.0 ? -1.0 : 1.0;
   const V3<double> nn = mk(tg[12], tg[13], tg[14]);
 
@@ -609,10 +640,11 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
     const Far64Rec& rq = rec[qi];
     const int ql = q0 + qi;
     const V3<double> d = mk(cp.x - rq.c[0], cp.y - rq.c[1], cp.z - rq.c[2]);
+    const double dd = dot(d, d);
     // near test: candidate filter on the centroid distance, exact classification (k_far)
     {
       const double lim = radp + rq.lim;
-      if (dot(d, d) <= lim * lim * 1.0001 + 1e-30) {
+      if (dd <= lim * lim * 1.0001 + 1e-30) {
         int cls = 4;
         if (P.qs_kind != BEAST_QS_DOUBLENUM) {
           const Geo t = load_geo(tg);
@@ -635,92 +667,243 @@ __global__ void __launch_bounds__(FAR_THREADS, 3) k_far64(FarParams P) {
     const double* pq = pts + (size_t)qi * ni * FAR64_PT;
     const V3<double> nq = mk(rq.n[0], rq.n[1], rq.n[2]);
     // moments over (1, u, v) of the test and (1, u, v) of the trial cell
-    C2<double> M[NT][NB], X[3];
+    C2<double> M[NT][NB], X[3], M00;
 #pragma unroll
     for (int m = 0; m < NT; ++m)
 #pragma unroll
       for (int n = 0; n < NB; ++n) M[m][n] = C2<double>{0, 0};
     X[0] = X[1] = X[2] = C2<double>{0, 0};
-    for (int a = 0; a < no; ++a) {
-      const V3<double> xi = mk(sxi[(3 * a) * FAR_THREADS + threadIdx.x], sxi[(3 * a + 1) * FAR_THREADS + threadIdx.x],
-                               sxi[(3 * a + 2) * FAR_THREADS + threadIdx.x]);
-      const V3<double> dx = d + xi;
-      C2<double> U[3];
-      U[0] = U[1] = U[2] = C2<double>{0, 0};
-#pragma unroll 2
-      for (int b = 0; b < ni; ++b) {
-        const double* pb = pq + b * FAR64_PT;
-        const V3<double> r = dx - mk(pb[0], pb[1], pb[2]);
-        const g64::Value v = g64::eval(dot(r, r), P.wave, tab);
-        double amp = v.iR;
-        if (gr != 0.0) amp *= exp(-gr * v.R);
-        double kr, ki;  // single layer: 4 pi G, the imaginary part times -sg; gradient: -4 pi c, times sg
-        if (GRAD) {
-          const double p1 = v.iR + gr, q = amp * v.iR;
-          kr = fma(p1, v.c, P.wave.k * v.s);
-          ki = fma(P.wave.k, v.c, -(p1 * v.s));
-          double f = q;
-          if (OPK == BEAST_HH_DLT) f *= dot(nn, r);
-          kr *= f;
-          ki *= f;
-        } else {
-          kr = amp * v.c;
-          ki = amp * v.s;
-        }
-        U[0].re = fma(pb[3], kr, U[0].re);
-        U[0].im = fma(pb[3], ki, U[0].im);
-        if (NB == 3) {
-          U[1].re = fma(pb[4], kr, U[1].re);
-          U[1].im = fma(pb[4], ki, U[1].im);
-          U[2].re = fma(pb[5], kr, U[2].re);
-          U[2].im = fma(pb[5], ki, U[2].im);
-        }
-      }
-      if (OPK == BEAST_HH_DL) {
-        const double f = dot(nq, dx);
-#pragma unroll
-        for (int n = 0; n < NB; ++n) U[n] = cscale(f, U[n]);
-      }
+    // integer moments: kernel values with 1/R scaled by a power of two of the pair, 62 fractional
+    // bits, truncated products with the mean of the truncation added up front.  A value out of range takes the pair to the FP64 sums below.
+    bool done = false;
+    if constexpr (FIX) {
+      int64_t Mr[NT][NB], Mi[NT][NB], Xr[3], Xi[3];
 #pragma unroll
       for (int m = 0; m < NT; ++m)
 #pragma unroll
+        for (int n = 0; n < NB; ++n) Mr[m][n] = Mi[m][n] = no / 2;
+      for (int n = 0; n < 3; ++n) Xr[n] = Xi[n] = no / 2;
+      // 1/R < 2^eI: from the distance of the circumspheres, for close cells from the points themselves
+      const float dm = sqrtf((float)dd), rad = (float)(radp + rq.lim);
+      float rlb = dm - rad;
+      if (dm < 3.f * rad) {
+        float m2 = 3e38f;
+        const float fx = (float)d.x, fy = (float)d.y, fz = (float)d.z;
+        for (int a = 0; a < no; ++a) {
+          const float ax = fx + sxf[(3 * a) * FAR_THREADS + threadIdx.x], ay = fy + sxf[(3 * a + 1) * FAR_THREADS + threadIdx.x],
+                      az = fz + sxf[(3 * a + 2) * FAR_THREADS + threadIdx.x];
+          for (int b = 0; b < ni; ++b) {
+            const float* pf = ptf + ((size_t)qi * ni + b) * 3;
+            const float x = ax - pf[0], y = ay - pf[1], z = az - pf[2];
+            m2 = fminf(m2, x * x + y * y + z * z);
+          }
+        }
+        rlb = sqrtf(m2);
+      }
+      const int eI = 127 - (int)(__float_as_uint(0.9999f * rlb) >> 23);
+      // the gradient's values are products of four factors: each is normalised and the product shifted to
+      // a common scale, iR^2 |1/R + i k| < 2^eK
+      const int ek = GRAD ? (int)((__double2hiint(P.wave.k) >> 20) & 0x7FF) - 1023 : 0;  // k < 2^(ek + 1)
+      const int64_t km = GRAD ? g64::to_fixed(P.wave.k, ek + 1) : 0;
+      const int eK = GRAD ? max(eI, ek + 1) + 1 + 2 * (eI - 1) : eI;
+      // the double layers' factor n . r (the normal's component does not change over its own cell):
+      // |n . r| < 2^eF
+      int eF = 0;
+      if (OPK == BEAST_HH_DL || OPK == BEAST_HH_DLT) {
+        const V3<double> n1 = OPK == BEAST_HH_DL ? nq : nn;
+        const float c = (float)dot(nn, nq), f = fabsf((float)dot(n1, d)) + 1e-6f * dm +
+                        sqrtf(fmaxf(1.f - c * c, 0.f) + 1e-6f) * (OPK == BEAST_HH_DL ? (float)radp : (float)rq.lim);
+        eF = (int)(__float_as_uint(1.0001f * f) >> 23) - 126;
+      }
+      // T = M 2^e0
+      const int e0 = GRAD ? eK + eF - 56 : eI - 58;
+      done = true;
+      for (int a = 0; a < no && done; ++a) {
+        const V3<double> dx = d + mk(sxi[(3 * a) * FAR_THREADS + threadIdx.x], sxi[(3 * a + 1) * FAR_THREADS + threadIdx.x],
+                                     sxi[(3 * a + 2) * FAR_THREADS + threadIdx.x]);
+        int64_t Ur[3], Ui[3];
+        for (int n = 0; n < 3; ++n) Ur[n] = Ui[n] = ni / 2;
+#pragma unroll 1
+        for (int b = 0; b < ni; ++b) {
+          const double* pb = pq + b * FAR64_PT;
+          const V3<double> r = dx - mk(pb[0], pb[1], pb[2]);
+          g64::ValueX v;
+          if (!g64::eval_fixed(dot(r, r), P.wave, tab, v) ||
+              (int)((__double2hiint(v.iR) >> 20) & 0x7FF) - 1022 > eI) {
+            done = false;
+            break;
+          }
+          int64_t kr, ki;
+          if (GRAD) {
+            const int E = (int)((__double2hiint(v.iR) >> 20) & 0x7FF) - 1023, eB = max(E + 1, ek + 1) + 1;
+            const int64_t im = g64::to_fixed(v.iR, E + 1);
+            const int64_t ib = im >> (eB - E - 1), kx = km >> min(eB - ek - 1, 63);
+            const int64_t br = g64::mulhi(ib, v.c) + g64::mulhi(kx, v.s), bi = g64::mulhi(kx, v.c) - g64::mulhi(ib, v.s);
+            int64_t q = g64::mulhi(im, im) << 2;
+            if (OPK == BEAST_HH_DLT) q = g64::mulhi(q, g64::to_fixed(dot(nn, r), eF)) << 2;
+            const int sh = eK - eB - 2 * E;
+            if (sh < 0) {
+              done = false;
+              break;
+            }
+            kr = (g64::mulhi(br << 2, q) << 2) >> min(sh, 63);
+            ki = (g64::mulhi(bi << 2, q) << 2) >> min(sh, 63);
+          } else {
+            const int64_t ir = g64::to_fixed(v.iR, eI);
+            kr = g64::mulhi(ir, v.c) << 2;
+            ki = g64::mulhi(ir, v.s) << 2;
+          }
+#pragma unroll
+          for (int n = 0; n < NB; ++n) {
+            Ur[n] += g64::mulhi(kr, ri_x[b][n]);
+            Ui[n] += g64::mulhi(ki, ri_x[b][n]);
+          }
+        }
+        // (the double layer's factor n_q . (d + xi) is common to the inner points)
+        const int64_t f = OPK == BEAST_HH_DL ? g64::to_fixed(dot(nq, dx), eF) : 0;
+#pragma unroll
         for (int n = 0; n < NB; ++n) {
-          M[m][n].re = fma(ro_s[a][m], U[n].re, M[m][n].re);
-          M[m][n].im = fma(ro_s[a][m], U[n].im, M[m][n].im);
-        }
-      if (NX) {
-        const double f = ro_s[a][0] * dot(xi, xi);
+          const int64_t ur = (OPK == BEAST_HH_DL ? g64::mulhi(Ur[n] << 2, f) : Ur[n]) << 2;
+          const int64_t ui = (OPK == BEAST_HH_DL ? g64::mulhi(Ui[n] << 2, f) : Ui[n]) << 2;
 #pragma unroll
-        for (int n = 0; n < 3; ++n) {
-          X[n].re = fma(f, U[n].re, X[n].re);
-          X[n].im = fma(f, U[n].im, X[n].im);
+          for (int m = 0; m < NT; ++m) {
+            Mr[m][n] += g64::mulhi(ur, ro_x[a][m]);
+            Mi[m][n] += g64::mulhi(ui, ro_x[a][m]);
+          }
+          if (NX) {
+            Xr[n] += g64::mulhi(ur, sxx[a * FAR_THREADS + threadIdx.x]);
+            Xi[n] += g64::mulhi(ui, sxx[a * FAR_THREADS + threadIdx.x]);
+          }
+        }
+      }
+      if (done) {
+        // barycentric coordinates as below, then doubles
+        M00 = C2<double>{g64::from_fixed(Mr[0][0], e0), g64::from_fixed(Mi[0][0], e0)};
+        if (NB == 3) {
+#pragma unroll
+          for (int m = 0; m < NT; ++m) {
+            const int64_t r0 = Mr[m][0], i0 = Mi[m][0];
+            Mr[m][0] = Mr[m][1];
+            Mr[m][1] = Mr[m][2];
+            Mr[m][2] = r0 - Mr[m][0] - Mr[m][1];
+            Mi[m][0] = Mi[m][1];
+            Mi[m][1] = Mi[m][2];
+            Mi[m][2] = i0 - Mi[m][0] - Mi[m][1];
+          }
+          if (NX) {
+            const int64_t r0 = Xr[0], i0 = Xi[0];
+            Xr[0] = Xr[1];
+            Xr[1] = Xr[2];
+            Xr[2] = r0 - Xr[0] - Xr[1];
+            Xi[0] = Xi[1];
+            Xi[1] = Xi[2];
+            Xi[2] = i0 - Xi[0] - Xi[1];
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+          if (NT == 3) {
+            const int64_t r0 = Mr[0][n], i0 = Mi[0][n];
+            Mr[0][n] = Mr[1][n];
+            Mr[1][n] = Mr[2][n];
+            Mr[2][n] = r0 - Mr[0][n] - Mr[1][n];
+            Mi[0][n] = Mi[1][n];
+            Mi[1][n] = Mi[2][n];
+            Mi[2][n] = i0 - Mi[0][n] - Mi[1][n];
+          }
+#pragma unroll
+          for (int m = 0; m < NT; ++m)
+            M[m][n] = C2<double>{g64::from_fixed(Mr[m][n], e0), g64::from_fixed(Mi[m][n], e0)};
+          if (NX) X[n] = C2<double>{g64::from_fixed(Xr[n], e0 + ex), g64::from_fixed(Xi[n], e0 + ex)};
         }
       }
     }
-    const C2<double> M00 = M[0][0];
-    // (1, u, v) -> the three barycentric coordinates, in the order 0 (u), 1 (v), 2
-    if (NB == 3) {
+    if (!done) {
+      for (int a = 0; a < no; ++a) {
+        const V3<double> xi = mk(sxi[(3 * a) * FAR_THREADS + threadIdx.x], sxi[(3 * a + 1) * FAR_THREADS + threadIdx.x],
+                                 sxi[(3 * a + 2) * FAR_THREADS + threadIdx.x]);
+        const V3<double> dx = d + xi;
+        C2<double> U[3];
+        U[0] = U[1] = U[2] = C2<double>{0, 0};
+#pragma unroll 2
+        for (int b = 0; b < ni; ++b) {
+          const double* pb = pq + b * FAR64_PT;
+          const V3<double> r = dx - mk(pb[0], pb[1], pb[2]);
+          g64::Value v;
+          if constexpr (FIX)
+            v = g64::eval_slow(dot(r, r), P.wave.k);
+          else
+            v = g64::eval(dot(r, r), P.wave, tab);
+          double amp = v.iR;
+          if (gr != 0.0) amp *= exp(-gr * v.R);
+          double kr, ki;  // single layer: 4 pi G, the imaginary part times -sg; gradient: -4 pi c, times sg
+          if (GRAD) {
+            const double p1 = v.iR + gr, q = amp * v.iR;
+            kr = fma(p1, v.c, P.wave.k * v.s);
+            ki = fma(P.wave.k, v.c, -(p1 * v.s));
+            double f = q;
+            if (OPK == BEAST_HH_DLT) f *= dot(nn, r);
+            kr *= f;
+            ki *= f;
+          } else {
+            kr = amp * v.c;
+            ki = amp * v.s;
+          }
+          U[0].re = fma(pb[3], kr, U[0].re);
+          U[0].im = fma(pb[3], ki, U[0].im);
+          if (NB == 3) {
+            U[1].re = fma(pb[4], kr, U[1].re);
+            U[1].im = fma(pb[4], ki, U[1].im);
+            U[2].re = fma(pb[5], kr, U[2].re);
+            U[2].im = fma(pb[5], ki, U[2].im);
+          }
+        }
+        if (OPK == BEAST_HH_DL) {
+          const double f = dot(nq, dx);
 #pragma unroll
-      for (int m = 0; m < NT; ++m) {
-        const C2<double> t = M[m][0];
-        M[m][0] = M[m][1];
-        M[m][1] = M[m][2];
-        M[m][2] = csub(csub(t, M[m][0]), M[m][1]);
-      }
-      if (NX) {
-        const C2<double> t = X[0];
-        X[0] = X[1];
-        X[1] = X[2];
-        X[2] = csub(csub(t, X[0]), X[1]);
-      }
-    }
-    if (NT == 3) {
+          for (int n = 0; n < NB; ++n) U[n] = cscale(f, U[n]);
+        }
 #pragma unroll
-      for (int n = 0; n < NB; ++n) {
-        const C2<double> t = M[0][n];
-        M[0][n] = M[1][n];
-        M[1][n] = M[2][n];
-        M[2][n] = csub(csub(t, M[0][n]), M[1][n]);
+        for (int m = 0; m < NT; ++m)
+#pragma unroll
+          for (int n = 0; n < NB; ++n) {
+            M[m][n].re = fma(ro_s[a][m], U[n].re, M[m][n].re);
+            M[m][n].im = fma(ro_s[a][m], U[n].im, M[m][n].im);
+          }
+        if (NX) {
+          const double f = ro_s[a][0] * dot(xi, xi);
+#pragma unroll
+          for (int n = 0; n < 3; ++n) {
+            X[n].re = fma(f, U[n].re, X[n].re);
+            X[n].im = fma(f, U[n].im, X[n].im);
+          }
+        }
+      }
+      M00 = M[0][0];
+      // (1, u, v) -> the three barycentric coordinates, in the order 0 (u), 1 (v), 2
+      if (NB == 3) {
+#pragma unroll
+        for (int m = 0; m < NT; ++m) {
+          const C2<double> t = M[m][0];
+          M[m][0] = M[m][1];
+          M[m][1] = M[m][2];
+          M[m][2] = csub(csub(t, M[m][0]), M[m][1]);
+        }
+        if (NX) {
+          const C2<double> t = X[0];
+          X[0] = X[1];
+          X[1] = X[2];
+          X[2] = csub(csub(t, X[0]), X[1]);
+        }
+      }
+      if (NT == 3) {
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+          const C2<double> t = M[0][n];
+          M[0][n] = M[1][n];
+          M[1][n] = M[2][n];
+          M[2][n] = csub(csub(t, M[0][n]), M[1][n]);
+        }
       }
     }
     auto put = [&](int i, int j, C2<double> z) { store_c<double>(P.zcell, zidx(zr[i], s_zc[qi][j], P.ldc), z, P.fmt); };
@@ -2655,20 +2838,30 @@ static int sm_count() {
 // of a CTA shared by 16 pairs per thread), halved while the grid has less than four CTAs per SM:
 // a thread's pairs run one after the other, and a small operator's few CTAs would leave most of the
 // chip's FP64 units idle.
-template <int OPK, int TK, int BK>
-static cudaError_t far64_t(FarParams P, int fmt, cudaStream_t st) {
+// The integer moments (FIX) for a real wavenumber at which most pairs are in their range: k times the
+// average cell radius at least 2^-5, a far pair's points being several radii apart (integer sines
+// start at kR = 2^-7).  Complex wavenumbers, static kernels and low frequencies take the FP64 sums.
+template <int OPK, int TK, int BK, bool FIX>
+static cudaError_t far64_launch(FarParams P, int fmt, cudaStream_t st) {
   const int64_t gx = (P.np + FAR_THREADS - 1) / FAR_THREADS;
   P.qt = FAR_QT;
   P.fmt = fmt;
   while (P.qt > 1 && gx * ((P.nq + P.qt - 1) / P.qt) < 4 * (int64_t)sm_count()) P.qt /= 2;
   P.wave = g64::make_wave(P.op.gi);
-  const size_t sm = sizeof(g64::Entry) * g64::TABLE + P.qt * (sizeof(Far64Rec) + sizeof(double) * FAR64_PT * P.ri.n) +
-                    sizeof(double) * 3 * FAR_THREADS * P.ro.n;
-  cudaError_t e = cudaFuncSetAttribute(k_far64<OPK, TK, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  size_t sm = sizeof(g64::Entry) * g64::TABLE + P.qt * (sizeof(Far64Rec) + sizeof(double) * FAR64_PT * P.ri.n) +
+              sizeof(double) * 3 * FAR_THREADS * P.ro.n;
+  if (FIX && OPK == BEAST_MW_NXDL) sm += sizeof(int64_t) * FAR_THREADS * P.ro.n;
+  if (FIX) sm += sizeof(float) * 3 * (P.qt * P.ri.n + FAR_THREADS * P.ro.n);
+  cudaError_t e = cudaFuncSetAttribute(k_far64<OPK, TK, BK, FIX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)gx, (unsigned)((P.nq + P.qt - 1) / P.qt));
-  k_far64<OPK, TK, BK><<<grid, FAR_THREADS, sm, st>>>(P);
+  k_far64<OPK, TK, BK, FIX><<<grid, FAR_THREADS, sm, st>>>(P);
   return cudaGetLastError();
+}
+template <int OPK, int TK, int BK>
+static cudaError_t far64_t(const FarParams& P, int fmt, cudaStream_t st) {
+  return P.op.gr == 0.0 && fabs(P.op.gi) * P.radius >= 0.03125 ? far64_launch<OPK, TK, BK, true>(P, fmt, st)
+                                                               : far64_launch<OPK, TK, BK, false>(P, fmt, st);
 }
 
 template <int OPK, int TK, int BK>
@@ -2868,6 +3061,7 @@ cudaError_t launch_far(const AsmArgs& a, const TriRuleDev& ro, const TriRuleDev&
   P.flag = a.flag;
   P.ro = ro;
   P.ri = ri;
+  P.radius = a.bs->mesh ? a.bs->mesh->radius : 0.0;
   if (P.np == 0 || P.nq == 0) return cudaSuccess;
   const int tk = a.ts->kind, bk = a.bs->kind;
   const int kind = a.op.kind;

@@ -179,9 +179,10 @@ G64_HD void inv_sqrt(double R2, double& iR, double& R) {
   R = fma(r, half(g), g);
 }
 
-// cos and sin of n + f steps, the fraction f in [-1/2, 1/2) as the 64-bit fixed-point number fh:fl
-// (plus rest)
-G64_HD void rotate(uint32_t n, uint32_t fh, uint32_t fl, float rest, const Entry* tab, double& c, double& s) {
+// what the fraction of a step, f in [-1/2, 1/2) as the 64-bit fixed-point number fh:fl (plus rest), adds
+// to the table point's sine and cosine A, B: float pairs (sh, sl), (ch, cl) with |sh| at least |sl|
+G64_HD void correction(uint32_t fh, uint32_t fl, float rest, float Ah, float Al, float Bh, float Bl, float& sh, float& sl,
+                       float& ch, float& cl) {
   // the fraction as 24 + 32 bits
   const float fa = fmul((float)(int32_t)(fh & 0xFFFFFF00u), 2.3283064365386963e-10f);
   const float fb = fmaf((float)((fh << 24) | (fl >> 8)), 1.3877787807814457e-17f, rest);
@@ -190,25 +191,32 @@ G64_HD void rotate(uint32_t n, uint32_t fh, uint32_t fl, float rest, const Entry
   const float p = fmul(th, th);
   const float pl = fmaf(th, th, -p) + 2.f * fmul(th, tl);
   // cos t - 1 and sin t
-  const float ch = fmul(-0.5f, p), cl = fmaf(-0.5f, pl, fmul(fmul(p, p), 1.f / 24.f));
-  const float sl = fmaf(fmul(th, p), fmaf(p, 1.f / 120.f, -1.f / 6.f), tl);
-  const int i = (int)(n & (QUARTER - 1)), q = (int)(n >> 10) & 3;
-  const Entry A = tab[i], B = tab[QUARTER - i];
+  const float kh = fmul(-0.5f, p), kl = fmaf(-0.5f, pl, fmul(fmul(p, p), 1.f / 24.f));
+  const float ul = fmaf(fmul(th, p), fmaf(p, 1.f / 120.f, -1.f / 6.f), tl);
   float h1, l1, h2, l2;
-  pair_mul(B.hi, B.lo, th, sl, h1, l1);
-  pair_mul(A.hi, A.lo, ch, cl, h2, l2);
+  pair_mul(Bh, Bl, th, ul, h1, l1);
+  pair_mul(Ah, Al, kh, kl, h2, l2);
   float h = fadd(h1, h2);
   float bb = fsub(h, h1);
   float l = fadd(fadd(fsub(h1, fsub(h, bb)), fsub(h2, bb)), fadd(l1, l2));
-  float t = fadd(h, l);
-  const double s0 = A.v + pair_to_double(t, fsub(l, fsub(t, h)));
-  pair_mul(B.hi, B.lo, ch, cl, h1, l1);
-  pair_mul(-A.hi, -A.lo, th, sl, h2, l2);
+  sh = fadd(h, l);
+  sl = fsub(l, fsub(sh, h));
+  pair_mul(Bh, Bl, kh, kl, h1, l1);
+  pair_mul(-Ah, -Al, th, ul, h2, l2);
   h = fadd(h1, h2);
   bb = fsub(h, h1);
   l = fadd(fadd(fsub(h1, fsub(h, bb)), fsub(h2, bb)), fadd(l1, l2));
-  t = fadd(h, l);
-  const double c0 = B.v + pair_to_double(t, fsub(l, fsub(t, h)));
+  ch = fadd(h, l);
+  cl = fsub(l, fsub(ch, h));
+}
+
+// cos and sin of n + f steps
+G64_HD void rotate(uint32_t n, uint32_t fh, uint32_t fl, float rest, const Entry* tab, double& c, double& s) {
+  const int i = (int)(n & (QUARTER - 1)), q = (int)(n >> 10) & 3;
+  const Entry A = tab[i], B = tab[QUARTER - i];
+  float sh, sl, ch, cl;
+  correction(fh, fl, rest, A.hi, A.lo, B.hi, B.lo, sh, sl, ch, cl);
+  const double s0 = A.v + pair_to_double(sh, sl), c0 = B.v + pair_to_double(ch, cl);
   // quarter turns
   const uint64_t us = bits((q & 1) ? c0 : s0), uc = bits((q & 1) ? s0 : c0);
   s = from_bits(us ^ ((uint64_t)(q >> 1) << 63));
@@ -257,6 +265,94 @@ G64_HD Value eval(double R2, const Wave& w, const Entry* tab) {
   return v;
 }
 
+// ---- the same in 64-bit fixed point ---------------------------------------------------------
+// Sums of kernel values times rule weights need no exponent of their own: as integers they cost two
+// instructions per addition and about a dozen per product where the FP64 pipe takes 64 issue slots
+// for either.  Values are int64 with 62 fractional bits.
+
+// round(x 2^62) of a float pair, |h| < 2^-9
+G64_HD int64_t pair_to_fixed(float h, float l) {
+#if defined(__CUDA_ARCH__)
+  const int i = __float2int_rn(fmul(h, 274877906944.f));  // 2^38
+#else
+  const int i = (int)lrintf(h * 274877906944.f);
+#endif
+  const float r = fmaf(-(float)i, 3.637978807091713e-12f, h) + l;
+#if defined(__CUDA_ARCH__)
+  const int k = __float2int_rn(fmul(r, 4611686018427387904.f));
+#else
+  const int k = (int)lrintf(r * 4611686018427387904.f);
+#endif
+  return ((int64_t)i << 24) + k;
+}
+// x 2^(62 - e) of a double with |x| < 2^e, truncated
+G64_HD int64_t to_fixed(double x, int e) {
+  const uint64_t u = bits(x);
+  const int E = (int)((u >> 52) & 0x7FF) - 1023;
+  const uint64_t m = E == -1023 ? 0 : (u & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+  const int sh = 10 + E - e;  // < 10
+  const uint64_t v = sh >= 0 ? m << (sh & 63) : (sh > -64 ? m >> (-sh & 63) : 0);
+  return (u >> 63) ? -(int64_t)v : (int64_t)v;
+}
+// x 2^e of an integer as a double, rounded to nearest (ties up); no FP64 instruction
+G64_HD double from_fixed(int64_t x, int e) {
+  const uint64_t sgn = (uint64_t)x & 0x8000000000000000ull;
+  const uint64_t u = x < 0 ? 0ull - (uint64_t)x : (uint64_t)x;
+  if (u == 0) return 0.0;
+#if defined(__CUDA_ARCH__)
+  const int lz = __clzll((long long)u);
+#else
+  const int lz = __builtin_clzll(u);
+#endif
+  const uint64_t m = u << lz;
+  const uint64_t r = (m >> 11) + ((m >> 10) & 1);  // 2^52 .. 2^53
+  return from_bits(sgn | (((uint64_t)(1023 + 63 - lz + e - 1) << 52) + r));
+}
+G64_HD int64_t mulhi(int64_t a, int64_t b) {
+#if defined(__CUDA_ARCH__)
+  return __mul64hi(a, b);
+#else
+  return (int64_t)(((__int128)a * b) >> 64);
+#endif
+}
+
+struct EntryX {
+  int64_t v;  // sin 2^62
+  float hi, lo;
+};
+G64_HD EntryX to_entryx(double x) {
+  const float h = (float)x;
+  return EntryX{x >= 1.0 ? (int64_t)1 << 62 : to_fixed(x, 0), h, (float)(x - (double)h)};
+}
+struct ValueX {
+  double iR;     // 1/R
+  int64_t c, s;  // cos(|k| R), sin(|k| R)
+};
+// false: R2 or the angle out of range (below 2^-8 the integer sine would lose relative accuracy)
+G64_HD bool eval_fixed(double R2, const Wave& w, const EntryX* tab, ValueX& v) {
+  if ((uint32_t)((uint32_t)(bits(R2) >> 52) - 923u) > 190u) return false;
+  double R;
+  inv_sqrt(R2, v.iR, R);
+  const double phi = R * w.steps;
+  const uint64_t u = bits(phi);
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
+  const int e = (int)(hi >> 20) - 1023;
+  if ((uint32_t)(e - 2) > 27u) return false;  // 4 <= phi < 2^30
+  const float rest = fmul(w.rest, from_fbits((uint32_t)(((bits(R) >> 32) - (896ull << 20)) << 3)));
+  const uint32_t xh = ((hi << 11) | (lo >> 21)) | 0x80000000u, xl = lo << 11;
+  const uint32_t fh = (xh << (e + 1)) | (xl >> (31 - e)), fl = xl << (e + 1);
+  const uint32_t n = (xh >> (31 - e)) + (fh >> 31);
+  const int i = (int)(n & (QUARTER - 1)), q = (int)(n >> 10) & 3;
+  const EntryX A = tab[i], B = tab[QUARTER - i];
+  float sh, sl, ch, cl;
+  correction(fh, fl, rest, A.hi, A.lo, B.hi, B.lo, sh, sl, ch, cl);
+  const int64_t s0 = A.v + pair_to_fixed(sh, sl), c0 = B.v + pair_to_fixed(ch, cl);
+  const int64_t us = (q & 1) ? c0 : s0, uc = (q & 1) ? s0 : c0;
+  v.s = (q >> 1) ? -us : us;
+  v.c = (((q + 1) >> 1) & 1) ? -uc : uc;
+  return true;
+}
+
 #if defined(__CUDACC__)
 // the table into shared memory, by the whole CTA (the caller synchronises)
 __device__ __forceinline__ void load_table(Entry* tab) {
@@ -265,6 +361,9 @@ __device__ __forceinline__ void load_table(Entry* tab) {
     const float h = (float)x;
     tab[i] = Entry{x, h, (float)(x - (double)h)};
   }
+}
+__device__ __forceinline__ void load_table(EntryX* tab) {
+  for (int i = threadIdx.x; i < TABLE; i += blockDim.x) tab[i] = to_entryx(sin_table_dev[i]);
 }
 #endif
 

@@ -86,6 +86,7 @@ struct beast_mesh {
   // the cells' children in a refinement (beast_mesh_set_children): [nc][nchild][9] or null
   double* children = nullptr;
   int nchild = 0;
+  double radius = 0.0;       // average distance of a cell's vertices from its centroid
 };
 
 // per active cell geometry, 16 doubles: v0 v1 v2 (9) | centroid (3) | unit normal (3) | area

@@ -37,6 +37,18 @@ void t_turn(long n, const double* phi, double* out) {
 void t_turn_signed(long n, const double* phi, double* out) {
   for (long i = 0; i < n; ++i) g64::turn_signed(phi[i], 0.f, tab, out[2 * i], out[2 * i + 1]);
 }
+void t_fixed(long n, const double* R2, double k, double* out, int* ok) {
+  static g64::EntryX tx[g64::TABLE];
+  for (int i = 0; i < g64::TABLE; ++i) tx[i] = g64::to_entryx(g64::sin_table_host[i]);
+  const g64::Wave w = g64::make_wave(k);
+  for (long i = 0; i < n; ++i) {
+    g64::ValueX v{0.0, 0, 0};
+    ok[i] = g64::eval_fixed(R2[i], w, tx, v);
+    out[3 * i] = v.iR; out[3 * i + 1] = (double)v.c / 4611686018427387904.0; out[3 * i + 2] = (double)v.s / 4611686018427387904.0;
+  }
+}
+int64_t t_to_fixed(double x, int e) { return g64::to_fixed(x, e); }
+double t_from_fixed(int64_t x, int e) { return g64::from_fixed(x, e); }
 double t_pair(float h, float l) { return g64::pair_to_double(h, l); }
 }
 """
@@ -52,6 +64,7 @@ def lib(tmp_path_factory):
     subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(so)])
     L = C.CDLL(str(so))
     L.t_pair.restype, L.t_pair.argtypes = C.c_double, [C.c_float, C.c_float]
+    L.t_to_fixed.restype, L.t_from_fixed.restype = C.c_int64, C.c_double
     L.t_init()
     return L
 
@@ -115,3 +128,35 @@ def test_turn_signed(lib):
     for p, (c, s) in zip(phi, out):
         th = mpmath.mpf(float(p)) * mpmath.pi / 2048
         assert abs(c - mpmath.cos(th)) <= 2.0 ** -52 and abs(s - mpmath.sin(th)) <= 2.0 ** -52
+
+
+@pytest.mark.parametrize("k", [0.7, 40.0, 1e4])
+def test_fixed_point_values(lib, k):
+    """cos and sin as 62-bit integers to 2^-52 plus the rounding of the argument; out of range below
+    four steps and above 2^30"""
+    rng = np.random.default_rng(6)
+    R2 = 10.0 ** rng.uniform(-6, 2, size=400)
+    out, ok = np.zeros((len(R2), 3)), np.zeros(len(R2), dtype=np.int32)
+    lib.t_fixed(C.c_long(len(R2)), R2.ctypes.data_as(C.c_void_p), C.c_double(k), out.ctypes.data_as(C.c_void_p),
+                ok.ctypes.data_as(C.c_void_p))
+    mpmath.mp.dps = 40
+    for r2, (iR, c, s), good in zip(R2, out, ok):
+        th = mpmath.sqrt(mpmath.mpf(float(r2))) * k
+        assert bool(good) == (4 <= th * 2048 / mpmath.pi < 2 ** 30)
+        if good:
+            tol = 2.0 ** -52 + float(th) * 2.0 ** -52
+            assert abs(c - mpmath.cos(th)) <= tol and abs(s - mpmath.sin(th)) <= tol
+
+
+def test_fixed_point_conversions(lib):
+    rng = np.random.default_rng(7)
+    x = rng.uniform(-1, 1, size=2000) * 2.0 ** rng.integers(-70, 1, size=2000)
+    x[:4] = [0.0, 0.5, -0.5, 1.0 - 2.0 ** -53]
+    for v in x:
+        for e in (0, 3):
+            f = lib.t_to_fixed(C.c_double(v), e)
+            assert abs(f * 2.0 ** (e - 62) - v) < 2.0 ** (e - 62) + abs(v) * 2.0 ** -53
+            assert lib.t_from_fixed(C.c_int64(f), 0) == float(f)
+    for v in [1, -1, 2 ** 53 + 1, -(2 ** 62) + 1, 2 ** 62, (1 << 63) - 1]:
+        r = lib.t_from_fixed(C.c_int64(v), -10)
+        assert abs(int(r * 1024) - v) * 2 ** 53 <= abs(v)
