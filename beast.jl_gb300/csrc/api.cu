@@ -1490,6 +1490,7 @@ int beast_batch_create(beast_ctx* ctx, const beast_qs_desc* qs, int64_t njobs, c
     }
     BatchJobDev& J = jt[j];
     J.op = to_params(&ops[j]);
+    batch_wave(&J);
     J.k2 = ops[j].gamma_re * ops[j].gamma_re + ops[j].gamma_im * ops[j].gamma_im;
     J.geo = s->geo;
     J.geof = s->geof;
@@ -1548,6 +1549,7 @@ int beast_batch_create(beast_ctx* ctx, const beast_qs_desc* qs, int64_t njobs, c
   L.precision = precision;
   L.zfmt = precision == BEAST_MIXED ? ZCELL_C64 : ZCELL_C128;
   L.op_kind = kind;
+  for (int64_t j = 0; j < njobs; ++j) L.complex_k |= ops[j].gamma_re != 0.0;
   L.near = b->near;
   L.near_cap = (int)std::min<int64_t>(near_cap, INT32_MAX);
   L.near_count = b->counter;
@@ -1561,6 +1563,7 @@ int beast_batch_create(beast_ctx* ctx, const beast_qs_desc* qs, int64_t njobs, c
   // (graph capture comes later)
   if (kind == BEAST_HH_SL && precision != BEAST_FP64 && qs->kind != BEAST_QS_DOUBLENUM) {
     cudaError_t e = ss_tables(&ctx->ss_tabs, *qs, ctx->stream, L.ssdf_tab, L.ssdf_items);
+    if (e == cudaSuccess) e = ssp_tables(&ctx->ss_tabs, *qs, ctx->stream, &L.ssp);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
       beast_batch_free(b);

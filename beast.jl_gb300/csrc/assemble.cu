@@ -25,6 +25,7 @@
 #include "fsplit.h"
 #include "green64.h"
 #include "internal.h"
+#include "pack2.h"
 #include "se_p1.h"
 #include "far_df.h"
 #include "se_core.h"
@@ -124,7 +125,8 @@ __global__ void k_geometry(const double* verts, const int* mcells, const int* ac
 // pair classification: quadrule(..., ::DoubleNumWiltonSauterQStrat)
 // returns 3/2/1 (common face/edge/vertex), -1 (Wilton SE) or 0 (far DQ)
 // ------------------------------------------------------------------------------------
-DEV int classify_exact(const Geo& t, const Geo& s, int qs_kind, double k2) {
+__device__ __noinline__ int classify_slow(const Geo* tp, const Geo* sp, int qs_kind, double k2) {
+  const Geo &t = *tp, &s = *sp;
   const double dtol = 1.0e3 * 2.220446049250313e-16;
   int hits = 0;
   double dmin2 = 1e308;
@@ -154,6 +156,58 @@ DEV int refines_class(int cls, int qs_kind) {
 }
 
 // squared distance below which a pair can be near (strategy threshold of the trial cell)
+// the same class without FP64 instructions (classify_slow has about 130 of them, and one candidate among
+// a warp's pairs makes the warp run them: 3 of the 10.5 ms of a batch of 24 Helmholtz systems): the
+// coordinates as FP32 pairs, shared vertices by their bits; what FP32 cannot decide goes to classify_slow
+DEV int classify_exact(const Geo& t, const Geo& s, int qs_kind, double k2) {
+  if (qs_kind == BEAST_QS_DOUBLENUM) return 0;
+  float th[9], tl[9], cmax = 0.f;
+  for (int i = 0; i < 3; ++i) {
+    fsplit::split_f64_fast(t.v[i].x, &th[3 * i], &tl[3 * i]);
+    fsplit::split_f64_fast(t.v[i].y, &th[3 * i + 1], &tl[3 * i + 1]);
+    fsplit::split_f64_fast(t.v[i].z, &th[3 * i + 2], &tl[3 * i + 2]);
+    cmax = fmaxf(cmax, fmaxf(fabsf(th[3 * i]), fmaxf(fabsf(th[3 * i + 1]), fabsf(th[3 * i + 2]))));
+  }
+  // vertices apart by more than this are not shared (the test's limit is 2.3e-13), and their distance is
+  // good to 1e-6 (the pairs' own error is 2^-47 of a coordinate)
+  const float apart = fmaxf(1e-20f, 1e-14f * cmax * cmax);
+  int hits = 0;
+  bool open = !(cmax < 1e15f);
+  float dmin2 = 3e38f;
+  for (int j = 0; j < 3; ++j) {
+    float sh[3], sl[3];
+    fsplit::split_f64_fast(s.v[j].x, &sh[0], &sl[0]);
+    fsplit::split_f64_fast(s.v[j].y, &sh[1], &sl[1]);
+    fsplit::split_f64_fast(s.v[j].z, &sh[2], &sl[2]);
+    for (int i = 0; i < 3; ++i) {
+      const float x = (th[3 * i] - sh[0]) + (tl[3 * i] - sl[0]), y = (th[3 * i + 1] - sh[1]) + (tl[3 * i + 1] - sl[1]),
+                  z = (th[3 * i + 2] - sh[2]) + (tl[3 * i + 2] - sl[2]);
+      const float d2 = fmaf(x, x, fmaf(y, y, z * z));
+      dmin2 = fminf(dmin2, d2);
+      if (!(d2 > apart)) {
+        const bool same = __double_as_longlong(t.v[i].x) == __double_as_longlong(s.v[j].x) &&
+                          __double_as_longlong(t.v[i].y) == __double_as_longlong(s.v[j].y) &&
+                          __double_as_longlong(t.v[i].z) == __double_as_longlong(s.v[j].z);
+        hits += same;
+        open |= !same;
+      }
+    }
+  }
+  if (!open) {
+    if (hits > 0) return hits;
+    if (qs_kind == BEAST_QS_SAUTER) return 0;
+    float ah, al, kh, kl;
+    fsplit::split_f64_fast(s.area, &ah, &al);
+    fsplit::split_f64_fast(k2, &kh, &kl);
+    const float a16 = 16.f * ah;
+    if (a16 > 1e-30f && a16 < 1e30f && kh < 1e30f && dmin2 < 1e30f) {
+      const float m = fmaxf(dmin2 * kh, dmin2 / a16);
+      if (m > 0.04f * 1.0001f) return 0;
+      if (m < 0.04f * 0.9999f && m > 1e-30f) return -1;
+    }
+  }
+  return classify_slow(&t, &s, qs_kind, k2);
+}
 DEV double near_threshold2(int qs_kind, double k2, double area) {
   if (qs_kind == BEAST_QS_DOUBLENUM) return -1.0;
   if (qs_kind == BEAST_QS_SAUTER) return 0.0;
@@ -226,12 +280,109 @@ DEV void store_c(void* z, int64_t idx, C2<R> v, int fmt) {
 // distance); then per inner rule point eta_b = y_b - c (3) and weight
 constexpr int QREC_HDR = 20;
 
+// sum over the point pairs of w_a w_b e^{-gr R} (cos gi R, sin gi R) / R: the Helmholtz single layer's
+// far pair on P0 in FP32, for k_far and k_far_batch alike.  Bound by its instructions: 23 per point pair
+// (69 before), the trial points two by two in packed FP32 (pack2.h), the constants 1 / (4 pi), alpha and
+// the areas left to the caller.  sin and cos: the nearest multiple of pi / 32 from a table (value and
+// rest) and the remainder by its Taylor polynomials, one rounding of a result of size one at the end.
+// Every rounding is written out, so that both kernels give the same bits.
+// Trial points: pairs (x x' y y' z z' w w'), an odd count filled up with a copy of weight 0.
+// tab: sin(m pi/32), its rest, cos, its rest, 64 values each; bound >= |gi| R over the pair.
+DEV C2<float> hh_sl_far_f(V3<float> d, const V3<float>* tau, const float* ro, int no, const float* pts, int ni, float gr,
+                          float gi, float bound, const float* tab) {
+  auto test_point = [&](int a) {
+    const float u = ro[3 * a], v = ro[3 * a + 1], w3 = __fsub_rn(__fsub_rn(1.f, u), v);
+    return mk(__fadd_rn(d.x, fmaf(u, tau[0].x, fmaf(v, tau[1].x, __fmul_rn(w3, tau[2].x)))),
+              __fadd_rn(d.y, fmaf(u, tau[0].y, fmaf(v, tau[1].y, __fmul_rn(w3, tau[2].y)))),
+              __fadd_rn(d.z, fmaf(u, tau[0].z, fmaf(v, tau[1].z, __fmul_rn(w3, tau[2].z)))));
+  };
+  float re, im;
+  if (gr == 0.f && bound < 32768.f) {
+    const pk::f2 magic = pk::both(12582912.f), g2 = pk::both(gi);  // 1.5 2^23: the nearest whole number
+    pk::f2 sr = pk::both(0.f), si = sr;
+    for (int a = 0; a < no; ++a) {
+      const V3<float> x = test_point(a);
+      const pk::f2 wa = pk::both(ro[3 * a + 2]), xx = pk::both(x.x), xy = pk::both(x.y), xz = pk::both(x.z);
+#pragma unroll 1
+      for (int b = 0; b < ni; b += 2) {
+        const ulonglong2 p0 = *reinterpret_cast<const ulonglong2*>(pts + 4 * b),
+                         p1 = *reinterpret_cast<const ulonglong2*>(pts + 4 * b + 4);
+        const pk::f2 rx = pk::sub(xx, pk::f2{p0.x}), ry = pk::sub(xy, pk::f2{p0.y}), rz = pk::sub(xz, pk::f2{p1.x});
+        const pk::f2 R2 = pk::fma(rx, rx, pk::fma(ry, ry, pk::mul(rz, rz)));
+        float i0, i1;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i0) : "f"(pk::lo(R2)));
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(pk::hi(R2)));
+        const pk::f2 iR = pk::make(i0, i1), ph = pk::mul(g2, pk::mul(R2, iR));
+        const pk::f2 f = pk::fma(ph, pk::both(10.185916357881302f), magic), m = pk::sub(f, magic);  // 32 / pi
+        const pk::f2 t = pk::fma(m, pk::both(2.7319617985750483e-09f), pk::fma(m, pk::both(-0.09817477315664291f), ph));
+        const pk::f2 t2 = pk::mul(t, t);
+        const pk::f2 st = pk::fma(pk::mul(t, t2), pk::both(-1.f / 6.f), t);
+        const pk::f2 ct = pk::mul(t2, pk::fma(t2, pk::both(1.f / 24.f), pk::both(-0.5f)));  // cos t - 1
+        const float* e0 = tab + ((unsigned)f.v & 63u);
+        const float* e1 = tab + ((unsigned)(f.v >> 32) & 63u);
+        const pk::f2 s = pk::make(e0[0], e1[0]), sl = pk::make(e0[64], e1[64]), c = pk::make(e0[128], e1[128]),
+                     cl = pk::make(e0[192], e1[192]);
+        const pk::f2 w = pk::mul(pk::mul(pk::f2{p1.y}, wa), iR);
+        const pk::f2 ns = pk::make(-pk::lo(s), -pk::hi(s));
+        si = pk::fma(w, pk::add(s, pk::fma(c, st, pk::fma(s, ct, sl))), si);
+        sr = pk::fma(w, pk::add(c, pk::fma(ns, st, pk::fma(c, ct, cl))), sr);
+      }
+    }
+    re = __fadd_rn(pk::lo(sr), pk::hi(sr));
+    im = __fadd_rn(pk::lo(si), pk::hi(si));
+    // (a distance below 1e-19 is flushed to 0 above: once more below)
+    if (fabsf(re) + fabsf(im) < 3e38f) return {re, im};
+  }
+  re = im = 0.f;
+  for (int a = 0; a < no; ++a) {
+    const V3<float> x = test_point(a);
+    for (int b = 0; b < ni; ++b) {
+      const float* p = pts + 8 * (b >> 1) + (b & 1);
+      const float rx = __fsub_rn(x.x, p[0]), ry = __fsub_rn(x.y, p[2]), rz = __fsub_rn(x.z, p[4]);
+      const float R2 = fmaf(rx, rx, fmaf(ry, ry, __fmul_rn(rz, rz)));
+      const float iR = rsqrtf(R2), R = __fmul_rn(R2, iR);
+      float s, c;
+      sincosf(__fmul_rn(gi, R), &s, &c);
+      float w = __fmul_rn(__fmul_rn(p[6], ro[3 * a + 2]), iR);
+      if (gr != 0.f) w = __fmul_rn(w, expf(__fmul_rn(-gr, R)));
+      re = fmaf(w, c, re);
+      im = fmaf(w, s, im);
+    }
+  }
+  return {re, im};
+}
+// |gi| R <= |gi| (|c_p - c_q| + both radii)
+DEV float hh_sl_bound_f(V3<float> d, float lim, float gi) {
+  const float dd = fmaf(d.x, d.x, fmaf(d.y, d.y, __fmul_rn(d.z, d.z)));
+  return __fmul_rn(fabsf(gi), __fadd_rn(__fmul_rn(1.001f, sqrtf(dd)), lim));
+}
+// a trial point's place in hh_sl_far_f's pairs
+DEV void hh_sl_stage_f(float* pts, int b, int ni, float x, float y, float z, float w) {
+  float* p = pts + 8 * (b >> 1) + (b & 1);
+  p[0] = x;
+  p[2] = y;
+  p[4] = z;
+  p[6] = w;
+  if (b == ni - 1 && (ni & 1)) {
+    p[1] = x;
+    p[3] = y;
+    p[5] = z;
+    p[7] = 0.f;
+  }
+}
+// its matrix entry: alpha A_p A_q / (4 pi) (re - i im)
+DEV C2<float> hh_sl_far_entry_f(C2<float> sum, C2<float> al, float Ap, float Aq) {
+  const float f = __fmul_rn(__fmul_rn(Ap, Aq), (float)I4PI), re = __fmul_rn(f, sum.re), im = __fmul_rn(f, sum.im);
+  return {fmaf(al.re, re, __fmul_rn(al.im, im)), fmaf(al.im, re, -__fmul_rn(al.re, im))};
+}
+
 template <int OPK, int TK, int BK, typename R, int FMT>
 __global__ void __launch_bounds__(FAR_THREADS) k_far(FarParams P) {
-  extern __shared__ unsigned char smraw[];
+  extern __shared__ __align__(16) unsigned char smraw[];
   R* sm = reinterpret_cast<R*>(smraw);
   const int ni = P.ri.n;
-  const int rec = QREC_HDR + 4 * ni;
+  constexpr bool SL_P0 = OPK == BEAST_HH_SL && TK == BEAST_P0 && BK == BEAST_P0;  // hh_sl_far_f
+  const int rec = QREC_HDR + 4 * (SL_P0 ? ni + (ni & 1) : ni);
   const int q0 = blockIdx.y * FAR_QT;
   const int nqt = min(FAR_QT, P.nq - q0);
   // rule points in the arithmetic type, converted once per CTA (a double -> float conversion
@@ -268,16 +419,26 @@ __global__ void __launch_bounds__(FAR_THREADS) k_far(FarParams P) {
     } else {
       int bb = b - 1;
       double u = P.ri.u[bb], v = P.ri.v[bb], w = 1.0 - u - v;
-      R* pt = r + QREC_HDR + 4 * bb;
-      pt[0] = (R)(u * (g[0] - cx) + v * (g[3] - cx) + w * (g[6] - cx));
-      pt[1] = (R)(u * (g[1] - cy) + v * (g[4] - cy) + w * (g[7] - cy));
-      pt[2] = (R)(u * (g[2] - cz) + v * (g[5] - cz) + w * (g[8] - cz));
-      pt[3] = (R)P.ri.w[bb];
+      const R x = (R)(u * (g[0] - cx) + v * (g[3] - cx) + w * (g[6] - cx));
+      const R y = (R)(u * (g[1] - cy) + v * (g[4] - cy) + w * (g[7] - cy));
+      const R z = (R)(u * (g[2] - cz) + v * (g[5] - cz) + w * (g[8] - cz));
+      if constexpr (SL_P0) {
+        hh_sl_stage_f(r + QREC_HDR, bb, ni, x, y, z, (R)P.ri.w[bb]);
+      } else {
+        R* pt = r + QREC_HDR + 4 * bb;
+        pt[0] = x;
+        pt[1] = y;
+        pt[2] = z;
+        pt[3] = (R)P.ri.w[bb];
+      }
     }
   }
   __shared__ int s_zc[FAR_QT][3];
   for (int k = threadIdx.x; k < nqt * 3; k += blockDim.x)
     s_zc[k / 3][k % 3] = (int)zcol_of(P.zcol, q0 + k / 3, (BK == BEAST_P0) ? 1 : 3, k % 3);
+  __shared__ float s_sc[SL_P0 ? 256 : 1];
+  if (SL_P0)
+    for (int k = threadIdx.x; k < 256; k += blockDim.x) s_sc[k] = dfl::sincos_tab_dev[k & 63][k >> 6];
   __syncthreads();
   // pp: the test cell's Zcell position (cells in the order of their first function, so that
   // the rows a warp of the gather reads are close together); p: the active cell
@@ -466,6 +627,11 @@ __global__ void __launch_bounds__(FAR_THREADS) k_far(FarParams P) {
           store_c<R>(P.zcell, zidx(zr[i], s_zc[qi][j], P.ldc), z, FMT);
         }
       }
+    } else if constexpr (SL_P0) {
+      store_c<R>(P.zcell, zidx(zr[0], s_zc[qi][0], P.ldc),
+                 hh_sl_far_entry_f(hh_sl_far_f(d, tau, ro_s, no, pts, ni, gr, gi, hh_sl_bound_f(d, radp + rq[19], gi), s_sc),
+                                   alpha, ApR, Aq),
+                 FMT);
     } else {
       // ---- Helmholtz kernels on P0/P1: per point pair with shape products
       C2<R> acc[9];
@@ -1291,19 +1457,8 @@ DEV void ss_node_f(int cls, int n, int item, const float* glx, const float* glw,
 
 // ss_node_f's maps in FP64 (X, Y, D = X - Y from the maps' own factors, weight): the node
 // tables of k_near_ss_df are built from it once
-DEV void ss_node_fd(int cls, int n, int item, const double* glx, const double* glw, double* X, double* Y,
+DEV void ss_node_at(int cls, int reg, double xi, double e1, double e2, double e3, double ww, double* X, double* Y,
                     double* D, double* w) {
-  const int nreg = cls == 1 ? 2 : 6;
-  const int reg = item % nreg;
-  int k = item / nreg;
-  const int i4 = k % n;
-  k /= n;
-  const int i3 = k % n;
-  k /= n;
-  const int i2 = k % n;
-  const int i1 = k / n;
-  const double xi = glx[i1], e1 = glx[i2], e2 = glx[i3], e3 = glx[i4];
-  const double ww = glw[i1] * glw[i2] * glw[i3] * glw[i4];
   double A[2], B[2], AB[2], wt;
   const int sub = reg >> 1;
   const bool swap = reg & 1;
@@ -1345,6 +1500,19 @@ DEV void ss_node_fd(int cls, int n, int item, const double* glx, const double* g
   }
   *w = wt;
 }
+DEV void ss_node_fd(int cls, int n, int item, const double* glx, const double* glw, double* X, double* Y,
+                    double* D, double* w) {
+  const int nreg = cls == 1 ? 2 : 6;
+  const int reg = item % nreg;
+  int k = item / nreg;
+  const int i4 = k % n;
+  k /= n;
+  const int i3 = k % n;
+  k /= n;
+  const int i2 = k % n;
+  const int i1 = k / n;
+  ss_node_at(cls, reg, glx[i1], glx[i2], glx[i3], glx[i4], glw[i1] * glw[i2] * glw[i3] * glw[i4], X, Y, D, w);
+}
 
 DEV V3<float> v3f(V3<double> a) { return V3<float>{(float)a.x, (float)a.y, (float)a.z}; }
 
@@ -1363,6 +1531,7 @@ struct NearParams {
   int ss32;  // Sauter-Schwab moments of RT Maxwell pairs in FP32 (mixed precision)
   int ssdf;  // Sauter-Schwab pairs of RT Maxwell operators in double-float (k_near_ss_df)
   const float2* ssdf_tab[4];  // per class 1..3: node table [7][items] (ss_table)
+  SspTables ssp;               // the same without the radial coordinate (k_ssp_table)
   int ssdf_items[4];
   int ss64;  // Sauter-Schwab pairs in k_near_ss64
   const double* ss64_tab[4];  // per class 1..3: node table [SS64_VALS][items]
@@ -1738,7 +1907,7 @@ DEV void near_pair(const NearParams& P, const NearPair np_, const double* s_glx,
   C2<double> acc[9];
   for (int k = 0; k < 9; ++k) acc[k] = C2<double>{0, 0};
   const bool dl_face = np_.cls == 3 && dl_type(P.op.kind);
-  if (np_.cls >= 5) return;  // k_near_refines
+  if (np_.cls >= 5 || np_.cls == -1) return;  // k_near_refines, k_near_se / k_near_batch_se
   if (np_.cls == 4) {
     // ---- DoubleNumQStrat pair close to its partner: the pair's own DoubleQuadRule
     // (src/quadrature/doublenumints.jl:12-43) point by point in FP64, lanes over point pairs.
@@ -1848,8 +2017,6 @@ DEV void near_pair(const NearParams& P, const NearPair np_, const double* s_glx,
       return;
     }
     ss_points(P, t, s, np_.cls, pt, ps, s_glx, s_glw, lane, acc);
-  } else if (np_.cls == -1) {
-    se_points(P, t, s, lane, acc);
   }
   // ---- warp reduction and store
   for (int k = 0; k < nt * nb; ++k) {
@@ -1879,6 +2046,104 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near(NearParams P) {
   const int64_t e = blockIdx.x * (int64_t)NEAR_WARPS + warp;
   if (e >= P.nnear) return;
   near_pair(P, P.near[e], s_glx, s_glw, lane);
+}
+
+// ---- singularity-extraction pairs (class -1), several per warp
+// A pair has one Wilton integral per outer point, about 2000 FP64 instructions, and a few regular
+// values: with a warp per pair three (default Helmholtz rules) or twelve lanes did all of it.  A warp
+// collects the pairs of this class from the list and gives every outer point a lane: 32 / no pairs
+// at once, each lane its point's regular values over the inner rule, then its analytic part; the
+// points of a pair are added in order.  (TK, BK: the spaces' kinds, -1: from P)
+struct SeArgs {
+  const OpParams& op;
+  const TriRuleDev &ro, &ri;
+  int* flag;
+  void* z;
+  int zfmt;
+  int64_t ldc;
+  const int *zrow, *zcol;
+};
+
+template <int TK, int BK>
+DEV void se_group(const SeArgs& A, int tk_, int bk_, bool active, const Geo& t, const Geo& s, int p, int q, int a,
+                  int lane) {
+  const int tk = TK >= 0 ? TK : tk_, bk = BK >= 0 ? BK : bk_;
+  const int nt = tk == BEAST_P0 ? 1 : 3, nb = bk == BEAST_P0 ? 1 : 3;
+  constexpr int NMAX = TK == BEAST_P0 && BK == BEAST_P0 ? 1 : 9;
+  C2<double> acc[NMAX];
+  for (int k = 0; k < NMAX; ++k) acc[k] = C2<double>{0, 0};
+  if (active) {
+    const double bx[3] = {A.ro.u[a], A.ro.v[a], 1.0 - A.ro.u[a] - A.ro.v[a]};
+    const double wx = A.ro.w[a] * t.area;
+    const V3<double> x = bx[0] * t.v[0] + bx[1] * t.v[1] + bx[2] * t.v[2];
+    Shp f, g;
+    shapes(tk, t, x, bx, f);
+#pragma unroll 1
+    for (int b = 0; b < A.ri.n; ++b) {
+      const double by[3] = {A.ri.u[b], A.ri.v[b], 1.0 - A.ri.u[b] - A.ri.v[b]};
+      const V3<double> y = by[0] * s.v[0] + by[1] * s.v[1] + by[2] * s.v[2];
+      shapes(bk, s, y, by, g);
+      integrand(REG + A.op.kind, A.op, x, y, t.n, s.n, tk, f, bk, g, wx * A.ri.w[b] * s.area, acc);
+    }
+    if (!se_singular(A.op, tk, bk, t, s, x, bx, wx, acc)) atomicOr(A.flag, 2);
+  }
+  const int base = lane - a;
+  for (int k = 0; k < nt * nb; ++k) {
+    double re = 0.0, im = 0.0;
+    for (int c = 0; c < A.ro.n; ++c) {
+      re += __shfl_sync(0xffffffffu, acc[k].re, (base + c) & 31);
+      im += __shfl_sync(0xffffffffu, acc[k].im, (base + c) & 31);
+    }
+    if (active && a == 0)
+      store_c<double>(A.z, zidx(zrow_of(A.zrow, p, nt, k / nb), zcol_of(A.zcol, q, nb, k % nb), A.ldc),
+                      C2<double>{re, im}, A.zfmt);
+  }
+}
+
+// the class -1 entries of list entries e0 .. e0 + 31 into a warp's queue, their indices in list order
+template <typename Cls>
+DEV int se_collect(int64_t e0, int64_t n, int lane, int* queue, int count, Cls cls) {
+  const bool se = e0 + lane < n && cls(e0 + lane) == -1;
+  const unsigned m = __ballot_sync(0xffffffffu, se);
+  if (se) queue[count + __popc(m & ((1u << lane) - 1u))] = (int)(e0 + lane);
+  __syncwarp();
+  return count + __popc(m);
+}
+
+// the class -1 pairs of a near list of n entries, dealt over the grid's warps: cls(e) gives an entry's
+// class, group(entry, active, point, lane) computes one point of one pair
+template <typename Cls, typename Group>
+DEV void se_walk(int64_t n, int no, int* queue, Cls cls, Group group) {
+  static_assert(RULE_MAXPTS <= 32, "a pair's outer points fit a warp");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 32 / no, g = lane / no, a = lane % no;
+  const int64_t step = (int64_t)gridDim.x * NEAR_WARPS * 32;
+  int count = 0;
+  for (int64_t e0 = (blockIdx.x * (int64_t)NEAR_WARPS + warp) * 32; e0 < n || count > 0; e0 += step) {
+    const bool last = e0 + step >= n;
+    if (e0 < n) count = se_collect(e0, n, lane, queue, count, cls);
+    int done = 0;
+    for (; count - done >= per || (last && count > done); done += per) {
+      const bool active = g < per && done + g < count;
+      group(queue[active ? done + g : done], active, a, lane);
+    }
+    const int left = max(count - done, 0), keep = lane < left ? queue[done + lane] : 0;
+    __syncwarp();
+    if (lane < left) queue[lane] = keep;
+    count = left;
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_se(NearParams P) {
+  __shared__ int s_queue[NEAR_WARPS][64];
+  const SeArgs A{P.op, P.ro, P.ri, P.flag, P.zcell, P.zfmt, P.ldc, P.zrow, P.zcol};
+  se_walk(P.nnear, P.ro.n, s_queue[threadIdx.x >> 5], [&](int64_t e) { return P.near[e].cls; },
+          [&](int e, bool active, int a, int lane) {
+            const NearPair np_ = P.near[e];
+            const Geo t = load_geo(P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE);
+            const Geo s = load_geo(P.bgeo + (int64_t)(P.qcells ? P.qcells[np_.q] : np_.q) * GEO_STRIDE);
+            se_group<-1, -1>(A, P.tk, P.bk, active, t, s, np_.p, np_.q, a, lane);
+          });
 }
 
 // the pairs of the refines strategies (classes 5 and 6), one per warp: a kernel of their own
@@ -2664,11 +2929,19 @@ cudaError_t launch_geometry(const beast_space* s, cudaStream_t st) {
 // straight to the job's matrix (row zrow[position], column zcol[trial cell]).  Near pairs go
 // to one list for the whole batch (k_near_batch).
 template <int OPK, typename R, int FMT>
-__global__ void k_far_batch(BatchLaunch L) {
-  extern __shared__ unsigned char smraw[];
-  R* sm = reinterpret_cast<R*>(smraw);
+__global__ void __maxnreg__(80) k_far_batch(BatchLaunch L) {
+  constexpr bool F32 = std::is_same<R, float>::value;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  g64::Entry* g_tab = reinterpret_cast<g64::Entry*>(smraw);                                     // FP64
+  R* sm = reinterpret_cast<R*>(smraw + (F32 ? 0 : g64::TABLE * sizeof(g64::Entry)));
+  __shared__ float s_sc[F32 ? 256 : 1];
+  if constexpr (F32) {
+    for (int k = threadIdx.x; k < 256; k += blockDim.x) s_sc[k] = dfl::sincos_tab_dev[k & 63][k >> 6];
+  } else {
+    g64::load_table(g_tab);
+  }
   const int ni = L.ri.n, no = L.ro.n;
-  const int rec = 8 + 4 * ni;  // per trial cell: centroid hi (3) lo (3), area, near radius; points
+  const int rec = 8 + 4 * (ni + (ni & 1));  // per trial cell: centroid hi (3) lo (3), area, near radius; points
   int* s_col = reinterpret_cast<int*>(sm + (size_t)L.tile_q * rec);
   __shared__ R ro_s[3 * RULE_MAXPTS];
   for (int k = threadIdx.x; k < no; k += blockDim.x) {
@@ -2676,9 +2949,18 @@ __global__ void k_far_batch(BatchLaunch L) {
     ro_s[3 * k + 1] = (R)L.ro.v[k];
     ro_s[3 * k + 2] = (R)L.ro.w[k];
   }
-  for (int t = blockIdx.x; t < L.ntiles; t += gridDim.x) {
+  // CTAs take runs of consecutive tiles in turn: over the tiles of one job and one group of test cells the
+  // test cell's geometry (about 25 FP64 instructions per thread) stays in registers.  (One run per CTA:
+  // the jobs' tiles differ in their share of near pairs, 20.0 ms against 16.9 for 24 Helmholtz systems)
+  const int run = max(1, min(8, L.ntiles / (4 * (int)gridDim.x)));
+  BatchTile last{-1, -1, -1, 0};
+  V3<R> chp, clp, tau[3], nn;
+  R ApR = 0, radp = 0;
+  int64_t zr = -1;
+  for (int t = blockIdx.x * run; t < L.ntiles; t += (t + 1) % run ? 1 : (gridDim.x - 1) * run + 1) {
     const BatchTile tile = L.tiles[t];
-    const BatchJobDev J = L.jobs[tile.job];
+    const BatchJobDev& J = L.jobs[tile.job];
+    const g64::Wave wave{fabs(J.op.gi), J.wave_steps, J.wave_rest};
     const int nqt = (int)min((int64_t)L.tile_q, J.ncells - tile.q0);
     __syncthreads();  // the previous tile's records are no longer read
     for (int k = threadIdx.x; k < nqt * (1 + ni); k += blockDim.x) {
@@ -2697,11 +2979,18 @@ __global__ void k_far_batch(BatchLaunch L) {
       } else {
         const int bb = b - 1;
         const double u = L.ri.u[bb], v = L.ri.v[bb], w = 1.0 - u - v;
-        R* pt = r + 8 + 4 * bb;
-        pt[0] = (R)(u * (g[0] - cx) + v * (g[3] - cx) + w * (g[6] - cx));
-        pt[1] = (R)(u * (g[1] - cy) + v * (g[4] - cy) + w * (g[7] - cy));
-        pt[2] = (R)(u * (g[2] - cz) + v * (g[5] - cz) + w * (g[8] - cz));
-        pt[3] = (R)L.ri.w[bb];
+        const R x = (R)(u * (g[0] - cx) + v * (g[3] - cx) + w * (g[6] - cx));
+        const R y = (R)(u * (g[1] - cy) + v * (g[4] - cy) + w * (g[7] - cy));
+        const R z = (R)(u * (g[2] - cz) + v * (g[5] - cz) + w * (g[8] - cz));
+        if constexpr (F32 && OPK == BEAST_HH_SL) {
+          hh_sl_stage_f(r + 8, bb, ni, x, y, z, (R)L.ri.w[bb]);
+        } else {
+          R* pt = r + 8 + 4 * bb;
+          pt[0] = x;
+          pt[1] = y;
+          pt[2] = z;
+          pt[3] = (R)L.ri.w[bb];
+        }
       }
     }
     __syncthreads();
@@ -2709,18 +2998,20 @@ __global__ void k_far_batch(BatchLaunch L) {
     if (pp >= J.ncells || threadIdx.x >= L.tile_m) continue;
     const int64_t p = J.tperm[pp];
     const double* tg = J.geo + p * GEO_STRIDE;
-    const double cpx = tg[9], cpy = tg[10], cpz = tg[11];
-    const V3<R> chp = mk((R)cpx, (R)cpy, (R)cpz);
-    const V3<R> clp = mk((R)(cpx - (double)(R)cpx), (R)(cpy - (double)(R)cpy), (R)(cpz - (double)(R)cpz));
-    V3<R> tau[3];
-    for (int i = 0; i < 3; ++i)
-      tau[i] = mk((R)(tg[3 * i] - cpx), (R)(tg[3 * i + 1] - cpy), (R)(tg[3 * i + 2] - cpz));
-    const V3<R> nn = mk((R)tg[12], (R)tg[13], (R)tg[14]);
-    const R ApR = (R)tg[15];
-    const R radp = (R)J.geof[4 * p + 3];
+    if (tile.job != last.job || tile.p0 != last.p0) {
+      last = tile;
+      const double cpx = tg[9], cpy = tg[10], cpz = tg[11];
+      chp = mk((R)cpx, (R)cpy, (R)cpz);
+      clp = mk((R)(cpx - (double)(R)cpx), (R)(cpy - (double)(R)cpy), (R)(cpz - (double)(R)cpz));
+      for (int i = 0; i < 3; ++i)
+        tau[i] = mk((R)(tg[3 * i] - cpx), (R)(tg[3 * i + 1] - cpy), (R)(tg[3 * i + 2] - cpz));
+      nn = mk((R)tg[12], (R)tg[13], (R)tg[14]);
+      ApR = (R)tg[15];
+      radp = (R)J.geof[4 * p + 3];
+      zr = J.zrow[pp];
+    }
     const R gr = (R)J.op.gr, gi = (R)J.op.gi;
     const C2<R> al{(R)J.op.ar, (R)J.op.ai};
-    const int64_t zr = J.zrow[pp];
     for (int qi = 0; qi < nqt; ++qi) {
       const R* rq = sm + qi * rec;
       const V3<R> d = mk((chp.x - rq[0]) + (clp.x - rq[3]), (chp.y - rq[1]) + (clp.y - rq[4]),
@@ -2744,7 +3035,12 @@ __global__ void k_far_batch(BatchLaunch L) {
         }
       }
       const R* pts = rq + 8;
-      const V3<R> nq = mk((R)0, (R)0, (R)0);  // trial normal: only the double layer needs it
+      if constexpr (F32 && OPK == BEAST_HH_SL) {
+        store_c<R>(J.Z, o, hh_sl_far_entry_f(hh_sl_far_f(d, tau, ro_s, no, pts, ni, gr, gi, hh_sl_bound_f(d, lim, gi), s_sc),
+                                                al, ApR, rq[6]),
+                   FMT);
+        continue;
+      }
       C2<R> acc{0, 0};
       for (int a = 0; a < no; ++a) {
         const R ua = ro_s[3 * a], va = ro_s[3 * a + 1], wa3 = (R)1 - ua - va;
@@ -2753,25 +3049,45 @@ __global__ void k_far_batch(BatchLaunch L) {
                             ua * tau[0].z + va * tau[1].z + wa3 * tau[2].z);
         const R wa = ro_s[3 * a + 2];
         const V3<R> dx = d + xi;
+        C2<R> inner{0, 0};
         for (int b = 0; b < ni; ++b) {
           const R* pb = pts + 4 * b;
           const V3<R> r = dx - mk(pb[0], pb[1], pb[2]);
           const R R2 = dot(r, r);
-          const R iR = rsq<R>(R2);
-          const C2<R> G = green<R>(gr, gi, R2 * iR, iR);
-          C2<R> K;
-          if (OPK == BEAST_HH_SL) {
-            K = cmul(al, G);
-          } else {  // transposed double layer: n_x . grad G (the double layer takes the trial
-                    // normal from the geometry below)
+          if constexpr (F32) {  // transposed double layer: n_x . grad G
+            const R iR = rsq<R>(R2);
+            const C2<R> G = green<R>(gr, gi, R2 * iR, iR);
             const C2<R> c = cmul(al, cscale(iR, cmul(C2<R>{-(gr + iR), -gi}, G)));
-            K = cscale(dot(nn, r), c);
+            acc = cadd(acc, cscale(pb[3] * wa, cscale(dot(nn, r), c)));
+          } else {  // as k_far64: 4 pi G, the imaginary part times -sign(gi); gradient: -4 pi c, times it
+            const g64::Value v = g64::eval(R2, wave, g_tab);
+            double amp = pb[3] * v.iR, kr, ki;
+            if (gr != 0.0) amp *= exp(-gr * v.R);
+            if (OPK == BEAST_HH_SL) {
+              kr = v.c;
+              ki = v.s;
+            } else {
+              const double p1 = v.iR + gr;
+              amp *= v.iR * dot(nn, r);
+              kr = fma(p1, v.c, wave.k * v.s);
+              ki = fma(wave.k, v.c, -(p1 * v.s));
+            }
+            inner.re = fma(amp, kr, inner.re);
+            inner.im = fma(amp, ki, inner.im);
           }
-          acc = cadd(acc, cscale(pb[3] * wa, K));
+        }
+        if constexpr (!F32) {
+          acc.re = fma(wa, inner.re, acc.re);
+          acc.im = fma(wa, inner.im, acc.im);
         }
       }
-      (void)nq;
-      store_c<R>(J.Z, o, cscale(ApR * rq[6], acc), FMT);
+      if constexpr (F32) {
+        store_c<R>(J.Z, o, cscale(ApR * rq[6], acc), FMT);
+      } else {
+        const double f = I4PI * ApR * rq[6] * (OPK == BEAST_HH_DLT ? -1.0 : 1.0);
+        const double fi = (OPK == BEAST_HH_DLT) == (gi < 0.0) ? -f : f;  // f sign(gi) or -f sign(gi)
+        store_c<R>(J.Z, o, cmul(al, C2<R>{f * acc.re, fi * acc.im}), FMT);
+      }
     }
   }
 }
@@ -2787,41 +3103,55 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch(BatchLaunch L) {
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = min(*L.near_count, L.near_cap);
+  NearParams P;  // the fields of the job that the pair is of are set below
+  P.qs = L.qs;
+  P.tk = BEAST_P0;
+  P.bk = BEAST_P0;
+  P.qcells = nullptr;
+  P.near = nullptr;
+  P.nnear = 0;
+  P.zfmt = L.zfmt;
+  P.ss32 = P.ss64 = P.ssdf = 0;
+  P.flag = L.flag;
+  P.ro = L.ron;
+  P.ri = L.rin;
+  P.bcells = P.tcells = nullptr;  // no refines strategies in a batch
+  P.bchildren = P.tchildren = nullptr;
+  P.bnchild = P.tnchild = 0;
   for (int64_t e = blockIdx.x * (int64_t)NEAR_WARPS + warp; e < n; e += (int64_t)gridDim.x * NEAR_WARPS) {
     const NearPairB nb = L.near[e];
-    const BatchJobDev J = L.jobs[nb.job];
-    NearParams P;
+    const BatchJobDev& J = L.jobs[nb.job];
+    if (nb.cls == -1 || (L.ssdf && J.op.gr == 0.0 && nb.cls >= 1 && nb.cls <= 3)) continue;  // k_near_batch_se / _df
     P.op = J.op;
-    P.qs = L.qs;
-    P.tk = BEAST_P0;
-    P.bk = BEAST_P0;
     P.tperm = J.tperm;
     P.tgeo = J.geo;
     P.bgeo = J.geo;
-    P.qcells = nullptr;
-    P.near = nullptr;
-    P.nnear = 0;
     P.zcell = J.Z;
-    P.zfmt = L.zfmt;
-    P.ss32 = P.ss64 = 0;
     P.ldc = J.ldz;
     P.zrow = J.zrow;
     P.zcol = J.zcol;
-    P.flag = L.flag;
-    P.ro = L.ron;
-    P.ri = L.rin;
-    P.ssdf = L.ssdf && J.op.gr == 0.0;  // those pairs run in k_near_batch_df
-    P.bcells = P.tcells = nullptr;  // no refines strategies in a batch
-    P.bchildren = P.tchildren = nullptr;
-    P.bnchild = P.tnchild = 0;
     near_pair(P, NearPair{nb.p, nb.q, nb.cls, 0}, s_glx, s_glw, lane);
   }
+}
+
+// the batch's singularity-extraction pairs (se_group)
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_se(BatchLaunch L) {
+  __shared__ int s_queue[NEAR_WARPS][64];
+  se_walk(min(*L.near_count, L.near_cap), L.ron.n, s_queue[threadIdx.x >> 5], [&](int64_t e) { return L.near[e].cls; },
+          [&](int e, bool active, int a, int lane) {
+            const NearPairB nb = L.near[e];
+            const BatchJobDev& J = L.jobs[nb.job];
+            const SeArgs A{J.op, L.ron, L.rin, L.flag, J.Z, L.zfmt, J.ldz, J.zrow, J.zcol};
+            const Geo t = load_geo(J.geo + (int64_t)J.tperm[nb.p] * GEO_STRIDE);
+            const Geo s = load_geo(J.geo + (int64_t)nb.q * GEO_STRIDE);
+            se_group<BEAST_P0, BEAST_P0>(A, BEAST_P0, BEAST_P0, active, t, s, nb.p, nb.q, a, lane);
+          });
 }
 
 template <int OPK, int TK, int BK, typename R, int FMT>
 static cudaError_t far_t(const FarParams& P, cudaStream_t st) {
   dim3 grid((unsigned)((P.np + FAR_THREADS - 1) / FAR_THREADS), (unsigned)((P.nq + FAR_QT - 1) / FAR_QT));
-  size_t sm = (size_t)FAR_QT * (QREC_HDR + 4 * P.ri.n) * sizeof(R);
+  size_t sm = (size_t)FAR_QT * (QREC_HDR + 4 * (P.ri.n + (P.ri.n & 1))) * sizeof(R);
   k_far<OPK, TK, BK, R, FMT><<<grid, FAR_THREADS, sm, st>>>(P);
   return cudaGetLastError();
 }
@@ -3110,29 +3440,41 @@ static cudaError_t upload_gl(cudaStream_t st) {
 
 cudaError_t launch_far_batch(const BatchLaunch& L, cudaStream_t st) {
   if (L.ntiles == 0) return cudaSuccess;
-  const size_t sm_f = (size_t)L.tile_q * (8 + 4 * L.ri.n) * sizeof(float) + sizeof(int) * L.tile_q;
-  const size_t sm_d = (size_t)L.tile_q * (8 + 4 * L.ri.n) * sizeof(double) + sizeof(int) * L.tile_q;
+  const int rec = 8 + 4 * (L.ri.n + (L.ri.n & 1));
+  const size_t sm_f = (size_t)L.tile_q * rec * sizeof(float) + sizeof(int) * L.tile_q;
+  const size_t sm_d = g64::TABLE * sizeof(g64::Entry) + (size_t)L.tile_q * rec * sizeof(double) +
+                      sizeof(int) * L.tile_q;
   const int th = ((L.tile_m + 31) / 32) * 32;
   const bool f32 = L.precision == BEAST_MIXED;
-  if (L.op_kind == BEAST_HH_SL) {
-    if (f32) k_far_batch<BEAST_HH_SL, float, ZCELL_C64><<<L.grid_far, th, sm_f, st>>>(L);
-    else k_far_batch<BEAST_HH_SL, double, ZCELL_C128><<<L.grid_far, th, sm_d, st>>>(L);
-  } else if (L.op_kind == BEAST_HH_DLT) {
-    if (f32) k_far_batch<BEAST_HH_DLT, float, ZCELL_C64><<<L.grid_far, th, sm_f, st>>>(L);
-    else k_far_batch<BEAST_HH_DLT, double, ZCELL_C128><<<L.grid_far, th, sm_d, st>>>(L);
-  } else {
-    return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
+  auto go = [&](void (*kernel)(BatchLaunch), size_t sm) {
+    if (sm > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, th, sm);
+    kernel<<<std::max(1, std::min(L.ntiles, sm_count() * per_sm)), th, sm, st>>>(L);
+    return cudaGetLastError();
+  };
+  if (L.op_kind == BEAST_HH_SL)
+    return f32 ? go(k_far_batch<BEAST_HH_SL, float, ZCELL_C64>, sm_f) : go(k_far_batch<BEAST_HH_SL, double, ZCELL_C128>, sm_d);
+  if (L.op_kind == BEAST_HH_DLT)
+    return f32 ? go(k_far_batch<BEAST_HH_DLT, float, ZCELL_C64>, sm_f) : go(k_far_batch<BEAST_HH_DLT, double, ZCELL_C128>, sm_d);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t upload_tables(cudaStream_t st) { return upload_gl(st); }
+
+void batch_wave(BatchJobDev* j) {
+  const g64::Wave w = g64::make_wave(j->op.gi);
+  j->wave_steps = w.steps;
+  j->wave_rest = w.rest;
+}
 
 __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_df(BatchLaunch L);  // below
 
 cudaError_t launch_near_batch(const BatchLaunch& L, cudaStream_t st) {
   // the Gauss-Legendre table is uploaded before (upload_tables): this launch may be captured
-  k_near_batch<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
+  // (double-float touching pairs of real wavenumbers: k_near_batch only where there are others)
+  if (!L.ssdf || L.qs_kind == BEAST_QS_DOUBLENUM || L.complex_k) k_near_batch<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
+  if (L.qs_kind == BEAST_QS_WILTON_SAUTER) k_near_batch_se<<<L.grid_near / 4, 32 * NEAR_WARPS, 0, st>>>(L);
   if (L.ssdf) k_near_batch_df<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
   return cudaGetLastError();
 }
@@ -3178,6 +3520,76 @@ static cudaError_t ss_table(std::map<int, void*>* cache, int cls, int n, cudaStr
   return cudaSuccess;
 }
 
+// ---- nodes without their radial coordinate
+// Every Sauter-Schwab map is x - y = xi rho(eta): the radial coordinate xi only scales x, y and the
+// distance.  For the n values of xi of one node eta = (eta1, eta2, eta3) and region,
+//   sum_xi w_xi xi^3 xi^j e^{-i k xi rho} / (xi rho) = (1/rho) sum_m c_jm u^m - i k sum_m s_jm u^m,
+//   u = (k rho)^2, c_jm = (-1)^m S_{2+j+2m} / (2m)!, s_jm = (-1)^m S_{3+j+2m} / (2m+1)!, S_p = sum_xi w_xi xi^p,
+// j = 0, 1, 2 the power of xi that the shapes bring in: two polynomials take the place of n square roots,
+// sines and cosines, and the coordinates are needed once per eta.  The same rule, summed in another
+// order; 11 terms leave 1e-15 at k rho = 2 (SSP_KR), above it the kernels take node by node.
+constexpr int SSP_TERMS = 11, SSP_ROWS = 6;  // rows: c_0, c_1, c_2, -s_0, -s_1, -s_2
+constexpr int SSP_VALS = 11;                 // X0, X1, Y0, Y1, D0, D1, w, X0 Y0, X0 Y1, X1 Y0, X1 Y1
+constexpr float SSP_KR = 2.f;
+__global__ void k_ssp_coef(int n, float2* out) {
+  const int row = threadIdx.x / SSP_TERMS, m = threadIdx.x % SSP_TERMS;
+  if (row >= SSP_ROWS) return;
+  const double *x = c_gl_x + c_gl_off[n - 1], *w = c_gl_w + c_gl_off[n - 1];
+  const int p = 2 + row % 3 + row / 3 + 2 * m;
+  double c = 0.0;
+  for (int i = 0; i < n; ++i) {
+    double t = w[i];
+    for (int k = 0; k < p; ++k) t *= x[i];
+    c += t;
+  }
+  for (int k = 2; k <= 2 * m + row / 3; ++k) c /= k;
+  if ((m + row / 3) & 1) c = -c;
+  const dfl::df v = df_of(c);
+  out[threadIdx.x] = make_float2(v.hi, v.lo);
+}
+__global__ void k_ssp_table(int cls, int n, int items, float2* tab) {
+  const int it = blockIdx.x * blockDim.x + threadIdx.x;
+  if (it >= items) return;
+  const int nreg = cls == 1 ? 2 : 6, k = it / nreg, i1 = k % n, i2 = k / n % n, i3 = k / n / n;
+  const double *x = c_gl_x + c_gl_off[n - 1], *g = c_gl_w + c_gl_off[n - 1];
+  double X[2], Y[2], D[2], w;
+  ss_node_at(cls, it % nreg, 1.0, x[i3], x[i2], x[i1], g[i3] * g[i2] * g[i1], X, Y, D, &w);
+  const double v[SSP_VALS] = {X[0], X[1], Y[0], Y[1], D[0], D[1], w, X[0] * Y[0], X[0] * Y[1], X[1] * Y[0], X[1] * Y[1]};
+  for (int q = 0; q < SSP_VALS; ++q) {
+    const dfl::df p = df_of(v[q]);
+    tab[(int64_t)q * items + it] = make_float2(p.hi, p.lo);
+  }
+}
+// the tables of a strategy's three orders: coef (64 per order: 6 rows of 11 terms, padded), tab and items per class
+cudaError_t ssp_tables(std::map<int, void*>* cache, const beast_qs_desc& qs, cudaStream_t st, SspTables* T) {
+  const int ord[4] = {0, qs.ss_vert, qs.ss_edge, qs.ss_face};
+  for (int c = 1; c <= 3; ++c) {
+    const int n = ord[c];
+    T->items[c] = (c == 1 ? 2 : 6) * n * n * n;
+    for (int what = 0; what < 2; ++what) {
+      const int key = what ? 16384 + n : 8192 + 64 * c + n;
+      auto f = cache->find(key);
+      if (f == cache->end()) {
+        void* p = nullptr;
+        cudaError_t e = cudaMalloc(&p, sizeof(float2) * (what ? SSP_ROWS * SSP_TERMS : SSP_VALS * T->items[c]));
+        if (e != cudaSuccess) return e;
+        if (what)
+          k_ssp_coef<<<1, 96, 0, st>>>(n, (float2*)p);
+        else
+          k_ssp_table<<<(T->items[c] + 127) / 128, 128, 0, st>>>(c, n, T->items[c], (float2*)p);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) {
+          cudaFree(p);
+          return e;
+        }
+        f = cache->emplace(key, p).first;
+      }
+      (what ? T->coef : T->tab)[c] = (const float2*)f->second;
+    }
+  }
+  return cudaSuccess;
+}
+
 cudaError_t ss_tables(std::map<int, void*>* cache, const beast_qs_desc& qs, cudaStream_t st, const float2** tab,
                       int* items) {
   cudaError_t e = upload_gl(st);
@@ -3198,24 +3610,9 @@ DEV void dfv3(const V3<double>& a, dfl::df* o) {
   o[2] = df_of(a.z);
 }
 
-// The moment form of k_near's Sauter-Schwab path for RT x RT Maxwell pairs, every node in
-// double-float arithmetic on the FP32 pipes (GB300's FP64 pipe is a small fraction of its FP32
-// rate): one warp per pair, lanes over the nodes, x - y from the maps' own factors (D = X - Y)
-// on double-float edge vectors, 1/R by the pair reciprocal square root, exp(-ikR) from the
-// shared-memory sine table; per-lane moments as running pair sums, the warp's totals as exact
-// pair sums, the 3 x 3 block from them in FP64 (nine lanes).  Real wavenumbers (the caller
-// keeps complex ones on k_near).
-// shared vertices of a touching pair first, in the same order (SauterSchwabQuadrature.reorder):
-// lanes 0..8 test one vertex pair each (shared vertices coincide exactly), the first three
-// hits in (i, j) order from the ballot
-DEV void ss_order_warp(const Geo& t, const Geo& s, int lane, int* pt, int* ps) {
-  const double dtol = 1.0e3 * 2.220446049250313e-16;
-  bool hit = false;
-  if (lane < 9) {
-    const V3<double> dd = t.v[lane / 3] - s.v[lane % 3];
-    hit = dot(dd, dd) < dtol * dtol;
-  }
-  const unsigned hmask = __ballot_sync(0xffffffffu, hit);
+// shared vertices of a touching pair first, in the same order (SauterSchwabQuadrature.reorder), from
+// the vertex pairs that coincide (bit 3 i + j): the first three hits
+DEV void ss_order_hits(unsigned hmask, int* pt, int* ps) {
   int hits = 0, ti[3], si[3];
   for (int b = 0; b < 9; ++b)
     if (((hmask >> b) & 1u) && hits < 3) {
@@ -3238,6 +3635,16 @@ DEV void ss_order_warp(const Geo& t, const Geo& s, int lane, int* pt, int* ps) {
     if (!used) ps[k++] = j;
   }
 }
+// lanes 0..8 test one vertex pair each (shared vertices coincide exactly)
+DEV void ss_order_warp(const Geo& t, const Geo& s, int lane, int* pt, int* ps) {
+  const double dtol = 1.0e3 * 2.220446049250313e-16;
+  bool hit = false;
+  if (lane < 9) {
+    const V3<double> dd = t.v[lane / 3] - s.v[lane % 3];
+    hit = dot(dd, dd) < dtol * dtol;
+  }
+  ss_order_hits(__ballot_sync(0xffffffffu, hit), pt, ps);
+}
 
 // the warp's total of a double-float value (exact pair sums over the butterfly), as FP64
 DEV double warp_total_df(dfl::df x) {
@@ -3247,6 +3654,116 @@ DEV double warp_total_df(dfl::df x) {
     x = dfl::add(x, y);
   }
   return fsplit::f2d(x.hi) + fsplit::f2d(x.lo);
+}
+
+// the order of the shared vertices and the edges et1 = t1 - t0, et2 = t2 - t1, es1, es2 of a touching pair
+// in that order, as pairs: twelve lanes a component each (an FP64 instruction takes a warp 64 issue slots)
+DEV void ssp_edges(const double* tg, const double* sg, int lane, int* pt, int* ps, dfl::df (*e)[3]) {
+  const double dtol = 1.0e3 * 2.220446049250313e-16;
+  bool hit = false;
+  if (lane < 9) {
+    const double *a = tg + 3 * (lane / 3), *b = sg + 3 * (lane % 3);
+    const V3<double> dd = mk(a[0] - b[0], a[1] - b[1], a[2] - b[2]);
+    hit = dot(dd, dd) < dtol * dtol;
+  }
+  ss_order_hits(__ballot_sync(0xffffffffu, hit), pt, ps);
+  dfl::df v = dfl::make(0.f);
+  if (lane < 12) {
+    const int k = lane / 3, c = lane % 3;
+    const double* g = k < 2 ? tg : sg;
+    const int i1 = k == 0 ? pt[1] : k == 1 ? pt[2] : k == 2 ? ps[1] : ps[2];
+    const int i0 = k == 0 ? pt[0] : k == 1 ? pt[1] : k == 2 ? ps[0] : ps[1];
+    v = df_of(g[3 * i1 + c] - g[3 * i0 + c]);
+  }
+#pragma unroll
+  for (int k = 0; k < 12; ++k)
+    e[k / 3][k % 3] = dfl::df{__shfl_sync(0xffffffffu, v.hi, k), __shfl_sync(0xffffffffu, v.lo, k)};
+}
+// k rho <= k (longest edge at the first shared vertex of either cell, added)
+DEV float ssp_bound(const dfl::df (*e)[3], float k) {
+  float l[2];
+  for (int c = 0; c < 2; ++c) {
+    const float x = e[2 * c][0].hi, y = e[2 * c][1].hi, z = e[2 * c][2].hi;
+    const float u = x + e[2 * c + 1][0].hi, v = y + e[2 * c + 1][1].hi, w = z + e[2 * c + 1][2].hi;
+    l[c] = sqrtf(fmaxf(x * x + y * y + z * z, u * u + v * v + w * w));
+  }
+  return fabsf(k) * (l[0] + l[1]) * 1.0001f;
+}
+// x - y at a node
+DEV void ssp_diff(int cls, const dfl::df (*e)[3], const dfl::df* v, dfl::df* r) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (cls == 3)
+      r[c] = dfl::adds(dfl::mulu(v[4], e[0][c]), dfl::mulu(v[5], e[1][c]));
+    else if (cls == 2)
+      r[c] = dfl::adds(dfl::mulu(v[4], e[0][c]), dfl::subs(dfl::mulu(v[1], e[1][c]), dfl::mulu(v[3], e[3][c])));
+    else
+      r[c] = dfl::subs(dfl::adds(dfl::mulu(v[0], e[0][c]), dfl::mulu(v[1], e[1][c])),
+                       dfl::adds(dfl::mulu(v[2], e[2][c]), dfl::mulu(v[3], e[3][c])));
+  }
+}
+// sum_m c_m u^m, u <= 4: the terms from m = 5 on (below 2e-5 of the first) in FP32
+DEV dfl::df ssp_poly(const float2* c, dfl::df u) {
+  float p = c[10].x;
+#pragma unroll
+  for (int m = 9; m >= 5; --m) p = fmaf(p, u.hi, c[m].x);
+  dfl::df q = dfl::addu(dfl::df{c[4].x, c[4].y}, dfl::mulu(u, p));
+#pragma unroll
+  for (int m = 3; m >= 0; --m) q = dfl::addu(dfl::df{c[m].x, c[m].y}, dfl::mulu(u, q));
+  return q;
+}
+// totals over the warp of N values per lane (N a power of two): half the values change lanes at each step,
+// N + log2(32 / N) - 1 pair sums instead of 5 N.  Lane l ends with the total of value l * N / 32.
+template <int N>
+DEV double ssp_totals(dfl::df* m, int lane) {
+#pragma unroll
+  for (int n = N / 2, o = 16; o > 0; n >>= 1, o >>= 1) {
+    if (n > 0) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < (n > 0 ? n : 1); ++k) {
+        const dfl::df send = up ? m[k] : m[k + n], keep = up ? m[k + n] : m[k];
+        m[k] = dfl::add(keep, dfl::df{__shfl_xor_sync(0xffffffffu, send.hi, o), __shfl_xor_sync(0xffffffffu, send.lo, o)});
+      }
+    } else {
+      m[0] = dfl::add(m[0], dfl::df{__shfl_xor_sync(0xffffffffu, m[0].hi, o), __shfl_xor_sync(0xffffffffu, m[0].lo, o)});
+    }
+  }
+  return fsplit::f2d(m[0].hi) + fsplit::f2d(m[0].lo);
+}
+
+DEV void ssp_load(float2 (*coef)[SSP_ROWS * SSP_TERMS], const SspTables& T) {
+  for (int k = threadIdx.x; k < 3 * SSP_ROWS * SSP_TERMS; k += blockDim.x)
+    coef[k / (SSP_ROWS * SSP_TERMS)][k % (SSP_ROWS * SSP_TERMS)] = T.coef[1 + k / (SSP_ROWS * SSP_TERMS)][k % (SSP_ROWS * SSP_TERMS)];
+}
+
+// the Helmholtz single layer's block of a touching P0 pair from ssp_tables; false: k rho above SSP_KR.
+// coef: the order's coefficients in shared memory
+DEV bool hh_sl_ss_poly(const OpParams& op, const double* tg, const double* sg, int cls, const float2* tab, int items,
+                       const float2* coef, int lane, C2<double>* z) {
+  int pt[3], ps[3];
+  dfl::df e[4][3];
+  ssp_edges(tg, sg, lane, pt, ps, e);
+  if (!(ssp_bound(e, (float)op.gi) <= SSP_KR)) return false;
+  const dfl::df kk = df_of(op.gi), k2 = dfl::mul(kk, kk);
+  dfl::df m[2] = {dfl::make(0.f), dfl::make(0.f)};
+  for (int it = lane; it < items; it += 32) {
+    dfl::df v[7], r[3];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      const float2 f = tab[q * items + it];
+      v[q] = dfl::df{f.x, f.y};
+    }
+    ssp_diff(cls, e, v, r);
+    const dfl::df R2 = dfl::dot3u(r, r), u = dfl::mulu(k2, R2);
+    dfl::acc(m[0], dfl::mulu(dfl::mulu(dfl::rsqrtu(R2), v[6]), ssp_poly(coef, u)));
+    dfl::acc(m[1], dfl::mulu(v[6], ssp_poly(coef + 3 * SSP_TERMS, u)));
+  }
+  m[0] = dfl::norm(m[0]);
+  m[1] = dfl::norm(m[1]);
+  const double x = ssp_totals<2>(m, lane), re = __shfl_sync(0xffffffffu, x, 0), im = op.gi * __shfl_sync(0xffffffffu, x, 16);
+  *z = cscale(4.0 * I4PI * (tg[15] * sg[15]), cmul(C2<double>{op.ar, op.ai}, C2<double>{re, im}));
+  return true;
 }
 
 // The Helmholtz single layer alpha G on a touching pair of P0 / P1 cells by the Sauter-Schwab
@@ -3330,17 +3847,24 @@ template <int TP1, int BP1>
 __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_hh_df(NearParams P) {
   __shared__ float s_tab[64][4];
   for (int k = threadIdx.x; k < 256; k += blockDim.x) s_tab[k >> 2][k & 3] = dfl::sincos_tab_dev[k >> 2][k & 3];
+  constexpr bool P0 = !TP1 && !BP1;
+  __shared__ float2 s_coef[P0 ? 3 : 1][SSP_ROWS * SSP_TERMS];
+  if constexpr (P0) ssp_load(s_coef, P.ssp);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t e = blockIdx.x * (int64_t)NEAR_WARPS + warp;
   if (e >= P.nnear) return;
   const NearPair np_ = P.near[e];
   if (!near_is_ssdf(P, np_.cls)) return;
-  const Geo t = load_geo(P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE);
-  const Geo s = load_geo(P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE);
+  const double *tg = P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE, *sg = P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE;
   constexpr int NT = TP1 ? 3 : 1, NB = BP1 ? 3 : 1;
   C2<double> z[NT * NB];
-  hh_sl_ss_df<TP1, BP1>(P.op, t, s, np_.cls, P.ssdf_tab[np_.cls], P.ssdf_items[np_.cls], s_tab, lane, z);
+  bool done = false;
+  if constexpr (P0)
+    done = hh_sl_ss_poly(P.op, tg, sg, np_.cls, P.ssp.tab[np_.cls], P.ssp.items[np_.cls], s_coef[np_.cls - 1], lane, z);
+  if (!done)
+    hh_sl_ss_df<TP1, BP1>(P.op, load_geo(tg), load_geo(sg), np_.cls, P.ssdf_tab[np_.cls], P.ssdf_items[np_.cls], s_tab,
+                          lane, z);
   if (lane == 0)
     for (int i = 0; i < NT; ++i)
       for (int j = 0; j < NB; ++j)
@@ -3353,6 +3877,8 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_hh_df(NearParams P) {
 __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_df(BatchLaunch L) {
   __shared__ float s_tab[64][4];
   for (int k = threadIdx.x; k < 256; k += blockDim.x) s_tab[k >> 2][k & 3] = dfl::sincos_tab_dev[k >> 2][k & 3];
+  __shared__ float2 s_coef[3][SSP_ROWS * SSP_TERMS];
+  ssp_load(s_coef, L.ssp);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = min(*L.near_count, L.near_cap);
@@ -3360,29 +3886,106 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_df(BatchLaunch L
     const NearPairB nb = L.near[e];
     const BatchJobDev& J = L.jobs[nb.job];
     if (!(J.op.gr == 0.0 && nb.cls >= 1 && nb.cls <= 3)) continue;
-    const Geo t = load_geo(J.geo + (int64_t)J.tperm[nb.p] * GEO_STRIDE);
-    const Geo s = load_geo(J.geo + (int64_t)nb.q * GEO_STRIDE);
+    const double *tg = J.geo + (int64_t)J.tperm[nb.p] * GEO_STRIDE, *sg = J.geo + (int64_t)nb.q * GEO_STRIDE;
     C2<double> z[1];
-    hh_sl_ss_df<0, 0>(J.op, t, s, nb.cls, L.ssdf_tab[nb.cls], L.ssdf_items[nb.cls], s_tab, lane, z);
+    if (!hh_sl_ss_poly(J.op, tg, sg, nb.cls, L.ssp.tab[nb.cls], L.ssp.items[nb.cls], s_coef[nb.cls - 1], lane, z))
+      hh_sl_ss_df<0, 0>(J.op, load_geo(tg), load_geo(sg), nb.cls, L.ssdf_tab[nb.cls], L.ssdf_items[nb.cls], s_tab, lane, z);
     if (lane == 0)
       store_c<double>(J.Z, zidx(zrow_of(J.zrow, nb.p, 1, 0), zcol_of(J.zcol, nb.q, 1, 0), J.ldz), z[0], L.zfmt);
   }
 }
 
+// the EFIE's 3 x 3 block of a touching RT pair from ssp_tables; false: k rho above SSP_KR.  With x - t0 =
+// xi xa, y - s0 = xi ya (t0 = s0 the first shared vertex), tau_i = t0 - t_i and sig_j = s0 - s_j
+//   z_ij = alpha (Q + tau_i.B + sig_j.A + tau_i.sig_j M0) + 4 beta M0,
+// M0 = sum G, A = sum G xi xa, B = sum G xi ya, Q = sum G xi^2 xa.ya: twelve real sums per warp (xa and ya
+// as combinations of the cells' edges, xa.ya of the edges' products) where x and y take sixteen.
+DEV bool efie_ss_poly(const NearParams& P, const NearPair& np_, const double* tg, const double* sg, const float2* coef,
+                      int lane) {
+  int pt[3], ps[3];
+  dfl::df e[4][3];
+  ssp_edges(tg, sg, lane, pt, ps, e);
+  if (!(ssp_bound(e, (float)P.op.gi) <= SSP_KR)) return false;
+  const int cls = np_.cls, items = P.ssp.items[cls];
+  const float2* tab = P.ssp.tab[cls];
+  const dfl::df kk = df_of(P.op.gi), k2 = dfl::mul(kk, kk);
+  dfl::df g[4];  // et_i . es_j
+#pragma unroll
+  for (int q = 0; q < 4; ++q) g[q] = dfl::dot3s(e[q >> 1], e[2 + (q & 1)]);
+  dfl::df m[16];  // M0, sum X0 F1, X1 F1, Y0 F1, Y1 F1, Q as (re, im); 12 .. 15 stay 0
+#pragma unroll
+  for (int q = 0; q < 16; ++q) m[q] = dfl::make(0.f);
+#pragma unroll 1
+  for (int it = lane; it < items; it += 32) {
+    dfl::df v[SSP_VALS], r[3];
+#pragma unroll
+    for (int q = 0; q < SSP_VALS; ++q) {
+      const float2 f = tab[q * items + it];
+      v[q] = dfl::df{f.x, f.y};
+    }
+    ssp_diff(cls, e, v, r);
+    const dfl::df R2 = dfl::dot3u(r, r), u = dfl::mulu(k2, R2), wr = dfl::mulu(dfl::rsqrtu(R2), v[6]);
+    dfl::acc(m[0], dfl::mulu(wr, ssp_poly(coef, u)));
+    dfl::acc(m[1], dfl::mulu(v[6], ssp_poly(coef + 3 * SSP_TERMS, u)));
+    const dfl::df f1r = dfl::mulu(wr, ssp_poly(coef + SSP_TERMS, u)), f1i = dfl::mulu(v[6], ssp_poly(coef + 4 * SSP_TERMS, u));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      dfl::acc(m[2 + 2 * q], dfl::mulu(v[q], f1r));
+      dfl::acc(m[3 + 2 * q], dfl::mulu(v[q], f1i));
+    }
+    dfl::df d = dfl::mulu(v[7], g[0]);
+#pragma unroll
+    for (int q = 1; q < 4; ++q) dfl::acc(d, dfl::mulu(v[7 + q], g[q]));
+    dfl::acc(m[10], dfl::mulu(d, dfl::mulu(wr, ssp_poly(coef + 2 * SSP_TERMS, u))));
+    dfl::acc(m[11], dfl::mulu(d, dfl::mulu(v[6], ssp_poly(coef + 5 * SSP_TERMS, u))));
+  }
+#pragma unroll
+  for (int q = 0; q < 12; ++q) m[q] = dfl::norm(m[q]);
+  const double x = ssp_totals<16>(m, lane) * (lane & 2 ? I4PI * P.op.gi : I4PI);  // odd values: imaginary parts
+  C2<double> S[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) S[q] = C2<double>{__shfl_sync(0xffffffffu, x, 4 * q), __shfl_sync(0xffffffffu, x, 4 * q + 2)};
+  if (lane < 9) {
+    const int i = lane / 3, j = lane % 3;
+    auto vert = [](const double* c, int k) { return mk(c[3 * k], c[3 * k + 1], c[3 * k + 2]); };
+    const V3<double> t0 = vert(tg, pt[0]), t1 = vert(tg, pt[1]), t2 = vert(tg, pt[2]), s0 = vert(sg, ps[0]),
+                     s1 = vert(sg, ps[1]), s2 = vert(sg, ps[2]);
+    const V3<double> ti = t0 - vert(tg, i), sj = s0 - vert(sg, j);
+    C2<double> f = cadd(S[5], cscale(dot(ti, sj), S[0]));
+    f = cadd(f, cadd(cscale(dot(sj, t1 - t0), S[1]), cscale(dot(sj, t2 - t1), S[2])));
+    f = cadd(f, cadd(cscale(dot(ti, s1 - s0), S[3]), cscale(dot(ti, s2 - s1), S[4])));
+    const C2<double> al{P.op.ar, P.op.ai}, be{P.op.br, P.op.bi};
+    store_c<double>(P.zcell, zidx(zrow_of(P.zrow, np_.p, 3, i), zcol_of(P.zcol, np_.q, 3, j), P.ldc),
+                    cadd(cmul(al, f), cscale(4.0, cmul(be, S[0]))), P.zfmt);
+  }
+  return true;
+}
+
+// The moment form of k_near's Sauter-Schwab path for RT x RT Maxwell pairs, every node in
+// double-float arithmetic on the FP32 pipes (GB300's FP64 pipe is a small fraction of its FP32
+// rate): one warp per pair, lanes over the nodes, x - y from the maps' own factors (D = X - Y)
+// on double-float edge vectors, 1/R by the pair reciprocal square root, exp(-ikR) from the
+// shared-memory sine table; per-lane moments as running pair sums, the warp's totals as exact
+// pair sums, the 3 x 3 block from them in FP64 (nine lanes).  Real wavenumbers (the caller
+// keeps complex ones on k_near).
 // five CTAs per SM (96 registers, a few spilled): measured 9.9 -> 9.6 ms per C2 solve against
 // four CTAs at 128 registers
 template <bool SL>
 __global__ void __launch_bounds__(32 * NEAR_WARPS, 5) k_near_ss_df(NearParams P) {
   __shared__ float s_tab[64][4];  // sin / cos(m pi/32)
   for (int k = threadIdx.x; k < 256; k += blockDim.x) s_tab[k >> 2][k & 3] = dfl::sincos_tab_dev[k >> 2][k & 3];
+  __shared__ float2 s_coef[SL ? 3 : 1][SSP_ROWS * SSP_TERMS];
+  if constexpr (SL) ssp_load(s_coef, P.ssp);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t e = blockIdx.x * (int64_t)NEAR_WARPS + warp;
   if (e >= P.nnear) return;
   const NearPair np_ = P.near[e];
   if (!near_is_ssdf(P, np_.cls)) return;
-  const Geo t = load_geo(P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE);
-  const Geo s = load_geo(P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE);
+  const double *tg = P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE, *sg = P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE;
+  if constexpr (SL)
+    if (efie_ss_poly(P, np_, tg, sg, s_coef[np_.cls - 1], lane)) return;
+  const Geo t = load_geo(tg), s = load_geo(sg);
   int pt[3], ps[3];
   ss_order_warp(t, s, lane, pt, ps);
   const int cls = np_.cls;
@@ -3777,6 +4380,7 @@ cudaError_t launch_near(const AsmArgs& a, int nnear, const TriRuleDev& ro, const
   }
   if (P.ssdf) {
     e = ss_tables(a.ss_tabs, a.qs, st, P.ssdf_tab, P.ssdf_items);
+    if (e == cudaSuccess) e = ssp_tables(a.ss_tabs, a.qs, st, &P.ssp);
     if (e != cudaSuccess) return e;
   }
   // every other Sauter-Schwab pair of the operators on RT (not n x K) and P0 / P1
@@ -3818,10 +4422,14 @@ cudaError_t launch_near(const AsmArgs& a, int nnear, const TriRuleDev& ro, const
     e = launch_near_ss64(P, st);
     if (e != cudaSuccess) return e;
   }
-  // (DoubleNumSauterQstrat lists touching pairs only: nothing is left for k_near then)
-  if (!(P.ss64 && P.qs.kind == BEAST_QS_SAUTER)) k_near<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
-  if (P.qs.kind == BEAST_QS_TEST_REFINES_TRIAL || P.qs.kind == BEAST_QS_TRIAL_REFINES_TEST)
-    k_near_refines<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
+  // k_near: the point-by-point pairs of DoubleNumQStrat and the touching pairs no other kernel takes
+  const bool refines = P.qs.kind == BEAST_QS_TEST_REFINES_TRIAL || P.qs.kind == BEAST_QS_TRIAL_REFINES_TEST;
+  const bool rt_sl = rt && a.op.kind == BEAST_MW_SL;  // (a double layer's common faces: zero blocks, k_near)
+  if (P.qs.kind == BEAST_QS_DOUBLENUM || refines || !(P.ss64 || (P.ssdf && (hh_sl || rt_sl)) || (P.ss32 && rt_sl)))
+    k_near<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
+  if (P.qs.kind == BEAST_QS_WILTON_SAUTER || refines)
+    k_near_se<<<std::min((nnear + 32 * NEAR_WARPS - 1) / (32 * NEAR_WARPS), 2 * sm_count()), 32 * NEAR_WARPS, 0, st>>>(P);
+  if (refines) k_near_refines<<<blocks, 32 * NEAR_WARPS, 0, st>>>(P);
   return cudaGetLastError();
 }
 

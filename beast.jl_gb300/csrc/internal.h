@@ -238,13 +238,23 @@ struct BatchJobDev {
   int64_t ncells;
   void* Z;             // the job's matrix (column-major, ld ldz)
   int64_t ldz;
+  double wave_steps;   // the wavenumber as green64.h takes it (batch_wave)
+  float wave_rest;
 };
+void batch_wave(BatchJobDev* j);
 struct BatchTile {
   int job, p0, q0, pad;  // test positions p0 .. p0 + tile_m, trial cells q0 .. q0 + tile_q
 };
 struct NearPairB {
   int job, p, q, cls;
 };
+// node tables of the Sauter-Schwab rules without their radial coordinate, per class 1..3 (k_ssp_table)
+struct SspTables {
+  const float2* tab[4] = {};
+  const float2* coef[4] = {};
+  int items[4] = {};
+};
+cudaError_t ssp_tables(std::map<int, void*>* cache, const beast_qs_desc& qs, cudaStream_t st, SspTables* T);
 struct BatchLaunch {
   const BatchJobDev* jobs;
   const BatchTile* tiles;
@@ -264,7 +274,9 @@ struct BatchLaunch {
   // single-layer Sauter-Schwab pairs in double-float (not on the FP64 path): node tables per
   // class 1..3 (ss_tables)
   int ssdf = 0;
+  int complex_k = 0;            // a job has a complex wavenumber
   const float2* ssdf_tab[4] = {nullptr, nullptr, nullptr, nullptr};
+  SspTables ssp;
   int ssdf_items[4] = {0, 0, 0, 0};
 };
 // the double-float Sauter-Schwab node tables of the strategy's orders (class 1..3: vertex,

@@ -1,0 +1,100 @@
+"""GPU: the pair kernels where their routes part -- singularity-extraction pairs several per warp, the
+FP32 far pairs of the Helmholtz single layer (packed points; odd point counts, complex and very large
+wavenumbers), touching pairs summed over their radial coordinate (k rho up to 2) or node by node (above),
+and the pair classification without FP64 instructions."""
+import numpy as np
+import pytest
+
+import beastgpu as bg
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+WS = bg.DoubleNumWiltonSauterQStrat
+
+
+def _mesh(level=1, seed=3):
+    return bg.ellipsoid(level, (1.0, 0.8, 1.3), perturb=0.02, rng=seed)
+
+
+@pytest.mark.parametrize("outer,inner", [(1, 1), (2, 3), (4, 2), (5, 5), (7, 3), (10, 6)])
+@pytest.mark.parametrize("kind", ["p0", "rt"])
+def test_singularity_extraction(kind, outer, inner):
+    """1 to 25 outer points: 32 pairs per warp to one; the FP64 contract against the oracle, 1e-10 with a
+    floor of 1e-3 of the largest entry"""
+    m = _mesh()
+    X = bg.lagrangecxd0(m) if kind == "p0" else bg.raviartthomas(m)
+    op = (bg.Helmholtz3D if kind == "p0" else bg.Maxwell3D).singlelayer(wavenumber=0.7)
+    qs = WS(2, 3, outer, inner, 3, 3, 3, 3)
+    for Y in (X, X.subset(np.arange(1))):
+        Z = bg.assemble(op, Y, X, quadstrat=qs, precision=bg.FP64)
+        Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), Y, X)
+        err = np.abs(Z - Zo) / (np.abs(Zo) + 1e-3 * np.abs(Zo).max())
+        assert err.max() < 1e-10
+
+
+@pytest.mark.parametrize("gamma", [2j, -3j, 0.4 + 2j, 0.0, 60j, 2e4j])
+@pytest.mark.parametrize("far", [(1, 1), (2, 3), (3, 5), (4, 7)])
+def test_fp32_far_pairs(far, gamma):
+    """a point's phase |gamma| R carries a few FP32 roundings, the rest of its term a dozen: 2^-24 (12 + 4
+    |gamma| R) of the sum of the terms' sizes, which the static kernel's entry is"""
+    X = bg.lagrangecxd0(_mesh(level=2))
+    H, qs = bg.Helmholtz3D.singlelayer, WS(far[0], far[1], 2, 3, 4, 4, 4, 4)
+    Z = bg.assemble(H(gamma=gamma), X, X, quadstrat=qs, precision=bg.MIXED)
+    Zr = bg.assemble(H(gamma=gamma), X, X, quadstrat=qs, precision=bg.FP64)
+    Zs = bg.assemble(H(gamma=0.0), X, X, quadstrat=qs, precision=bg.FP64).real
+    assert np.all(np.abs(Z - Zr) <= 2.0**-24 * (12 + 4 * abs(gamma) * 2.7) * Zs)
+
+
+@pytest.mark.parametrize("precision", [bg.MIXED, bg.FP64])
+@pytest.mark.parametrize("kind", ["sl", "dlt"])
+def test_batch_of_one_small_tile(kind, precision):
+    """the batch's kernels against the per-mesh ones: runs of tiles that end in the middle of a mesh"""
+    ms = [_mesh(level, seed) for level, seed in ((0, 1), (2, 2), (1, 3), (2, 4))]
+    H = bg.Helmholtz3D
+    make = H.singlelayer if kind == "sl" else H.doublelayer_transposed
+    spaces, ops = [bg.lagrangecxd0(m) for m in ms], [make(gamma=g) for g in (1j, 0.3 + 2j, -4j, 0.0)]
+    b = bg.Batch(ops, spaces, precision=precision, tile_m=32, tile_q=5)
+    try:
+        Zs = [Z.cpu().numpy() for Z in b.assemble()]
+    finally:
+        b.close()
+    tol = 1e-13 if precision == bg.FP64 else 2.0**-21  # a few FP32 roundings of a far entry
+    for op, X, Z in zip(ops, spaces, Zs):
+        ref = bg.assemble(op, X, X, precision=precision)
+        assert np.abs(Z - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("k", [0.0, 0.3, -2.0, 2.5, 6.0])
+@pytest.mark.parametrize("orders", [(1, 1, 1), (2, 3, 5), (4, 4, 4), (7, 5, 6)])
+@pytest.mark.parametrize("kind", ["p0", "rt"])
+def test_radial_sums(kind, orders, k):
+    """pair arithmetic's sine (1e-11) bounds a node's error; a Maxwell entry adds blocks that are up to ten
+    times its size"""
+    m = _mesh()
+    X = bg.lagrangecxd0(m) if kind == "p0" else bg.raviartthomas(m)
+    if kind == "p0":
+        op = bg.Helmholtz3D.singlelayer(gamma=1j * k)
+    else:
+        op = bg.Maxwell3D.singlelayer(gamma=1j * k, alpha=-1.3j, beta=0.7)
+    qs = WS(2, 3, 2, 3, orders[0], orders[1], orders[2], 3)
+    Z = bg.assemble(op, X, X, quadstrat=qs, precision=bg.MIXED_ACCURATE)
+    Zr = bg.assemble(op, X, X, quadstrat=qs, precision=bg.FP64)
+    assert np.abs(Z - Zr).max() <= (1e-11 if kind == "p0" else 1e-10) * np.abs(Zr).max()
+
+
+def test_classification():
+    """vertices that are shared to rounding only, and meshes far from size one, are classified as before:
+    the assembly scales, and does not change with the last bits of the vertices"""
+    m = _mesh()
+    H = bg.Helmholtz3D.singlelayer
+    Z = bg.assemble(H(wavenumber=2.0), bg.lagrangecxd0(m), bg.lagrangecxd0(m), precision=bg.FP64)
+    rng = np.random.default_rng(1)
+    v = m.vertices[m.cells].reshape(-1, 3)
+    loose = bg.Mesh(v * (1.0 + 1e-15 * rng.integers(-1, 2, v.shape)), np.arange(len(v)).reshape(-1, 3))
+    X = bg.lagrangecxd0(loose)
+    assert np.abs(bg.assemble(H(wavenumber=2.0), X, X, precision=bg.FP64) - Z).max() <= 1e-12 * np.abs(Z).max()
+    for e in (-30, -20, 25):
+        X = bg.lagrangecxd0(bg.Mesh(np.ldexp(m.vertices, e), m.cells))
+        Zs = bg.assemble(H(wavenumber=np.ldexp(2.0, -e)), X, X, precision=bg.FP64)
+        assert np.abs(np.ldexp(Zs.real, -3 * e) + 1j * np.ldexp(Zs.imag, -3 * e) - Z).max() <= 1e-12 * np.abs(Z).max()
