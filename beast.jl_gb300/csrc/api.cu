@@ -309,6 +309,7 @@ int beast_mesh_upload(beast_ctx* ctx, const double* verts, int64_t nv, const int
   m->ctx = ctx;
   m->nv = nv;
   m->nc = nc;
+  double lmin = 1e300, lmax = 0.0;
   for (int64_t i = 0; i < nc; ++i) {
     const double *a = verts + 3 * (int64_t)c[3 * i], *b = verts + 3 * (int64_t)c[3 * i + 1], *g = verts + 3 * (int64_t)c[3 * i + 2];
     double r2 = 0.0;
@@ -317,7 +318,16 @@ int beast_mesh_upload(beast_ctx* ctx, const double* verts, int64_t nv, const int
       r2 += (a[k] - z) * (a[k] - z) + (b[k] - z) * (b[k] - z) + (g[k] - z) * (g[k] - z);
     }
     m->radius += std::sqrt(r2 / 3.0) / nc;
+    const double* v[3] = {a, b, g};
+    for (int s = 0; s < 3; ++s) {
+      double l2 = 0.0;
+      for (int k = 0; k < 3; ++k) l2 += (v[s][k] - v[(s + 1) % 3][k]) * (v[s][k] - v[(s + 1) % 3][k]);
+      lmin = std::min(lmin, l2);
+      lmax = std::max(lmax, l2);
+    }
   }
+  m->edge_min = std::sqrt(lmin);
+  m->edge_max = nc > 0 ? std::sqrt(lmax) : 1e300;
   cudaError_t e = cudaMalloc(&m->verts, sizeof(double) * 3 * nv);
   if (e == cudaSuccess) e = cudaMalloc(&m->cells, sizeof(int) * 3 * nc);
   if (e == cudaSuccess) e = cudaMemcpyAsync(m->verts, verts, sizeof(double) * 3 * nv, cudaMemcpyHostToDevice, ctx->stream);

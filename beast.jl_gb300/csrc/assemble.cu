@@ -1532,6 +1532,10 @@ struct NearParams {
   int ssdf;  // Sauter-Schwab pairs of RT Maxwell operators in double-float (k_near_ss_df)
   const float2* ssdf_tab[4];  // per class 1..3: node table [7][items] (ss_table)
   SspTables ssp;               // the same without the radial coordinate (k_ssp_table)
+  int ssx;                     // k_near_ssx takes k_near_ss64's pairs
+  const double* ssx_tab[4];
+  const int64_t* ssx_coef[4];
+  int ssx_items[4];
   int ssdf_items[4];
   int ss64;  // Sauter-Schwab pairs in k_near_ss64
   const double* ss64_tab[4];  // per class 1..3: node table [SS64_VALS][items]
@@ -4143,6 +4147,64 @@ __global__ void k_ss64_table(int cls, int n, int items, double* tab) {
     for (int k = 0; k < 3; ++k) tab[(int64_t)(4 + 3 * m + k) * items + it] = w * lx[m] * ly[k];
 }
 
+// the block of a touching pair from its moments over (1, X0, X1) (1, Y0, Y1), tot_[2 (NB m + n)] re and im (the
+// sums of k_near_ss64's kr, ki); a shape pair per lane, T_ scratch of the warp
+template <int OPK, int TK, int BK>
+DEV void ss64_block(const NearParams& P, const NearPair& np_, int lane, const int* pt, const int* ps, const double* tg,
+                    const double* sgeo, const double* tot_, C2<double>* T_) {
+  constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL;
+  constexpr bool GRAD = OPK != BEAST_MW_SL && OPK != BEAST_HH_SL;
+  constexpr int NT = TK == BEAST_P0 ? 1 : 3, NB = BK == BEAST_P0 ? 1 : 3, NM = NT * NB;
+  const double sg = P.op.gi < 0.0 ? -1.0 : 1.0;
+  auto vert = [](const double* g, int k) { return mk(g[3 * k], g[3 * k + 1], g[3 * k + 2]); };
+  const V3<double> A0 = vert(tg, pt[0]), A1 = vert(tg, pt[1]), A2 = vert(tg, pt[2]);
+  const V3<double> B0 = vert(sgeo, ps[0]), B1 = vert(sgeo, ps[1]), B2 = vert(sgeo, ps[2]);
+  // (1, X0, X1) -> barycentric (1 - X0, X0 - X1, X1) on both cells, a shape pair per lane
+  const int m_ = lane / NB, n_ = lane % NB;
+  if (lane < NM) {
+    auto tot = [&](int m, int n) { return C2<double>{tot_[2 * (m * NB + n)], tot_[2 * (m * NB + n) + 1]}; };
+    auto row = [&](int m) {
+      return NB == 3 && n_ < 2 ? csub(tot(m, n_), tot(m, n_ + 1)) : tot(m, n_);
+    };
+    C2<double> T = row(m_);
+    if (NT == 3 && m_ < 2) T = csub(T, row(m_ + 1));
+    T_[lane] = T;
+  }
+  __syncwarp();
+  if (lane < NM) {
+    const int i = NT == 3 ? pt[m_] : 0, j = NB == 3 ? ps[n_] : 0;
+    C2<double> z;
+    if (!RT) {
+      const double c = I4PI * 4.0 * tg[15] * sgeo[15] * (OPK == BEAST_HH_DLT ? -1.0 : 1.0);
+      const C2<double> T = T_[lane];
+      z = cmul(C2<double>{P.op.ar, P.op.ai}, C2<double>{c * T.re, c * (GRAD ? sg : -sg) * T.im});
+    } else {
+      double fr = 0.0, fi = 0.0;
+      auto tv = [&](int m) { return m == 0 ? A0 : (m == 1 ? A1 : A2); };
+      auto sv = [&](int n) { return n == 0 ? B0 : (n == 1 ? B1 : B2); };
+      const V3<double> ti = tv(m_), sj = sv(n_);
+#pragma unroll
+      for (int dm = 1; dm < 3; ++dm)
+#pragma unroll
+        for (int dn = 1; dn < 3; ++dn) {
+          const int m = (m_ + dm) % 3, n = (n_ + dn) % 3;
+          const V3<double> em = tv(m) - ti, en = sv(n) - sj;
+          const double w = OPK == BEAST_MW_SL ? dot(em, en) : dot(em, cross(tv(m) - sv(n), en));
+          const C2<double> T = T_[3 * m + n];
+          fr = fma(w, T.re, fr);
+          fi = fma(w, T.im, fi);
+        }
+      if (OPK == BEAST_MW_SL) {
+        const C2<double> f{I4PI * fr, -sg * I4PI * fi}, m0{4.0 * I4PI * tot_[0], -sg * 4.0 * I4PI * tot_[1]};
+        z = cadd(cmul(C2<double>{P.op.ar, P.op.ai}, f), cmul(C2<double>{P.op.br, P.op.bi}, m0));
+      } else {
+        z = C2<double>{-I4PI * fr, -I4PI * sg * fi};
+      }
+    }
+    store_c<double>(P.zcell, zidx(zrow_of(P.zrow, np_.p, NT, i), zcol_of(P.zcol, np_.q, NB, j), P.ldc), z, P.zfmt);
+  }
+}
+
 template <int OPK, int TK, int BK, int PPC>
 __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
   constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL;
@@ -4155,7 +4217,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
   g64::load_table(tab);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double gr = P.op.gr, sg = P.op.gi < 0.0 ? -1.0 : 1.0;
+  const double gr = P.op.gr;
   for (int step = 0; step < 2 * PPC; ++step) {
     const int64_t e = blockIdx.x * (int64_t)PPC + step % PPC;
     if (e >= P.nnear) continue;
@@ -4165,8 +4227,8 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
     const int items = P.ss64_items[cls];
     const bool heavy = items >= SS64_HEAVY;  // uniform over the CTA
     if (heavy != (step < PPC) || (!heavy && warp != step % PPC)) continue;
-    const Geo t = load_geo(P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE);
-    const Geo s = load_geo(P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE);
+    const double *tg = P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE, *sgeo = P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE;
+    const Geo t = load_geo(tg), s = load_geo(sgeo);
     int pt[3], ps[3];
     ss_order_warp(t, s, lane, pt, ps);
     const V3<double> A0 = t.v[pt[0]], A1 = t.v[pt[1]], A2 = t.v[pt[2]];
@@ -4237,56 +4299,268 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
       if (warp > 0) continue;  // (its own rows of s_red and s_tot are read by no other warp)
     }
     __syncwarp();
-    // (1, X0, X1) -> barycentric (1 - X0, X0 - X1, X1) on both cells, a shape pair per lane
-    const int m_ = lane / NB, n_ = lane % NB;
-    if (lane < NM) {
-      auto tot = [&](int m, int n) { return C2<double>{s_tot[warp][2 * (m * NB + n)], s_tot[warp][2 * (m * NB + n) + 1]}; };
-      auto row = [&](int m) {
-        return NB == 3 && n_ < 2 ? csub(tot(m, n_), tot(m, n_ + 1)) : tot(m, n_);
-      };
-      C2<double> T = row(m_);
-      if (NT == 3 && m_ < 2) T = csub(T, row(m_ + 1));
-      s_T[warp][lane] = T;
-    }
-    __syncwarp();
-    if (lane < NM) {
-      const int i = NT == 3 ? pt[m_] : 0, j = NB == 3 ? ps[n_] : 0;
-      C2<double> z;
-      if (!RT) {
-        const double c = I4PI * 4.0 * t.area * s.area * (OPK == BEAST_HH_DLT ? -1.0 : 1.0);
-        const C2<double> T = s_T[warp][lane];
-        z = cmul(C2<double>{P.op.ar, P.op.ai}, C2<double>{c * T.re, c * (GRAD ? sg : -sg) * T.im});
-      } else {
-        double fr = 0.0, fi = 0.0;
-        auto tv = [&](int m) { return m == 0 ? A0 : (m == 1 ? A1 : A2); };
-        auto sv = [&](int n) { return n == 0 ? B0 : (n == 1 ? B1 : B2); };
-        const V3<double> ti = tv(m_), sj = sv(n_);
-#pragma unroll
-        for (int dm = 1; dm < 3; ++dm)
-#pragma unroll
-          for (int dn = 1; dn < 3; ++dn) {
-            const int m = (m_ + dm) % 3, n = (n_ + dn) % 3;
-            const V3<double> em = tv(m) - ti, en = sv(n) - sj;
-            const double w = OPK == BEAST_MW_SL ? dot(em, en) : dot(em, cross(tv(m) - sv(n), en));
-            const C2<double> T = s_T[warp][3 * m + n];
-            fr = fma(w, T.re, fr);
-            fi = fma(w, T.im, fi);
-          }
-        if (OPK == BEAST_MW_SL) {
-          const C2<double> f{I4PI * fr, -sg * I4PI * fi}, m0{4.0 * I4PI * s_tot[warp][0], -sg * 4.0 * I4PI * s_tot[warp][1]};
-          z = cadd(cmul(C2<double>{P.op.ar, P.op.ai}, f), cmul(C2<double>{P.op.br, P.op.bi}, m0));
-        } else {
-          z = C2<double>{-I4PI * fr, -I4PI * sg * fi};
-        }
-      }
-      store_c<double>(P.zcell, zidx(zrow_of(P.zrow, np_.p, NT, i), zcol_of(P.zcol, np_.q, NB, j), P.ldc), z, P.zfmt);
-    }
+    ss64_block<OPK, TK, BK>(P, np_, lane, pt, ps, tg, sgeo, s_tot[warp], s_T[warp]);
     __syncwarp();  // s_red, s_tot and s_T are written again by the next pair
   }
 }
 
+// ---- the same pairs without the radial coordinate (the formulas above k_ssp_coef), FP64
+// Per node eta the distance vector, its square and 1/rho in FP64 (about 20 instructions for the n nodes of
+// k_near_ss64, 36 .. 48 each); the polynomials in u = (k rho)^2, their products with a = w / rho^p and the
+// moments over the coordinates' products in 64-bit integers.  With the gradient the radial sums are those
+// of (cos t + t sin t, t cos t - sin t), t = k xi rho:
+//   G        re w / rho    c_jm = (-1)^m S_{2+j+2m} / (2m)!             im k w        (-1)^m S_{3+j+2m} / (2m+1)!
+//   grad G   re w / rho^3  c_jm = (-1)^m (1-2m) S_{j+2m} / (2m)!        im k w / rho^2  (-1)^m 2m S_{1+j+2m} / (2m+1)!
+// (one more power of xi with the double layers' factor n . rho).  Both sums of |a| over the pair's nodes,
+// taken first in FP32, set the integers' scales; integer sums do not depend on their order, so a pair may
+// be one warp's or four's.  12 terms leave 1e-17 at k rho = 2; the host takes this kernel where
+// k (longest test edge + longest trial edge) <= 2, and k_near_ss64 elsewhere.  Measured: EFIE, 43,900
+// pairs at orders 5, 5, 4: 4.57 -> 2.04 ms; double layer on P1, 75,100 pairs at order 4: 7.56 -> 2.70.
+constexpr int SSX_TERMS = 12, SSX_ROWS = 6;
+// table rows: k_ss64_table's four coordinates at xi = 1, the weight without w_xi xi^3; X0, X1, Y0, Y1, X0 Y0,
+// X0 Y1, X1 Y0, X1 Y1 as integers; after them the first five in FP32
+constexpr int SSX_VALS = 13;
+__global__ void k_ssx_table(int cls, int n, int items, double* tab) {
+  const int it = blockIdx.x * blockDim.x + threadIdx.x;
+  if (it >= items) return;
+  const int nreg = cls == 1 ? 2 : 6, k = it / nreg, i1 = k % n, i2 = k / n % n, i3 = k / n / n;
+  const double *x = c_gl_x + c_gl_off[n - 1], *g = c_gl_w + c_gl_off[n - 1];
+  double X[2], Y[2], D[2], w;
+  ss_node_at(cls, it % nreg, 1.0, x[i3], x[i2], x[i1], g[i3] * g[i2] * g[i1], X, Y, D, &w);
+  const double co[5] = {cls == 1 ? X[0] : D[0], cls == 3 ? D[1] : X[1], cls == 1 ? Y[0] : 0.0, cls == 3 ? 0.0 : Y[1], w};
+  const double p[8] = {X[0], X[1], Y[0], Y[1], X[0] * Y[0], X[0] * Y[1], X[1] * Y[0], X[1] * Y[1]};
+  float* tabf = reinterpret_cast<float*>(tab + (int64_t)SSX_VALS * items);
+  for (int q = 0; q < 5; ++q) {
+    tab[(int64_t)q * items + it] = co[q];
+    tabf[(int64_t)q * items + it] = (float)co[q];
+  }
+  for (int q = 0; q < 8; ++q)
+    tab[(int64_t)(5 + q) * items + it] = __longlong_as_double(p[q] >= 1.0 ? (int64_t)1 << 62 : g64::to_fixed(p[q], 0));
+}
+// kind 0: G, 1: grad G, 2: grad G with one more power of xi; coefficients of (u / 4)^m
+__global__ void k_ssx_coef(int n, int kind, int64_t* out) {
+  const int row = threadIdx.x / SSX_TERMS, m = threadIdx.x % SSX_TERMS, im = row / 3;
+  if (row >= SSX_ROWS) return;
+  const double *x = c_gl_x + c_gl_off[n - 1], *w = c_gl_w + c_gl_off[n - 1];
+  const int p = (kind == 0 ? 2 : kind - 1) + row % 3 + im + 2 * m;
+  double c = 0.0;
+  for (int i = 0; i < n; ++i) {
+    double t = w[i];
+    for (int k = 0; k < p; ++k) t *= x[i];
+    c += t;
+  }
+  for (int k = 2; k <= 2 * m + im; ++k) c /= k;
+  for (int k = 0; k < m; ++k) c *= 4.0;
+  if (kind) c *= im ? 2 * m : 1 - 2 * m;
+  if (m & 1) c = -c;
+  out[threadIdx.x] = fabs(c) >= 1.0 ? (c < 0 ? -1 : 1) * ((int64_t)1 << 62) : g64::to_fixed(c, 0);
+}
+DEV int64_t ssx_poly(const int64_t* c, int64_t u) {
+  int64_t q = c[SSX_TERMS - 1];
+#pragma unroll
+  for (int m = SSX_TERMS - 2; m >= 0; --m) q = c[m] + (g64::mulhi(u, q) << 2);
+  return q;
+}
+DEV double shfl_d(double x, int lane) { return __shfl_sync(0xffffffffu, x, lane); }
+
+// W: warps per pair, 4 while there are fewer pairs than eight per SM
+template <int OPK, int TK, int BK, int W>
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
+  constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL;
+  constexpr bool GRAD = OPK != BEAST_MW_SL && OPK != BEAST_HH_SL;
+  constexpr int NT = TK == BEAST_P0 ? 1 : 3, NB = BK == BEAST_P0 ? 1 : 3, NM = NT * NB;
+  constexpr int NJ = (NT > 1) + (NB > 1) + 1;  // powers of xi
+  __shared__ int64_t s_coef[3][SSX_ROWS * SSX_TERMS];
+  __shared__ int64_t s_red[NEAR_WARPS][2 * NM][33], s_sum[NEAR_WARPS][2 * NM];
+  __shared__ double s_tot[NEAR_WARPS][2 * NM];
+  __shared__ C2<double> s_T[NEAR_WARPS][NM];
+  for (int k = threadIdx.x; k < 3 * SSX_ROWS * SSX_TERMS; k += blockDim.x)
+    s_coef[k / (SSX_ROWS * SSX_TERMS)][k % (SSX_ROWS * SSX_TERMS)] =
+        P.ssx_coef[1 + k / (SSX_ROWS * SSX_TERMS)][k % (SSX_ROWS * SSX_TERMS)];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t e = W == 1 ? blockIdx.x * (int64_t)NEAR_WARPS + warp : blockIdx.x;
+  if (e >= P.nnear) return;
+  const NearPair np_ = P.near[e];
+  const int cls = np_.cls;
+  if (cls < 1 || cls > 3 || (cls == 3 && dl_type(OPK))) return;  // other paths / identically zero
+  const double *tg = P.tgeo + (int64_t)P.tperm[np_.p] * GEO_STRIDE, *sgeo = P.bgeo + (int64_t)P.qcells[np_.q] * GEO_STRIDE;
+  // shared vertices first, and the edges et1, et2, es1, es2: a component per lane
+  int pt[3], ps[3];
+  V3<double> E[4];
+  {
+    const double dtol = 1.0e3 * 2.220446049250313e-16;
+    bool hit = false;
+    if (lane < 9) {
+      const double *a = tg + 3 * (lane / 3), *b = sgeo + 3 * (lane % 3);
+      const V3<double> dd = mk(a[0] - b[0], a[1] - b[1], a[2] - b[2]);
+      hit = dot(dd, dd) < dtol * dtol;
+    }
+    ss_order_hits(__ballot_sync(0xffffffffu, hit), pt, ps);
+    double v = 0.0;
+    if (lane < 12) {
+      const int k = lane / 3, c = lane % 3;
+      const double* g = k < 2 ? tg : sgeo;
+      const int i1 = k == 0 ? pt[1] : k == 1 ? pt[2] : k == 2 ? ps[1] : ps[2];
+      const int i0 = k == 0 ? pt[0] : k == 1 ? pt[1] : k == 2 ? ps[0] : ps[1];
+      v = g[3 * i1 + c] - g[3 * i0 + c];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) E[k] = mk(shfl_d(v, 3 * k), shfl_d(v, 3 * k + 1), shfl_d(v, 3 * k + 2));
+  }
+  const int items = P.ssx_items[cls];
+  const double* nodes = P.ssx_tab[cls];
+  const float* tabf = reinterpret_cast<const float*>(nodes + (int64_t)SSX_VALS * items);
+  const double* ng = OPK == BEAST_HH_DL ? sgeo + 12 : tg + 12;
+  const V3<double> nv = mk(ng[0], ng[1], ng[2]);
+  // ---- the scales: sums of |a| (every warp of the pair takes them over all nodes, in the same order)
+  float sa = 0.f, sb = 0.f;
+  {
+    float f[4][3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      f[k][0] = (float)E[k].x;
+      f[k][1] = (float)E[k].y;
+      f[k][2] = (float)E[k].z;
+    }
+    const float n0 = (float)nv.x, n1 = (float)nv.y, n2 = (float)nv.z;
+    for (int it = lane; it < items; it += 32) {
+      const float a = tabf[it], b = tabf[items + it], c = tabf[2 * items + it],
+                  d = tabf[3 * items + it], w = fabsf(tabf[4 * items + it]);
+      const float x = a * f[0][0] + b * f[1][0] - (c * f[2][0] + d * f[3][0]),
+                  y = a * f[0][1] + b * f[1][1] - (c * f[2][1] + d * f[3][1]),
+                  z = a * f[0][2] + b * f[1][2] - (c * f[2][2] + d * f[3][2]);
+      const float ir = rsqrtf(x * x + y * y + z * z);
+      float q = w;
+      if (GRAD) {
+        q *= ir * ir;
+        if (!RT) q *= fabsf(n0 * x + n1 * y + n2 * z) + 1e-6f / ir;
+      }
+      sb += q;
+      sa += q * ir;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sa += __shfl_xor_sync(0xffffffffu, sa, o);
+      sb += __shfl_xor_sync(0xffffffffu, sb, o);
+    }
+  }
+  const int ea = (int)(__float_as_uint(1.01f * sa) >> 23) - 126, eb = (int)(__float_as_uint(1.01f * sb) >> 23) - 126;
+  const double k4 = 0.25 * P.wave.k * P.wave.k;
+  // ---- the nodes
+  int64_t Mr[NM], Mi[NM];
+#pragma unroll
+  for (int k = 0; k < NM; ++k) Mr[k] = Mi[k] = 0;
+  const int64_t* cf = s_coef[cls - 1];
+  for (int it = W == 1 ? lane : (int)threadIdx.x; it < items; it += 32 * W) {
+    const double* nd = nodes + it;
+    V3<double> r = nd[0] * E[0] + nd[items] * E[1];
+    if (cls != 3) {
+      r = r - nd[3 * items] * E[3];
+      if (cls == 1) r = r - nd[2 * items] * E[2];
+    }
+    const double R2 = dot(r, r);
+    double iR, R;
+    if ((uint32_t)((uint32_t)(g64::bits(R2) >> 52) - 923u) > 190u)
+      iR = rsqrt(R2);
+    else
+      g64::inv_sqrt(R2, iR, R);
+    double b = nd[4 * items];
+    if (GRAD) {
+      b *= iR * iR;
+      if (!RT) b *= dot(nv, r);
+    }
+    const int64_t a = g64::to_fixed(b * iR, ea), bx = g64::to_fixed(b, eb), u = g64::to_fixed(R2 * k4, 0);
+    const int64_t* pp = reinterpret_cast<const int64_t*>(nd) + 5 * items;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      int64_t tr = g64::mulhi(a, ssx_poly(cf + SSX_TERMS * j, u)), ti = g64::mulhi(bx, ssx_poly(cf + SSX_TERMS * (3 + j), u));
+      if (j == 0) {
+        Mr[0] += tr;
+        Mi[0] += ti;
+      }
+      tr <<= 2;
+      ti <<= 2;
+#pragma unroll
+      for (int m = 0; m < NT; ++m)
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+          if (j > 0 && (m > 0) + (n > 0) == j) {
+            const int64_t x = pp[(m && n ? 2 + 2 * m + n - 1 : m ? m - 1 : 1 + n) * items];
+            Mr[m * NB + n] += g64::mulhi(tr, x);
+            Mi[m * NB + n] += g64::mulhi(ti, x);
+          }
+    }
+  }
+  // ---- totals: lane k sums value k of the 32 lanes (a truncation of half a unit per node made good)
+#pragma unroll
+  for (int k = 0; k < NM; ++k) {
+    s_red[warp][2 * k][lane] = Mr[k];
+    s_red[warp][2 * k + 1][lane] = Mi[k];
+  }
+  __syncwarp();
+  int64_t tot = 0;
+  if (lane < 2 * NM)
+    for (int l = 0; l < 32; ++l) tot += s_red[warp][lane][l];
+  if (W > 1) {
+    if (lane < 2 * NM) s_sum[warp][lane] = tot;
+    __syncthreads();
+    if (warp > 0) return;
+    if (lane < 2 * NM) tot = (s_sum[0][lane] + s_sum[1][lane]) + (s_sum[2][lane] + s_sum[3][lane]);
+  }
+  if (lane < 2 * NM) {
+    const double x = g64::from_fixed(tot + items / 2, (lane & 1 ? eb : ea) - 60);
+    s_tot[warp][lane] = lane & 1 ? P.wave.k * x : x;
+  }
+  __syncwarp();
+  ss64_block<OPK, TK, BK>(P, np_, lane, pt, ps, tg, sgeo, s_tot[warp], s_T[warp]);
+}
+
+template <int OPK, int TK, int BK>
+static cudaError_t near_ssx_t(const NearParams& P, cudaStream_t st) {
+  if (P.nnear < 8 * sm_count())
+    k_near_ssx<OPK, TK, BK, NEAR_WARPS><<<(unsigned)P.nnear, 32 * NEAR_WARPS, 0, st>>>(P);
+  else
+    k_near_ssx<OPK, TK, BK, 1><<<(unsigned)((P.nnear + NEAR_WARPS - 1) / NEAR_WARPS), 32 * NEAR_WARPS, 0, st>>>(P);
+  return cudaGetLastError();
+}
+
+static cudaError_t ssx_tables(std::map<int, void*>* cache, const beast_qs_desc& qs, int kind, cudaStream_t st, NearParams* P) {
+  const int ord[4] = {0, qs.ss_vert, qs.ss_edge, qs.ss_face};
+  for (int c = 1; c <= 3; ++c) {
+    const int n = ord[c];
+    P->ssx_items[c] = (c == 1 ? 2 : 6) * n * n * n;
+    for (int what = 0; what < 2; ++what) {
+      const int key = what ? 40960 + 64 * kind + n : 32768 + 64 * c + n;
+      auto f = cache->find(key);
+      if (f == cache->end()) {
+        void* p = nullptr;
+        cudaError_t e = cudaMalloc(&p, what ? sizeof(int64_t) * SSX_ROWS * SSX_TERMS
+                                            : (sizeof(double) * SSX_VALS + sizeof(float) * 5) * (size_t)P->ssx_items[c]);
+        if (e != cudaSuccess) return e;
+        if (what)
+          k_ssx_coef<<<1, 96, 0, st>>>(n, kind, (int64_t*)p);
+        else
+          k_ssx_table<<<(P->ssx_items[c] + 127) / 128, 128, 0, st>>>(c, n, P->ssx_items[c], (double*)p);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) {
+          cudaFree(p);
+          return e;
+        }
+        f = cache->emplace(key, p).first;
+      }
+      if (what)
+        P->ssx_coef[c] = (const int64_t*)f->second;
+      else
+        P->ssx_tab[c] = (const double*)f->second;
+    }
+  }
+  return cudaSuccess;
+}
+
 template <int OPK, int TK, int BK>
 static cudaError_t near_ss64_t(const NearParams& P, cudaStream_t st) {
+  if (P.ssx) return near_ssx_t<OPK, TK, BK>(P, st);
   if (P.nnear < 8 * sm_count())
     k_near_ss64<OPK, TK, BK, 1><<<(unsigned)P.nnear, 32 * NEAR_WARPS, 0, st>>>(P);
   else
@@ -4389,8 +4663,17 @@ cudaError_t launch_near(const AsmArgs& a, int nnear, const TriRuleDev& ro, const
   const bool hh = a.op.kind == BEAST_HH_SL || a.op.kind == BEAST_HH_DL || a.op.kind == BEAST_HH_DLT;
   P.ss64 = (a.qs.kind == BEAST_QS_WILTON_SAUTER || a.qs.kind == BEAST_QS_SAUTER) && a.ss_tabs != nullptr &&
            ((rt && sl_dl && !P.ss32) || (hh && a.ts->kind != BEAST_RT && a.bs->kind != BEAST_RT)) && !P.ssdf;
+  // k_near_ssx: real wavenumbers up to k rho = 2, cells of ordinary size (its FP32 sums take 1/rho^3)
+  const beast_mesh *tm = a.ts->mesh, *bm = a.bs->mesh;
+  P.ssx = P.ss64 && a.op.gr == 0.0 && tm && bm && fabs(a.op.gi) * (tm->edge_max + bm->edge_max) <= 2.0 &&
+          std::min(tm->edge_min, bm->edge_min) > 0x1p-20 && std::max(tm->edge_max, bm->edge_max) < 0x1p20;
+  if (P.ssx && ssx_tables(a.ss_tabs, a.qs, a.op.kind == BEAST_MW_SL || a.op.kind == BEAST_HH_SL ? 0 : rt ? 1 : 2, st, &P) !=
+                   cudaSuccess) {
+    cudaGetLastError();
+    P.ssx = 0;
+  }
   // (orders up to 10: a node table of at most 6 MB; without the memory for it, k_near)
-  if (P.ss64 && (a.qs.ss_vert > 10 || a.qs.ss_edge > 10 || a.qs.ss_face > 10 ||
+  if (P.ss64 && !P.ssx && (a.qs.ss_vert > 10 || a.qs.ss_edge > 10 || a.qs.ss_face > 10 ||
                  ss64_tables(a.ss_tabs, a.qs, st, P.ss64_tab, P.ss64_items) != cudaSuccess)) {
     cudaGetLastError();
     P.ss64 = 0;

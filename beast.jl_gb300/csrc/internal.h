@@ -87,6 +87,7 @@ struct beast_mesh {
   double* children = nullptr;
   int nchild = 0;
   double radius = 0.0;       // average distance of a cell's vertices from its centroid
+  double edge_min = 0.0, edge_max = 1e300;  // shortest and longest edge of a cell
 };
 
 // per active cell geometry, 16 doubles: v0 v1 v2 (9) | centroid (3) | unit normal (3) | area

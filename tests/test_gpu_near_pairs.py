@@ -98,3 +98,34 @@ def test_classification():
         X = bg.lagrangecxd0(bg.Mesh(np.ldexp(m.vertices, e), m.cells))
         Zs = bg.assemble(H(wavenumber=np.ldexp(2.0, -e)), X, X, precision=bg.FP64)
         assert np.abs(np.ldexp(Zs.real, -3 * e) + 1j * np.ldexp(Zs.imag, -3 * e) - Z).max() <= 1e-12 * np.abs(Z).max()
+
+
+@pytest.mark.parametrize("k", [0.0, 0.004, -0.5, 0.9])
+@pytest.mark.parametrize("orders", [(1, 1, 1), (2, 3, 5), (11, 4, 4)])
+@pytest.mark.parametrize("kind,spaces", [("mwsl", "rtrt"), ("mwdl", "rtrt"), ("sl", "p0p0"), ("sl", "p1p0"), ("dl", "p1p1"),
+                                         ("dl", "p0p1"), ("dlt", "p0p0"), ("dlt", "p1p0")])
+def test_radial_sums_fp64(kind, spaces, orders, k):
+    """k rho below 2 on the whole mesh: the integer sums, against the oracle with the FP64 contract"""
+    m = _mesh()
+    make = {"p0": bg.lagrangecxd0, "p1": bg.lagrangec0d1, "rt": bg.raviartthomas}
+    H, M = bg.Helmholtz3D, bg.Maxwell3D
+    op = {"mwsl": lambda: M.singlelayer(gamma=1j * k, alpha=-1.3j, beta=0.7), "mwdl": lambda: M.doublelayer(gamma=1j * k),
+          "sl": lambda: H.singlelayer(gamma=1j * k), "dl": lambda: H.doublelayer(gamma=1j * k),
+          "dlt": lambda: H.doublelayer_transposed(gamma=1j * k)}[kind]()
+    X, Y, qs = make[spaces[:2]](m), make[spaces[2:]](m), WS(2, 3, 2, 3, orders[0], orders[1], orders[2], 3)
+    Z = bg.assemble(op, X, Y, quadstrat=qs, precision=bg.FP64)
+    Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), X, Y)
+    err = np.abs(Z - Zo) / (np.abs(Zo) + 1e-3 * np.abs(Zo).max())
+    assert err.max() < 1e-10
+
+
+@pytest.mark.parametrize("kind", ["sl", "dl"])
+def test_few_and_many_pairs(kind):
+    """four warps per pair and one give the same bits (integer sums)"""
+    X = bg.lagrangecxd0(_mesh(level=3))
+    op = (bg.Helmholtz3D.singlelayer if kind == "sl" else bg.Helmholtz3D.doublelayer)(wavenumber=3.0)
+    Z = bg.assemble(op, X, X, precision=bg.FP64)
+    rows = np.arange(0, X.numfunctions(), 97)
+    Zs = bg.assemble(op, X.subset(rows), X, precision=bg.FP64)
+    near = np.abs(Zs) > 0.05 * np.abs(Zs).max(axis=1, keepdims=True)
+    assert near.any(axis=1).all() and np.array_equal(Zs[near], Z[rows][near])
