@@ -28,6 +28,7 @@
 #include "pack2.h"
 #include "se_p1.h"
 #include "far_df.h"
+#include "far_df2.h"
 #include "se_core.h"
 
 namespace {
@@ -3229,10 +3230,33 @@ DEV dfl::df df_of(double x) {
 // at compile time (the default 3 x 4 far rules; efie_far_pair_fast), else the general core.
 // BETA: the balanced core (efie_far_pair_beta: Green's function values and the beta term of
 // the pair in double-float, the alpha terms in FP32; BEAST_MIXED_BALANCED)
-// (five CTAs per SM for the cores of the default rule sizes: 96 registers, no spills)
+// The balanced core takes the trial points two by two (far_df2.h): bound by the FP32 pipe, which
+// issue slots shared with the table's loads and moves keep two thirds busy; 13520 cells: 22.0 -> 21.2 ms
+// packed, 19.2 with the finer sine table.
+// (five CTAs per SM for the double-float core of the default rule sizes: 96 registers, no spills; four
+// for the packed one: 124 registers, 19.2 ms against 19.5 with five)
 template <int NO, int NI, bool BETA = false>
-__global__ void __launch_bounds__(FAR_THREADS, NO > 0 ? 5 : 1) k_far_efie_df(FarParams P) {
+__global__ void __launch_bounds__(FAR_THREADS, BETA ? 4 : NO > 0 ? 5 : 1) k_far_efie_df(FarParams P) {
   __shared__ FarDfRecord rec[FAR_QT];
+  constexpr bool PAIRS = BETA && NI % 2 == 0;
+  constexpr int NIP = PAIRS ? NI : 2, NOP = PAIRS ? NO : 1;
+  __shared__ __align__(16) dfl::EtaPairs<NIP> s_eta[PAIRS ? FAR_QT : 1];
+  __shared__ __align__(16) float4 s_wab2[NOP][NIP / 2];
+  __shared__ float s_tab2[PAIRS ? 2048 : 1];  // sin hi, lo, cos hi, lo of 2 pi k / 512 (sincos_tab2)
+  if (PAIRS)
+    for (int k = threadIdx.x; k < 512; k += blockDim.x) {
+      // from the FP64 table's quarter turn: sin(m) = sin(Q - m), the quadrant's sign
+      auto sine = [](int m) {
+        const int i = m & (g64::QUARTER - 1), quad = (m / g64::QUARTER) & 3;
+        const double x = g64::sin_table_dev[quad & 1 ? g64::QUARTER - i : i];
+        return df_of(quad & 2 ? -x : x);
+      };
+      const dfl::df s = sine(8 * k), c = sine(8 * k + g64::QUARTER);
+      s_tab2[k] = s.hi;
+      s_tab2[512 + k] = s.lo;
+      s_tab2[1024 + k] = c.hi;
+      s_tab2[1536 + k] = c.lo;
+    }
   __shared__ float s_tab[64][4];  // sin / cos(m pi/32): lanes read different entries
   __shared__ int s_zc[FAR_QT][3];
   constexpr int NOW = NO > 0 ? NO : 1, NIW = NI > 0 ? NI : 1;
@@ -3244,6 +3268,10 @@ __global__ void __launch_bounds__(FAR_THREADS, NO > 0 ? 5 : 1) k_far_efie_df(Far
       for (int a = 0; a < NO; ++a) w1[a] = df_of(P.ro.w[a]);
       for (int b = 0; b < NI; ++b) w2[b] = df_of(P.ri.w[b]);
       dfl::efie_far_weights<NOW, NIW>(w1, w2, s_wab);
+      if constexpr (PAIRS)
+        for (int a = 0; a < NO; ++a)
+          for (int b = 0; b < NI; b += 2)
+            s_wab2[a][b / 2] = make_float4(s_wab[a][b].hi, s_wab[a][b + 1].hi, s_wab[a][b].lo, s_wab[a][b + 1].lo);
     }
   }
   const int ni = P.ri.n, no = P.ro.n;
@@ -3274,6 +3302,17 @@ __global__ void __launch_bounds__(FAR_THREADS, NO > 0 ? 5 : 1) k_far_efie_df(Far
       r.eta[bb][2] = df_of(u * (g[2] - cz) + v * (g[5] - cz) + w * (g[8] - cz));
       r.w[bb] = df_of(P.ri.w[bb]);
       r.eta2[bb] = dfl::dot3s(r.eta[bb], r.eta[bb]);
+      if constexpr (PAIRS) {
+        dfl::EtaPairs<NIP>& E = s_eta[qi];
+        auto at = [&](float2& x) -> float& { return (bb & 1) ? x.y : x.x; };
+        for (int c = 0; c < 3; ++c) {
+          at(E.hi[bb / 2][c]) = r.eta[bb][c].hi;
+          at(E.lo[bb / 2][c]) = r.eta[bb][c].lo;
+          E.dup[bb][c] = make_float2(r.eta[bb][c].hi, r.eta[bb][c].hi);
+        }
+        at(E.s_hi[bb / 2]) = r.eta2[bb].hi;
+        at(E.s_lo[bb / 2]) = r.eta2[bb].lo;
+      }
     }
   }
   for (int k = threadIdx.x; k < nqt * 3; k += blockDim.x) s_zc[k / 3][k % 3] = (int)zcol_of(P.zcol, q0 + k / 3, 3, k % 3);
@@ -3335,12 +3374,20 @@ __global__ void __launch_bounds__(FAR_THREADS, NO > 0 ? 5 : 1) k_far_efie_df(Far
       }
     }
     dfl::cdf z[9];
-    if constexpr (NO > 0 && BETA)
-      dfl::efie_far_pair_beta<NO, NI>(d, tau, r.sig, xi, s_wab, r.eta, r.eta2, kk, alpha, beta, s_tab, z);
-    else if constexpr (NO > 0)
-      dfl::efie_far_pair_fast<NO, NI>(d, tau, r.sig, xi, s_wab, r.eta, r.eta2, kk, alpha, beta, s_tab, z);
-    else
-      dfl::efie_far_pair(d, tau, r.sig, no, xi, wo, ni, r.eta, r.w, kk, alpha, beta, z);
+    // (phases of 2^14 and above keep sincos_tab's range)
+    bool packed = false;
+    if constexpr (PAIRS) {
+      packed = fabsf(kk.hi) * (fabsf(d[0].hi) + fabsf(d[1].hi) + fabsf(d[2].hi) + radp + r.lim) < 16384.f;
+      if (packed) dfl::efie_far_pair_beta2<NO, NI>(d, tau, r.sig, xi, s_wab2, s_eta[qi], kk, alpha, beta, s_tab2, z);
+    }
+    if (!packed) {
+      if constexpr (NO > 0 && BETA)
+        dfl::efie_far_pair_beta<NO, NI>(d, tau, r.sig, xi, s_wab, r.eta, r.eta2, kk, alpha, beta, s_tab, z);
+      else if constexpr (NO > 0)
+        dfl::efie_far_pair_fast<NO, NI>(d, tau, r.sig, xi, s_wab, r.eta, r.eta2, kk, alpha, beta, s_tab, z);
+      else
+        dfl::efie_far_pair(d, tau, r.sig, no, xi, wo, ni, r.eta, r.w, kk, alpha, beta, z);
+    }
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) {
         const dfl::cdf& v = z[3 * i + j];

@@ -218,6 +218,40 @@ struct cf {  // complex FP32 (host and device)
 };
 DF_HD float f32(df a) { return add_rn(a.hi, a.lo); }
 DF_HD cf cmulf(cf a, cf b) { return {fmaf(a.x, b.x, -mul_rn(a.y, b.y)), fmaf(a.x, b.y, mul_rn(a.y, b.x))}; }
+// the balanced mode's 3 x 3 block from the pair's moments (M0 normalised)
+DF_HD void efie_beta_block(cdf M0, cf M1, const cf* V1, const cf* V2, const df (*tau)[3], const df (*sig)[3], cdf alpha,
+                           cdf beta, cdf* out) {
+  // alpha term in FP32: a4 (M1 - sig_j.V1 - tau_i.V2 + (tau_i.sig_j) M0)
+  const cf a4 = cf{0.25f * f32(alpha.re), 0.25f * f32(alpha.im)};
+  const cf C = cmulf(a4, M1), D = cmulf(a4, cf{f32(M0.re), f32(M0.im)});
+  float ts[3][3], ss[3][3];
+  for (int i = 0; i < 3; ++i)
+    for (int c = 0; c < 3; ++c) {
+      ts[i][c] = f32(tau[i][c]);
+      ss[i][c] = f32(sig[i][c]);
+    }
+  cf S[3], Tm[3];
+  for (int j = 0; j < 3; ++j) {
+    cf sv = cf{0.f, 0.f}, tv = cf{0.f, 0.f};
+    for (int c = 0; c < 3; ++c) {
+      sv.x = fmaf(ss[j][c], V1[c].x, sv.x);
+      sv.y = fmaf(ss[j][c], V1[c].y, sv.y);
+      tv.x = fmaf(ts[j][c], V2[c].x, tv.x);
+      tv.y = fmaf(ts[j][c], V2[c].y, tv.y);
+    }
+    S[j] = cmulf(a4, sv);
+    Tm[j] = cmulf(a4, tv);
+  }
+  // beta term in double-float, once per pair
+  const cdf bM0 = cmulu(beta, M0);
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) {
+      const float g = fmaf(ts[i][0], ss[j][0], fmaf(ts[i][1], ss[j][1], ts[i][2] * ss[j][2]));
+      const float zr = C.x - S[j].x - Tm[i].x + g * D.x;
+      const float zi = C.y - S[j].y - Tm[i].y + g * D.y;
+      out[3 * i + j] = cdf{add(bM0.re, zr), add(bM0.im, zi)};
+    }
+}
 template <int NO, int NI>
 DF_HD void efie_far_pair_beta(const df* d, const df (*tau)[3], const df (*sig)[3], const df (*xi)[3],
                               const df (*wab)[NI], const df (*eta)[3], const df* eta2, df k, cdf alpha, cdf beta,
@@ -279,37 +313,7 @@ DF_HD void efie_far_pair_beta(const df* d, const df (*tau)[3], const df (*sig)[3
       V1[c].y = fmaf(U0.y, xf[c], V1[c].y);
     }
   }
-  M0 = cnorm(M0);
-  // alpha term in FP32: a4 (M1 - sig_j.V1 - tau_i.V2 + (tau_i.sig_j) M0)
-  const cf a4 = cf{0.25f * f32(alpha.re), 0.25f * f32(alpha.im)};
-  const cf C = cmulf(a4, M1), D = cmulf(a4, cf{f32(M0.re), f32(M0.im)});
-  float ts[3][3], ss[3][3];
-  for (int i = 0; i < 3; ++i)
-    for (int c = 0; c < 3; ++c) {
-      ts[i][c] = f32(tau[i][c]);
-      ss[i][c] = f32(sig[i][c]);
-    }
-  cf S[3], Tm[3];
-  for (int j = 0; j < 3; ++j) {
-    cf sv = cf{0.f, 0.f}, tv = cf{0.f, 0.f};
-    for (int c = 0; c < 3; ++c) {
-      sv.x = fmaf(ss[j][c], V1[c].x, sv.x);
-      sv.y = fmaf(ss[j][c], V1[c].y, sv.y);
-      tv.x = fmaf(ts[j][c], V2[c].x, tv.x);
-      tv.y = fmaf(ts[j][c], V2[c].y, tv.y);
-    }
-    S[j] = cmulf(a4, sv);
-    Tm[j] = cmulf(a4, tv);
-  }
-  // beta term in double-float, once per pair
-  const cdf bM0 = cmulu(beta, M0);
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      const float g = fmaf(ts[i][0], ss[j][0], fmaf(ts[i][1], ss[j][1], ts[i][2] * ss[j][2]));
-      const float zr = C.x - S[j].x - Tm[i].x + g * D.x;
-      const float zi = C.y - S[j].y - Tm[i].y + g * D.y;
-      out[3 * i + j] = cdf{add(bM0.re, zr), add(bM0.im, zi)};
-    }
+  efie_beta_block(cnorm(M0), M1, V1, V2, tau, sig, alpha, beta, out);
 }
 
 }  // namespace dfl

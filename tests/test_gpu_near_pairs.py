@@ -129,3 +129,15 @@ def test_few_and_many_pairs(kind):
     Zs = bg.assemble(op, X.subset(rows), X, precision=bg.FP64)
     near = np.abs(Zs) > 0.05 * np.abs(Zs).max(axis=1, keepdims=True)
     assert near.any(axis=1).all() and np.array_equal(Zs[near], Z[rows][near])
+
+
+@pytest.mark.parametrize("k,tol", [(0.5, 1e-10), (2.0, 1e-10), (300.0, 1e-9), (3e4, 1e-7)])
+def test_balanced_beta_term(k, tol):
+    """the beta term alone: pair arithmetic (4e-12 per value and 2^-45 of the phase; an entry adds blocks up
+    to ten times its size), phases below and above the packed core's 2^14"""
+    X = bg.raviartthomas(_mesh())
+    make = lambda g: bg.Maxwell3D.singlelayer(gamma=g, alpha=0.0, beta=1.0)
+    Z = bg.assemble(make(1j * k), X, X, precision=bg.MIXED_BALANCED)
+    Zr = bg.assemble(make(1j * k), X, X, precision=bg.FP64)
+    scale = np.abs(bg.assemble(make(0.0), X, X, precision=bg.FP64)).max()
+    assert np.abs(Z - Zr).max() <= tol * scale
