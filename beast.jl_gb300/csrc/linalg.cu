@@ -613,9 +613,8 @@ __device__ __forceinline__ int pidx(int c) {  // conflict-free index of the publ
 // SYM: only the lower triangle of the block is current (symmetric updates); the upper one
 // is taken from it by symmetry, the elimination on U^T is skipped and, U = D L^T,
 // U^{-1} = (L^{-1})^T D^{-1} is formed from L^{-1} and the pivots at the end.
-// TR x TC: the tile a thread owns (rows x columns): 4 x 4 (256 threads), 2 x 4 (512) or 2 x 2
-// (1024 threads: a quarter of the serial instructions per warp and step of 4 x 4, which is what
-// bounds this latency-bound chain).  The arithmetic per element is the same for every tile.
+// TR x TC: the tile a thread owns (rows x columns): 4 x 4 (256 threads) or 2 x 4 (512); 2 x 2 tiles:
+// k_lu_inv64_pair.  The arithmetic per element is the same for every tile.
 template <typename T, bool SYM, int TR = 4, int TC = TR>
 __global__ void __launch_bounds__(TRI * TRI / (TR * TC)) k_lu_inv64(T* A, int64_t lda, int64_t j0, int kb, int* info,
                                                                    T* inv) {
@@ -730,6 +729,225 @@ __global__ void __launch_bounds__(TRI * TRI / (TR * TC)) k_lu_inv64(T* A, int64_
       }
       __syncthreads();
     }
+  }
+  // U (upper part of S1) joins the L factor in Ls; the factored block goes back to A
+#pragma unroll
+  for (int i = 0; i < TR; ++i)
+#pragma unroll
+    for (int j = 0; j < TC; ++j)
+      if (c0 + j >= r0 + i) Ls[(r0 + i) * LD + c0 + j] = s1[i][j];
+  __syncthreads();
+  for (int e = tid; e < kb * kb; e += NT) {
+    const int r = e % kb, c = e / kb;
+    A[(j0 + r) + (j0 + c) * lda] = Ls[r * LD + c];
+  }
+  __syncthreads();
+  // Linv (column-major, inv[c * 64 + r] = Linv[r][c]) through Ls; Uinv = X^T, so row r of X
+  // is column r of Uinv (inv[4096 + r * 64 + c] = X[r][c]), written by the tile owners;
+  // symmetric: X[r][c] = Linv[r][c] / d_r
+  if (SYM) {
+    __shared__ T s_dinv[TRI];
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+      for (int j = 0; j < TC; ++j)
+        if (c0 + j == r0 + i) {  // the tile holding the pivot of row r0 + i
+          T di;
+          crecip(s1[i][j], di);  // nonzero: the elimination checked every pivot
+          s_dinv[r0 + i] = di;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TR; ++i) {
+      const T di = s_dinv[r0 + i];
+#pragma unroll
+      for (int j = 0; j < TC; ++j) {
+        const int r = r0 + i, c = c0 + j;
+        s2[i][j] = c < r ? cmulx(s1[i][j], di) : (c == r ? di : zero);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TR; ++i)
+#pragma unroll
+    for (int j = 0; j < TC; ++j) {
+      const int r = r0 + i, c = c0 + j;
+      Ls[r * LD + c] = c < r ? s1[i][j] : (c == r ? one : zero);
+      inv[TRI * TRI + r * TRI + c] = s2[i][j];
+    }
+  __syncthreads();
+  for (int e = tid; e < TRI * TRI; e += NT) {
+    const int r = e & (TRI - 1), c = e >> 6;
+    inv[e] = Ls[r * LD + c];
+  }
+}
+
+// two neighbouring complex values of shared memory (the first at an even place) in one load
+__device__ __forceinline__ void ld_two(const float2* p, float2& a, float2& b) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a = make_float2(v.x, v.y);
+  b = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void ld_two(const double2* p, double2& a, double2& b) {
+  a = p[0];
+  b = p[1];
+}
+
+// k_lu_inv64 on 2 x 2 tiles (1024 threads), two steps per barrier.  A step of that kernel is 57 instructions
+// a warp on eight warps per scheduler and then a chain through shared memory and the barrier (28 us a
+// block, 55% of it issuing).  Here the tile that holds the 2 x 2 pivot block eliminates in it before it
+// publishes, and every thread forms the second pivot row's and column's entries that it needs itself:
+// the same operations on every element, in the same order, as one step at a time.  25.9 us a block; the
+// chain pivot - publish - barrier is now what the warps wait for (per panel, job of 30,720: 48.6 -> 46.1).
+template <typename T, bool SYM>
+__global__ void __launch_bounds__(TRI * TRI / 4) k_lu_inv64_pair(T* A, int64_t lda, int64_t j0, int kb, int* info, T* inv) {
+  constexpr bool sym = SYM;
+  constexpr int TR = 2, TC = 2, NT = TRI * TRI / 4, LD = TRI + 1;
+  extern __shared__ unsigned char smraw[];
+  T* Ls = reinterpret_cast<T*>(smraw);  // 64 x LD: staging, then the L factor, then Linv
+  __shared__ __align__(16) T p1[2][2][TRI], p2[2][2][SYM ? 2 : TRI], lc[2][TRI][2], dv[2][4];  // dv: d0, d1, l10, u01
+  __shared__ int s_zero[2];  // 1-based column of a zero pivot, by parity of the pair of steps
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int tid = threadIdx.x, rb = tid >> 5, cb = tid & 31;
+  const int r0 = TR * rb, c0 = TC * cb;
+  const T zero = cmk<T>(0.0, 0.0), one = cmk<T>(1.0, 0.0);
+  for (int e = tid; e < TRI * TRI; e += NT) {
+    const int r = e & (TRI - 1), c = e >> 6;
+    const int rr = (sym && c > r) ? c : r, cc = (sym && c > r) ? r : c;
+    Ls[r * LD + c] = (r < kb && c < kb) ? A[(j0 + rr) + (j0 + cc) * lda] : (r == c ? one : zero);
+  }
+  if (tid < 2) s_zero[tid] = 0;
+  __syncthreads();
+  T s1[TR][TC], s2[TR][TC];
+#pragma unroll
+  for (int i = 0; i < TR; ++i)
+#pragma unroll
+    for (int j = 0; j < TC; ++j) {
+      s1[i][j] = Ls[(r0 + i) * LD + c0 + j];
+      s2[i][j] = (r0 + i == c0 + j) ? one : zero;
+    }
+  // rows and columns 2 kq, 2 kq + 1 of S1 (the column of the first pivot as the second row has it after the
+  // first step), the pivots' reciprocals and the block's multiplier
+  auto publish = [&](int b, int kq) {
+    if (rb == kq) {
+      if (cb == kq) {
+        T d0 = zero, d1 = zero;
+        const bool ok = crecip(s1[0][0], d0);
+        const T l = cmulx(s1[1][0], d0);
+        T piv = s1[1][1];
+        cfms(piv, l, s1[0][1]);
+        if (!ok)
+          s_zero[b] = 2 * kq + 1;
+        else if (!crecip(piv, d1))
+          s_zero[b] = 2 * kq + 2;
+        dv[b][0] = d0;
+        dv[b][1] = d1;
+        dv[b][2] = l;
+        dv[b][3] = s1[0][1];
+        T nl;
+        nl.x = -l.x;
+        nl.y = -l.y;
+        p1[b][0][c0] = zero;
+        p1[b][1][c0] = nl;
+      } else {
+        p1[b][0][c0] = s1[0][0];
+        p1[b][1][c0] = s1[1][0];
+      }
+      p1[b][0][c0 + 1] = s1[0][1];
+      p1[b][1][c0 + 1] = s1[1][1];
+      if constexpr (!SYM)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) p2[b][i][c0 + j] = s2[i][j];
+    } else if (cb == kq) {
+#pragma unroll
+      for (int i = 0; i < TR; ++i) {
+        lc[b][r0 + i][0] = s1[i][0];
+        lc[b][r0 + i][1] = s1[i][1];
+      }
+    }
+  };
+  publish(0, 0);
+  __syncthreads();  // the staging buffer is free from here on (L factor)
+#pragma unroll 1
+  for (int kq = 0; kq < TRI / 2; ++kq) {
+    const int b = kq & 1, k = 2 * kq;
+    if (s_zero[b]) {  // uniform
+      if (tid == 0) atomicCAS(info, 0, (int)(j0 + s_zero[b]));
+      return;
+    }
+    if (rb >= kq) {
+      T d0, d1, l10, u01, q0[TC], q1[TC], x0[TC], x1[TC];
+      ld_two(&dv[b][0], d0, d1);
+      ld_two(&dv[b][2], l10, u01);
+      ld_two(&p1[b][0][c0], q0[0], q0[1]);
+      ld_two(&p1[b][1][c0], q1[0], q1[1]);
+      if constexpr (!SYM) {
+        ld_two(&p2[b][0][c0], x0[0], x0[1]);
+        ld_two(&p2[b][1][c0], x1[0], x1[1]);
+      }
+      const T m01 = cmulx(u01, d0);  // the multiplier of X's row k + 1
+      if (rb == kq) {  // row k + 1: the first step
+#pragma unroll
+        for (int j = 0; j < TC; ++j) {
+          cfms(s1[1][j], l10, q0[j]);
+          if constexpr (!SYM) {
+            cfms(s2[1][j], m01, x0[j]);
+            s2[0][j] = cmulx(s2[0][j], d0);
+            s2[1][j] = cmulx(s2[1][j], d1);
+          }
+        }
+        if (cb == kq) {
+          s1[1][0].x = -l10.x;
+          s1[1][0].y = -l10.y;
+          Ls[(k + 1) * LD + k] = l10;
+        }
+      } else {
+        // the second pivot row after the first step (its entry at column k is there already, at k + 1 none)
+#pragma unroll
+        for (int j = 0; j < TC; ++j) {
+          cfms(q1[j], l10, q0[j]);
+          if constexpr (!SYM) cfms(x1[j], m01, x0[j]);
+        }
+        if (cb == kq) q1[1] = zero;
+#pragma unroll
+        for (int i = 0; i < TR; ++i) {
+          T a0, a1;
+          ld_two(&lc[b][r0 + i][0], a0, a1);
+          const T l0 = cmulx(a0, d0);
+          cfms(a1, l0, u01);
+          const T l1 = cmulx(a1, d1);
+#pragma unroll
+          for (int j = 0; j < TC; ++j) cfms(s1[i][j], l0, q0[j]);
+          if (cb == kq) {
+            s1[i][0].x = -l0.x;
+            s1[i][0].y = -l0.y;
+          }
+#pragma unroll
+          for (int j = 0; j < TC; ++j) cfms(s1[i][j], l1, q1[j]);
+          if (cb == kq) {
+            s1[i][1].x = -l1.x;
+            s1[i][1].y = -l1.y;
+            Ls[(r0 + i) * LD + k] = l0;
+            Ls[(r0 + i) * LD + k + 1] = l1;
+          }
+          if constexpr (!SYM) {
+            const T u0 = p1[b][0][r0 + i];
+            T u1 = p1[b][1][r0 + i];
+            cfms(u1, l10, u0);
+            const T m0 = cmulx(u0, d0), m1 = cmulx(u1, d1);
+#pragma unroll
+            for (int j = 0; j < TC; ++j) {
+              cfms(s2[i][j], m0, x0[j]);
+              cfms(s2[i][j], m1, x1[j]);
+            }
+          }
+        }
+      }
+      if (kq + 1 < TRI / 2) publish(b ^ 1, kq + 1);
+    }
+    __syncthreads();
   }
   // U (upper part of S1) joins the L factor in Ls; the factored block goes back to A
 #pragma unroll
@@ -2322,8 +2540,8 @@ int lu_factor_t(beast_ctx* ctx, int64_t n, T* A, int64_t lda, int* ipiv, int* in
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_getrf64<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
-  BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64<T, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
-  BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64<T, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
+  BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64_pair<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
+  BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64_pair<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64<T, false, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_lu_inv64<T, true, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)getrf_sm));
   // the diagonal-block elimination with 2 x 2 tiles on 1024 threads (default), 2 x 4 tiles on 512
@@ -2354,9 +2572,9 @@ int lu_factor_t(beast_ctx* ctx, int64_t n, T* A, int64_t lda, int* ipiv, int* in
   int* dstatus = dinfo + 1;                        // a panel wait that ran out
   auto diag = [&](bool sy, int64_t jd, int kd, T* out_inv, cudaStream_t s_) {
     if (dtile == 22 && sy)
-      k_lu_inv64<T, true, 2><<<1, TRI * TRI / 4, getrf_sm, s_>>>(A, lda, jd, kd, dinfo, out_inv);
+      k_lu_inv64_pair<T, true><<<1, TRI * TRI / 4, getrf_sm, s_>>>(A, lda, jd, kd, dinfo, out_inv);
     else if (dtile == 22)
-      k_lu_inv64<T, false, 2><<<1, TRI * TRI / 4, getrf_sm, s_>>>(A, lda, jd, kd, dinfo, out_inv);
+      k_lu_inv64_pair<T, false><<<1, TRI * TRI / 4, getrf_sm, s_>>>(A, lda, jd, kd, dinfo, out_inv);
     else if (dtile == 24 && sy)
       k_lu_inv64<T, true, 2, 4><<<1, TRI * TRI / 8, getrf_sm, s_>>>(A, lda, jd, kd, dinfo, out_inv);
     else if (dtile == 24)

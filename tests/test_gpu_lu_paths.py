@@ -69,3 +69,26 @@ def test_gmres_zero_right_hand_side_and_limit():
     assert it == 0 and np.array_equal(x, np.zeros(70))
     with pytest.raises(bg.BeastError):
         bg.gmres(A, np.ones(70), reltol=1e-14, restart=4, maxiter=6)
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("n,col", [(300, 64), (300, 65), (300, 127), (65, 64), (130, 129)])
+def test_zero_pivot_of_a_pair(n, col, symmetric, monkeypatch):
+    """the diagonal block's elimination takes two pivots at a time: a zero first or second pivot, also the
+    last one of a matrix, ends as it does one pivot at a time (4 x 4 tiles)"""
+    import torch
+    rng = np.random.default_rng(n + col)
+    A = np.diag(rng.uniform(1.0, 2.0, n) + 1j * rng.uniform(-1.0, 1.0, n)).astype(np.complex64)
+    A[col, col] = 0.0
+    b = rng.normal(size=n) + 0j
+    if not symmetric:
+        A[1, 0] = 0.5
+    out = []
+    for tile in ("4", "2"):
+        monkeypatch.setenv("BEAST_LU_DIAG_TILE", tile)
+        try:
+            x, it, res = bg.solve(torch.from_numpy(np.ascontiguousarray(A.T)).cuda().T, b, precision=bg.MIXED)
+            out.append(("solved", x.tobytes()))
+        except bg.BeastError as e:
+            out.append(("refused", str(e)))
+    assert out[0] == out[1]
