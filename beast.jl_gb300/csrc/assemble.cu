@@ -1,15 +1,16 @@
 // assemble.cu -- GB300 kernels of the Galerkin assembly path.
 //
 // Pipeline of one beast_assemble call (per trial-dof chunk):
-//   k_far     every (test cell p, trial cell q) pair of the chunk: pair classification
-//             (quadrule, src/quadrature/doublenumwiltonsauterqstrat.jl:32-69) and, for far
-//             pairs, the DoubleQuadRule block (src/quadrature/doublenumints.jl:12-43) in FP64
-//             or FP32.  The per-point-pair work is reduced algebraically: for RT shapes
-//             f_i = (x - v_i)/2A the 3x3 block is a fixed combination of 8 (single layer) or
-//             10/16 (double layer, n x K) complex moments of the kernel, accumulated with
-//             coordinates relative to the cell centroids.  Near pairs go to a list.
-//   k_near    one warp per listed pair: Sauter-Schwab (touching) or Wilton singularity
-//             extraction (near), FP64 (src/quadrature/sauterschwabints.jl:156-182,
+//   far kernels: every (test cell p, trial cell q) pair of the chunk is classified (quadrule,
+//             src/quadrature/doublenumwiltonsauterqstrat.jl:32-69); far pairs get their
+//             DoubleQuadRule block (src/quadrature/doublenumints.jl:12-43), near pairs go to a list.
+//             k_far64 in FP64 (moments over the cells' barycentric coordinates, kernel values on
+//             green64.h, the sums in 64-bit integers where the wavenumber allows), k_far in FP32,
+//             k_far_efie_df for the EFIE in double-float.
+//   near kernels: touching pairs by Sauter-Schwab rules (src/quadrature/sauterschwabints.jl:156-182):
+//             k_near_ssx (FP64, radial coordinate summed out), k_near_ss64 (FP64 node by node),
+//             k_near_ss_df / k_near_hh_df (double-float), k_near_ss32 (mixed), k_near for the rest;
+//             close ones by Wilton singularity extraction (k_near_se,
 //             src/quadrature/singularityextractionints.jl:4-22).
 //   k_gather  Z[m,n] = sum over the shapes of dof m and dof n of a*b*Zcell: the RT/P0/P1
 //             local-to-global scatter (src/integralop.jl:173-184) as an owner-computes
@@ -306,9 +307,9 @@ DEV C2<float> hh_sl_far_f(V3<float> d, const V3<float>* tau, const float* ro, in
       const pk::f2 wa = pk::both(ro[3 * a + 2]), xx = pk::both(x.x), xy = pk::both(x.y), xz = pk::both(x.z);
 #pragma unroll 1
       for (int b = 0; b < ni; b += 2) {
-        const ulonglong2 p0 = *reinterpret_cast<const ulonglong2*>(pts + 4 * b),
-                         p1 = *reinterpret_cast<const ulonglong2*>(pts + 4 * b + 4);
-        const pk::f2 rx = pk::sub(xx, pk::f2{p0.x}), ry = pk::sub(xy, pk::f2{p0.y}), rz = pk::sub(xz, pk::f2{p1.x});
+        const float4 p0 = *reinterpret_cast<const float4*>(pts + 4 * b), p1 = *reinterpret_cast<const float4*>(pts + 4 * b + 4);
+        const pk::f2 rx = pk::sub(xx, pk::make(p0.x, p0.y)), ry = pk::sub(xy, pk::make(p0.z, p0.w)),
+                     rz = pk::sub(xz, pk::make(p1.x, p1.y));
         const pk::f2 R2 = pk::fma(rx, rx, pk::fma(ry, ry, pk::mul(rz, rz)));
         float i0, i1;
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i0) : "f"(pk::lo(R2)));
@@ -319,11 +320,11 @@ DEV C2<float> hh_sl_far_f(V3<float> d, const V3<float>* tau, const float* ro, in
         const pk::f2 t2 = pk::mul(t, t);
         const pk::f2 st = pk::fma(pk::mul(t, t2), pk::both(-1.f / 6.f), t);
         const pk::f2 ct = pk::mul(t2, pk::fma(t2, pk::both(1.f / 24.f), pk::both(-0.5f)));  // cos t - 1
-        const float* e0 = tab + ((unsigned)f.v & 63u);
-        const float* e1 = tab + ((unsigned)(f.v >> 32) & 63u);
+        const float* e0 = tab + (__float_as_uint(pk::lo(f)) & 63u);
+        const float* e1 = tab + (__float_as_uint(pk::hi(f)) & 63u);
         const pk::f2 s = pk::make(e0[0], e1[0]), sl = pk::make(e0[64], e1[64]), c = pk::make(e0[128], e1[128]),
                      cl = pk::make(e0[192], e1[192]);
-        const pk::f2 w = pk::mul(pk::mul(pk::f2{p1.y}, wa), iR);
+        const pk::f2 w = pk::mul(pk::mul(pk::make(p1.z, p1.w), wa), iR);
         const pk::f2 ns = pk::make(-pk::lo(s), -pk::hi(s));
         si = pk::fma(w, pk::add(s, pk::fma(c, st, pk::fma(s, ct, sl))), si);
         sr = pk::fma(w, pk::add(c, pk::fma(ns, st, pk::fma(c, ct, cl))), sr);
@@ -3231,7 +3232,7 @@ DEV dfl::df df_of(double x) {
 // BETA: the balanced core (efie_far_pair_beta: Green's function values and the beta term of
 // the pair in double-float, the alpha terms in FP32; BEAST_MIXED_BALANCED)
 // The balanced core takes the trial points two by two (far_df2.h): bound by the FP32 pipe, which
-// issue slots shared with the table's loads and moves keep two thirds busy; 13520 cells: 22.0 -> 21.2 ms
+// issue slots shared with the table's loads and moves keep two thirds busy; 14580 cells: 22.0 -> 21.2 ms
 // packed, 19.2 with the finer sine table.
 // (five CTAs per SM for the double-float core of the default rule sizes: 96 registers, no spills; four
 // for the packed one: 124 registers, 19.2 ms against 19.5 with five)

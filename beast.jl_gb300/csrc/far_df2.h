@@ -61,8 +61,8 @@ __device__ __forceinline__ void sincos_tab2(df2 th, const float* tab, df2* s, df
   f2 e = pk::sub(th.lo, pk::fma(n, pk::both(0.012271846644580364f), np));
   e = pk::fma(n, pk::both(3.4149522099014007e-10f), e);
   e = pk::fma(n, pk::both(1.3399410234420952e-17f), e);
-  const float* e0 = tab + ((unsigned)f.v & 511u);
-  const float* e1 = tab + ((unsigned)(f.v >> 32) & 511u);
+  const float* e0 = tab + (__float_as_uint(pk::lo(f)) & 511u);
+  const float* e1 = tab + (__float_as_uint(pk::hi(f)) & 511u);
   const f2 sh = pk::make(e0[0], e1[0]), sl = pk::make(e0[512], e1[512]), ch = pk::make(e0[1024], e1[1024]),
            cl = pk::make(e0[1536], e1[1536]);
   const f2 tt = pk::add(t, e), t2 = pk::mul(tt, tt);
@@ -84,7 +84,7 @@ struct EtaPairs {
   float2 hi[NI / 2][3], lo[NI / 2][3], s_hi[NI / 2], s_lo[NI / 2];
   float2 dup[NI][3];
 };
-__device__ __forceinline__ f2 ld(const float2& x) { return f2{*reinterpret_cast<const unsigned long long*>(&x)}; }
+__device__ __forceinline__ f2 ld(const float2& x) { return f2{x}; }
 
 // wab[a][b / 2]: high parts of (b, b + 1), low parts
 template <int NO, int NI>

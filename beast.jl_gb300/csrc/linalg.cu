@@ -10,9 +10,10 @@
 //   k_laswp    the panel's row interchanges applied to the other columns
 //   k_trsm_tile   U12 = L11^{-1} A12 and (unpivoted path, after k_getrf64 on the diagonal
 //                 block) L21 = A21 U11^{-1}
-//   k_lu_inv64 + k_panel_apply   the unpivoted c64 panel: diagonal block LU with the
+//   k_lu_inv64(_pair) + k_panel_apply   the unpivoted c64 panel: diagonal block LU with the
 //                 inverses of its triangles, then both triangular solves as products
-//   k_gemm     A22 -= L21 U12 (complex, tiled through shared memory)
+//   A22 -= L21 U12: on the tensor cores (tc_gemm.cu for c64, tc_gemm64.cu for c128), else
+//                 k_gemm (complex, tiled through shared memory)
 // The element type is complex FP64 (c128) or complex FP32 (c64).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
