@@ -295,7 +295,7 @@ def compare_fp64(args):
     """Plain FP64 (c128 matrix, FP64 quadrature, FP64 LU) against the mixed path on the same
     workload: solves/s of each (CUDA events around assemble + excitation + solve; the mixed
     path after one warm-up solve, the FP64 path as one run after it, its LU alone taking
-    minutes), and each arm's relative difference from the FP64 one in the surface current, the
+    seconds), and each arm's relative difference from the FP64 one in the surface current, the
     far field (181 directions in the xz-plane) and, for the mixed arm, the matrix (Frobenius)."""
     import torch
     import beastgpu as bg
