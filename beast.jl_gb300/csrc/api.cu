@@ -1566,8 +1566,7 @@ int beast_batch_create(beast_ctx* ctx, const beast_qs_desc* qs, int64_t njobs, c
   L.flag = b->counter + 1;
   L.tile_m = tile_m;
   L.tile_q = tile_q;
-  // persistent grids: a few CTAs per SM (the far kernel holds ~130 registers per thread)
-  L.grid_far = std::max(1, std::min(L.ntiles, ctx->num_sms * std::max(1, 512 / std::max(64, tile_m))));
+  // persistent grids: a few CTAs per SM (the far kernel: as many as its registers let an SM hold)
   L.grid_near = ctx->num_sms * 8;
   // the single layer's Sauter-Schwab pairs in double-float off the FP64 path: node tables now
   // (graph capture comes later)

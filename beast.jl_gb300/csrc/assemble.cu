@@ -38,12 +38,6 @@ namespace {
 
 
 // exp(-gamma R) / (4 pi R) for gamma = gr + i gi
-DEV C2<double> green_d(double gr, double gi, double R, double iR) {
-  double s, c;
-  sincos(gi * R, &s, &c);
-  double a = (gr == 0.0 ? 1.0 : exp(-gr * R)) * I4PI * iR;
-  return {a * c, -a * s};
-}
 DEV C2<float> green_f(float gr, float gi, float R, float iR) {
   float s, c;
   sincosf(gi * R, &s, &c);
@@ -53,19 +47,11 @@ DEV C2<float> green_f(float gr, float gi, float R, float iR) {
 template <typename R>
 DEV C2<R> green(R gr, R gi, R Rr, R iR);
 template <>
-DEV C2<double> green<double>(double gr, double gi, double Rr, double iR) {
-  return green_d(gr, gi, Rr, iR);
-}
-template <>
 DEV C2<float> green<float>(float gr, float gi, float Rr, float iR) {
   return green_f(gr, gi, Rr, iR);
 }
 template <typename R>
 DEV R rsq(R x);
-template <>
-DEV double rsq<double>(double x) {
-  return rsqrt(x);
-}
 template <>
 DEV float rsq<float>(float x) {
   return rsqrtf(x);

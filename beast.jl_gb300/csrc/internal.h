@@ -271,7 +271,7 @@ struct BatchLaunch {
   int* near_count;
   int* flag;
   int tile_m, tile_q;           // test cells per CTA (= threads), trial cells staged per CTA
-  int grid_far, grid_near;      // persistent CTAs
+  int grid_near;                // persistent CTAs of the near kernels
   // single-layer Sauter-Schwab pairs in double-float (not on the FP64 path): node tables per
   // class 1..3 (ss_tables)
   int ssdf = 0;
