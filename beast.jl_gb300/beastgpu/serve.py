@@ -42,12 +42,12 @@ from . import lib as L
 def job_footprint(n, nrhs=1, precision=L.MIXED, workspace=0):
     """device bytes a job holds at its peak: the matrix, the factor copy, the tensor-core
     operands of the largest trailing update (12 bytes per row and column of K <= 1024 on the mixed
-    paths, 96 of K <= 256 in FP64), the right-hand sides / solutions /
+    paths, 108 of K <= 256 in FP64), the right-hand sides / solutions /
     refinement vectors, the context's assembly workspace, and 64 MiB of small buffers"""
     zel = 8 if precision == L.MIXED else 16
     fel = 16 if precision == L.FP64 else 8
     if precision == L.FP64:
-        tc = 96 * 256 * n if n > 64 else 0
+        tc = 108 * 256 * n if n > 64 else 0
     else:
         tc = 12 * 1024 * n if n > 1024 else 0
     return int(zel * n * n + fel * n * n + tc + 16 * n * (2 * nrhs + 4) + workspace + (64 << 20))

@@ -1573,14 +1573,13 @@ __global__ void __launch_bounds__(256) k_convert_lower_c128(int64_t n, const dou
 
 // ---- C -= A B  (complex; C m x n, A m x k, B k x n; all column-major with ld) -------------
 constexpr int GT = 64, GK = 8;
+// the GT x GT tile at (bm, bn), by a CTA of 256 threads
 template <typename T, typename R>
-__global__ void __launch_bounds__(256) k_gemm_sub(T* C, int64_t ldc, const T* Am, int64_t lda,
-                                                  const T* Bm, int64_t ldb, int64_t m, int64_t n,
-                                                  int k) {
+__device__ __forceinline__ void gemm_tile(T* C, int64_t ldc, const T* Am, int64_t lda, const T* Bm, int64_t ldb, int64_t m,
+                                          int64_t n, int k, int64_t bm, int64_t bn) {
   __shared__ R As[2][GK][GT + 1];
   __shared__ R Bs[2][GK][GT + 1];
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int64_t bm = blockIdx.x * (int64_t)GT, bn = blockIdx.y * (int64_t)GT;
   R cr[4][4], ci[4][4];
   for (int i = 0; i < 4; ++i)
     for (int j = 0; j < 4; ++j) cr[i][j] = ci[i][j] = 0;
@@ -1629,6 +1628,22 @@ __global__ void __launch_bounds__(256) k_gemm_sub(T* C, int64_t ldc, const T* Am
         C[r + c * ldc] = cmk<T>(v.x - cr[i][j], v.y - ci[i][j]);
       }
     }
+}
+template <typename T, typename R>
+__global__ void __launch_bounds__(256) k_gemm_sub(T* C, int64_t ldc, const T* Am, int64_t lda, const T* Bm, int64_t ldb,
+                                                  int64_t m, int64_t n, int k) {
+  gemm_tile<T, R>(C, ldc, Am, lda, Bm, ldb, m, n, k, blockIdx.x * (int64_t)GT, blockIdx.y * (int64_t)GT);
+}
+// the tiles that tc_gemm64.cu leaves to the FP64 units: *count of GT rows x per GT columns, by (row, column) index
+__global__ void __launch_bounds__(256) k_gemm_tiles(const int2* list, const int* count, int per, double2* C, int64_t ldc,
+                                                    const double2* Am, int64_t lda, const double2* Bm, int64_t ldb,
+                                                    int64_t m, int64_t n, int k) {
+  const int64_t items = (int64_t)*count * per;
+  for (int64_t i = blockIdx.x; i < items; i += gridDim.x) {
+    const int2 t = list[i / per];
+    const int64_t bn = ((int64_t)t.y * per + i % per) * GT;
+    if (bn < n) gemm_tile<double2, double>(C, ldc, Am, lda, Bm, ldb, m, n, k, t.x * (int64_t)GT, bn);
+  }
 }
 
 // ---- triangular solves on one right-hand side ------------------------------------------
@@ -2906,6 +2921,13 @@ int lu_solve_fixed_scratch(beast_ctx* ctx, int64_t n, const T* A, int64_t lda, c
 }
 
 }  // namespace
+
+// tnt: columns of a listed tile (a multiple of GT); its rows are GT
+cudaError_t gemm64_tiles(const int2* list, const int* count, int tnt, double2* C, int64_t ldc, const double2* A, int64_t lda,
+                         const double2* B, int64_t ldb, int64_t m, int64_t n, int k, int grid, cudaStream_t st) {
+  k_gemm_tiles<<<(unsigned)grid, 256, 0, st>>>(list, count, tnt / GT, C, ldc, A, lda, B, ldb, m, n, k);
+  return cudaGetLastError();
+}
 
 int lu_factor_dev(beast_ctx* ctx, int64_t n, void* A, int64_t lda, int dtype, int* ipiv, int* info,
                   bool pivot, bool sym) {

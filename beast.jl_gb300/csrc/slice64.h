@@ -6,6 +6,16 @@
 //   x 2^-e = sum_i d_i 2^(-6 - 7 i) + r,   -64 <= d_i <= 64,   |r| <= 2^-56,
 // each exactly an FP16 number.  A product of two digits is at most 2^12, so a sum of up to 4096 of
 // them is an integer of at most 2^24 that FP32 accumulation holds exactly, whatever the order.
+//
+// Balance.  The digits cut a value relative to its row's largest, so a sum over k of a_ik b_kj whose
+// terms meet large a with small b (rows of a matrix in different units: a_ik ~ d_i / d_k, b_kj ~ d_k)
+// would lose what FP64 keeps.  The sum is therefore taken over (a_ik 2^-s_k) (b_kj 2^s_k) with 2^s_k
+// the power of two above the largest |a_ik| of column k: exact, and the same for every scaling of the
+// rows and columns by powers of two.
+// Spread.  What no such scaling levels (blocks of unknowns that are hardly coupled) is measured: the
+// sum S_ij over k of p_ik q_kj, p and q the magnitudes relative to 2^e of their row and column.  The
+// digits' error is at most about 2^-54 of the row's times the column's largest value, so relative to
+// sum |a_ik b_kj| it stays near FP64's own where S_ij is not far below one.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -42,6 +52,23 @@ SL_HD int row_exponent(uint32_t hi) {
   return (E > 0 ? E : 1) - 1022;
 }
 
+// s_k of a column whose largest abs_hi is hi (0 for a column that holds an infinity or a NaN)
+SL_HD int balance_exponent(uint32_t hi) {
+  const int e = row_exponent(hi);
+  return e == EXP_NONFINITE ? 0 : e;
+}
+// the exponent of x 2^s as a key that is ordered like it (a zero below every other value, what is not
+// finite above), and the exponent e of a row from its largest key: every |x| 2^s of the row < 2^e
+constexpr int KEY_ZERO = -(1 << 20);
+SL_HD int scaled_key(double x, int s) {
+  const int E = (int)(abs_hi(x) >> 20);
+  if (E >= 2047) return EXP_NONFINITE;
+  return (bits_of(x) << 1) == 0 ? KEY_ZERO : (E > 0 ? E : 1) - 1022 + s;
+}
+SL_HD int key_exponent(int key) {
+  return key >= EXP_NONFINITE / 2 ? EXP_NONFINITE : (key == KEY_ZERO ? -1021 : key);
+}
+
 // round(x 2^(55 - e)), ties up in magnitude; |x| < 2^e
 SL_HD int64_t fixed55(double x, int e) {
   const uint64_t u = bits_of(x);
@@ -66,6 +93,19 @@ SL_HD void digits(int64_t X, int d[SLICES]) {
     X = (X - d[i]) >> 7;
   }
   d[0] = (int)X;
+}
+
+// the magnitude of a complex value from its two fixed-point parts, relative to 2^e: 2^-24 at least (the
+// smallest FP16 number) unless both are exactly zero, at most 1
+constexpr float SPREAD_MIN = 0x1p-24f;
+// a tile with a sum 0 < S < SPREAD_LIMIT goes to the FP64 units.  Boundary-operator matrices (EFIE, MFIE
+// and Helmholtz, orders 480 to 6,007) have no sum below 2^-9.4; two blocks of unknowns coupled by 2^-9
+// lose 6 in the accuracy of the weak one there, by 2^-13 a hundred.
+constexpr float SPREAD_LIMIT = 0x1p-10f;
+SL_HD float spread_magnitude(int64_t X, int64_t Y, bool zero) {
+  const int64_t x = X < 0 ? -X : X, y = Y < 0 ? -Y : Y;
+  const float p = (float)(int32_t)((x > y ? x : y) >> 25) * 0x1p-30f;
+  return zero ? 0.f : (p > SPREAD_MIN ? p : SPREAD_MIN);
 }
 
 // the FP64 value -D 2^sh of an integer-valued FP32 number D, built from its bits (a conversion

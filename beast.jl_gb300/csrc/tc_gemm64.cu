@@ -12,10 +12,16 @@
 // = [[re, -im], [im, re]], B' columns hold (re, im) per k).  D_l is a sum of at most (l + 1) 2K
 // products of magnitude at most 2^12: with K <= 256 an integer of at most 2^24, exact in the FP32
 // accumulators.  What is dropped (digits beyond 2^-56 of the row's and the column's largest
-// magnitude, pairs i + j > 7) is below the rounding of an FP64 sum of the same length: measured
-// against 64-bit products in tests/test_gpu_lu_paths.py.
+// magnitude, pairs i + j > 7) is small against those two magnitudes, not against every entry's own sum.
+// Two things keep it below an FP64 sum's own rounding (slice64.h):
+//   - the columns of A are levelled by powers of two and the rows of B by their inverses before the
+//     digits are taken (k_balance): rows of a matrix in different units lose nothing.  Without it an
+//     order-300 system with half its rows scaled by 1e-8 came out with an error of 1e-9 (1e-15 with);
+//   - a ninth slice holds the entries' magnitudes; their product S is taken first, and a tile with a sum
+//     that is small against the tile's scale goes to the FP64 units (gemm64_tiles).
+// measured against LAPACK's solutions in tests/test_gpu_lu_paths.py.
 //
-// k_tc_gemm64: persistent CTAs over 128 x TNT tiles of C'; the levels run from the smallest
+// k_tc_gemm64: persistent CTAs over 128 x TNT tiles of C'; after S the levels run from the smallest
 // contribution (l = 7) to the largest, each as one K loop over its l + 1 digit pairs through the
 // 4-stage TMA ring into one of two TMEM accumulators, while four epilogue warps add the previous
 // level to C (one FP64 addition per value: -D 2^sh is built from the bits of D).  A tile's C
@@ -33,13 +39,19 @@
 #include "slice64.h"
 #include "tc_ptx.h"
 
+// the listed tiles of the update on the FP64 units (linalg.cu)
+cudaError_t gemm64_tiles(const int2* list, const int* count, int tnt, double2* C, int64_t ldc, const double2* A, int64_t lda,
+                         const double2* B, int64_t ldb, int64_t m, int64_t n, int k, int grid, cudaStream_t st);
+
 namespace {
 
 using slice64::SLICES;
+constexpr int PLANES = SLICES + 1;  // the digits and the magnitudes
 
 constexpr int TM = 128, TK = 64, STAGES = 4;
 constexpr int KMAX = 256;  // complex columns of A per launch: (l + 1) 2K 2^12 <= 2^24 for l = 7
 constexpr int A_BYTES = TM * TK * 2;
+constexpr int SPREAD = SLICES;  // the level of the magnitudes' product
 constexpr int GROUP = 8;  // row tiles taken together, column by column
 
 template <int TNT>
@@ -57,26 +69,31 @@ __device__ __forceinline__ void tile_at(int tile, int ntm, int ntn, int& mt, int
 }
 
 // M2 = 2M real rows of C' at Cr (ldr doubles per column), N columns; A' slice i at rows i M2, B'
-// slice j at rows j N of their tensor maps; nk stages of TK halves per digit pair
+// slice j at rows j N of their tensor maps; nk stages of TK halves per digit pair.  Tiles left to the FP64
+// units: their (row, column) tile indices in list, their number in count
 template <int TNT>
 __global__ void __launch_bounds__(192, 1)
     k_tc_gemm64(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double* Cr,
-                int64_t ldr, int M2, int N, const int* __restrict__ ea, const int* __restrict__ eb, int nk, int* status) {
+                int64_t ldr, int M2, int N, const int* __restrict__ ea, const int* __restrict__ eb, int nk, int2* list, int* count,
+                int* status) {
   constexpr int STAGE_BYTES = Tile<TNT>::STAGE_BYTES;
   extern __shared__ unsigned char smraw[];
   const uint32_t base = (smem_u32(smraw) + 1023u) & ~1023u;
   unsigned char* gbase = smraw + (base - smem_u32(smraw));
-  // full[STAGES], empty[STAGES], tfull[2], tempty[2], done
+  // full[STAGES], empty[STAGES], tfull[2], tempty[2], done, spread
   uint64_t* bars = reinterpret_cast<uint64_t*>(gbase + STAGES * STAGE_BYTES);
-  const int B_FULL = 0, B_EMPTY = STAGES, B_TFULL = 2 * STAGES, B_TEMPTY = 2 * STAGES + 2, B_DONE = 2 * STAGES + 4;
+  const int B_FULL = 0, B_EMPTY = STAGES, B_TFULL = 2 * STAGES, B_TEMPTY = 2 * STAGES + 2, B_DONE = 2 * STAGES + 4,
+            B_SPREAD = 2 * STAGES + 5;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 7);
-  __shared__ int s_abort_mem;
+  __shared__ int s_abort_mem, s_wide_mem[2];
+  volatile int* s_wide = s_wide_mem;  // by parity of a CTA's tiles: 1 + the last one left to the FP64 units
   volatile int* s_abort = &s_abort_mem;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntm = (M2 + TM - 1) / TM, ntn = (N + TNT - 1) / TNT, ntiles = ntm * ntn;
 
   if (threadIdx.x == 0) {
     *s_abort = 0;
+    s_wide[0] = s_wide[1] = 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(bars + B_FULL + s), 1);
       mbar_init(smem_u32(bars + B_EMPTY + s), 1);
@@ -86,6 +103,7 @@ __global__ void __launch_bounds__(192, 1)
       mbar_init(smem_u32(bars + B_TEMPTY + a), 4);  // one arrival per epilogue warp
     }
     mbar_init(smem_u32(bars + B_DONE), 1);
+    mbar_init(smem_u32(bars + B_SPREAD), 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -105,15 +123,15 @@ __global__ void __launch_bounds__(192, 1)
     for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x) {
       int mt, nt;
       tile_at(tile, ntm, ntn, mt, nt);
-      for (int l = SLICES - 1; l >= 0 && !*s_abort; --l)
-        for (int i = 0; i <= l && !*s_abort; ++i)
+      for (int l = SPREAD; l >= 0 && !*s_abort; --l)
+        for (int i = l == SPREAD ? SPREAD : 0; i <= l && !*s_abort; ++i)
           for (int kb = 0; kb < nk; ++kb, ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(smem_u32(bars + B_EMPTY + s), ((it / STAGES) & 1) ^ 1, status, s_abort)) break;
             const uint32_t sa = base + s * STAGE_BYTES, full = smem_u32(bars + B_FULL + s);
             mbar_expect_tx(full, STAGE_BYTES);
             tma_load_2d(sa, &tmA, kb * TK, i * M2 + mt * TM, full);
-            tma_load_2d(sa + A_BYTES, &tmB, kb * TK, (l - i) * N + nt * TNT, full);
+            tma_load_2d(sa + A_BYTES, &tmB, kb * TK, (l == SPREAD ? SPREAD : l - i) * N + nt * TNT, full);
           }
     }
     // no copy may still be landing in shared memory when the CTA exits (bounded, whatever the
@@ -127,12 +145,12 @@ __global__ void __launch_bounds__(192, 1)
     uint32_t it = 0;
     int t = 0;  // levels of all tiles, in order
     for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x)
-      for (int l = SLICES - 1; l >= 0 && !*s_abort; --l, ++t) {
+      for (int l = SPREAD; l >= 0 && !*s_abort; --l, ++t) {
         const int a = t & 1;
         if (!mbar_wait(smem_u32(bars + B_TEMPTY + a), ((t >> 1) & 1) ^ 1, status, s_abort)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + (uint32_t)(a * TNT);
-        const int steps = (l + 1) * nk;
+        const int steps = l == SPREAD ? nk : (l + 1) * nk;
         for (int kb = 0; kb < steps; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(smem_u32(bars + B_FULL + s), (it / STAGES) & 1, status, s_abort)) break;
@@ -153,9 +171,9 @@ __global__ void __launch_bounds__(192, 1)
   } else if (warp >= 2) {
     // ---- epilogue: warp w owns TMEM lanes 32 (w % 4) .. +31, a thread one real row of the tile
     const int q = warp & 3;
-    int t = 0;
+    int t = 0, ord = 0;
     bool live = true;
-    for (int tile = blockIdx.x; tile < ntiles && live; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < ntiles && live; tile += gridDim.x, ++ord) {
       int mt, nt;
       tile_at(tile, ntm, ntn, mt, nt);
       const int row = mt * TM + q * 32 + lane, n0 = nt * TNT;
@@ -163,7 +181,8 @@ __global__ void __launch_bounds__(192, 1)
       const int er = in ? ea[row >> 1] : 0;
       double* c0 = Cr + row + (int64_t)n0 * ldr;
       const int ncol = min(TNT, N - n0);
-      for (int l = SLICES - 1; l >= 0; --l, ++t) {
+      bool wide = false;  // the tile goes to the FP64 units: its levels are waited for and left out
+      for (int l = SPREAD; l >= 0; --l, ++t) {
         const int a = t & 1;
         if (!mbar_wait(smem_u32(bars + B_TFULL + a), (t >> 1) & 1, status, s_abort)) {
           live = false;
@@ -171,6 +190,38 @@ __global__ void __launch_bounds__(192, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * TNT);
+        auto release = [&]() {  // accumulator read: hand it back to the MMA warp
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bars + B_TEMPTY + a)) : "memory");
+        };
+        if (l == SPREAD) {
+          bool small = false;
+          for (int c = 0; c < ncol; c += 16) {
+            float v[16];
+            tmem_ld16(tb + (uint32_t)c, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) small |= c + j < ncol && v[j] > 0.f && v[j] < slice64::SPREAD_LIMIT;
+          }
+          release();
+          // the four warps agree
+          if (__any_sync(0xffffffffu, in && small) && lane == 0) s_wide[ord & 1] = ord + 1;
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bars + B_SPREAD)) : "memory");
+          if (!mbar_wait(smem_u32(bars + B_SPREAD), ord & 1, status, s_abort)) {
+            live = false;
+            break;
+          }
+          wide = s_wide[ord & 1] == ord + 1;
+          if (wide && q == 0 && lane == 0) list[atomicAdd(count, 1)] = make_int2(mt, nt);
+          continue;
+        }
+        if (wide) {
+          release();
+          continue;
+        }
         const int sh0 = er - 12 - 7 * l;
         for (int c = 0; c < ncol; c += 16) {
           float v[16];
@@ -196,11 +247,7 @@ __global__ void __launch_bounds__(192, 1)
             }
           }
         }
-        // accumulator read: hand it back to the MMA warp
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bars + B_TEMPTY + a)) : "memory");
+        release();
       }
     }
   }
@@ -221,25 +268,62 @@ __device__ __forceinline__ __half2 digits_h2(int lo, int hi) {
   return __hsub2(h, __half2half2(__ushort_as_half((unsigned short)0x6600)));
 }
 
+// s_k of the columns of A: the power of two above a column's largest magnitude, a column per CTA
+__global__ void __launch_bounds__(512) k_balance(const double2* A, int64_t lda, int64_t M, int* sk, int* count) {
+  __shared__ uint32_t red[16];
+  const double2* col = A + (int64_t)blockIdx.x * lda;
+  uint32_t mx = 0;
+#pragma unroll 4
+  for (int64_t m = threadIdx.x; m < M; m += 512) {
+    const double2 a = col[m];
+    mx = max(mx, max(slice64::abs_hi(a.x), slice64::abs_hi(a.y)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int j = 1; j < 16; ++j) mx = max(mx, red[j]);
+    sk[blockIdx.x] = slice64::balance_exponent(mx);
+    if (blockIdx.x == 0) *count = 0;
+  }
+}
+
+// the eight digits of (x, y) and the pair's magnitude: put(slice, digits of x, digits of y, magnitude)
+template <typename Put>
+__device__ __forceinline__ void slice_value(double2 a, int e, Put put) {
+  int dr[SLICES], di[SLICES];
+  const int64_t X = slice64::fixed55(a.x, e), Y = slice64::fixed55(a.y, e);
+  slice64::digits(X, dr);
+  slice64::digits(Y, di);
+#pragma unroll
+  for (int s = 0; s < SLICES; ++s) put(s, dr[s], di[s], 0.f);
+  const bool zero = ((slice64::bits_of(a.x) | slice64::bits_of(a.y)) << 1) == 0;
+  put(SPREAD, 0, 0, slice64::spread_magnitude(X, Y, zero));
+}
+
 // A' slices of 32 rows of A per CTA: row maxima, then 32 x 64 tiles transposed through shared
 // memory so that every warp writes whole row segments of each slice
-__device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, int M, int K, __half2* Ap, int* ea) {
-  __shared__ uint32_t red[8][33];
+__device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, int M, int K, const int* sk, __half2* Ap,
+                                        int* ea) {
+  __shared__ int red[8][33];
   __shared__ double2 tile[32][65];
-  __shared__ int s_e[32];
+  __shared__ int s_e[32], s_k[KMAX];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int m0 = bid * 32, m = m0 + lane;
-  uint32_t mx = 0;
+  if (threadIdx.x < K) s_k[threadIdx.x] = sk[threadIdx.x];
+  __syncthreads();
+  int key = slice64::KEY_ZERO;
   if (m < M)
     for (int k = w; k < K; k += 8) {
       const double2 a = A[m + (int64_t)k * lda];
-      mx = max(mx, max(slice64::abs_hi(a.x), slice64::abs_hi(a.y)));
+      key = max(key, max(slice64::scaled_key(a.x, -s_k[k]), slice64::scaled_key(a.y, -s_k[k])));
     }
-  red[w][lane] = mx;
+  red[w][lane] = key;
   __syncthreads();
   if (w == 0) {
-    for (int j = 1; j < 8; ++j) mx = max(mx, red[j][lane]);
-    s_e[lane] = slice64::row_exponent(mx);
+    for (int j = 1; j < 8; ++j) key = max(key, red[j][lane]);
+    s_e[lane] = slice64::key_exponent(key);
     if (m < M) ea[m] = s_e[lane];
   }
   __syncthreads();
@@ -259,16 +343,12 @@ __device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, 
         for (int h = 0; h < 2; ++h) {
           const int kk = lane + 32 * h, k = k0 + kk;
           if (k < K) {
-            const double2 a = tile[r][kk];
-            int dr[SLICES], di[SLICES];
-            slice64::digits(slice64::fixed55(a.x, e), dr);
-            slice64::digits(slice64::fixed55(a.y, e), di);
             __half2* row0 = Ap + (int64_t)(2 * mr) * K + k;  // 2K halves = K half2 per row
-#pragma unroll
-            for (int s = 0; s < SLICES; ++s) {
-              row0[(int64_t)s * 2 * M * K] = digits_h2(dr[s], -di[s]);
-              row0[(int64_t)s * 2 * M * K + K] = digits_h2(di[s], dr[s]);
-            }
+            slice_value(tile[r][kk], e + s_k[k], [&](int s, int dr, int di, float p) {
+              __half2* row = row0 + (int64_t)s * 2 * M * K;
+              row[0] = s < SLICES ? digits_h2(dr, -di) : __floats2half2_rn(p, 0.f);
+              row[K] = s < SLICES ? digits_h2(di, dr) : __floats2half2_rn(p, 0.f);
+            });
           }
         }
       }
@@ -278,94 +358,106 @@ __device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, 
 }
 
 // B' slices, one warp per column
-__device__ __forceinline__ void slice_b(int bid, const double2* B, int64_t ldb, int K, int N, __half2* Bp, int* eb) {
+__device__ __forceinline__ void slice_b(int bid, const double2* B, int64_t ldb, int K, int N, const int* sk, __half2* Bp,
+                                        int* eb) {
   const int lane = threadIdx.x & 31;
   const int j = bid * 8 + (threadIdx.x >> 5);
   if (j >= N) return;
   const double2* col = B + (int64_t)j * ldb;
-  uint32_t mx = 0;
-  for (int k = lane; k < K; k += 32) mx = max(mx, max(slice64::abs_hi(col[k].x), slice64::abs_hi(col[k].y)));
+  int key = slice64::KEY_ZERO;
+  for (int k = lane; k < K; k += 32) key = max(key, max(slice64::scaled_key(col[k].x, sk[k]), slice64::scaled_key(col[k].y, sk[k])));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const int e = slice64::row_exponent(mx);
+  for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
+  const int e = slice64::key_exponent(key);
   if (lane == 0) eb[j] = e;
-  for (int k = lane; k < K; k += 32) {
-    const double2 b = col[k];
-    int dr[SLICES], di[SLICES];
-    slice64::digits(slice64::fixed55(b.x, e), dr);
-    slice64::digits(slice64::fixed55(b.y, e), di);
-#pragma unroll
-    for (int s = 0; s < SLICES; ++s) Bp[((int64_t)s * N + j) * K + k] = digits_h2(dr[s], di[s]);
-  }
+  for (int k = lane; k < K; k += 32)
+    slice_value(col[k], e - sk[k], [&](int s, int dr, int di, float q) {
+      Bp[((int64_t)s * N + j) * K + k] = s < SLICES ? digits_h2(dr, di) : __floats2half2_rn(q, 0.f);
+    });
 }
 
 // both operands in one launch: CTAs [0, nA) 32 rows of A each, the rest 8 columns of B each
 __global__ void __launch_bounds__(256) k_slice(const double2* A, int64_t lda, const double2* B, int64_t ldb, int M,
-                                               int N, int K, __half2* Ap, int* ea, __half2* Bp, int* eb, int nA) {
+                                               int N, int K, const int* sk, __half2* Ap, int* ea, __half2* Bp, int* eb,
+                                               int nA) {
   if ((int)blockIdx.x < nA)
-    slice_a(blockIdx.x, A, lda, M, K, Ap, ea);
+    slice_a(blockIdx.x, A, lda, M, K, sk, Ap, ea);
   else
-    slice_b(blockIdx.x - nA, B, ldb, K, N, Bp, eb);
+    slice_b(blockIdx.x - nA, B, ldb, K, N, sk, Bp, eb);
 }
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 template <int TNT>
 int run(beast_ctx* ctx, const CUtensorMap& tmA, const __half2* Bp, double* Cr, int64_t ldr, int M2, int N, int K,
-        const int* ea, const int* eb) {
+        const int* ea, const int* eb, int2* list, int* count) {
   CUtensorMap tmB;
-  if (!make_map(&tmB, Bp, (uint64_t)2 * K, (uint64_t)SLICES * N, (uint64_t)2 * K * 2, TK, TNT, true,
+  if (!make_map(&tmB, Bp, (uint64_t)2 * K, (uint64_t)PLANES * N, (uint64_t)2 * K * 2, TK, TNT, true,
                 CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
     return beast_fail(ctx, BEAST_ERR_CUDA, "tensor map encode (B' slices) failed");
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tc_gemm64<TNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<TNT>::SMEM));
   const int tiles = ((M2 + TM - 1) / TM) * ((N + TNT - 1) / TNT);
   k_tc_gemm64<TNT><<<std::min(tiles, std::max(1, ctx->num_sms)), 192, Tile<TNT>::SMEM, ctx->stream>>>(
-      tmA, tmB, Cr, ldr, M2, N, ea, eb, 2 * K / TK, ctx->d_flag);
+      tmA, tmB, Cr, ldr, M2, N, ea, eb, 2 * K / TK, list, count, ctx->d_flag);
   BEAST_CUDA_TRY(ctx, cudaGetLastError());
   return BEAST_OK;
 }
 
 }  // namespace
 
-// bytes of workspace of an update with at most M rows and N columns
+// tiles of an M x N update at most (TNT = 64), and the workspace it takes
+static int64_t max_tiles(int64_t M, int64_t N) { return ((2 * M + TM - 1) / TM) * ((N + 63) / 64); }
 size_t tc_gemm64_work_bytes(int64_t M, int64_t N, int K) {
   const int64_t k = std::min(K, KMAX);
-  return al256((size_t)SLICES * M * k * 8) + al256((size_t)SLICES * N * k * 4) + al256((size_t)M * 4) + al256((size_t)N * 4);
+  return al256((size_t)PLANES * M * k * 8) + al256((size_t)PLANES * N * k * 4) + al256((size_t)M * 4) + al256((size_t)N * 4) +
+         al256(KMAX * 4) + al256((size_t)max_tiles(M, N) * 8 + 8);
 }
 
 // C -= A B (complex128): C at (M x N, ldc), A (M x K, lda), B (K x N, ldb), K a multiple of 32,
 // taken KMAX columns at a time.  A wait that runs out sets bit 4 of the context's status word.
 int tc_gemm64_sub(beast_ctx* ctx, double2* C, int64_t ldc, const double2* A, int64_t lda, const double2* B, int64_t ldb,
                   int64_t M, int64_t N, int K, void* work, size_t work_bytes) {
-  if (K % 32 != 0 || 2 * M * SLICES > INT32_MAX || N * SLICES > INT32_MAX || tc_gemm64_work_bytes(M, N, K) > work_bytes)
+  if (K % 32 != 0 || 2 * M * PLANES > INT32_MAX || N * PLANES > INT32_MAX || tc_gemm64_work_bytes(M, N, K) > work_bytes)
     return beast_fail(ctx, BEAST_ERR_ARG, "sliced FP64 update: unsupported block");
   for (int k0 = 0; k0 < K; k0 += KMAX) {
     const int k = std::min(KMAX, K - k0);
     char* w = static_cast<char*>(work);
-    __half2* Ap = reinterpret_cast<__half2*>(w);
-    w += al256((size_t)SLICES * M * k * 8);
-    __half2* Bp = reinterpret_cast<__half2*>(w);
-    w += al256((size_t)SLICES * N * k * 4);
-    int* ea = reinterpret_cast<int*>(w);
-    int* eb = reinterpret_cast<int*>(w + al256((size_t)M * 4));
+    auto take = [&](size_t bytes) {
+      char* p = w;
+      w += al256(bytes);
+      return p;
+    };
+    __half2* Ap = reinterpret_cast<__half2*>(take((size_t)PLANES * M * k * 8));
+    __half2* Bp = reinterpret_cast<__half2*>(take((size_t)PLANES * N * k * 4));
+    int* ea = reinterpret_cast<int*>(take((size_t)M * 4));
+    int* eb = reinterpret_cast<int*>(take((size_t)N * 4));
+    int* sk = reinterpret_cast<int*>(take(KMAX * 4));
+    int* count = reinterpret_cast<int*>(w);
+    int2* list = reinterpret_cast<int2*>(w) + 1;
+    const double2 *Ak = A + (int64_t)k0 * lda, *Bk = B + k0;
     {
-      // operands read once, 8 digits of 2 (A') and 1 (B') FP16 pairs written per element
-      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (16 + 64) + (double)N * k * (16 + 32));
+      // A read twice and B once, nine planes of 2 (A') and 1 (B') FP16 pairs written per element
+      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (32 + 72) + (double)N * k * (16 + 36));
       const int nA = (int)((M + 31) / 32), nB = (int)((N + 7) / 8);
-      k_slice<<<(unsigned)(nA + nB), 256, 0, ctx->stream>>>(A + (int64_t)k0 * lda, lda, B + k0, ldb, (int)M, (int)N, k, Ap,
-                                                            ea, Bp, eb, nA);
+      k_balance<<<(unsigned)k, 512, 0, ctx->stream>>>(Ak, lda, M, sk, count);
+      k_slice<<<(unsigned)(nA + nB), 256, 0, ctx->stream>>>(Ak, lda, Bk, ldb, (int)M, (int)N, k, sk, Ap, ea, Bp, eb, nA);
       BEAST_CUDA_TRY(ctx, cudaGetLastError());
     }
     CUtensorMap tmA;
-    if (!make_map(&tmA, Ap, (uint64_t)2 * k, (uint64_t)SLICES * 2 * M, (uint64_t)2 * k * 2, TK, TM, true,
+    if (!make_map(&tmA, Ap, (uint64_t)2 * k, (uint64_t)PLANES * 2 * M, (uint64_t)2 * k * 2, TK, TM, true,
                   CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
       return beast_fail(ctx, BEAST_ERR_CUDA, "tensor map encode (A' slices) failed");
-    ProfScope ps(ctx, PK_TCGEMM, 8.0 * k * (double)M * N);
-    const int64_t wide = ((2 * M + TM - 1) / TM) * ((N + 255) / 256);
-    double* Cr = reinterpret_cast<double*>(C);
-    const int rc = wide >= ctx->num_sms ? run<256>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb)
-                                        : run<64>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb);
-    if (rc) return rc;
+    const bool wide = ((2 * M + TM - 1) / TM) * ((N + 255) / 256) >= ctx->num_sms;
+    {
+      ProfScope ps(ctx, PK_TCGEMM, 8.0 * k * (double)M * N);
+      double* Cr = reinterpret_cast<double*>(C);
+      const int rc = wide ? run<256>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb, list, count)
+                          : run<64>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb, list, count);
+      if (rc) return rc;
+    }
+    ProfScope ps(ctx, PK_GEMM, 0.0);
+    BEAST_CUDA_TRY(ctx, gemm64_tiles(list, count, wide ? 256 : 64, C, ldc, Ak, lda, Bk, ldb, M, N, k,
+                                     std::max(1, 2 * ctx->num_sms), ctx->stream));
   }
   return BEAST_OK;
 }

@@ -51,6 +51,75 @@ def test_fp64_solve_is_invariant_under_column_scaling():
     assert np.array_equal(y * s, x)
 
 
+@pytest.mark.parametrize("n", [97, 577, 1345, 2113])
+def test_fp64_solve_backward_error_of_a_64_bit_lu(n):
+    """20 u: LAPACK leaves 2 to 10 u of these; one digit level less would be 300 u"""
+    A = _matrix(n, False, n + 7, dominance=0.0)
+    b = np.random.default_rng(n + 1).normal(size=(n, 2)) + 0j
+    x, _, _ = bg.solve(A, b, precision=bg.FP64)
+    assert np.linalg.norm(A @ x - b) <= 20 * 2.0 ** -53 * np.linalg.norm(A) * np.linalg.norm(x)
+
+
+def _exact(A, b, scale):
+    """the solution of A x = b to well below 64-bit rounding: residuals in extended precision, corrections
+    from a matrix without its row scale"""
+    M = np.linalg.inv(A / scale[:, None])
+    x = np.zeros(b.shape, dtype=np.clongdouble)
+    Al, bl = A.astype(np.clongdouble), b.astype(np.clongdouble)
+    for _ in range(5):
+        x = x + M @ ((bl - Al @ x) / scale).astype(np.complex128)
+    return x
+
+
+def _row_scales(n, which, rng):
+    s = np.ones(n)
+    if which == "border":  # half of them, the border inside a panel
+        s[n // 2 + 6:] = 2.0 ** -27
+    elif which == "shuffled":
+        s[rng.permutation(n)[: n // 2]] = 2.0 ** -40
+    elif which == "377":  # an unscaled electric / magnetic system
+        s[rng.permutation(n)[: n // 3]] = 377.0 ** -2
+    else:
+        s = 2.0 ** rng.integers(-40, 41, size=n)
+    return s
+
+
+@pytest.mark.parametrize("n", [300, 1089])
+@pytest.mark.parametrize("which", ["border", "shuffled", "377", "random"])
+def test_fp64_solve_of_scaled_rows(n, which):
+    """rows in different units: the forward error is that of a 64-bit LU with the same pivot rule (LAPACK's,
+    within a factor of 4 for the sums' other order and pivots that differ in near ties)"""
+    rng = np.random.default_rng(n)
+    s = _row_scales(n, which, rng)
+    A = _matrix(n, False, n, dominance=2.0) * s[:, None]
+    b = s * (rng.normal(size=n) + 1j * rng.normal(size=n))
+    x, _, _ = bg.solve(A, b, precision=bg.FP64)
+    ref = _exact(A, b, s)
+    err = np.linalg.norm(x - ref) / np.linalg.norm(ref)
+    lapack = np.linalg.norm(np.linalg.solve(A, b) - ref) / np.linalg.norm(ref)
+    assert err <= 4 * lapack
+
+
+@pytest.mark.parametrize("n,coupling,part", [(300, -20, 0.5), (2113, -33, 0.5), (2113, -33, 0.1)])
+def test_fp64_solve_of_weakly_coupled_blocks(n, coupling, part):
+    """two blocks of unknowns, numbered at random or one after the other, coupled by 2^coupling: no scaling of rows
+    and columns levels that, so the updates go to the FP64 units (all tiles, or those of the border); the part of
+    the solution that only the coupling excites keeps its own relative accuracy (LAPACK's, within a factor of 4)"""
+    rng = np.random.default_rng(n)
+    order = rng.permutation(n) if part == 0.5 else np.arange(n)
+    a, c = order[: int(part * n)], order[int(part * n):]
+    A = _matrix(n, False, n, dominance=2.0)
+    A[np.ix_(a, c)] *= 2.0 ** coupling
+    A[np.ix_(c, a)] *= 2.0 ** coupling
+    b = np.zeros(n, dtype=np.complex128)
+    b[c] = rng.normal(size=len(c)) + 1j * rng.normal(size=len(c))
+    x, _, _ = bg.solve(A, b, precision=bg.FP64)
+    ref, lap = _exact(A, b, np.ones(n)), np.linalg.solve(A, b)
+    for part_ in (a, c):
+        err, lapack = (np.linalg.norm(y[part_] - ref[part_]) for y in (x, lap))
+        assert err <= 4 * lapack
+
+
 @pytest.mark.parametrize("n,restart,dtype", [(1, 0, "c128"), (37, 5, "c128"), (63, 0, "c64"), (64, 1, "c128"), (65, 33, "c128"),
                                              (301, 0, "c64"), (1030, 7, "c128"), (2111, 0, "c128")])
 def test_gmres_at_the_edges_of_its_row_blocks(n, restart, dtype):
