@@ -181,10 +181,24 @@ __device__ __forceinline__ void panel_best(unsigned long long& key, int& idx, in
     }
   }
 }
+// |z|^2 in a range where it and its reciprocal are normal numbers
+__device__ __forceinline__ bool square_in_range(double den) { return den >= 0x1p-1000 && den <= 0x1p1000; }
+// 1 / z for any z by a power of two taken out of it (infinite below 2^-1024); zero for zero, NaN for what is
+// not finite
+__device__ __noinline__ double2 recip_scaled(double2 z) {
+  const double m = fmax(fabs(z.x), fabs(z.y));
+  if (m == 0.0) return make_double2(0.0, 0.0);
+  if (!(m <= 1.7976931348623157e308) || isnan(z.x) || isnan(z.y)) return make_double2(nan(""), nan(""));
+  const int e = ilogb(m);
+  const double x = scalbn(z.x, -e), y = scalbn(z.y, -e), den = x * x + y * y;
+  return make_double2(scalbn(x / den, -e), scalbn(-y / den, -e));
+}
 // (1 / piv) in the factorisation's arithmetic, by one division (an FP64 division is 30 instructions
-// on the column's chain); zero when |piv|^2 is zero
+// on the column's chain); zero for a zero pivot
 __device__ __forceinline__ double2 panel_recip(double2 piv) {
-  const double den = piv.x * piv.x + piv.y * piv.y, id = den != 0.0 ? 1.0 / den : 0.0;
+  const double den = piv.x * piv.x + piv.y * piv.y;
+  if (!square_in_range(den)) return recip_scaled(piv);
+  const double id = 1.0 / den;
   return make_double2(piv.x * id, -piv.y * id);
 }
 __device__ __forceinline__ float2 panel_recip(float2 piv) {
@@ -348,14 +362,15 @@ __global__ void __launch_bounds__(256) k_panel(T* A, int64_t lda, int64_t n, int
       if (lane == 0) {
         s_p = p;
         s_inv = inv;
-        s_go[jj & 1] = inv.x != 0 || inv.y != 0;
+        const bool over = isinf(inv.x) || isinf(inv.y);  // a pivot too small for its reciprocal: as a zero one
+        s_go[jj & 1] = !over && (inv.x != 0 || inv.y != 0);
         if (!ok) {
           s_bad = 1;
           atomicOr(status, 1);
         }
         if (blockIdx.x == 0) {
           ipiv[j] = p;
-          if (sing && *info == 0) *info = (int)j + 1;
+          if ((sing || over) && *info == 0) *info = (int)j + 1;
         }
       }
     }
@@ -1769,6 +1784,8 @@ __global__ void k_invert_diag(const T* A, int64_t lda, int64_t n, T* dinv) {
       T q;
       q.x = (v.x * d.x + v.y * d.y) / den;
       q.y = (v.y * d.x - v.x * d.y) / den;
+      if constexpr (sizeof(T) == 16)
+        if (!square_in_range(den) && (d.x != 0 || d.y != 0)) q = cmulx(v, recip_scaled(d));
       v = q;
     }
     x[i] = v;

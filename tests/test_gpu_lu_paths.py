@@ -60,6 +60,24 @@ def test_fp64_solve_backward_error_of_a_64_bit_lu(n):
     assert np.linalg.norm(A @ x - b) <= 20 * 2.0 ** -53 * np.linalg.norm(A) * np.linalg.norm(x)
 
 
+@pytest.mark.parametrize("n", [40, 300])
+@pytest.mark.parametrize("e", [-900, -520, -512, 508, 520, 900])
+def test_fp64_solve_far_from_one(n, e):
+    """matrices scaled by 2^e, where the square of a pivot or its reciprocal leaves the FP64 range: the
+    solution is the unscaled one's (a few roundings of the reciprocals apart, condition about 10)"""
+    A = _matrix(n, False, n, dominance=2.0)
+    b = np.random.default_rng(n).normal(size=n) + 0j
+    x, _, _ = bg.solve(A, b, precision=bg.FP64)
+    y, _, _ = bg.solve(A * 2.0 ** e, b, precision=bg.FP64)
+    assert np.linalg.norm(y * 2.0 ** e - x) <= 1e-13 * np.linalg.norm(x)
+
+
+def test_fp64_solve_refuses_a_pivot_without_a_reciprocal():
+    A = np.diag([1.0, 2.0, 1e-309, 3.0]).astype(np.complex128)
+    with pytest.raises(bg.BeastError):
+        bg.solve(A, np.ones(4), precision=bg.FP64)
+
+
 def _exact(A, b, scale):
     """the solution of A x = b to well below 64-bit rounding: residuals in extended precision, corrections
     from a matrix without its row scale"""
