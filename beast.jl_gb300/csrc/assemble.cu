@@ -4346,7 +4346,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
 //   G        re w / rho    c_jm = (-1)^m S_{2+j+2m} / (2m)!             im k w        (-1)^m S_{3+j+2m} / (2m+1)!
 //   grad G   re w / rho^3  c_jm = (-1)^m (1-2m) S_{j+2m} / (2m)!        im k w / rho^2  (-1)^m 2m S_{1+j+2m} / (2m+1)!
 // (one more power of xi with the double layers' factor n . rho).  Both sums of |a| over the pair's nodes,
-// taken first in FP32, set the integers' scales; integer sums do not depend on their order, so a pair may
+// taken first in FP32 (in FP64 where that cannot tell the distances), set the integers' scales; integer sums do not depend on their order, so a pair may
 // be one warp's or four's.  12 terms leave 1e-17 at k rho = 2; the host takes this kernel where
 // k (longest test edge + longest trial edge) <= 2, and k_near_ss64 elsewhere.  Measured: EFIE, 43,900
 // pairs at orders 5, 5, 4: 4.57 -> 2.04 ms; double layer on P1, 75,100 pairs at order 4: 7.56 -> 2.70.
@@ -4447,28 +4447,36 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
   const float* tabf = reinterpret_cast<const float*>(nodes + (int64_t)SSX_VALS * items);
   const double* ng = OPK == BEAST_HH_DL ? sgeo + 12 : tg + 12;
   const V3<double> nv = mk(ng[0], ng[1], ng[2]);
-  // ---- the scales: sums of |a| (every warp of the pair takes them over all nodes, in the same order)
-  float sa = 0.f, sb = 0.f;
+  // ---- the scales: sums of |a| (every warp of the pair takes them over all nodes, in the same order), in FP32
+  // where that knows rho well: to 3 parts in 1000 of 1/rho^3 while rho is at least 2^-10 of the terms it is the sum
+  // of.  A node below that (cells nearly on top of each other) takes the sums to FP64; they bound the integers.
+  auto exponent = [](double x) { return (int)((__double2hiint(1.01 * x) >> 20) & 0x7FF) - 1022; };
+  int ea, eb;
+  bool finite = true;
   {
-    float f[4][3];
+    float sa = 0.f, sb = 0.f, f[4][3], len2[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       f[k][0] = (float)E[k].x;
       f[k][1] = (float)E[k].y;
       f[k][2] = (float)E[k].z;
+      len2[k] = f[k][0] * f[k][0] + f[k][1] * f[k][1] + f[k][2] * f[k][2];
     }
     const float n0 = (float)nv.x, n1 = (float)nv.y, n2 = (float)nv.z;
+    bool flat = false;
     for (int it = lane; it < items; it += 32) {
       const float a = tabf[it], b = tabf[items + it], c = tabf[2 * items + it],
                   d = tabf[3 * items + it], w = fabsf(tabf[4 * items + it]);
       const float x = a * f[0][0] + b * f[1][0] - (c * f[2][0] + d * f[3][0]),
                   y = a * f[0][1] + b * f[1][1] - (c * f[2][1] + d * f[3][1]),
                   z = a * f[0][2] + b * f[1][2] - (c * f[2][2] + d * f[3][2]);
-      const float ir = rsqrtf(x * x + y * y + z * z);
+      const float rho2 = x * x + y * y + z * z, ir = rsqrtf(rho2);
+      const float size2 = a * a * len2[0] + b * b * len2[1] + c * c * len2[2] + d * d * len2[3];
+      flat |= !(rho2 > 0x1p-20f * size2);
       float q = w;
       if (GRAD) {
         q *= ir * ir;
-        if (!RT) q *= fabsf(n0 * x + n1 * y + n2 * z) + 1e-6f / ir;
+        if (!RT) q *= fabsf(n0 * x + n1 * y + n2 * z) + 1e-6f * sqrtf(size2);  // (the rounding of n . r)
       }
       sb += q;
       sa += q * ir;
@@ -4478,8 +4486,35 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
       sa += __shfl_xor_sync(0xffffffffu, sa, o);
       sb += __shfl_xor_sync(0xffffffffu, sb, o);
     }
+    double da = fsplit::f2d(sa), db = fsplit::f2d(sb);
+    if (__any_sync(0xffffffffu, flat)) {
+      da = db = 0.0;
+      for (int it = lane; it < items; it += 32) {
+        const double* nd = nodes + it;
+        V3<double> r = nd[0] * E[0] + nd[items] * E[1];
+        if (cls != 3) {
+          r = r - nd[3 * items] * E[3];
+          if (cls == 1) r = r - nd[2 * items] * E[2];
+        }
+        const double iR = rsqrt(dot(r, r));
+        double q = fabs(nd[4 * items]);
+        if (GRAD) {
+          q *= iR * iR;
+          if (!RT) q *= fabs(dot(nv, r));
+        }
+        db += q;
+        da += q * iR;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        da += __shfl_xor_sync(0xffffffffu, da, o);
+        db += __shfl_xor_sync(0xffffffffu, db, o);
+      }
+      finite = isfinite(da) && isfinite(db);
+    }
+    ea = exponent(da);
+    eb = exponent(db);
   }
-  const int ea = (int)(__float_as_uint(1.01f * sa) >> 23) - 126, eb = (int)(__float_as_uint(1.01f * sb) >> 23) - 126;
   const double k4 = 0.25 * P.wave.k * P.wave.k;
   // ---- the nodes
   int64_t Mr[NM], Mi[NM];
@@ -4544,7 +4579,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
   }
   if (lane < 2 * NM) {
     const double x = g64::from_fixed(tot + items / 2, (lane & 1 ? eb : ea) - 60);
-    s_tot[warp][lane] = lane & 1 ? P.wave.k * x : x;
+    s_tot[warp][lane] = !finite ? nan("") : lane & 1 ? P.wave.k * x : x;
   }
   __syncwarp();
   ss64_block<OPK, TK, BK>(P, np_, lane, pt, ps, tg, sgeo, s_tot[warp], s_T[warp]);

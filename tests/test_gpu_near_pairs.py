@@ -141,3 +141,30 @@ def test_balanced_beta_term(k, tol):
     Zr = bg.assemble(make(1j * k), X, X, precision=bg.FP64)
     scale = np.abs(bg.assemble(make(0.0), X, X, precision=bg.FP64)).max()
     assert np.abs(Z - Zr).max() <= tol * scale
+
+
+
+def _overlap(h, order):
+    """two cells with one shared vertex, the second the first scaled by one over the largest Gauss node and turned by
+    h about an axis in its plane: one quadrature node finds a distance of h"""
+    g = 0.5 + 0.5 * np.polynomial.legendre.leggauss(order)[0].max()
+    t = np.array([[1.0, 0.2, 0.3], [0.1, 0.9, -0.4]])
+    u, n = t.sum(0) / np.linalg.norm(t.sum(0)), np.cross(t[0], t[1]) / np.linalg.norm(np.cross(t[0], t[1]))
+    s = t / g + h * (t @ np.cross(n, u))[:, None] * n + h * n
+    return bg.Mesh(np.vstack([np.zeros(3), t, s]), np.array([[0, 1, 2], [0, 3, 4]], dtype=np.int32))
+
+
+@pytest.mark.parametrize("h", [1e-2, 1e-6, 1e-9])
+@pytest.mark.parametrize("kind", ["sl", "dl", "dlt"])
+def test_touching_cells_on_top_of_each_other(kind, h):
+    """the radially summed FP64 pairs size their integers from FP32 distances, which cells nearly on top of each other
+    leave no digits of: against the oracle within the FP64 contract plus the roundings of a distance h between
+    coordinates of size one, 40 u / h of the largest entry"""
+    m = _overlap(h, 4)
+    X = bg.lagrangecxd0(m)
+    op = {"sl": bg.Helmholtz3D.singlelayer, "dl": bg.Helmholtz3D.doublelayer,
+          "dlt": bg.Helmholtz3D.doublelayer_transposed}[kind](wavenumber=0.3)
+    qs = bg.DoubleNumSauterQstrat(2, 3, 4, 4, 4, 4)
+    Z = bg.assemble(op, X, X, quadstrat=qs, precision=bg.FP64)
+    Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), X, X)
+    assert np.abs(Z - Zo).max() <= (1e-10 + 40 * 2.0**-53 / h) * np.abs(Zo).max()
