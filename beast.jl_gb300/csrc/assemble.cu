@@ -4182,8 +4182,14 @@ __global__ void k_ss64_table(int cls, int n, int items, double* tab) {
 }
 
 // the block of a touching pair from its moments over (1, X0, X1) (1, Y0, Y1), tot_[2 (NB m + n)] re and im (the
-// sums of k_near_ss64's kr, ki); a shape pair per lane, T_ scratch of the warp
-template <int OPK, int TK, int BK>
+// sums of k_near_ss64's kr, ki); a shape pair per lane, T_ scratch of the warp.
+// Maxwell double layer: with x = o + X, y = o + Y from the shared vertex o, a_i = o - t_i, b_j = o - s_j
+//   f_i . ((x - y) x g_j) = (X x Y) . (a_i - b_j) + (X - Y) . (b_j x a_i),
+// where both X x Y and X - Y are small with |x - y|: the kernel's 1 / |x - y|^3 meets no large terms that cancel
+// (moments over the barycentric coordinates lost a factor of 4 on regular cells and 50 on flat ones).  On a common
+// edge X - Y = D0 e + X1 et2 - Y1 es2 and X x Y has no X0 Y0 term; the moment of D0 takes the place of (1, 1).
+// HAVE_T: T_ holds the moments over the barycentric coordinates already
+template <int OPK, int TK, int BK, bool HAVE_T = false>
 DEV void ss64_block(const NearParams& P, const NearPair& np_, int lane, const int* pt, const int* ps, const double* tg,
                     const double* sgeo, const double* tot_, C2<double>* T_) {
   constexpr bool RT = OPK == BEAST_MW_SL || OPK == BEAST_MW_DL;
@@ -4193,9 +4199,38 @@ DEV void ss64_block(const NearParams& P, const NearPair& np_, int lane, const in
   auto vert = [](const double* g, int k) { return mk(g[3 * k], g[3 * k + 1], g[3 * k + 2]); };
   const V3<double> A0 = vert(tg, pt[0]), A1 = vert(tg, pt[1]), A2 = vert(tg, pt[2]);
   const V3<double> B0 = vert(sgeo, ps[0]), B1 = vert(sgeo, ps[1]), B2 = vert(sgeo, ps[2]);
+  if constexpr (OPK == BEAST_MW_DL) {
+    if (lane < NM) {
+      const int cls = np_.cls;
+      auto tot = [&](int m, int n, double c, V3<double> v, V3<double>& re, V3<double>& im) {
+        re = re + (c * tot_[2 * (m * NB + n)]) * v;
+        im = im + (c * tot_[2 * (m * NB + n) + 1]) * v;
+      };
+      const V3<double> e1 = A1 - A0, e2 = A2 - A1, h1 = B1 - B0, h2 = B2 - B1;
+      V3<double> Vr = mk(0.0, 0.0, 0.0), Vi = Vr, Wr = Vr, Wi = Vr;  // sums of X - Y and X x Y
+      if (cls == 2) {
+        tot(0, 0, 1.0, e1, Vr, Vi);
+      } else {
+        tot(1, 0, 1.0, e1, Vr, Vi);
+        tot(0, 1, -1.0, h1, Vr, Vi);
+        tot(1, 1, 1.0, cross(e1, h1), Wr, Wi);
+      }
+      tot(2, 0, 1.0, e2, Vr, Vi);
+      tot(0, 2, -1.0, h2, Vr, Vi);
+      tot(1, 2, 1.0, cross(e1, h2), Wr, Wi);
+      tot(2, 1, 1.0, cross(e2, h1), Wr, Wi);
+      tot(2, 2, 1.0, cross(e2, h2), Wr, Wi);
+      const int m_ = lane / NB, n_ = lane % NB;
+      const V3<double> ai = A0 - vert(tg, pt[m_]), bj = B0 - vert(sgeo, ps[n_]), ab = ai - bj, c = cross(bj, ai);
+      const double fr = dot(Wr, ab) + dot(Vr, c), fi = dot(Wi, ab) + dot(Vi, c);
+      store_c<double>(P.zcell, zidx(zrow_of(P.zrow, np_.p, NT, pt[m_]), zcol_of(P.zcol, np_.q, NB, ps[n_]), P.ldc),
+                      C2<double>{-I4PI * fr, -I4PI * sg * fi}, P.zfmt);
+    }
+    return;
+  }
   // (1, X0, X1) -> barycentric (1 - X0, X0 - X1, X1) on both cells, a shape pair per lane
   const int m_ = lane / NB, n_ = lane % NB;
-  if (lane < NM) {
+  if (!HAVE_T && lane < NM) {
     auto tot = [&](int m, int n) { return C2<double>{tot_[2 * (m * NB + n)], tot_[2 * (m * NB + n) + 1]}; };
     auto row = [&](int m) {
       return NB == 3 && n_ < 2 ? csub(tot(m, n_), tot(m, n_ + 1)) : tot(m, n_);
@@ -4223,17 +4258,13 @@ DEV void ss64_block(const NearParams& P, const NearPair& np_, int lane, const in
         for (int dn = 1; dn < 3; ++dn) {
           const int m = (m_ + dm) % 3, n = (n_ + dn) % 3;
           const V3<double> em = tv(m) - ti, en = sv(n) - sj;
-          const double w = OPK == BEAST_MW_SL ? dot(em, en) : dot(em, cross(tv(m) - sv(n), en));
+          const double w = dot(em, en);
           const C2<double> T = T_[3 * m + n];
           fr = fma(w, T.re, fr);
           fi = fma(w, T.im, fi);
         }
-      if (OPK == BEAST_MW_SL) {
-        const C2<double> f{I4PI * fr, -sg * I4PI * fi}, m0{4.0 * I4PI * tot_[0], -sg * 4.0 * I4PI * tot_[1]};
-        z = cadd(cmul(C2<double>{P.op.ar, P.op.ai}, f), cmul(C2<double>{P.op.br, P.op.bi}, m0));
-      } else {
-        z = C2<double>{-I4PI * fr, -I4PI * sg * fi};
-      }
+      const C2<double> f{I4PI * fr, -sg * I4PI * fi}, m0{4.0 * I4PI * tot_[0], -sg * 4.0 * I4PI * tot_[1]};
+      z = cadd(cmul(C2<double>{P.op.ar, P.op.ai}, f), cmul(C2<double>{P.op.br, P.op.bi}, m0));
     }
     store_c<double>(P.zcell, zidx(zrow_of(P.zrow, np_.p, NT, i), zcol_of(P.zcol, np_.q, NB, j), P.ldc), z, P.zfmt);
   }
@@ -4302,7 +4333,8 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
         for (int m = 0; m < NT; ++m)
 #pragma unroll
           for (int n = 0; n < NB; ++n) {
-            const double w = nd[(int64_t)(4 + 3 * m + n) * items];
+            double w = nd[(int64_t)(4 + 3 * m + n) * items];
+            if (OPK == BEAST_MW_DL && m + n == 0) w *= nd[0];  // D0 (ss64_block)
             M[m * NB + n].re = fma(w, kr, M[m * NB + n].re);
             M[m * NB + n].im = fma(w, ki, M[m * NB + n].im);
           }
@@ -4542,7 +4574,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
     const int64_t a = g64::to_fixed(b * iR, ea), bx = g64::to_fixed(b, eb), u = g64::to_fixed(R2 * k4, 0);
     const int64_t* pp = reinterpret_cast<const int64_t*>(nd) + 5 * items;
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
+    for (int j = OPK == BEAST_MW_DL ? 1 : 0; j < NJ; ++j) {
       int64_t tr = g64::mulhi(a, ssx_poly(cf + SSX_TERMS * j, u)), ti = g64::mulhi(bx, ssx_poly(cf + SSX_TERMS * (3 + j), u));
       if (j == 0) {
         Mr[0] += tr;
@@ -4550,6 +4582,11 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
       }
       tr <<= 2;
       ti <<= 2;
+      if (OPK == BEAST_MW_DL && j == 1) {  // D0 (ss64_block)
+        const int64_t x = g64::to_fixed(nd[0], 0);
+        Mr[0] += g64::mulhi(tr, x);
+        Mi[0] += g64::mulhi(ti, x);
+      }
 #pragma unroll
       for (int m = 0; m < NT; ++m)
 #pragma unroll
@@ -4577,12 +4614,31 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
     if (warp > 0) return;
     if (lane < 2 * NM) tot = (s_sum[0][lane] + s_sum[1][lane]) + (s_sum[2][lane] + s_sum[3][lane]);
   }
+  // (1, X0, X1) -> barycentric coordinates in the integers: the differences are exact
+  auto value = [&](int64_t v, int im) {
+    const double x = g64::from_fixed(v, (im ? eb : ea) - 60);
+    return !finite ? nan("") : im ? P.wave.k * x : x;
+  };
+  if (W > 1) __syncwarp();
   if (lane < 2 * NM) {
-    const double x = g64::from_fixed(tot + items / 2, (lane & 1 ? eb : ea) - 60);
-    s_tot[warp][lane] = !finite ? nan("") : lane & 1 ? P.wave.k * x : x;
+    tot += items / 2;
+    s_sum[warp][lane] = tot;
+    s_tot[warp][lane] = value(tot, lane & 1);
   }
   __syncwarp();
-  ss64_block<OPK, TK, BK>(P, np_, lane, pt, ps, tg, sgeo, s_tot[warp], s_T[warp]);
+  if (lane < NM) {
+    const int m = lane / NB, n = lane % NB;
+    auto part = [&](int im) {
+      auto row = [&](int r) {
+        const int64_t* t = s_sum[warp] + 2 * r * NB + im;
+        return NB == 3 && n < 2 ? t[2 * n] - t[2 * n + 2] : t[2 * n];
+      };
+      return value(NT == 3 && m < 2 ? row(m) - row(m + 1) : row(m), im);
+    };
+    s_T[warp][lane] = C2<double>{part(0), part(1)};
+  }
+  __syncwarp();
+  ss64_block<OPK, TK, BK, true>(P, np_, lane, pt, ps, tg, sgeo, s_tot[warp], s_T[warp]);
 }
 
 template <int OPK, int TK, int BK>

@@ -168,3 +168,20 @@ def test_touching_cells_on_top_of_each_other(kind, h):
     Z = bg.assemble(op, X, X, quadstrat=qs, precision=bg.FP64)
     Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), X, X)
     assert np.abs(Z - Zo).max() <= (1e-10 + 40 * 2.0**-53 / h) * np.abs(Zo).max()
+
+
+@pytest.mark.parametrize("wavenumber", [0.4, 3.0])
+def test_maxwell_double_layer_on_long_thin_cells(wavenumber):
+    """a staircase of strips of length 1 and width h = 1e-3, neighbours at right angles (k rho up to 2 and above: both
+    FP64 kernels of touching pairs): the kernel's 1 / |x - y|^3 meets no cancelling terms beyond the roundings of h
+    itself, 40 u / h of the largest entry"""
+    h = 1e-3
+    yz = np.cumsum([[0, 0]] + [[h, 0], [0, h]] * 3, axis=0)
+    v = np.array([[x, y, z] for y, z in yz for x in (0.0, 1.0)])
+    c = [t for i in range(len(yz) - 1) for t in ([2 * i, 2 * i + 1, 2 * i + 2], [2 * i + 1, 2 * i + 3, 2 * i + 2])]
+    q, _ = np.linalg.qr(np.random.default_rng(2).normal(size=(3, 3)))
+    X = bg.raviartthomas(bg.Mesh(v @ q, np.array(c, dtype=np.int32)))
+    op, qs = bg.Maxwell3D.doublelayer(wavenumber=wavenumber), bg.DoubleNumSauterQstrat(2, 3, 4, 4, 4, 4)
+    Z = bg.assemble(op, X, X, quadstrat=qs, precision=bg.FP64)
+    Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), X, X)
+    assert np.abs(Z - Zo).max() <= 40 * 2.0**-53 / h * np.abs(Zo).max()
