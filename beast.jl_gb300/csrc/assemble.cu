@@ -4403,23 +4403,45 @@ __global__ void k_ssx_table(int cls, int n, int items, double* tab) {
   for (int q = 0; q < 8; ++q)
     tab[(int64_t)(5 + q) * items + it] = __longlong_as_double(p[q] >= 1.0 ? (int64_t)1 << 62 : g64::to_fixed(p[q], 0));
 }
-// kind 0: G, 1: grad G, 2: grad G with one more power of xi; coefficients of (u / 4)^m
+// a sum of two doubles (built once per context: not a matter of speed)
+struct Dd {
+  double h, l;
+};
+DEV Dd dd_norm(double h, double l) {
+  const double s = h + l;
+  return Dd{s, l - (s - h)};
+}
+DEV Dd dd_mul(Dd a, double x) {
+  const double p = a.h * x;
+  return dd_norm(p, fma(a.h, x, -p) + a.l * x);
+}
+DEV Dd dd_div(Dd a, double x) {
+  const double q = a.h / x;
+  return dd_norm(q, (fma(-q, x, a.h) + a.l) / x);
+}
+DEV Dd dd_add(Dd a, Dd b) {
+  const double s = a.h + b.h, z = s - a.h;
+  return dd_norm(s, ((a.h - (s - z)) + (b.h - z)) + (a.l + b.l));
+}
+// kind 0: G, 1: grad G, 2: grad G with one more power of xi; coefficients of (u / 4)^m, to the last of their 62 bits
+// (their rounding is common to all nodes; as doubles they set the error of a double layer's entries)
 __global__ void k_ssx_coef(int n, int kind, int64_t* out) {
   const int row = threadIdx.x / SSX_TERMS, m = threadIdx.x % SSX_TERMS, im = row / 3;
   if (row >= SSX_ROWS) return;
   const double *x = c_gl_x + c_gl_off[n - 1], *w = c_gl_w + c_gl_off[n - 1];
   const int p = (kind == 0 ? 2 : kind - 1) + row % 3 + im + 2 * m;
-  double c = 0.0;
+  Dd c{0.0, 0.0};
   for (int i = 0; i < n; ++i) {
-    double t = w[i];
-    for (int k = 0; k < p; ++k) t *= x[i];
-    c += t;
+    Dd t{w[i], 0.0};
+    for (int k = 0; k < p; ++k) t = dd_mul(t, x[i]);
+    c = dd_add(c, t);
   }
-  for (int k = 2; k <= 2 * m + im; ++k) c /= k;
-  for (int k = 0; k < m; ++k) c *= 4.0;
-  if (kind) c *= im ? 2 * m : 1 - 2 * m;
-  if (m & 1) c = -c;
-  out[threadIdx.x] = fabs(c) >= 1.0 ? (c < 0 ? -1 : 1) * ((int64_t)1 << 62) : g64::to_fixed(c, 0);
+  for (int k = 2; k <= 2 * m + im; ++k) c = dd_div(c, k);
+  for (int k = 0; k < m; ++k) c = dd_mul(c, 4.0);
+  if (kind) c = dd_mul(c, im ? 2 * m : 1 - 2 * m);
+  if (m & 1) c = dd_mul(c, -1.0);
+  const int64_t h = fabs(c.h) >= 1.0 ? (c.h < 0 ? -1 : 1) * ((int64_t)1 << 62) : g64::to_fixed(c.h, 0);
+  out[threadIdx.x] = fabs(c.h) > 1.0 ? h : h + __double2ll_rn(c.l * 0x1p62);
 }
 DEV int64_t ssx_poly(const int64_t* c, int64_t u) {
   int64_t q = c[SSX_TERMS - 1];
@@ -4580,8 +4602,8 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ssx(NearParams P) {
         Mr[0] += tr;
         Mi[0] += ti;
       }
-      tr <<= 2;
-      ti <<= 2;
+      tr = (tr << 2) + 2;  // (with the mean of the truncation, which would add up over the nodes)
+      ti = (ti << 2) + 2;
       if (OPK == BEAST_MW_DL && j == 1) {  // D0 (ss64_block)
         const int64_t x = g64::to_fixed(nd[0], 0);
         Mr[0] += g64::mulhi(tr, x);

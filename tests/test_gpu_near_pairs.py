@@ -185,3 +185,13 @@ def test_maxwell_double_layer_on_long_thin_cells(wavenumber):
     Z = bg.assemble(op, X, X, quadstrat=qs, precision=bg.FP64)
     Zo = O.assemble(O.make_op(op.kind, op.gamma, op.alpha, op.beta), O.OrcQs(*qs.orders()), X, X)
     assert np.abs(Z - Zo).max() <= 40 * 2.0**-53 / h * np.abs(Zo).max()
+
+
+def test_integer_sums_of_touching_pairs_do_not_drift():
+    """touching P1 pairs are differences of integer moments, sums of thousands of truncated products: the static kernel
+    against the same rule node by node in FP64 (a real part of 1e-300 takes that route), 4 u of the largest entry
+    each: 1 / R, the weight and the three factors of a block"""
+    X = bg.lagrangec0d1(_mesh())
+    qs = WS(2, 3, 6, 7, 5, 5, 4, 3)
+    Z, Zn = (bg.assemble(bg.Helmholtz3D.singlelayer(gamma=g), X, X, quadstrat=qs, precision=bg.FP64) for g in (0.0, 1e-300))
+    assert np.abs(Z - Zn).max() <= 8 * 2.0**-53 * np.abs(Zn).max()
