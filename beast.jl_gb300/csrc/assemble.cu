@@ -3174,7 +3174,7 @@ static cudaError_t far64_launch(FarParams P, int fmt, cudaStream_t st) {
               sizeof(double) * 3 * FAR_THREADS * P.ro.n;
   if (FIX && OPK == BEAST_MW_NXDL) sm += sizeof(int64_t) * FAR_THREADS * P.ro.n;
   if (FIX) sm += sizeof(float) * 3 * (P.qt * P.ri.n + FAR_THREADS * P.ro.n);
-  cudaError_t e = cudaFuncSetAttribute(k_far64<OPK, TK, BK, FIX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_shared((const void*)k_far64<OPK, TK, BK, FIX>);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)gx, (unsigned)((P.nq + P.qt - 1) / P.qt));
   k_far64<OPK, TK, BK, FIX><<<grid, FAR_THREADS, sm, st>>>(P);
@@ -3485,7 +3485,8 @@ cudaError_t launch_far_batch(const BatchLaunch& L, cudaStream_t st) {
   const int th = ((L.tile_m + 31) / 32) * 32;
   const bool f32 = L.precision == BEAST_MIXED;
   auto go = [&](void (*kernel)(BatchLaunch), size_t sm) {
-    if (sm > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_shared((const void*)kernel);
+    if (e != cudaSuccess) return e;
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, th, sm);
     kernel<<<std::max(1, std::min(L.ntiles, sm_count() * per_sm)), th, sm, st>>>(L);

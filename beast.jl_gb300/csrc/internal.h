@@ -90,6 +90,19 @@ struct beast_mesh {
   double edge_min = 0.0, edge_max = 1e300;  // shortest and longest edge of a cell
 };
 
+// allows a kernel all the dynamic shared memory that the device gives it.  The limit belongs to the kernel, not to
+// a launch: set to one launch's size it is taken from under the launch of another host thread.
+inline cudaError_t allow_shared(const void* kernel) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+  return e;
+}
+
 // per active cell geometry, 16 doubles: v0 v1 v2 (9) | centroid (3) | unit normal (3) | area
 enum { GEO_STRIDE = 16 };
 

@@ -2564,7 +2564,7 @@ int lu_factor_t(beast_ctx* ctx, int64_t n, T* A, int64_t lda, int* ipiv, int* in
   }
   const size_t panel_smem = (size_t)(std::max<int64_t>(rows0, PANEL_ROWS) * (nb + 1) + 3 * nb) * sizeof(T);
   if (pivot)
-    BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem));
+    BEAST_CUDA_TRY(ctx, allow_shared((const void*)k_panel<T>));
   // unpivoted c64 with 64-wide panels: k_lu_inv64 also inverts the block's triangles and
   // k_panel_apply does both triangular solves (and the FP16 operands of the in-block update)
   const bool apply_path = !pivot && sizeof(T) == 8 && nb == TRI;
