@@ -1220,6 +1220,25 @@ int beast_solve_dense(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int
   return rc;
 }
 
+// what a GMRES call holds: every way out of the call waits for the stream (a copy into the context's pinned buffer
+// may be on its way) and gives it back
+struct GmresHold {
+  cudaStream_t st;
+  cudaEvent_t ready = nullptr;
+  std::vector<void*> bufs;
+  cudaError_t alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMallocAsync(p, bytes, st);
+    if (e == cudaSuccess) bufs.push_back(*p);
+    return e;
+  }
+  ~GmresHold() {
+    cudaStreamSynchronize(st);
+    if (ready) cudaEventDestroy(ready);
+    for (void* p : bufs) cudaFreeAsync(p, st);
+    cudaStreamSynchronize(st);
+  }
+};
+
 // restarted GMRES: classical Gram-Schmidt with one reorthogonalisation (linalg.cu, no host round
 // trip inside an iteration) and Givens rotations on the host (the Hessenberg matrix is tiny).  The
 // host reads an iteration's coefficients while the next basis vector's matvec, queued before the
@@ -1236,15 +1255,16 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
   const int c64 = a_dtype == BEAST_C64;
   double *V = nullptr, *w = nullptr, *db = nullptr, *dx = nullptr, *h = nullptr, *nrm = nullptr;
   void* work = nullptr;
-  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&V, (size_t)n * (m + 1) * 16, st));
-  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&w, n * 16, st));
-  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&h, (size_t)(m + 2) * 32 + 64, st));
-  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&nrm, 64, st));
-  BEAST_CUDA_TRY(ctx, cudaMallocAsync(&work, gmres_work_bytes(n, m), st));
+  std::lock_guard<std::mutex> pinned_lock(ctx->pinned_mtx);  // released after hold has waited
+  GmresHold hold{st};
+  BEAST_CUDA_TRY(ctx, hold.alloc((void**)&V, (size_t)n * (m + 1) * 16));
+  BEAST_CUDA_TRY(ctx, hold.alloc((void**)&w, n * 16));
+  BEAST_CUDA_TRY(ctx, hold.alloc((void**)&h, (size_t)(m + 2) * 32 + 64));
+  BEAST_CUDA_TRY(ctx, hold.alloc((void**)&nrm, 64));
+  BEAST_CUDA_TRY(ctx, hold.alloc((void**)&work, gmres_work_bytes(n, m)));
   unsigned int* count = reinterpret_cast<unsigned int*>(nrm + 4);
   BEAST_CUDA_TRY(ctx, cudaMemsetAsync(nrm, 0, 64, st));
   const size_t pin = (size_t)(m + 2) * 32 + 64;
-  std::lock_guard<std::mutex> pinned_lock(ctx->pinned_mtx);
   if (ctx->pinned_size < pin) {
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     ctx->pinned = nullptr;
@@ -1253,11 +1273,11 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
     ctx->pinned_size = pin;
   }
   double* hh = static_cast<double*>(ctx->pinned);
-  cudaEvent_t ready;
-  BEAST_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+  BEAST_CUDA_TRY(ctx, cudaEventCreateWithFlags(&hold.ready, cudaEventDisableTiming));
+  const cudaEvent_t ready = hold.ready;
   if (bx_loc != BEAST_DEVICE) {
-    BEAST_CUDA_TRY(ctx, cudaMallocAsync(&db, n * 16, st));
-    BEAST_CUDA_TRY(ctx, cudaMallocAsync(&dx, n * 16, st));
+    BEAST_CUDA_TRY(ctx, hold.alloc((void**)&db, n * 16));
+    BEAST_CUDA_TRY(ctx, hold.alloc((void**)&dx, n * 16));
     BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(db, b, n * 16, cudaMemcpyHostToDevice, st));
   } else {
     db = (double*)b;
@@ -1281,7 +1301,7 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
     int k = 0, slabs = 0;
     BEAST_CUDA_TRY(ctx, gmres_matvec(n, A, lda, c64, w, nrm, V, work, &slabs, st));
     for (; k < m && it < maxiter; ++k) {
-      BEAST_CUDA_TRY(ctx, gmres_orthogonalise(n, k, m, slabs, V, w, work, count, h, st));
+      BEAST_CUDA_TRY(ctx, gmres_orthogonalise(n, k, slabs, V, w, work, count, h, st));
       const int kk = k + 1;
       BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(hh, h, (size_t)kk * 32 + 8, cudaMemcpyDeviceToHost, st));
       BEAST_CUDA_TRY(ctx, cudaEventRecord(ready, st));
@@ -1323,19 +1343,8 @@ int beast_gmres(beast_ctx* ctx, int64_t n, const void* A, int64_t lda, int a_dty
     BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(h, yh.data(), k * 16, cudaMemcpyHostToDevice, st));
     BEAST_CUDA_TRY(ctx, vec_gemv_sub(n, k, V, n, h, dx, st));
   }
-  cudaEventDestroy(ready);
   if (bx_loc != BEAST_DEVICE) BEAST_CUDA_TRY(ctx, cudaMemcpyAsync(x, dx, n * 16, cudaMemcpyDeviceToHost, st));
   BEAST_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-  cudaFreeAsync(V, st);
-  cudaFreeAsync(w, st);
-  cudaFreeAsync(h, st);
-  cudaFreeAsync(nrm, st);
-  cudaFreeAsync(work, st);
-  if (bx_loc != BEAST_DEVICE) {
-    cudaFreeAsync(db, st);
-    cudaFreeAsync(dx, st);
-  }
-  cudaStreamSynchronize(st);
   if (iters) *iters = it;
   if (resid) *resid = rel;
   if (rel > reltol) return beast_fail(ctx, BEAST_ERR_NOCONV, "GMRES did not converge");

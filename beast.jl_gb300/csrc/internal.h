@@ -343,7 +343,7 @@ cudaError_t vec_norm2(int64_t n, const double* x, double* out, cudaStream_t st);
 size_t gmres_work_bytes(int64_t n, int m);
 cudaError_t gmres_matvec(int64_t n, const void* A, int64_t lda, int a_c64, const double* w, const double* norm2,
                          double* vk, void* work, int* slabs, cudaStream_t st);
-cudaError_t gmres_orthogonalise(int64_t n, int k, int m, int slabs, const double* V, double* w, void* work,
+cudaError_t gmres_orthogonalise(int64_t n, int k, int slabs, const double* V, double* w, void* work,
                                 unsigned int* count, double* out, cudaStream_t st);
 // w -= V h (m columns)
 cudaError_t vec_gemv_sub(int64_t n, int m, const double* V, int64_t ldv, const double* h,

@@ -3064,7 +3064,7 @@ cudaError_t gmres_matvec(int64_t n, const void* A, int64_t lda, int a_c64, const
   return cudaGetLastError();
 }
 // w = A v_k from the slabs, orthogonalised twice against v_0 .. v_k: out = h1 (k + 1 complex), h2, |w|^2
-cudaError_t gmres_orthogonalise(int64_t n, int k, int m, int slabs, const double* V, double* w, void* work,
+cudaError_t gmres_orthogonalise(int64_t n, int k, int slabs, const double* V, double* w, void* work,
                                 unsigned int* count, double* out, cudaStream_t st) {
   double* slab = static_cast<double*>(work);
   double* part = slab + (size_t)MV_MAX_SLABS * n * 2 + (size_t)n * 2;
@@ -3073,7 +3073,6 @@ cudaError_t gmres_orthogonalise(int64_t n, int k, int m, int slabs, const double
   k_gm_step<<<nb, GM_THREADS, 0, st>>>(0, n, k + 1, slabs, slab, V, w, nullptr, part, count, out);
   k_gm_step<<<nb, GM_THREADS, 0, st>>>(1, n, k + 1, slabs, slab, V, w, out, part, count, h2);
   k_gm_step<<<nb, GM_THREADS, 0, st>>>(2, n, k + 1, slabs, slab, V, w, h2, part, count, h2 + 2 * (k + 1));
-  (void)m;
   return cudaGetLastError();
 }
 

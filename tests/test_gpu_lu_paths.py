@@ -158,6 +158,35 @@ def test_gmres_zero_right_hand_side_and_limit():
         bg.gmres(A, np.ones(70), reltol=1e-14, restart=4, maxiter=6)
 
 
+_GMRES_OOM = r"""
+import ctypes as C, torch, beastgpu as bg
+ctx = bg.get_context(0)
+def used():
+    v = [C.c_size_t() for _ in range(4)]
+    ctx.check(ctx.lib.beast_pool_stats(ctx.handle, *[C.byref(x) for x in v]))
+    return v[2].value
+t = torch.zeros(64, dtype=torch.complex128, device="cuda")
+_, total = torch.cuda.mem_get_info()
+n = int(0.6 * total) // 1060  # the matvec's sums take 1 KiB a row, the basis of 66 vectors as much: 1.2 of the memory
+before = used()
+it, res = C.c_int(), C.c_double()
+rc = ctx.lib.beast_gmres(ctx.handle, n, t.data_ptr(), n, bg.C128, t.data_ptr(), t.data_ptr(), bg.lib.DEVICE, 1e-8, 65,
+                         65, C.byref(it), C.byref(res))
+print(rc == bg.lib.ERR_OOM, used() - before)
+"""
+
+
+def test_gmres_out_of_memory_gives_everything_back():
+    """a call that fails in the middle of its allocations (an order beyond the device's memory; nothing of it is read)
+    leaves none of them behind"""
+    import os
+    import subprocess
+    import sys
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join(sys.path))
+    r = subprocess.run([sys.executable, "-c", _GMRES_OOM], env=env, capture_output=True, text=True, timeout=300)
+    assert r.stdout.split() == ["True", "0"], (r.stdout, r.stderr[-2000:])
+
+
 @pytest.mark.parametrize("symmetric", [True, False])
 @pytest.mark.parametrize("n,col", [(300, 64), (300, 65), (300, 127), (65, 64), (130, 129)])
 def test_zero_pivot_of_a_pair(n, col, symmetric, monkeypatch):
