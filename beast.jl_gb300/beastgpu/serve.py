@@ -39,18 +39,31 @@ import numpy as np
 from . import lib as L
 
 
+def _solve_scratch(n, nrhs, element):
+    """device bytes of a solve with given factors of `element` bytes a value: the matvec's 64 partial sums a row and
+    its split vector, the triangular solves of up to eight right-hand sides at a time, right-hand sides, solutions
+    and refinement vectors"""
+    return n * (1040 + 8 * element) + 16 * n * (2 * nrhs + 4)
+
+
+def update_operands(n, precision):
+    """device bytes of the tensor-core operands of the largest trailing update: 12 bytes per row and column of K <= 1024
+    on the mixed paths, 108 of K <= 256 in FP64"""
+    if precision == L.FP64:
+        return 108 * 256 * n if n > 64 else 0
+    return 12 * 1024 * n if n > 1024 else 0
+
+
 def job_footprint(n, nrhs=1, precision=L.MIXED, workspace=0):
-    """device bytes a job holds at its peak: the matrix, the factor copy, the tensor-core
-    operands of the largest trailing update (12 bytes per row and column of K <= 1024 on the mixed
-    paths, 108 of K <= 256 in FP64), the right-hand sides / solutions /
-    refinement vectors, the context's assembly workspace, and 64 MiB of small buffers"""
+    """device bytes a job holds at its peak: the matrix, the factor copy (whole 128-byte lines a column) with its
+    pivots and the inverses of its diagonal blocks, the tensor-core operands, the solve's scratch, the panels' exchange
+    slots, the context's assembly workspace, and 64 MiB of small buffers"""
     zel = 8 if precision == L.MIXED else 16
     fel = 16 if precision == L.FP64 else 8
-    if precision == L.FP64:
-        tc = 108 * 256 * n if n > 64 else 0
-    else:
-        tc = 12 * 1024 * n if n > 1024 else 0
-    return int(zel * n * n + fel * n * n + tc + 16 * n * (2 * nrhs + 4) + workspace + (64 << 20))
+    factor = fel * n * n + n * (128 + 128 * fel + 8)
+    slots = 36 << 20 if n > 64 else 0
+    return int(zel * n * n + factor + update_operands(n, precision) + _solve_scratch(n, nrhs, fel) + slots + workspace +
+               (64 << 20))
 
 
 def _upload(ctx, m, X):
@@ -287,8 +300,13 @@ class Server:
             t.start()
 
     def _default_footprint(self, job):
-        return job_footprint(job["space"].numfunctions(), len(job.get("waves", ())) or 1,
-                             job.get("precision", L.MIXED), self.workspace)
+        n, precision = job["space"].numfunctions(), job.get("precision", L.MIXED)
+        fp = job_footprint(n, len(job.get("waves", ())) or 1, precision, self.workspace)
+        # without memory for their operands the FP64 updates run on the FP64 units: such a job is not refused, it runs
+        # with nothing beside it
+        if precision == L.FP64 and fp > self.budget >= fp - update_operands(n, precision):
+            return self.budget
+        return fp
 
     # ---- admission
     def submit(self, job):
@@ -346,9 +364,10 @@ class Server:
             self._cv.notify_all()
 
     def _resident_footprint(self, job):
-        """a job on a resident system: the excitations, solutions and refinement vectors"""
+        """a job on a resident system: the solve's scratch"""
         n = job["space"].numfunctions()
-        return int(16 * n * (2 * (len(job.get("waves", ())) or 1) + 4) + (16 << 20))
+        fel = 16 if job.get("precision", L.MIXED) == L.FP64 else 8
+        return int(_solve_scratch(n, len(job.get("waves", ())) or 1, fel) + (16 << 20))
 
     def _worker(self, s):
         ctx = self._ctxs[s]

@@ -100,6 +100,35 @@ def test_job_footprint_counts_the_matrix_and_its_factor_copy():
     assert 32 * n * n < fp64 < 32 * n * n + (1 << 30)
 
 
+@pytest.mark.parametrize("precision", [L.MIXED, L.MIXED_BALANCED, L.FP64])
+def test_job_footprint_counts_the_scratch(precision):
+    """what the library allocates beside the matrix, its factors and the updates' operands: 64 matvec sums of 16 bytes a
+    row, the inverses of two 64 x 64 triangles for every 64 rows, eight right-hand sides of the triangular solves and,
+    for a pivoted panel on 152 SMs, 64 columns of (2 G^2 + 2 G + 2 (G + 1) 64) 8-byte slots"""
+    n, G = 122880, 152
+    zel, fel = (8 if precision == L.MIXED else 16), (16 if precision == L.FP64 else 8)
+    operands = 108 * 256 * n if precision == L.FP64 else 12 * 1024 * n
+    scratch = 64 * 16 * n + 16 * n + 2 * 64 * fel * n + 8 * fel * n + 64 * 8 * (2 * G * G + 2 * G + 2 * (G + 1) * 64)
+    fp = job_footprint(n, 1, precision)
+    assert fp - (zel + fel) * n * n - operands >= scratch + (64 << 20)
+    assert fp <= (zel + fel) * n * n + operands + scratch + (128 << 20)
+
+
+def test_an_fp64_job_without_room_for_its_update_operands_runs_alone():
+    class Space:
+        def numfunctions(self):
+            return 20000
+
+    job = {"name": "j", "space": Space(), "precision": L.FP64}
+    full = job_footprint(20000, 1, L.FP64)
+    rec = Recorder()
+    with Server(slots=1, hbm_budget=full - (100 << 20), make_context=lambda: None, runner=rec, workspace=0) as s:
+        assert s.submit(job).result(timeout=10) == "j"
+    with Server(slots=1, hbm_budget=full - (2 << 30), make_context=lambda: None, runner=rec, workspace=0) as s:
+        with pytest.raises(ValueError):
+            s.submit(job).result(timeout=10)
+
+
 def test_a_cancelled_pending_job_never_runs():
     rec = Recorder(hold=0.1)
     with server(rec, slots=1, budget=100) as s:
