@@ -2925,7 +2925,7 @@ int lu_solve_t(beast_ctx* ctx, int64_t n, const T* A, int64_t lda, const int* pe
 // ---- allocation-free triangular solve ----------------------------------------------------
 // Scratch of beast_lu_solve_noalloc: one right-hand side of up to NOALLOC_MAX_N complex128
 // values (the permuted right-hand side, then the backward sweep's output).
-// Held by every GPU that loads the library, for the life of the process.
+// Held by every GPU that loads the library, for the life of the process; calls take turns on it.
 constexpr int64_t NOALLOC_MAX_N = 65536;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_MAX_N * 16];
 
@@ -3157,6 +3157,9 @@ extern "C" int beast_lu_solve_noalloc(beast_ctx* ctx, const beast_lu* lu, int64_
   BEAST_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   unsigned char* scratch = noalloc_scratch(ctx);
   if (!scratch) return beast_fail(ctx, BEAST_ERR_CUDA, "cudaGetSymbolAddress of the fixed scratch failed");
+  // one call at a time per GPU (contexts and host threads share the scratch); every way out has waited for the stream
+  static std::mutex turn[64];
+  std::lock_guard<std::mutex> lk(turn[ctx->device]);
   int rc;
   if (lu->dtype == BEAST_C64)
     rc = lu_solve_fixed_scratch<float2, float>(ctx, lu->n, (const float2*)lu->A, lu->lda, lu->ipiv + lu->n,
@@ -3166,6 +3169,9 @@ extern "C" int beast_lu_solve_noalloc(beast_ctx* ctx, const beast_lu* lu, int64_
     rc = lu_solve_fixed_scratch<double2, double>(ctx, lu->n, (const double2*)lu->A, lu->lda,
                                                  lu->ipiv + lu->n, (double2*)B, ldb, nrhs, scratch,
                                                  (const double2*)lu_dinv(lu->ipiv, lu->n));
-  if (rc) return rc;
+  if (rc) {
+    cudaStreamSynchronize(ctx->stream);
+    return rc;
+  }
   return trsv_check(ctx);
 }

@@ -54,3 +54,34 @@ def test_fp64_solves_of_different_order():
         return lambda c: bg.solve(A, b, precision=bg.FP64, ctx=c)[0]
 
     _together([job(70), job(640), job(150)], 60)
+
+
+def test_noalloc_solves_take_turns():
+    """the triangular solves without an allocation share one scratch array a GPU: contexts on threads of their own, at
+    orders that end in different places of it"""
+    import ctypes as C
+
+    import torch
+
+    def job(n):
+        rng = np.random.default_rng(n)
+        A = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)) + 4 * n**0.5 * np.eye(n)
+        At = torch.from_numpy(np.ascontiguousarray(A.T)).cuda()
+        b = torch.from_numpy(rng.normal(size=n) + 0j).cuda()
+        torch.cuda.synchronize()
+        held = {}
+
+        def run(c):
+            if c not in held:
+                F, h = At.clone(), C.c_void_p()
+                torch.cuda.synchronize()
+                c.check(c.lib.beast_lu_factor(c.handle, n, F.data_ptr(), n, bg.C128, C.byref(h)))
+                held[c] = F, h
+            x = b.clone()
+            torch.cuda.synchronize()
+            c.check(c.lib.beast_lu_solve_noalloc(c.handle, held[c][1], 1, x.data_ptr(), n))
+            return x.cpu().numpy()
+
+        return run
+
+    _together([job(700), job(1100), job(300)], 40)
