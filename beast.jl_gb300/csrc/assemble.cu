@@ -2812,12 +2812,12 @@ __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, i
     s_q[k][4] = r.w[k] * v;
   }
   __syncthreads();
-  const int64_t p = blockIdx.x, npts = gridDim.x;
+  const int64_t p = blockIdx.y, npts = gridDim.y, chunk = blockIdx.x;
   const V3<double> y = mk(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
   const double sg = gi < 0.0 ? -1.0 : 1.0;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  const int64_t c1 = min(ncells, (blockIdx.y + 1) * (int64_t)FF_CHUNK);
-  for (int64_t c = blockIdx.y * (int64_t)FF_CHUNK + threadIdx.x; c < c1; c += FF_THREADS) {
+  const int64_t c1 = min(ncells, (chunk + 1) * FF_CHUNK);
+  for (int64_t c = chunk * FF_CHUNK + threadIdx.x; c < c1; c += FF_THREADS) {
     const FarCell& f = cells[c];
     const V3<double> a = mk(f.a[0], f.a[1], f.a[2]), b = mk(f.b[0], f.b[1], f.b[2]);
     const double pa = dot(y, a), pb = dot(y, b);
@@ -2870,7 +2870,7 @@ __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, i
       for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x < 6) part[(blockIdx.y * npts + p) * 6 + threadIdx.x] = red[threadIdx.x][0];
+  if (threadIdx.x < 6) part[(chunk * npts + p) * 6 + threadIdx.x] = red[threadIdx.x][0];
 }
 
 // the chunks' sums, then (y x F) x y
@@ -4931,8 +4931,9 @@ cudaError_t launch_farfield(const beast_space* s, const double* u, const double*
                             double gr, double gi, const TriRuleDev& r, double* ff, cudaStream_t st) {
   if (npts == 0) return cudaSuccess;
   const int nchunk = (int)((s->ncells + FF_CHUNK - 1) / FF_CHUNK);
-  // directions in slabs whose partial sums take at most 64 MB
-  const int64_t slab = std::max<int64_t>(1, std::min<int64_t>(npts, (64ll << 20) / (48 * std::max(nchunk, 1))));
+  // directions in slabs whose partial sums take at most 64 MB, and no more than a grid's second dimension (the chunks,
+  // whose number has no such bound, are the first)
+  const int64_t slab = std::max<int64_t>(1, std::min<int64_t>({npts, 65535, (64ll << 20) / (48ll * std::max(nchunk, 1))}));
   FarCell* cells = nullptr;
   double* part = nullptr;
   cudaError_t e = cudaMallocAsync(&cells, sizeof(FarCell) * (size_t)s->ncells + 256, st);
@@ -4949,7 +4950,7 @@ cudaError_t launch_farfield(const beast_space* s, const double* u, const double*
   for (int64_t p0 = 0; p0 < npts; p0 += slab) {
     const int64_t n = std::min(slab, npts - p0);
     if (nchunk > 0)
-      k_farfield<<<dim3((unsigned)n, (unsigned)nchunk), FF_THREADS, 0, st>>>(cells, s->ncells, pts + 3 * p0, gr, gi, wave, r,
+      k_farfield<<<dim3((unsigned)nchunk, (unsigned)n), FF_THREADS, 0, st>>>(cells, s->ncells, pts + 3 * p0, gr, gi, wave, r,
                                                                              part);
     k_farfield_sum<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, nchunk, n, pts + 3 * p0, ff + 6 * p0);
   }

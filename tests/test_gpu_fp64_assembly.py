@@ -103,3 +103,15 @@ def test_farfield(level, npts, gamma):
     ff = bg.farfield(X, u, d, gamma)
     fo = _farfield_sum(X, u, d, gamma)
     assert np.abs(ff - fo).max() <= 1e-12 * np.abs(fo).max()
+
+
+def test_farfield_of_more_directions_than_a_grid_dimension():
+    """directions come in slabs of at most 65535: those of a long list are bit for bit those of a short one"""
+    X = bg.raviartthomas(bg.ellipsoid(0, (1.0, 0.8, 1.3)))
+    rng = np.random.default_rng(0)
+    u = rng.normal(size=X.numfunctions()) + 1j * rng.normal(size=X.numfunctions())
+    d = rng.normal(size=(131073, 3))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    ff = bg.farfield(X, u, d, 2j)
+    pick = [0, 1, 65534, 65535, 65536, 131069, 131070, 131071, 131072]
+    assert np.array_equal(ff[pick], bg.farfield(X, u, d[pick], 2j))
