@@ -48,22 +48,20 @@ def _solve_scratch(n, nrhs, element):
 
 def update_operands(n, precision):
     """device bytes of the tensor-core operands of the largest trailing update: 12 bytes per row and column of K <= 1024
-    on the mixed paths, 108 of K <= 256 in FP64"""
+    on the mixed paths, 112 of K <= 256 in FP64"""
     if precision == L.FP64:
-        return 108 * 256 * n if n > 64 else 0
+        return 112 * 256 * n if n > 64 else 0
     return 12 * 1024 * n if n > 1024 else 0
 
 
 def job_footprint(n, nrhs=1, precision=L.MIXED, workspace=0):
     """device bytes a job holds at its peak: the matrix, the factor copy (whole 128-byte lines a column) with its
-    pivots and the inverses of its diagonal blocks, the tensor-core operands, the solve's scratch, the panels' exchange
-    slots, the context's assembly workspace, and 64 MiB of small buffers"""
+    pivots and the inverses of its diagonal blocks, the tensor-core operands, the solve's scratch, the context's
+    assembly workspace, and 64 MiB of small buffers (34 of them a pivoted panel's exchange slots)"""
     zel = 8 if precision == L.MIXED else 16
     fel = 16 if precision == L.FP64 else 8
     factor = fel * n * n + n * (128 + 128 * fel + 8)
-    slots = 36 << 20 if n > 64 else 0
-    return int(zel * n * n + factor + update_operands(n, precision) + _solve_scratch(n, nrhs, fel) + slots + workspace +
-               (64 << 20))
+    return int(zel * n * n + factor + update_operands(n, precision) + _solve_scratch(n, nrhs, fel) + workspace + (64 << 20))
 
 
 def _upload(ctx, m, X):

@@ -1649,16 +1649,13 @@ __global__ void __launch_bounds__(256) k_gemm_sub(T* C, int64_t ldc, const T* Am
                                                   int64_t m, int64_t n, int k) {
   gemm_tile<T, R>(C, ldc, Am, lda, Bm, ldb, m, n, k, blockIdx.x * (int64_t)GT, blockIdx.y * (int64_t)GT);
 }
-// the tiles that tc_gemm64.cu leaves to the FP64 units: *count of GT rows x per GT columns, by (row, column) index
-__global__ void __launch_bounds__(256) k_gemm_tiles(const int2* list, const int* count, int per, double2* C, int64_t ldc,
+// the GT x GT tiles that tc_gemm64.cu leaves to the FP64 units, by (row, column) index
+__global__ void __launch_bounds__(256) k_gemm_tiles(const int2* list, const int* count, double2* C, int64_t ldc,
                                                     const double2* Am, int64_t lda, const double2* Bm, int64_t ldb,
                                                     int64_t m, int64_t n, int k) {
-  const int64_t items = (int64_t)*count * per;
-  for (int64_t i = blockIdx.x; i < items; i += gridDim.x) {
-    const int2 t = list[i / per];
-    const int64_t bn = ((int64_t)t.y * per + i % per) * GT;
-    if (bn < n) gemm_tile<double2, double>(C, ldc, Am, lda, Bm, ldb, m, n, k, t.x * (int64_t)GT, bn);
-  }
+  const int items = *count;
+  for (int i = blockIdx.x; i < items; i += gridDim.x)
+    gemm_tile<double2, double>(C, ldc, Am, lda, Bm, ldb, m, n, k, list[i].x * (int64_t)GT, list[i].y * (int64_t)GT);
 }
 
 // ---- triangular solves on one right-hand side ------------------------------------------
@@ -2939,10 +2936,10 @@ int lu_solve_fixed_scratch(beast_ctx* ctx, int64_t n, const T* A, int64_t lda, c
 
 }  // namespace
 
-// tnt: columns of a listed tile (a multiple of GT); its rows are GT
-cudaError_t gemm64_tiles(const int2* list, const int* count, int tnt, double2* C, int64_t ldc, const double2* A, int64_t lda,
+cudaError_t gemm64_tiles(const int2* list, const int* count, double2* C, int64_t ldc, const double2* A, int64_t lda,
                          const double2* B, int64_t ldb, int64_t m, int64_t n, int k, int grid, cudaStream_t st) {
-  k_gemm_tiles<<<(unsigned)grid, 256, 0, st>>>(list, count, tnt / GT, C, ldc, A, lda, B, ldb, m, n, k);
+  static_assert(GT == 64, "tc_gemm64.cu lists blocks of 64");
+  k_gemm_tiles<<<(unsigned)grid, 256, 0, st>>>(list, count, C, ldc, A, lda, B, ldb, m, n, k);
   return cudaGetLastError();
 }
 

@@ -15,7 +15,8 @@
 // Spread.  What no such scaling levels (blocks of unknowns that are hardly coupled) is measured: the
 // sum S_ij over k of p_ik q_kj, p and q the magnitudes relative to 2^e of their row and column.  The
 // digits' error is at most about 2^-54 of the row's times the column's largest value, so relative to
-// sum |a_ik b_kj| it stays near FP64's own where S_ij is not far below one.
+// sum |a_ik b_kj| it stays near FP64's own where S_ij is not far below one (and relative to the entry the sum is
+// subtracted from where that is not).
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -69,12 +70,12 @@ SL_HD int key_exponent(int key) {
   return key >= EXP_NONFINITE / 2 ? EXP_NONFINITE : (key == KEY_ZERO ? -1021 : key);
 }
 
-// round(x 2^(55 - e)), ties up in magnitude; |x| < 2^e
-SL_HD int64_t fixed55(double x, int e) {
+// round(x 2^(b - e)), ties up in magnitude; |x| < 2^e, b <= 62
+SL_HD int64_t fixed_point(double x, int e, int b) {
   const uint64_t u = bits_of(x);
   const int E = (int)((u >> 52) & 0x7FF);
   const uint64_t m = (u & 0xFFFFFFFFFFFFFull) | (E ? 1ull << 52 : 0ull);
-  const int sh = (E ? E : 1) - 1020 - e;  // x = m 2^(E - 1075); sh <= 2
+  const int sh = (E ? E : 1) - 1075 + b - e;  // x = m 2^(E - 1075); sh <= b - 53
   uint64_t X;
   if (sh >= 0)
     X = m << sh;
@@ -84,6 +85,10 @@ SL_HD int64_t fixed55(double x, int e) {
     X = 0;
   return (u >> 63) ? -(int64_t)X : (int64_t)X;
 }
+
+// the fixed-point number of the eight digits, and of nine
+SL_HD int64_t fixed55(double x, int e) { return fixed_point(x, e, 55); }
+SL_HD int64_t fixed62(double x, int e) { return fixed_point(x, e, 62); }
 
 // the digits of X, most significant first
 SL_HD void digits(int64_t X, int d[SLICES]) {
@@ -95,17 +100,29 @@ SL_HD void digits(int64_t X, int d[SLICES]) {
   d[0] = (int)X;
 }
 
-// the magnitude of a complex value from its two fixed-point parts, relative to 2^e: 2^-24 at least (the
-// smallest FP16 number) unless both are exactly zero, at most 1
+// the nine digits of X = fixed62: the ninth is taken off, the rest is the eight digits' number
+SL_HD void digits9(int64_t X, int d[SLICES + 1]) {
+  d[SLICES] = (int)((X + 64) & 127) - 64;
+  digits((X - d[SLICES]) >> 7, d);
+}
+
+// the magnitude of a complex value from its two parts (fixed62), relative to 2^e: 2^-24 at least (the smallest FP16
+// number) unless both are exactly zero, at most 1
 constexpr float SPREAD_MIN = 0x1p-24f;
-// a tile with a sum 0 < S < SPREAD_LIMIT goes to the FP64 units.  Boundary-operator matrices (EFIE, MFIE
-// and Helmholtz, orders 480 to 6,007) have no sum below 2^-9.4; two blocks of unknowns coupled by 2^-9
-// lose 6 in the accuracy of the weak one there, by 2^-13 a hundred.
-constexpr float SPREAD_LIMIT = 0x1p-10f;
 SL_HD float spread_magnitude(int64_t X, int64_t Y, bool zero) {
   const int64_t x = X < 0 ? -X : X, y = Y < 0 ? -Y : Y;
-  const float p = (float)(int32_t)((x > y ? x : y) >> 25) * 0x1p-30f;
+  const float p = (float)(int32_t)((x > y ? x : y) >> 32) * 0x1p-30f;
   return zero ? 0.f : (p > SPREAD_MIN ? p : SPREAD_MIN);
+}
+// An entry with a sum 0 < S < 2^-SPREAD_BITS that is itself below the same part of its scale needs the ninth digit,
+// below 2^-SPREAD_BITS_FP64 the FP64 units.  (An FP64 update rounds to 2^-53 of the entry or the sum, whichever is
+// larger; eight digits cut at 2^-55 of the scale, nine at 2^-62.)  Two blocks of unknowns coupled by 2^-9 lose a factor
+// of 6 in the accuracy of the weak one at these limits; at 2^-13 it would be a hundred.
+constexpr int SPREAD_BITS = 10, SPREAD_BITS_FP64 = 17;
+// max(|x|, |y|) < 2^(e - bits)
+SL_HD bool spread_small(double x, double y, int e, int bits) {
+  const uint32_t a = abs_hi(x), b = abs_hi(y);
+  return (int)((a > b ? a : b) >> 20) - 1022 <= e - bits;
 }
 
 // the FP64 value -D 2^sh of an integer-valued FP32 number D, built from its bits (a conversion

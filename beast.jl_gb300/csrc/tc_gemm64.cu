@@ -17,8 +17,12 @@
 //   - the columns of A are levelled by powers of two and the rows of B by their inverses before the
 //     digits are taken (k_balance): rows of a matrix in different units lose nothing.  Without it an
 //     order-300 system with half its rows scaled by 1e-8 came out with an error of 1e-9 (1e-15 with);
-//   - a ninth slice holds the entries' magnitudes; their product S is taken first, and a tile with a sum
-//     that is small against the tile's scale goes to the FP64 units (gemm64_tiles).
+//   - the product S of the entries' magnitudes is taken first.  Where a sum and its entry of C are both below 2^-10
+//     of the row's and the column's scale, the block of 64 columns takes the ninth digit (nine more pairs), and below
+//     2^-17 it goes to the FP64 units, 64 x 64 at a time (gemm64_tiles).  Hardly any block does in EFIE and Helmholtz
+//     matrices of real wavenumbers, a few hundredths take the ninth digit in second-kind ones of flat surfaces, a tenth
+//     under a kernel that decays by e^6 over the surface; under one that decays by e^40 half the work is the FP64
+//     units' and a solve takes as long as on those alone at worst.
 // measured against LAPACK's solutions in tests/test_gpu_lu_paths.py.
 //
 // k_tc_gemm64: persistent CTAs over 128 x TNT tiles of C'; after S the levels run from the smallest
@@ -39,19 +43,30 @@
 #include "slice64.h"
 #include "tc_ptx.h"
 
-// the listed tiles of the update on the FP64 units (linalg.cu)
-cudaError_t gemm64_tiles(const int2* list, const int* count, int tnt, double2* C, int64_t ldc, const double2* A, int64_t lda,
+// the listed 64 x 64 blocks of the update on the FP64 units (linalg.cu)
+cudaError_t gemm64_tiles(const int2* list, const int* count, double2* C, int64_t ldc, const double2* A, int64_t lda,
                          const double2* B, int64_t ldb, int64_t m, int64_t n, int k, int grid, cudaStream_t st);
 
 namespace {
 
 using slice64::SLICES;
-constexpr int PLANES = SLICES + 1;  // the digits and the magnitudes
+constexpr int PLANES = SLICES + 1;  // digits held of each operand
 
 constexpr int TM = 128, TK = 64, STAGES = 4;
 constexpr int KMAX = 256;  // complex columns of A per launch: (l + 1) 2K 2^12 <= 2^24 for l = 7
 constexpr int A_BYTES = TM * TK * 2;
-constexpr int SPREAD = SLICES;  // the level of the magnitudes' product
+// the accumulations of a tile, in order: the magnitudes, levels 7 .. 0, and level 8 in two (nine pairs would not be
+// exact in one) where a block asks for it
+constexpr int STEPS = SLICES + 1, NINE_A = 5;
+struct Step {
+  int level, i0, i1;  // pairs (i, level - i) for i0 <= i < i1
+};
+__device__ __forceinline__ Step step_at(int st) {
+  const int l = SLICES - st;  // 0: the magnitudes
+  if (st == 0) return Step{0, 0, 1};
+  if (st < STEPS) return Step{l, 0, l + 1};
+  return st == STEPS ? Step{SLICES, 0, NINE_A} : Step{SLICES, NINE_A, PLANES};
+}
 constexpr int GROUP = 8;  // row tiles taken together, column by column
 
 template <int TNT>
@@ -69,13 +84,15 @@ __device__ __forceinline__ void tile_at(int tile, int ntm, int ntn, int& mt, int
 }
 
 // M2 = 2M real rows of C' at Cr (ldr doubles per column), N columns; A' slice i at rows i M2, B'
-// slice j at rows j N of their tensor maps; nk stages of TK halves per digit pair.  Tiles left to the FP64
-// units: their (row, column) tile indices in list, their number in count
+// slice j at rows j N of their tensor maps; nk stages of TK halves per digit pair.  tmP, tmQ: the magnitudes of A (a
+// row per complex row) and B, nkS stages.  Blocks left to the FP64
+// units: their (row, column) indices in units of 64 in list, their number in count
 template <int TNT>
 __global__ void __launch_bounds__(192, 1)
-    k_tc_gemm64(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double* Cr,
-                int64_t ldr, int M2, int N, const int* __restrict__ ea, const int* __restrict__ eb, int nk, int2* list, int* count,
-                int* status) {
+    k_tc_gemm64(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, double* Cr, int64_t ldr,
+                int M2, int N, const int* __restrict__ ea, const int* __restrict__ eb, int nk, int nkS, int2* list,
+                int* count, int* status) {
   constexpr int STAGE_BYTES = Tile<TNT>::STAGE_BYTES;
   extern __shared__ unsigned char smraw[];
   const uint32_t base = (smem_u32(smraw) + 1023u) & ~1023u;
@@ -85,15 +102,16 @@ __global__ void __launch_bounds__(192, 1)
   const int B_FULL = 0, B_EMPTY = STAGES, B_TFULL = 2 * STAGES, B_TEMPTY = 2 * STAGES + 2, B_DONE = 2 * STAGES + 4,
             B_SPREAD = 2 * STAGES + 5;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 7);
-  __shared__ int s_abort_mem, s_wide_mem[2];
-  volatile int* s_wide = s_wide_mem;  // by parity of a CTA's tiles: 1 + the last one left to the FP64 units
+  __shared__ int s_abort_mem, s_wide_mem[2][4];
+  // by parity of a CTA's tiles, per epilogue warp: groups of 64 columns left to the FP64 units (bits 0 .. 3) and with the
+  // ninth digit (bits 4 .. 7)
+  volatile int(*s_wide)[4] = s_wide_mem;
   volatile int* s_abort = &s_abort_mem;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntm = (M2 + TM - 1) / TM, ntn = (N + TNT - 1) / TNT, ntiles = ntm * ntn;
 
   if (threadIdx.x == 0) {
     *s_abort = 0;
-    s_wide[0] = s_wide[1] = 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(bars + B_FULL + s), 1);
       mbar_init(smem_u32(bars + B_EMPTY + s), 1);
@@ -117,22 +135,39 @@ __global__ void __launch_bounds__(192, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
+  // true when tile number ord of this CTA asks for the ninth digit (known once its magnitudes are read); false at once
+  // when a wait has given up
+  auto nine = [&](int ord) {
+    if (!mbar_wait(smem_u32(bars + B_SPREAD), ord & 1, status, s_abort)) return false;
+    volatile int* w = s_wide[ord & 1];
+    return ((w[0] | w[1] | w[2] | w[3]) >> 4) != 0;
+  };
+
   if (warp == 0 && lane == 0) {
     // ---- TMA producer
     uint32_t it = 0;
-    for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x) {
+    int ord = 0;
+    for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x, ++ord) {
       int mt, nt;
       tile_at(tile, ntm, ntn, mt, nt);
-      for (int l = SPREAD; l >= 0 && !*s_abort; --l)
-        for (int i = l == SPREAD ? SPREAD : 0; i <= l && !*s_abort; ++i)
-          for (int kb = 0; kb < nk; ++kb, ++it) {
+      for (int st = 0; st < STEPS + 2 && !*s_abort; ++st) {
+        if (st == STEPS && !nine(ord)) break;
+        const Step p = step_at(st);
+        for (int i = p.i0; i < p.i1 && !*s_abort; ++i)
+          for (int kb = 0; kb < (st == 0 ? nkS : nk); ++kb, ++it) {
             const int s = it % STAGES;
             if (!mbar_wait(smem_u32(bars + B_EMPTY + s), ((it / STAGES) & 1) ^ 1, status, s_abort)) break;
             const uint32_t sa = base + s * STAGE_BYTES, full = smem_u32(bars + B_FULL + s);
             mbar_expect_tx(full, STAGE_BYTES);
-            tma_load_2d(sa, &tmA, kb * TK, i * M2 + mt * TM, full);
-            tma_load_2d(sa + A_BYTES, &tmB, kb * TK, (l == SPREAD ? SPREAD : l - i) * N + nt * TNT, full);
+            if (st == 0) {
+              tma_load_2d(sa, &tmP, kb * TK, mt * (TM / 2), full);
+              tma_load_2d(sa + A_BYTES, &tmQ, kb * TK, nt * TNT, full);
+            } else {
+              tma_load_2d(sa, &tmA, kb * TK, i * M2 + mt * TM, full);
+              tma_load_2d(sa + A_BYTES, &tmB, kb * TK, (p.level - i) * N + nt * TNT, full);
+            }
           }
+      }
     }
     // no copy may still be landing in shared memory when the CTA exits (bounded, whatever the
     // abort state)
@@ -143,14 +178,16 @@ __global__ void __launch_bounds__(192, 1)
     // ---- MMA issuer: D f32, A / B f16, both K-major, M = 128, N = TNT
     const uint32_t idesc = (1u << 4) | ((uint32_t)(TNT >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
     uint32_t it = 0;
-    int t = 0;  // levels of all tiles, in order
-    for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x)
-      for (int l = SPREAD; l >= 0 && !*s_abort; --l, ++t) {
+    int t = 0, ord = 0;  // accumulations of all tiles, in order
+    for (int tile = blockIdx.x; tile < ntiles && !*s_abort; tile += gridDim.x, ++ord)
+      for (int st = 0; st < STEPS + 2 && !*s_abort; ++st, ++t) {
+        if (st == STEPS && !nine(ord)) break;
+        const Step p = step_at(st);
         const int a = t & 1;
         if (!mbar_wait(smem_u32(bars + B_TEMPTY + a), ((t >> 1) & 1) ^ 1, status, s_abort)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + (uint32_t)(a * TNT);
-        const int steps = l == SPREAD ? nk : (l + 1) * nk;
+        const int steps = st == 0 ? nkS : (p.i1 - p.i0) * nk;
         for (int kb = 0; kb < steps; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(smem_u32(bars + B_FULL + s), (it / STAGES) & 1, status, s_abort)) break;
@@ -181,8 +218,8 @@ __global__ void __launch_bounds__(192, 1)
       const int er = in ? ea[row >> 1] : 0;
       double* c0 = Cr + row + (int64_t)n0 * ldr;
       const int ncol = min(TNT, N - n0);
-      bool wide = false;  // the tile goes to the FP64 units: its levels are waited for and left out
-      for (int l = SPREAD; l >= 0; --l, ++t) {
+      int wide = 0;  // as s_wide, of all four warps
+      for (int st = 0; st < (wide >> 4 ? STEPS + 2 : STEPS); ++st, ++t) {
         const int a = t & 1;
         if (!mbar_wait(smem_u32(bars + B_TFULL + a), (t >> 1) & 1, status, s_abort)) {
           live = false;
@@ -196,34 +233,61 @@ __global__ void __launch_bounds__(192, 1)
           if (lane == 0)
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bars + B_TEMPTY + a)) : "memory");
         };
-        if (l == SPREAD) {
-          bool small = false;
-          for (int c = 0; c < ncol; c += 16) {
+        if (st == 0) {
+          // small sums whose entry of C is small too, a thread a complex row (the first two warps; the accumulator's
+          // other rows are the next tile's)
+          const int cr = mt * (TM / 2) + q * 32 + lane;
+          const bool inc = q < 2 && 2 * cr < M2;
+          const int ec = inc ? ea[cr] : 0;
+          const double* cz = Cr + 2 * (int64_t)cr + (int64_t)n0 * ldr;
+          int found = 0;
+          for (int c = 0; c < ncol && q < 2; c += 16) {
             float v[16];
             tmem_ld16(tb + (uint32_t)c, v);
+            uint32_t low = 0;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) small |= c + j < ncol && v[j] > 0.f && v[j] < slice64::SPREAD_LIMIT;
+            for (int j = 0; j < 16; ++j)
+              low |= (uint32_t)(v[j] > 0.f && v[j] < 1.f / (1 << slice64::SPREAD_BITS)) << j;
+            const int g = c >> 6;
+            if (!inc) low = 0;
+            for (; low && !((found >> g) & 1); low &= low - 1) {
+              const int jj = __ffs(low) - 1, j = c + jj;
+              if (j >= ncol) break;
+              const double x = cz[j * ldr], y = cz[j * ldr + 1];
+              const int e = ec + eb[n0 + j];
+              float s = 0.f;
+#pragma unroll
+              for (int u = 0; u < 16; ++u) s = u == jj ? v[u] : s;
+              if (!slice64::spread_small(x, y, e, slice64::SPREAD_BITS)) continue;
+              found |= 16 << g;
+              if (s < 1.f / (1 << slice64::SPREAD_BITS_FP64) && slice64::spread_small(x, y, e, slice64::SPREAD_BITS_FP64))
+                found |= 1 << g;
+            }
+            __syncwarp();  // (the accumulator is read by the whole warp)
           }
           release();
           // the four warps agree
-          if (__any_sync(0xffffffffu, in && small) && lane == 0) s_wide[ord & 1] = ord + 1;
-          __syncwarp();
-          if (lane == 0)
+          found = (int)__reduce_or_sync(0xffffffffu, (unsigned)found);
+          if (lane == 0) {
+            s_wide[ord & 1][q] = found & ~((found & 15) << 4);
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bars + B_SPREAD)) : "memory");
+          }
           if (!mbar_wait(smem_u32(bars + B_SPREAD), ord & 1, status, s_abort)) {
             live = false;
             break;
           }
-          wide = s_wide[ord & 1] == ord + 1;
-          if (wide && q == 0 && lane == 0) list[atomicAdd(count, 1)] = make_int2(mt, nt);
+          wide = s_wide[ord & 1][0] | s_wide[ord & 1][1] | s_wide[ord & 1][2] | s_wide[ord & 1][3];
+          if (q == 0 && lane == 0)
+            for (int g = 0; g < TNT / 64; ++g)
+              if ((wide >> g) & 1) list[atomicAdd(count, 1)] = make_int2(mt, nt * (TNT / 64) + g);
           continue;
         }
-        if (wide) {
-          release();
-          continue;
-        }
+        // columns of this accumulation: level 8 those with the ninth digit, none of the FP64 units' any
+        const int skip = (wide & 15) | (st >= STEPS ? ~(wide >> 4) & 15 : 0);
+        const int l = step_at(st).level;
         const int sh0 = er - 12 - 7 * l;
         for (int c = 0; c < ncol; c += 16) {
+          if ((skip >> (c >> 6)) & 1) continue;
           float v[16];
           double z[16];
           tmem_ld16(tb + (uint32_t)c, v);
@@ -289,23 +353,23 @@ __global__ void __launch_bounds__(512) k_balance(const double2* A, int64_t lda, 
   }
 }
 
-// the eight digits of (x, y) and the pair's magnitude: put(slice, digits of x, digits of y, magnitude)
+// the nine digits of (x, y): put(slice, digit of x, digit of y); returns the pair's magnitude
 template <typename Put>
-__device__ __forceinline__ void slice_value(double2 a, int e, Put put) {
-  int dr[SLICES], di[SLICES];
-  const int64_t X = slice64::fixed55(a.x, e), Y = slice64::fixed55(a.y, e);
-  slice64::digits(X, dr);
-  slice64::digits(Y, di);
+__device__ __forceinline__ __half slice_value(double2 a, int e, Put put) {
+  int dr[PLANES], di[PLANES];
+  const int64_t X = slice64::fixed62(a.x, e), Y = slice64::fixed62(a.y, e);
+  slice64::digits9(X, dr);
+  slice64::digits9(Y, di);
 #pragma unroll
-  for (int s = 0; s < SLICES; ++s) put(s, dr[s], di[s], 0.f);
+  for (int s = 0; s < PLANES; ++s) put(s, dr[s], di[s]);
   const bool zero = ((slice64::bits_of(a.x) | slice64::bits_of(a.y)) << 1) == 0;
-  put(SPREAD, 0, 0, slice64::spread_magnitude(X, Y, zero));
+  return __float2half_rn(slice64::spread_magnitude(X, Y, zero));
 }
 
 // A' slices of 32 rows of A per CTA: row maxima, then 32 x 64 tiles transposed through shared
 // memory so that every warp writes whole row segments of each slice
 __device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, int M, int K, const int* sk, __half2* Ap,
-                                        int* ea) {
+                                        __half* P, int* ea) {
   __shared__ int red[8][33];
   __shared__ double2 tile[32][65];
   __shared__ int s_e[32], s_k[KMAX];
@@ -344,10 +408,10 @@ __device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, 
           const int kk = lane + 32 * h, k = k0 + kk;
           if (k < K) {
             __half2* row0 = Ap + (int64_t)(2 * mr) * K + k;  // 2K halves = K half2 per row
-            slice_value(tile[r][kk], e + s_k[k], [&](int s, int dr, int di, float p) {
+            P[(int64_t)mr * K + k] = slice_value(tile[r][kk], e + s_k[k], [&](int s, int dr, int di) {
               __half2* row = row0 + (int64_t)s * 2 * M * K;
-              row[0] = s < SLICES ? digits_h2(dr, -di) : __floats2half2_rn(p, 0.f);
-              row[K] = s < SLICES ? digits_h2(di, dr) : __floats2half2_rn(p, 0.f);
+              row[0] = digits_h2(dr, -di);
+              row[K] = digits_h2(di, dr);
             });
           }
         }
@@ -359,7 +423,7 @@ __device__ __forceinline__ void slice_a(int bid, const double2* A, int64_t lda, 
 
 // B' slices, one warp per column
 __device__ __forceinline__ void slice_b(int bid, const double2* B, int64_t ldb, int K, int N, const int* sk, __half2* Bp,
-                                        int* eb) {
+                                        __half* Q, int* eb) {
   const int lane = threadIdx.x & 31;
   const int j = bid * 8 + (threadIdx.x >> 5);
   if (j >= N) return;
@@ -371,46 +435,47 @@ __device__ __forceinline__ void slice_b(int bid, const double2* B, int64_t ldb, 
   const int e = slice64::key_exponent(key);
   if (lane == 0) eb[j] = e;
   for (int k = lane; k < K; k += 32)
-    slice_value(col[k], e - sk[k], [&](int s, int dr, int di, float q) {
-      Bp[((int64_t)s * N + j) * K + k] = s < SLICES ? digits_h2(dr, di) : __floats2half2_rn(q, 0.f);
-    });
+    Q[(int64_t)j * K + k] = slice_value(
+        col[k], e - sk[k], [&](int s, int dr, int di) { Bp[((int64_t)s * N + j) * K + k] = digits_h2(dr, di); });
 }
 
 // both operands in one launch: CTAs [0, nA) 32 rows of A each, the rest 8 columns of B each
 __global__ void __launch_bounds__(256) k_slice(const double2* A, int64_t lda, const double2* B, int64_t ldb, int M,
-                                               int N, int K, const int* sk, __half2* Ap, int* ea, __half2* Bp, int* eb,
-                                               int nA) {
+                                               int N, int K, const int* sk, __half2* Ap, __half* P, int* ea,
+                                               __half2* Bp, __half* Q, int* eb, int nA) {
   if ((int)blockIdx.x < nA)
-    slice_a(blockIdx.x, A, lda, M, K, sk, Ap, ea);
+    slice_a(blockIdx.x, A, lda, M, K, sk, Ap, P, ea);
   else
-    slice_b(blockIdx.x - nA, B, ldb, K, N, sk, Bp, eb);
+    slice_b(blockIdx.x - nA, B, ldb, K, N, sk, Bp, Q, eb);
 }
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 template <int TNT>
-int run(beast_ctx* ctx, const CUtensorMap& tmA, const __half2* Bp, double* Cr, int64_t ldr, int M2, int N, int K,
-        const int* ea, const int* eb, int2* list, int* count) {
-  CUtensorMap tmB;
+int run(beast_ctx* ctx, const CUtensorMap& tmA, const CUtensorMap& tmP, const __half2* Bp, const __half* Q, double* Cr,
+        int64_t ldr, int M2, int N, int K, const int* ea, const int* eb, int2* list, int* count) {
+  CUtensorMap tmB, tmQ;
   if (!make_map(&tmB, Bp, (uint64_t)2 * K, (uint64_t)PLANES * N, (uint64_t)2 * K * 2, TK, TNT, true,
-                CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
+                CU_TENSOR_MAP_DATA_TYPE_FLOAT16) ||
+      !make_map(&tmQ, Q, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, TK, TNT, true, CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
     return beast_fail(ctx, BEAST_ERR_CUDA, "tensor map encode (B' slices) failed");
   BEAST_CUDA_TRY(ctx, cudaFuncSetAttribute(k_tc_gemm64<TNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<TNT>::SMEM));
   const int tiles = ((M2 + TM - 1) / TM) * ((N + TNT - 1) / TNT);
   k_tc_gemm64<TNT><<<std::min(tiles, std::max(1, ctx->num_sms)), 192, Tile<TNT>::SMEM, ctx->stream>>>(
-      tmA, tmB, Cr, ldr, M2, N, ea, eb, 2 * K / TK, list, count, ctx->d_flag);
+      tmA, tmB, tmP, tmQ, Cr, ldr, M2, N, ea, eb, 2 * K / TK, (K + TK - 1) / TK, list, count, ctx->d_flag);
   BEAST_CUDA_TRY(ctx, cudaGetLastError());
   return BEAST_OK;
 }
 
 }  // namespace
 
-// tiles of an M x N update at most (TNT = 64), and the workspace it takes
-static int64_t max_tiles(int64_t M, int64_t N) { return ((2 * M + TM - 1) / TM) * ((N + 63) / 64); }
+// 64 x 64 blocks of an M x N update, and the workspace it takes
+static int64_t max_blocks(int64_t M, int64_t N) { return ((2 * M + TM - 1) / TM) * ((N + 63) / 64); }
 size_t tc_gemm64_work_bytes(int64_t M, int64_t N, int K) {
   const int64_t k = std::min(K, KMAX);
-  return al256((size_t)PLANES * M * k * 8) + al256((size_t)PLANES * N * k * 4) + al256((size_t)M * 4) + al256((size_t)N * 4) +
-         al256(KMAX * 4) + al256((size_t)max_tiles(M, N) * 8 + 8);
+  return al256((size_t)PLANES * M * k * 8) + al256((size_t)PLANES * N * k * 4) + al256((size_t)M * k * 2) +
+         al256((size_t)N * k * 2) + al256((size_t)M * 4) + al256((size_t)N * 4) +
+         al256(KMAX * 4) + al256((size_t)max_blocks(M, N) * 8 + 8);
 }
 
 // C -= A B (complex128): C at (M x N, ldc), A (M x K, lda), B (K x N, ldb), K a multiple of 32,
@@ -429,6 +494,8 @@ int tc_gemm64_sub(beast_ctx* ctx, double2* C, int64_t ldc, const double2* A, int
     };
     __half2* Ap = reinterpret_cast<__half2*>(take((size_t)PLANES * M * k * 8));
     __half2* Bp = reinterpret_cast<__half2*>(take((size_t)PLANES * N * k * 4));
+    __half* P = reinterpret_cast<__half*>(take((size_t)M * k * 2));
+    __half* Q = reinterpret_cast<__half*>(take((size_t)N * k * 2));
     int* ea = reinterpret_cast<int*>(take((size_t)M * 4));
     int* eb = reinterpret_cast<int*>(take((size_t)N * 4));
     int* sk = reinterpret_cast<int*>(take(KMAX * 4));
@@ -436,28 +503,30 @@ int tc_gemm64_sub(beast_ctx* ctx, double2* C, int64_t ldc, const double2* A, int
     int2* list = reinterpret_cast<int2*>(w) + 1;
     const double2 *Ak = A + (int64_t)k0 * lda, *Bk = B + k0;
     {
-      // A read twice and B once, nine planes of 2 (A') and 1 (B') FP16 pairs written per element
-      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (32 + 72) + (double)N * k * (16 + 36));
+      // A read twice and B once, nine digits of 2 (A') and 1 (B') FP16 pairs and a magnitude written per element
+      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (32 + 74) + (double)N * k * (16 + 38));
       const int nA = (int)((M + 31) / 32), nB = (int)((N + 7) / 8);
       k_balance<<<(unsigned)k, 512, 0, ctx->stream>>>(Ak, lda, M, sk, count);
-      k_slice<<<(unsigned)(nA + nB), 256, 0, ctx->stream>>>(Ak, lda, Bk, ldb, (int)M, (int)N, k, sk, Ap, ea, Bp, eb, nA);
+      k_slice<<<(unsigned)(nA + nB), 256, 0, ctx->stream>>>(Ak, lda, Bk, ldb, (int)M, (int)N, k, sk, Ap, P, ea, Bp, Q,
+                                                            eb, nA);
       BEAST_CUDA_TRY(ctx, cudaGetLastError());
     }
-    CUtensorMap tmA;
+    CUtensorMap tmA, tmP;
     if (!make_map(&tmA, Ap, (uint64_t)2 * k, (uint64_t)PLANES * 2 * M, (uint64_t)2 * k * 2, TK, TM, true,
-                  CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
+                  CU_TENSOR_MAP_DATA_TYPE_FLOAT16) ||
+        !make_map(&tmP, P, (uint64_t)k, (uint64_t)M, (uint64_t)k * 2, TK, TM, true, CU_TENSOR_MAP_DATA_TYPE_FLOAT16))
       return beast_fail(ctx, BEAST_ERR_CUDA, "tensor map encode (A' slices) failed");
     const bool wide = ((2 * M + TM - 1) / TM) * ((N + 255) / 256) >= ctx->num_sms;
     {
       ProfScope ps(ctx, PK_TCGEMM, 8.0 * k * (double)M * N);
       double* Cr = reinterpret_cast<double*>(C);
-      const int rc = wide ? run<256>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb, list, count)
-                          : run<64>(ctx, tmA, Bp, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb, list, count);
+      const int rc = wide ? run<256>(ctx, tmA, tmP, Bp, Q, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb, list, count)
+                          : run<64>(ctx, tmA, tmP, Bp, Q, Cr, 2 * ldc, (int)(2 * M), (int)N, k, ea, eb, list, count);
       if (rc) return rc;
     }
     ProfScope ps(ctx, PK_GEMM, 0.0);
-    BEAST_CUDA_TRY(ctx, gemm64_tiles(list, count, wide ? 256 : 64, C, ldc, Ak, lda, Bk, ldb, M, N, k,
-                                     std::max(1, 2 * ctx->num_sms), ctx->stream));
+    BEAST_CUDA_TRY(ctx, gemm64_tiles(list, count, C, ldc, Ak, lda, Bk, ldb, M, N, k, std::max(1, 2 * ctx->num_sms),
+                                     ctx->stream));
   }
   return BEAST_OK;
 }

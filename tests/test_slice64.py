@@ -28,7 +28,11 @@ int t_scaled(long n, const double* x, const int* s, int* d) {
 }
 int t_balance(double x) { return slice64::balance_exponent(slice64::abs_hi(x)); }
 float t_spread(double x, double y, int e) {
-  return slice64::spread_magnitude(slice64::fixed55(x, e), slice64::fixed55(y, e), x == 0.0 && y == 0.0);
+  return slice64::spread_magnitude(slice64::fixed62(x, e), slice64::fixed62(y, e), x == 0.0 && y == 0.0);
+}
+int t_small(double x, double y, int e) { return slice64::spread_small(x, y, e, 10); }
+void t_nine(long n, const double* x, int e, int* d) {
+  for (long i = 0; i < n; ++i) slice64::digits9(slice64::fixed62(x[i], e), d + 9 * i);
 }
 int t_exp(double x) { return slice64::row_exponent(slice64::abs_hi(x)); }
 }
@@ -46,6 +50,7 @@ def lib(tmp_path_factory):
     h = C.CDLL(str(so))
     h.t_neg.restype, h.t_neg.argtypes = C.c_double, [C.c_float, C.c_int]
     h.t_exp.argtypes = h.t_balance.argtypes = [C.c_double]
+    h.t_small.argtypes = [C.c_double, C.c_double, C.c_int]
     h.t_spread.restype, h.t_spread.argtypes = C.c_float, [C.c_double, C.c_double, C.c_int]
     return h
 
@@ -150,3 +155,25 @@ def test_balanced_update_of_scaled_rows(lib):
         p = sum(u * v for u, v in zip(A, B)) * Fraction(2) ** (ea + eb - 110)
         err.append(float(abs(p - exact) / Fraction(d[-1])))
     assert err[0] <= K * 2.0 ** -53 and err[1] >= 1e6 * err[0]
+
+
+def test_small_entries(lib):
+    """max(|x|, |y|) below 2^-10 of 2^e: zeros and subnormals of any ordinary scale are, infinities are not"""
+    for e in (0, 7, -300):
+        t = 2.0 ** (e - 10)
+        assert lib.t_small(0.99 * t, 0.0, e) and lib.t_small(0.0, -0.99 * t, e) and lib.t_small(0.0, 0.0, e)
+        assert not lib.t_small(t, 0.0, e) and not lib.t_small(0.0, -1.5 * t, e)
+        assert lib.t_small(5e-324, 0.0, e) and not lib.t_small(float("inf"), 0.0, e)
+
+
+def test_nine_digits_hold_the_value(lib):
+    """the digits of the wider form: all of a value to 2^-63 of its row's largest, each at most 64"""
+    from fractions import Fraction
+    rng = np.random.default_rng(11)
+    x = np.concatenate([[0.0, 1.0 - 2.0**-53, -(1.0 - 2.0**-53), 2.0**-70], rng.uniform(-1, 1, 500) * 2.0 ** -rng.integers(0, 60, 500)])
+    d = np.zeros((len(x), 9), dtype=np.int32)
+    lib.t_nine(C.c_long(len(x)), x.ctypes.data_as(C.c_void_p), 0, d.ctypes.data_as(C.c_void_p))
+    assert np.abs(d).max() <= 64
+    for v, row in zip(x, d):
+        X = sum(int(k) << (7 * (8 - i)) for i, k in enumerate(row))
+        assert abs(Fraction(float(v)) - Fraction(X, 2**62)) <= Fraction(1, 2**63)
