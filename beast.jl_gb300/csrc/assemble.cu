@@ -143,7 +143,6 @@ DEV int refines_class(int cls, int qs_kind) {
   return cls;
 }
 
-// squared distance below which a pair can be near (strategy threshold of the trial cell)
 // the same class without FP64 instructions (classify_slow has about 130 of them, and one candidate among
 // a warp's pairs makes the warp run them: 3 of the 10.5 ms of a batch of 24 Helmholtz systems): the
 // coordinates as FP32 pairs, shared vertices by their bits; what FP32 cannot decide goes to classify_slow
@@ -196,6 +195,7 @@ DEV int classify_exact(const Geo& t, const Geo& s, int qs_kind, double k2) {
   }
   return classify_slow(&t, &s, qs_kind, k2);
 }
+// squared distance below which a pair can be near (strategy threshold of the trial cell)
 DEV double near_threshold2(int qs_kind, double k2, double area) {
   if (qs_kind == BEAST_QS_DOUBLENUM) return -1.0;
   if (qs_kind == BEAST_QS_SAUTER) return 0.0;
@@ -3162,7 +3162,8 @@ static int sm_count() {
 // chip's FP64 units idle.
 // The integer moments (FIX) for a real wavenumber at which most pairs are in their range: k times the
 // average cell radius at least 2^-5, a far pair's points being several radii apart (integer sines
-// start at kR = 2^-7).  Complex wavenumbers, static kernels and low frequencies take the FP64 sums.
+// start at kR = 0.0061, four steps of their table).  Complex wavenumbers, static kernels and low frequencies
+// take the FP64 sums.
 template <int OPK, int TK, int BK, bool FIX>
 static cudaError_t far64_launch(FarParams P, int fmt, cudaStream_t st) {
   const int64_t gx = (P.np + FAR_THREADS - 1) / FAR_THREADS;

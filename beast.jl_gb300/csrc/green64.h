@@ -328,7 +328,7 @@ struct ValueX {
   double iR;     // 1/R
   int64_t c, s;  // cos(|k| R), sin(|k| R)
 };
-// false: R2 or the angle out of range (below 2^-8 the integer sine would lose relative accuracy)
+// false: R2 or the angle out of range (below 4 steps, kR = 0.0061, the integer sine would lose relative accuracy)
 G64_HD bool eval_fixed(double R2, const Wave& w, const EntryX* tab, ValueX& v) {
   if ((uint32_t)((uint32_t)(bits(R2) >> 52) - 923u) > 190u) return false;
   double R;

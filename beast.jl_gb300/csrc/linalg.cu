@@ -294,7 +294,9 @@ __global__ void __launch_bounds__(256) k_panel(T* A, int64_t lda, int64_t n, int
         const float inv = 1.0f / (float)ncol;
         const int tot = (nloc - ibeg) * ncol;
         for (int e = tid - 32; e < tot; e += 224) {
-          const int q = (int)(((float)e + 0.5f) * inv);  // e / ncol (e < 2^14)
+          // e / ncol: a CTA's rows x columns take at most 220 KB, so e < 2^15 and the product is within 2^-7 / ncol of
+          // (e + 1/2) / ncol
+          const int q = (int)(((float)e + 0.5f) * inv);
           const int i = ibeg + q, k = jj + 1 + (e - q * ncol);
           if (i == li || i == lj) continue;
           T c = S[i * ld + k];

@@ -504,7 +504,7 @@ int tc_gemm64_sub(beast_ctx* ctx, double2* C, int64_t ldc, const double2* A, int
     const double2 *Ak = A + (int64_t)k0 * lda, *Bk = B + k0;
     {
       // A read twice and B once, nine digits of 2 (A') and 1 (B') FP16 pairs and a magnitude written per element
-      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (32 + 74) + (double)N * k * (16 + 38));
+      ProfScope ps(ctx, PK_CONVERT, (double)M * k * (32 + 74) + (double)N * k * (16 + 38), 2);
       const int nA = (int)((M + 31) / 32), nB = (int)((N + 7) / 8);
       k_balance<<<(unsigned)k, 512, 0, ctx->stream>>>(Ak, lda, M, sk, count);
       k_slice<<<(unsigned)(nA + nB), 256, 0, ctx->stream>>>(Ak, lda, Bk, ldb, (int)M, (int)N, k, sk, Ap, P, ea, Bp, Q,
