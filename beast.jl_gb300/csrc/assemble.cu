@@ -2798,7 +2798,7 @@ __global__ void k_farfield_cells(const double* geo, const int* ad_dof, const dou
 }
 
 __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, int64_t ncells, const double* pts, double gr,
-                                                         double gi, g64::Wave wave, TriRuleDev r, double* part) {
+                                                         double gi, g64::Wave wave, TriRuleDev r, int chunk0, double* part) {
   __shared__ __align__(16) g64::Entry tab[g64::TABLE];
   __shared__ double s_q[RULE_MAXPTS][5];  // u, v, w, w u, w v
   __shared__ double red[6][FF_THREADS];
@@ -2812,7 +2812,7 @@ __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, i
     s_q[k][4] = r.w[k] * v;
   }
   __syncthreads();
-  const int64_t p = blockIdx.y, npts = gridDim.y, chunk = blockIdx.x;
+  const int64_t p = blockIdx.x, npts = gridDim.x, chunk = chunk0 + (int64_t)blockIdx.y;
   const V3<double> y = mk(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
   const double sg = gi < 0.0 ? -1.0 : 1.0;
   double acc[6] = {0, 0, 0, 0, 0, 0};
@@ -4932,9 +4932,8 @@ cudaError_t launch_farfield(const beast_space* s, const double* u, const double*
                             double gr, double gi, const TriRuleDev& r, double* ff, cudaStream_t st) {
   if (npts == 0) return cudaSuccess;
   const int nchunk = (int)((s->ncells + FF_CHUNK - 1) / FF_CHUNK);
-  // directions in slabs whose partial sums take at most 64 MB, and no more than a grid's second dimension (the chunks,
-  // whose number has no such bound, are the first)
-  const int64_t slab = std::max<int64_t>(1, std::min<int64_t>({npts, 65535, (64ll << 20) / (48ll * std::max(nchunk, 1))}));
+  // directions in slabs whose partial sums take at most 64 MB
+  const int64_t slab = std::max<int64_t>(1, std::min<int64_t>(npts, (64ll << 20) / (48ll * std::max(nchunk, 1))));
   FarCell* cells = nullptr;
   double* part = nullptr;
   cudaError_t e = cudaMallocAsync(&cells, sizeof(FarCell) * (size_t)s->ncells + 256, st);
@@ -4950,9 +4949,9 @@ cudaError_t launch_farfield(const beast_space* s, const double* u, const double*
   const g64::Wave wave = g64::make_wave(gi);
   for (int64_t p0 = 0; p0 < npts; p0 += slab) {
     const int64_t n = std::min(slab, npts - p0);
-    if (nchunk > 0)
-      k_farfield<<<dim3((unsigned)nchunk, (unsigned)n), FF_THREADS, 0, st>>>(cells, s->ncells, pts + 3 * p0, gr, gi, wave, r,
-                                                                             part);
+    for (int c0 = 0; c0 < nchunk; c0 += 65535)  // (a grid's second dimension ends there)
+      k_farfield<<<dim3((unsigned)n, (unsigned)std::min(65535, nchunk - c0)), FF_THREADS, 0, st>>>(
+          cells, s->ncells, pts + 3 * p0, gr, gi, wave, r, c0, part);
     k_farfield_sum<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, nchunk, n, pts + 3 * p0, ff + 6 * p0);
   }
   e = cudaGetLastError();

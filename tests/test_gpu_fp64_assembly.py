@@ -105,8 +105,8 @@ def test_farfield(level, npts, gamma):
     assert np.abs(ff - fo).max() <= 1e-12 * np.abs(fo).max()
 
 
-def test_farfield_of_more_directions_than_a_grid_dimension():
-    """directions come in slabs of at most 65535: those of a long list are bit for bit those of a short one"""
+def test_farfield_of_many_directions():
+    """more directions than a grid's second dimension: those of a long list are bit for bit those of a short one"""
     X = bg.raviartthomas(bg.ellipsoid(0, (1.0, 0.8, 1.3)))
     rng = np.random.default_rng(0)
     u = rng.normal(size=X.numfunctions()) + 1j * rng.normal(size=X.numfunctions())
