@@ -4380,8 +4380,9 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_ss64(NearParams P) {
 //   G        re w / rho    c_jm = (-1)^m S_{2+j+2m} / (2m)!             im k w        (-1)^m S_{3+j+2m} / (2m+1)!
 //   grad G   re w / rho^3  c_jm = (-1)^m (1-2m) S_{j+2m} / (2m)!        im k w / rho^2  (-1)^m 2m S_{1+j+2m} / (2m+1)!
 // (one more power of xi with the double layers' factor n . rho).  Both sums of |a| over the pair's nodes,
-// taken first in FP32 (in FP64 where that cannot tell the distances), set the integers' scales; integer sums do not depend on their order, so a pair may
-// be one warp's or four's.  12 terms leave 1e-17 at k rho = 2; the host takes this kernel where
+// taken first in FP32 (in FP64 where that cannot tell the distances), set the integers' scales; integer sums do
+// not depend on their order, so a pair may be one warp's or four's.  What bounds it is latency: 255 registers let an
+// SM hold eight warps, and no pipe is busy for more than a quarter of the time.  12 terms leave 1e-17 at k rho = 2; the host takes this kernel where
 // k (longest test edge + longest trial edge) <= 2, and k_near_ss64 elsewhere.  Measured: EFIE, 43,900
 // pairs at orders 5, 5, 4: 4.57 -> 2.04 ms; double layer on P1, 75,100 pairs at order 4: 7.56 -> 2.70.
 constexpr int SSX_TERMS = 12, SSX_ROWS = 6;

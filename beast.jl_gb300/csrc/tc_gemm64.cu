@@ -4,9 +4,9 @@
 //
 // GB300 runs FP64 at 1/1500 of its FP16 tensor rate (measured: the shared-memory tiled FP64 kernel
 // this replaces ran at 0.69 TFLOP/s, 90% of an FP64 solve of order 6007).  Each operand row /
-// column is therefore written as eight 7-bit digits of a fixed-point number (slice64.h; Ozaki et
+// column is therefore written in 7-bit digits of a fixed-point number (slice64.h; Ozaki et
 // al., Numer. Algorithms 59 (2012), with the tensor-core form of Mukunoki et al., ISC 2020) and
-// the product summed digit by digit:
+// the product summed digit by digit, eight of the nine digits unless a block asks for the last:
 //   C' = sum_l 2^(-12 - 7 l) D_l,   D_l = sum_{i + j = l} A'_i B'_j,   l = 0 .. 7
 // on the real 2x2 form of the complex product (the layout of tc_gemm.cu: A' has rows 2m, 2m+1
 // = [[re, -im], [im, re]], B' columns hold (re, im) per k).  D_l is a sum of at most (l + 1) 2K
@@ -26,7 +26,7 @@
 // measured against LAPACK's solutions in tests/test_gpu_lu_paths.py.
 //
 // k_tc_gemm64: persistent CTAs over 128 x TNT tiles of C'; after S the levels run from the smallest
-// contribution (l = 7) to the largest, each as one K loop over its l + 1 digit pairs through the
+// contribution (l = 7) to the largest (and l = 8 where it is asked for), each as one K loop over its l + 1 digit pairs through the
 // 4-stage TMA ring into one of two TMEM accumulators, while four epilogue warps add the previous
 // level to C (one FP64 addition per value: -D 2^sh is built from the bits of D).  A tile's C
 // values belong to one CTA and are added to in a fixed order: the result is deterministic.
