@@ -3084,8 +3084,8 @@ __global__ void __maxnreg__(80) k_far_batch(BatchLaunch L) {
   }
 }
 
-// near pairs of a batch: one warp per pair, pairs dealt over the warps of a fixed grid
-// (the list length is read on the device, so the launch needs no host round trip)
+// near pairs of a batch under DoubleNumQStrat (close pairs point by point): one warp per pair, pairs dealt over the
+// warps of a fixed grid (the list length is read on the device, so the launch needs no host round trip)
 __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch(BatchLaunch L) {
   __shared__ double s_glx[210], s_glw[210];
   for (int k = threadIdx.x; k < 210; k += blockDim.x) {
@@ -3113,7 +3113,6 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch(BatchLaunch L) {
   for (int64_t e = blockIdx.x * (int64_t)NEAR_WARPS + warp; e < n; e += (int64_t)gridDim.x * NEAR_WARPS) {
     const NearPairB nb = L.near[e];
     const BatchJobDev& J = L.jobs[nb.job];
-    if (nb.cls == -1 || (L.ssdf && J.op.gr == 0.0 && nb.cls >= 1 && nb.cls <= 3)) continue;  // k_near_batch_se / _df
     P.op = J.op;
     P.tperm = J.tperm;
     P.tgeo = J.geo;
@@ -3508,12 +3507,16 @@ void batch_wave(BatchJobDev* j) {
   j->wave_rest = w.rest;
 }
 
-__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_df(BatchLaunch L);  // below
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_ss(BatchLaunch L);  // below
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_df(BatchLaunch L);
 
 cudaError_t launch_near_batch(const BatchLaunch& L, cudaStream_t st) {
   // the Gauss-Legendre table is uploaded before (upload_tables): this launch may be captured
-  // (double-float touching pairs of real wavenumbers: k_near_batch only where there are others)
-  if (!L.ssdf || L.qs_kind == BEAST_QS_DOUBLENUM || L.complex_k) k_near_batch<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
+  // (double-float touching pairs of real wavenumbers: k_near_batch_ss only where there are others)
+  if (L.qs_kind == BEAST_QS_DOUBLENUM)
+    k_near_batch<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
+  else if (!L.ssdf || L.complex_k)
+    k_near_batch_ss<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
   if (L.qs_kind == BEAST_QS_WILTON_SAUTER) k_near_batch_se<<<L.grid_near / 4, 32 * NEAR_WARPS, 0, st>>>(L);
   if (L.ssdf) k_near_batch_df<<<L.grid_near, 32 * NEAR_WARPS, 0, st>>>(L);
   return cudaGetLastError();
@@ -3912,7 +3915,74 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_hh_df(NearParams P) {
                         z[i * NB + j], P.zfmt);
 }
 
-// the batch's P0 single-layer Sauter-Schwab pairs in double-float (the pairs k_near_batch
+// the batch's touching pairs in FP64, one warp per pair, lanes over the nodes: what the double-float kernel below does
+// not take (transposed double layers, FP64 batches, complex wavenumbers).  Bound by FP64 instructions; x - y comes from
+// the maps' own factors on the edges, and the areas, alpha and 1 / (4 pi) enter once per pair, where the general
+// integrand of k_near forms both points and a full complex product per node: two jobs of 720 cells, transposed double
+// layer, 3.14 .. 3.62 ms with that (by the compiler's choice of registers), 2.42 here.
+__global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_ss(BatchLaunch L) {
+  __shared__ double s_glx[210], s_glw[210];
+  for (int k = threadIdx.x; k < 210; k += blockDim.x) {
+    s_glx[k] = c_gl_x[k];
+    s_glw[k] = c_gl_w[k];
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = min(*L.near_count, L.near_cap);
+  for (int64_t e = blockIdx.x * (int64_t)NEAR_WARPS + warp; e < n; e += (int64_t)gridDim.x * NEAR_WARPS) {
+    const NearPairB nb = L.near[e];
+    const BatchJobDev& J = L.jobs[nb.job];
+    const OpParams op = J.op;
+    if (nb.cls < 1 || (L.ssdf && op.gr == 0.0)) continue;  // k_near_batch_se, k_near_batch_df
+    const bool grad = op.kind == BEAST_HH_DLT;
+    const double *tg = J.geo + (int64_t)J.tperm[nb.p] * GEO_STRIDE, *sg = J.geo + (int64_t)nb.q * GEO_STRIDE;
+    const Geo t = load_geo(tg), s = load_geo(sg);
+    C2<double> acc{0, 0};
+    if (!(grad && nb.cls == 3)) {  // (identically zero)
+      int pt[3], ps[3];
+      ss_order_warp(t, s, lane, pt, ps);
+      const V3<double> e1 = t.v[pt[1]] - t.v[pt[0]], e2 = t.v[pt[2]] - t.v[pt[1]];
+      const V3<double> h1 = s.v[ps[1]] - s.v[ps[0]], h2 = s.v[ps[2]] - s.v[ps[1]];
+      const int ord = nb.cls == 3 ? L.qs.ss_face : (nb.cls == 2 ? L.qs.ss_edge : L.qs.ss_vert);
+      const int items = (nb.cls == 1 ? 2 : 6) * ord * ord * ord * ord;
+      const double *glx = s_glx + c_gl_off[ord - 1], *glw = s_glw + c_gl_off[ord - 1];
+      for (int it = lane; it < items; it += 32) {
+        double X[2], Y[2], D[2], w;
+        ss_node_fd(nb.cls, ord, it, glx, glw, X, Y, D, &w);
+        V3<double> r;
+        if (nb.cls == 3)
+          r = D[0] * e1 + D[1] * e2;
+        else if (nb.cls == 2)
+          r = D[0] * e1 + (X[1] * e2 - Y[1] * h2);
+        else
+          r = (X[0] * e1 + X[1] * e2) - (Y[0] * h1 + Y[1] * h2);
+        const double R2 = dot(r, r), iR = rsqrt(R2), R = R2 * iR;
+        double sn, cs;
+        sincos(op.gi * R, &sn, &cs);
+        double amp = w * iR;
+        if (op.gr != 0.0) amp *= exp(-op.gr * R);
+        if (grad) {  // n_x . grad G = -(gamma + 1/R) G (n_x . r) / R
+          amp *= -iR * dot(t.n, r);
+          const double p = op.gr + iR;
+          acc.re = fma(amp, fma(p, cs, op.gi * sn), acc.re);
+          acc.im = fma(amp, fma(op.gi, cs, -(p * sn)), acc.im);
+        } else {
+          acc.re = fma(amp, cs, acc.re);
+          acc.im = fma(-amp, sn, acc.im);
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        acc.re += __shfl_xor_sync(0xffffffffu, acc.re, o);
+        acc.im += __shfl_xor_sync(0xffffffffu, acc.im, o);
+      }
+    }
+    if (lane == 0)
+      store_c<double>(J.Z, zidx(zrow_of(J.zrow, nb.p, 1, 0), zcol_of(J.zcol, nb.q, 1, 0), J.ldz),
+                      cscale(4.0 * I4PI * t.area * s.area, cmul(C2<double>{op.ar, op.ai}, acc)), L.zfmt);
+  }
+}
+
+// the batch's P0 single-layer Sauter-Schwab pairs in double-float (the pairs k_near_batch_ss
 // skips), persistent over the device-counted near list
 __global__ void __launch_bounds__(32 * NEAR_WARPS) k_near_batch_df(BatchLaunch L) {
   __shared__ float s_tab[64][4];
