@@ -2798,7 +2798,7 @@ __global__ void k_farfield_cells(const double* geo, const int* ad_dof, const dou
 }
 
 __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, int64_t ncells, const double* pts, double gr,
-                                                         double gi, g64::Wave wave, TriRuleDev r, int chunk0, double* part) {
+                                                         double gi, g64::Wave wave, TriRuleDev r, double* part) {
   __shared__ __align__(16) g64::Entry tab[g64::TABLE];
   __shared__ double s_q[RULE_MAXPTS][5];  // u, v, w, w u, w v
   __shared__ double red[6][FF_THREADS];
@@ -2812,12 +2812,12 @@ __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, i
     s_q[k][4] = r.w[k] * v;
   }
   __syncthreads();
-  const int64_t p = blockIdx.x, npts = gridDim.x, chunk = chunk0 + (int64_t)blockIdx.y;
+  const int64_t p = blockIdx.x, npts = gridDim.x;
   const V3<double> y = mk(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
   const double sg = gi < 0.0 ? -1.0 : 1.0;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  const int64_t c1 = min(ncells, (chunk + 1) * FF_CHUNK);
-  for (int64_t c = chunk * FF_CHUNK + threadIdx.x; c < c1; c += FF_THREADS) {
+  const int64_t c1 = min(ncells, (blockIdx.y + 1) * (int64_t)FF_CHUNK);
+  for (int64_t c = blockIdx.y * (int64_t)FF_CHUNK + threadIdx.x; c < c1; c += FF_THREADS) {
     const FarCell& f = cells[c];
     const V3<double> a = mk(f.a[0], f.a[1], f.a[2]), b = mk(f.b[0], f.b[1], f.b[2]);
     const double pa = dot(y, a), pb = dot(y, b);
@@ -2870,7 +2870,7 @@ __global__ void __launch_bounds__(FF_THREADS) k_farfield(const FarCell* cells, i
       for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x < 6) part[(chunk * npts + p) * 6 + threadIdx.x] = red[threadIdx.x][0];
+  if (threadIdx.x < 6) part[(blockIdx.y * npts + p) * 6 + threadIdx.x] = red[threadIdx.x][0];
 }
 
 // the chunks' sums, then (y x F) x y
@@ -5022,7 +5022,8 @@ cudaError_t launch_farfield(const beast_space* s, const double* u, const double*
     const int64_t n = std::min(slab, npts - p0);
     for (int c0 = 0; c0 < nchunk; c0 += 65535)  // (a grid's second dimension ends there)
       k_farfield<<<dim3((unsigned)n, (unsigned)std::min(65535, nchunk - c0)), FF_THREADS, 0, st>>>(
-          cells, s->ncells, pts + 3 * p0, gr, gi, wave, r, c0, part);
+          cells + (int64_t)c0 * FF_CHUNK, s->ncells - (int64_t)c0 * FF_CHUNK, pts + 3 * p0, gr, gi, wave, r,
+          part + 6 * n * c0);
     k_farfield_sum<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, nchunk, n, pts + 3 * p0, ff + 6 * p0);
   }
   e = cudaGetLastError();
